@@ -1,13 +1,11 @@
-// Token-sequential KDA scan: the decode step (T = 1) and inference prefill.
+// Token-sequential KDA recurrence: the decode step (T = 1) and the token scan (inference prefill, a
+// few tokens per sequence, the fp32-accurate evaluation of chunk_kda).
 //
 // Replaces the reference's Triton scan `_kda_recurrent_fwd_kernel`
 // (attn_gym/linear/kda/fwd/triton/recurrent.py:41-153).  Per token, per (sequence, head):
 //     S <- diag(2^g) S ;  d = beta (v - S^T k) ;  S <- S + k d^T ;  o = scale S^T q
-// One CTA owns a [K x 32*VEC] column slab of the fp32 state and keeps it in registers for
-// the whole scan: warp w holds rows w, w+8, ...; lane l holds VEC adjacent columns, so a
-// warp touches one contiguous 128*VEC-byte row segment per load (VEC = 4: 512 B, LDG.128).
-// The two K-reductions of a step (S^T k and S^T q, both taken on the decayed state) share
-// one shared-memory exchange:  o = scale (S_d^T q + (q.k) d).
+// The two K-reductions of a step (S^T k and S^T q, both taken on the decayed state) share one
+// exchange:  o = scale (S_d^T q + (q.k) d).
 // The decode step is pure state streaming: 2*K*V*4 bytes per (sequence, head) per step.
 #include "kda_common.cuh"
 #include "kda_sm100.cuh"
@@ -29,38 +27,62 @@ struct ScanParams {
   float scale;
 };
 
-template <int KR, int VEC, int MINB>
-__global__ void __launch_bounds__(256, MINB) kda_scan_kernel(const ScanParams p) {
-  constexpr int BV = 32 * VEC;
-  constexpr int NW = 8;
-  __shared__ float s_q[2][256], s_k[2][256], s_d[2][256];
-  __shared__ float s_red[2][2][NW][BV];
-  __shared__ float s_qk[2][NW];
-  __shared__ float s_beta[2];
+// ------------------------------------------------------------------------------------------------
+// Token scan.  Every computing warp owns 4 VC columns of the fp32 state and keeps them in registers for
+// the whole scan: lane (lk = lane / 4, cv = lane % 4) holds VC adjacent columns and the key rows
+// 4 (lk + 8 i) .. + 3, i < KR / 4, as pairs of rows for the packed fp32 arithmetic.  The K-reductions
+// are three shuffles, so no token needs a barrier.  The CTA's warps share one (sequence, head): its
+// operands are fetched TT tokens at a time, one tile ahead of their use (raw bits in registers), and
+// published to shared memory as fp32 (q scaled, 2^g) with one barrier per tile.
+//
+// A long scan of few sequences is bound by the latency of one token: the dependent chain of decay,
+// reduction, three shuffles and update, 0.15 us of a warp that issues nothing else.  So NP warps of
+// their own fetch, publish and store (NP = 0: the computing warps do it), and the next token's operands
+// are read from shared memory before the shuffles.  T = 512, H = 4, K = V = 64: 726 us with eight warps
+// sharing a column slab, two CTA barriers and a shared-memory exchange per token; 135 us in this split
+// with scalar arithmetic and no moving warps, 114 us with packed arithmetic, 79 us with moving warps.
+// A short scan of many sequences is bound by the state traffic and by how much of it two CTAs per SM
+// can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 141 us before, 60 us
+// now.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
+// CUM: the gate is the cumulative one of chunk_kda; the per-token gate is its difference inside the
+// 64-token chunks of a sequence.
+// ------------------------------------------------------------------------------------------------
+template <int KR, int VC, int NW, int NP, int TT, bool CUM, int MINB>
+__global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const ScanParams p) {
+  constexpr int NT = 32 * (NP ? NP : NW);          // threads that fetch and publish operands
+  constexpr int KP = 8 * KR, CT = 4 * VC * NW;
+  constexpr int NE = TT * KP / NT;                 // operand elements per thread, array and tile
+  constexpr int NV = (TT * CT + NT - 1) / NT;      // value and output elements per thread and tile
+  constexpr int NR = KR / 4;
+  constexpr bool kPrefetch = VC == 1 && KR <= 16;
+  static_assert(TT * KP % NT == 0 && TT <= 32, "tile split");
+  __shared__ __align__(16) float s_q[2][TT][KP], s_k[2][TT][KP], s_d[2][TT][KP];
+  __shared__ float s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int vtiles = (p.V + BV - 1) / BV;
-  const int vt = blockIdx.x % vtiles;
-  const int sh = blockIdx.x / vtiles;
-  const int head = sh % p.H, seq = sh / p.H;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cv = lane & 3, lk = lane >> 2;
+  const bool computes = warp < NW, moves = NP == 0 || warp >= NW;
+  const int tid = NP ? (int)threadIdx.x - 32 * NW : (int)threadIdx.x;     // index among the moving threads
   const int K = p.K, V = p.V, H = p.H;
+  const int vtiles = (V + CT - 1) / CT;
+  const int vt = blockIdx.x % vtiles, sh = blockIdx.x / vtiles;
+  const int head = sh % H, seq = sh / H;
   int64_t bos, eos;
   if (p.cu_seqlens) { bos = p.cu_seqlens[seq]; eos = p.cu_seqlens[seq + 1]; }
   else { bos = (int64_t)seq * p.T; eos = bos + p.T; }
-  const int c0 = vt * BV + lane * VEC;
+  const int cta0 = vt * CT, wc = 4 * VC * warp + VC * cv, c0 = cta0 + wc;    // this lane's first column
 
   int64_t slot = seq;
   bool active = true;
   if (p.state_indices) {
-    int si = p.state_indices[seq];
+    const int si = p.state_indices[seq];
     active = si > 0 && si < p.num_slots;   // non-positive (or out of range) slots are padding
     slot = si;
   }
   if (!active) {  // padding rows produce zero output and leave the pool untouched
-    if (warp == 0)
-      for (int64_t t = bos; t < eos; ++t)
-        for (int j = 0; j < VEC; ++j)
-          if (c0 + j < V) store_from_float(p.out, p.dt_out, (t * H + head) * V + c0 + j, 0.f);
+    for (int64_t t = bos; t < eos; ++t)
+      for (int c = cta0 + (int)threadIdx.x; c < min(cta0 + CT, V); c += 32 * (NW + NP))
+        store_from_float(p.out, p.dt_out, (t * H + head) * V + c, 0.f);
     return;
   }
   const bool paged = p.state_indices != nullptr;
@@ -69,130 +91,250 @@ __global__ void __launch_bounds__(256, MINB) kda_scan_kernel(const ScanParams p)
   float* sout = paged ? const_cast<float*>(sin)
                       : (p.ht ? p.ht + ((int64_t)seq * H + head) * K * V : nullptr);
 
-  float S[KR][VEC];
-#pragma unroll
-  for (int i = 0; i < KR; ++i) {
-    int r = i * NW + warp;
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) S[i][j] = 0.f;
-    if (sin && r < K) {
-      if (VEC == 4 && c0 + 3 < V) {
-        float4 x = *reinterpret_cast<const float4*>(sin + (int64_t)r * V + c0);
-        S[i][0] = x.x; S[i][1] = x.y; S[i][2] = x.z; S[i][3] = x.w;
-      } else if (VEC == 2 && c0 + 1 < V) {
-        float2 x = *reinterpret_cast<const float2*>(sin + (int64_t)r * V + c0);
-        S[i][0] = x.x; S[i][1] = x.y;
-      } else {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j)
-          if (c0 + j < V) S[i][j] = sin[(int64_t)r * V + c0 + j];
-      }
-    }
-  }
-
-  // stage token `t` into parity buffer `b`: q*scale, k, 2^g, beta
-  auto stage = [&](int64_t t, int b) {
-    int64_t base = (t * H + head) * K;
-    for (int r = tid; r < K; r += 256) {
-      s_q[b][r] = load_as_float(p.q, p.dt_q, base + r) * p.scale;
-      s_k[b][r] = load_as_float(p.k, p.dt_k, base + r);
-      s_d[b][r] = exp2f(load_as_float(p.g, p.dt_g, base + r));
-    }
-    if (tid == 0) s_beta[b] = load_as_float(p.beta, p.dt_beta, t * H + head);
+  // ---- operand tiles: raw bits in registers, published as fp32 ----------------------------------------
+  // (a warp's elements of one n belong to one token, so tokens past the end cost it nothing)
+  uint32_t rq[NE], rk[NE], rg[NE], rp[CUM ? NE : 1], rv[NV], rb = 0;
+  auto bits = [](const void* base, int dt, int64_t at, int off) -> uint32_t {
+    if (dt == KDA_F32) return (reinterpret_cast<const uint32_t*>(base) + at)[off];
+    return (reinterpret_cast<const unsigned short*>(base) + at)[off];
   };
-
-  if (bos < eos) stage(bos, 0);
-  for (int64_t t = bos; t < eos; ++t) {
-    const int b = (int)((t - bos) & 1);
-    float vv[VEC];
+  auto fetch = [&](int64_t t0) {
+    const int ntok = (int)min((int64_t)TT, eos - t0);
+    const int64_t kbase = (t0 * H + head) * K, vbase = (t0 * H + head) * V + cta0;
 #pragma unroll
-    for (int j = 0; j < VEC; ++j)
-      vv[j] = (c0 + j < V) ? load_as_float(p.v, p.dt_v, (t * H + head) * V + c0 + j) : 0.f;
-    __syncthreads();  // staged token visible; previous step's readers are done
-    float pk[VEC], pq[VEC], pqk = 0.f;
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) { pk[j] = 0.f; pq[j] = 0.f; }
-#pragma unroll
-    for (int i = 0; i < KR; ++i) {
-      int r = i * NW + warp;
-      if (r < K) {
-        float d = s_d[b][r], kk = s_k[b][r], qq = s_q[b][r];
-        pqk += qq * kk;
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) {
-          float s = S[i][j] * d;
-          S[i][j] = s;
-          pk[j] += kk * s;
-          pq[j] += qq * s;
-        }
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + n * NT, tok = e / KP, r = e % KP, off = tok * H * K + r;
+      rq[n] = rk[n] = rg[n] = 0;
+      if (CUM) rp[n] = 0;
+      if (tok < ntok && r < K) {
+        rq[n] = bits(p.q, p.dt_q, kbase, off);
+        rk[n] = bits(p.k, p.dt_k, kbase, off);
+        rg[n] = bits(p.g, p.dt_g, kbase, off);
+        if (CUM && (((int)(t0 - bos) + tok) & (kChunk - 1)) != 0) rp[n] = bits(p.g, p.dt_g, kbase, off - H * K);
       }
     }
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-      s_red[b][0][warp][lane * VEC + j] = pk[j];
-      s_red[b][1][warp][lane * VEC + j] = pq[j];
+    for (int n = 0; n < NV; ++n) {
+      const int e = tid + n * NT, tok = e / CT, c = e % CT;
+      rv[n] = (tok < ntok && cta0 + c < V) ? bits(p.v, p.dt_v, vbase, tok * H * V + c) : 0;
     }
-    if (lane == 0) s_qk[b][warp] = pqk;
-    if (t + 1 < eos) stage(t + 1, b ^ 1);  // overlaps the exchange below
-    __syncthreads();
-    float qk = 0.f;
+    if (tid < ntok) rb = bits(p.beta, p.dt_beta, t0 * H + head, tid * H);
+  };
+  auto publish = [&](int b, int ntok) {
 #pragma unroll
-    for (int w = 0; w < NW; ++w) qk += s_qk[b][w];
-    const float bt = s_beta[b];
-    float delta[VEC];
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-      float a = 0.f, o = 0.f;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        a += s_red[b][0][w][lane * VEC + j];
-        o += s_red[b][1][w][lane * VEC + j];
-      }
-      delta[j] = bt * (vv[j] - a);
-      o += qk * delta[j];
-      if (warp == 0 && c0 + j < V)
-        store_from_float(p.out, p.dt_out, (t * H + head) * V + c0 + j, o);
-    }
-#pragma unroll
-    for (int i = 0; i < KR; ++i) {
-      int r = i * NW + warp;
-      if (r < K) {
-        float kk = s_k[b][r];
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) S[i][j] += kk * delta[j];
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + n * NT, tok = e / KP, r = e % KP;
+      if (NP || tok < ntok) {        // (a long scan's tiles are whole but for the last one)
+        s_q[b][tok][r] = raw_to_float(rq[n], p.dt_q) * p.scale;
+        s_k[b][tok][r] = raw_to_float(rk[n], p.dt_k);
+        float g = raw_to_float(rg[n], p.dt_g);
+        if (CUM) g -= raw_to_float(rp[n], p.dt_g);
+        s_d[b][tok][r] = exp2f(g);
       }
     }
-  }
-
-  if (sout) {
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      const int e = tid + n * NT;
+      if (e / CT < ntok) s_v[b][e / CT][e % CT] = raw_to_float(rv[n], p.dt_v);
+    }
+    if (tid < ntok) s_beta[b][tid] = raw_to_float(rb, p.dt_beta);
+  };
+  if (moves) fetch(bos);
+  // ---- state slab: S[i][j] holds the rows 2 i, 2 i + 1 of this lane's list in column j -----------------------
+  f32x2 S[KR / 2][VC];
+  {
+    float x[2][VC];
 #pragma unroll
     for (int i = 0; i < KR; ++i) {
-      int r = i * NW + warp;
-      if (r < K) {
-        if (VEC == 4 && c0 + 3 < V) {
-          *reinterpret_cast<float4*>(sout + (int64_t)r * V + c0) =
-              make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-        } else if (VEC == 2 && c0 + 1 < V) {
-          *reinterpret_cast<float2*>(sout + (int64_t)r * V + c0) = make_float2(S[i][0], S[i][1]);
+      const int r = 4 * (lk + 8 * (i >> 2)) + (i & 3);
+      float (&xr)[VC] = x[i & 1];
+#pragma unroll
+      for (int j = 0; j < VC; ++j) xr[j] = 0.f;
+      if (computes && sin && r < K) {
+        if (VC > 1) {             // (V is a multiple of 4 then, and so is every column offset)
+          if (c0 < V) {
+            if (VC == 4) {
+              const float4 f = *reinterpret_cast<const float4*>(sin + (int64_t)r * V + c0);
+              xr[0] = f.x; xr[1 % VC] = f.y; xr[2 % VC] = f.z; xr[3 % VC] = f.w;
+            } else {
+              const float2 f = *reinterpret_cast<const float2*>(sin + (int64_t)r * V + c0);
+              xr[0] = f.x; xr[1 % VC] = f.y;
+            }
+          }
         } else {
 #pragma unroll
-          for (int j = 0; j < VEC; ++j)
-            if (c0 + j < V) sout[(int64_t)r * V + c0 + j] = S[i][j];
+          for (int j = 0; j < VC; ++j)
+            if (c0 + j < V) xr[j] = sin[(int64_t)r * V + c0 + j];
+        }
+      }
+      if (i & 1) {
+#pragma unroll
+        for (int j = 0; j < VC; ++j) S[i >> 1][j] = pack2(x[0][j], x[1][j]);
+      }
+    }
+  }
+
+  auto flush = [&](int64_t t0, int b, int ntok) {      // the outputs of a tile
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      const int e = tid + n * NT, tok = e / CT, c = e % CT;
+      if (tok < ntok && cta0 + c < V)
+        store_from_float(p.out, p.dt_out, (t0 * H + head) * V + cta0 + (tok * H * V + c), s_o[b][tok][c]);
+    }
+  };
+  if (moves) publish(0, (int)min((int64_t)TT, eos - bos));
+  __syncthreads();
+  int b = 0;
+  for (int64_t t0 = bos; t0 < eos; t0 += TT, b ^= 1) {
+    const bool more = t0 + TT < eos;
+    const int ntok = more ? TT : (int)(eos - t0);
+    if (moves && more) fetch(t0 + TT);
+    if (NP && moves && t0 > bos) flush(t0 - TT, b ^ 1, TT);
+    if (computes) {
+    // The operands of a long scan's next token are read from shared memory between the two halves of
+    // a step, where their latency hides behind the shuffles.
+    f32x2 q[KR / 2], k[KR / 2], d[KR / 2];
+    auto read = [&](int tok, f32x2 (&qd)[KR / 2], f32x2 (&kd)[KR / 2], f32x2 (&dd)[KR / 2]) {
+      const ulonglong2* qs = reinterpret_cast<const ulonglong2*>(s_q[b][tok]) + lk;
+      const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
+      const ulonglong2* ds = reinterpret_cast<const ulonglong2*>(s_d[b][tok]) + lk;
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        const ulonglong2 a = qs[8 * i], c = ks[8 * i], e = ds[8 * i];
+        qd[2 * i] = a.x; qd[2 * i + 1] = a.y;
+        kd[2 * i] = c.x; kd[2 * i + 1] = c.y;
+        dd[2 * i] = e.x; dd[2 * i + 1] = e.y;
+      }
+    };
+    if (kPrefetch) read(0, q, k, d);
+#pragma unroll(kPrefetch ? 2 : 1)
+    for (int tok = 0; tok < ntok; ++tok) {
+      f32x2 pk[VC], pq[VC], pqk = 0;       // (zero bits: +0, +0) even rows in the low half, odd in the high
+#pragma unroll
+      for (int j = 0; j < VC; ++j) pk[j] = pq[j] = 0;
+      const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
+#pragma unroll
+      for (int i = 0; i < KR / 2; ++i) {
+        if (!kPrefetch && i % 2 == 0) {
+          const ulonglong2 x = reinterpret_cast<const ulonglong2*>(s_q[b][tok])[lk + 4 * i], y = ks[4 * i],
+                           z = reinterpret_cast<const ulonglong2*>(s_d[b][tok])[lk + 4 * i];
+          q[i] = x.x; q[i + 1] = x.y; k[i] = y.x; k[i + 1] = y.y; d[i] = z.x; d[i + 1] = z.y;
+        }
+        pqk = fma2(q[i], k[i], pqk);
+#pragma unroll
+        for (int j = 0; j < VC; ++j) {
+          S[i][j] = mul2(S[i][j], d[i]);
+          pk[j] = fma2(k[i], S[i][j], pk[j]);
+          pq[j] = fma2(q[i], S[i][j], pq[j]);
+        }
+      }
+      float a[VC], o[VC];
+      const float2 x = unpack2(pqk);
+      float qk = x.x + x.y;
+#pragma unroll
+      for (int j = 0; j < VC; ++j) {
+        const float2 y = unpack2(pk[j]), z = unpack2(pq[j]);
+        a[j] = y.x + y.y;
+        o[j] = z.x + z.y;
+      }
+      f32x2 qn[KR / 2], kn[KR / 2], dn[KR / 2];
+      if (kPrefetch) read(tok + 1 < TT ? tok + 1 : tok, qn, kn, dn);
+#pragma unroll
+      for (int m = 4; m < 32; m <<= 1) {
+#pragma unroll
+        for (int j = 0; j < VC; ++j) {
+          a[j] += __shfl_xor_sync(0xffffffffu, a[j], m);
+          o[j] += __shfl_xor_sync(0xffffffffu, o[j], m);
+        }
+        qk += __shfl_xor_sync(0xffffffffu, qk, m);
+      }
+      const float bt = s_beta[b][tok];
+      float mine = 0.f;                    // lane row lk < VC keeps column lk of its group
+      f32x2 delta2[VC];
+#pragma unroll
+      for (int j = 0; j < VC; ++j) {
+        const float delta = bt * (s_v[b][tok][wc + j] - a[j]);
+        const float out = fmaf(qk, delta, o[j]);
+        if (lk == j) mine = out;
+        delta2[j] = pack2(delta, delta);
+      }
+#pragma unroll
+      for (int i = 0; i < KR / 2; ++i) {
+        if (!kPrefetch && i % 2 == 0) { const ulonglong2 y = ks[4 * i]; k[i] = y.x; k[i + 1] = y.y; }
+#pragma unroll
+        for (int j = 0; j < VC; ++j) S[i][j] = fma2(k[i], delta2[j], S[i][j]);
+      }
+      if (lk < VC) s_o[b][tok][wc + lk] = mine;
+      if (kPrefetch) {
+#pragma unroll
+        for (int i = 0; i < KR / 2; ++i) { q[i] = qn[i]; k[i] = kn[i]; d[i] = dn[i]; }
+      }
+    }
+    }
+    if (moves && more) publish(b ^ 1, (int)min((int64_t)TT, eos - t0 - TT));   // those buffers were last read before the previous barrier
+    __syncthreads();
+    if (moves && (NP == 0 || !more)) flush(t0, b, ntok);
+  }
+
+  if (sout && computes) {
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+      const int r = 4 * (lk + 8 * (i >> 2)) + (i & 3);
+      float x[VC];
+#pragma unroll
+      for (int j = 0; j < VC; ++j) {
+        const float2 y = unpack2(S[i >> 1][j]);
+        x[j] = (i & 1) ? y.y : y.x;
+      }
+      if (r < K) {
+        if (VC > 1) {
+          if (c0 < V) {
+            if (VC == 4) *reinterpret_cast<float4*>(sout + (int64_t)r * V + c0) = make_float4(x[0], x[1 % VC], x[2 % VC], x[3 % VC]);
+            else *reinterpret_cast<float2*>(sout + (int64_t)r * V + c0) = make_float2(x[0], x[1 % VC]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < VC; ++j)
+            if (c0 + j < V) sout[(int64_t)r * V + c0 + j] = x[j];
         }
       }
     }
   }
 }
 
-template <int KR, int VEC, int MINB = 1>
-static int launch_scan(const ScanParams& p, cudaStream_t stream) {
-  constexpr int BV = 32 * VEC;
-  int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + BV - 1) / BV);
+static int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    return 148;
+  return sms;
+}
+
+template <int KR, int VC, int NW, int NP, int MINB>
+static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream) {
+  constexpr int CT = 4 * VC * NW, KP = 8 * KR;
+  // 24 KiB of operands in two buffers (K = 128: 8 tokens); the wide form also buffers 128 columns of v and o
+  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : 1024 / KP;
+  const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + CT - 1) / CT);
   if (blocks <= 0) return KDA_OK;
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
   StageScope timing(kStageRecurrent, stream);
-  kda_scan_kernel<KR, VEC, MINB><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  if (cumulative) kda_scan_kernel<KR, VC, NW, NP, TT, true, MINB><<<(unsigned)blocks, 32 * (NW + NP), 0, stream>>>(p);
+  else kda_scan_kernel<KR, VC, NW, NP, TT, false, MINB><<<(unsigned)blocks, 32 * (NW + NP), 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
+// Columns per lane: one (16 columns per CTA, the shortest chain from token to token) while those CTAs take
+// at most two turns on the SMs, else four (128 columns per CTA, 16-byte state accesses).  K = V = 128, us for
+// one / four columns per lane: 32 chains 13.8 / 12.7 at 2 tokens, 28 / 33 at 32, 128 / 187 at 256;
+// 64 chains 19.5 / 13.3, 46 / 34, 249 / 188; 256 chains 48 / 14, 141 / 50, 961 / 325.
+static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s) {
+  const int sms = device_sms();
+  const bool aligned = (((uintptr_t)p.h0 | (uintptr_t)p.ht) & 15) == 0 && p.V % 4 == 0 && p.slot_stride % 4 == 0;
+  const bool wide = aligned && (int64_t)p.nseq * p.H * ((p.V + 15) / 16) > 2 * sms;
+  if (p.K <= 32) return wide ? launch_scan<4, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<4, 1, 4, 4, 1>(p, cumulative, s);
+  if (p.K <= 64) return wide ? launch_scan<8, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<8, 1, 4, 4, 1>(p, cumulative, s);
+  if (p.K <= 128) return wide ? launch_scan<16, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<16, 1, 4, 4, 1>(p, cumulative, s);
+  return launch_scan<32, 1, 4, 4, 2>(p, cumulative, s);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -491,8 +633,6 @@ extern "C" int kda_recurrent_fwd(const void* q, const void* k, const void* v, co
   p.nseq = nseq; p.T = tokens_per_row; p.H = heads; p.K = key_dim; p.V = value_dim;
   p.scale = scale;
   cudaStream_t s = (cudaStream_t)stream;
-  // Wide column slabs (float4 rows) when the state rows allow 16-byte accesses and there are
-  // enough (sequence, head) pairs to fill the machine; otherwise 32-column slabs for parallelism.
   // the decode step proper: one token per sequence, K = V = 128, state in and out
   const bool decode = tokens_per_row == 1 && !cu_seqlens && key_dim == 128 && value_dim == 128 &&
                       initial_state && (state_indices || final_state) && nseq * (int64_t)heads < (1 << 24) &&
@@ -500,17 +640,23 @@ extern "C" int kda_recurrent_fwd(const void* q, const void* k, const void* v, co
                       (!state_indices || (slot_stride % 128 == 0 && slot_stride >= (int64_t)heads * 16384 &&
                                           (int64_t)num_slots * (slot_stride / 128) < (1LL << 31)));
   if (decode) return launch_decode(p, s);
-  bool vec4 = (value_dim % 4 == 0) && (slot_stride % 4 == 0) &&
-              ((int64_t)nseq * heads * ((value_dim + 127) / 128) >= 296 || value_dim > 1024);
-  int kr = (key_dim + 7) / 8;
-  if (vec4) {
-    if (kr <= 4) return launch_scan<4, 4>(p, s);
-    if (kr <= 8) return launch_scan<8, 4>(p, s);
-    if (kr <= 16) return launch_scan<16, 4, 2>(p, s);  // two CTAs per SM: loads overlap stores
-    return launch_scan<32, 1>(p, s);
-  }
-  if (kr <= 4) return launch_scan<4, 1>(p, s);
-  if (kr <= 8) return launch_scan<8, 1>(p, s);
-  if (kr <= 16) return launch_scan<16, 1>(p, s);
-  return launch_scan<32, 1>(p, s);
+  return launch_scan_any(p, false, s);
+}
+
+// The recurrence on the cumulative gate of chunk_kda (dense or packed, no paged pool).
+extern "C" int kda_chunk_scan_fwd(const void* q, const void* k, const void* v, const void* cum_gate,
+                                  const void* beta, int dt_q, int dt_k, int dt_v, int dt_gate, int dt_beta,
+                                  const float* initial_state, float* final_state, void* out, int dt_out,
+                                  const int32_t* cu_seqlens, int nseq, int tokens_per_row, int heads,
+                                  int key_dim, int value_dim, float scale, void* stream) {
+  using namespace kda;
+  if (!q || !k || !v || !cum_gate || !beta || !out) return KDA_ERR_ARG;
+  if (nseq < 0 || heads <= 0 || key_dim <= 0 || key_dim > 256 || value_dim <= 0) return KDA_ERR_ARG;
+  ScanParams p{};
+  p.q = q; p.k = k; p.v = v; p.g = cum_gate; p.beta = beta;
+  p.dt_q = dt_q; p.dt_k = dt_k; p.dt_v = dt_v; p.dt_g = dt_gate; p.dt_beta = dt_beta;
+  p.h0 = initial_state; p.ht = final_state; p.out = out; p.dt_out = dt_out;
+  p.cu_seqlens = cu_seqlens; p.nseq = nseq; p.T = tokens_per_row; p.H = heads; p.K = key_dim; p.V = value_dim;
+  p.scale = scale;
+  return launch_scan_any(p, true, (cudaStream_t)stream);
 }

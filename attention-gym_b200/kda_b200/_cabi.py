@@ -37,6 +37,8 @@ _SIGNATURES = {
     "kda_recurrent_fwd": (c_int, [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_void_p, c_void_p, c_int,
                                   c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
                                   c_int, c_float, c_void_p]),
+    "kda_chunk_scan_fwd": (c_int, [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_void_p, c_void_p, c_int,
+                                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
     "kda_gate_cumsum_fwd": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int64,
                                     c_void_p]),

@@ -18,6 +18,7 @@ from __future__ import annotations
 import torch
 
 from .fused import chunk_forward as _fused_chunk_forward
+from .ops import chunk_scan_op as _chunk_scan_op
 from .ops import recurrent_forward as _fused_recurrent_forward
 from .reference_impl import reference_kda
 from .types import Impl, resolve_impl
@@ -28,20 +29,6 @@ def _narrow_offsets(cu_seqlens):
     if cu_seqlens is not None and cu_seqlens.dtype == torch.int64:
         return cu_seqlens.to(torch.int32)
     return cu_seqlens
-
-
-def _per_token_gate(cumulative_gate, cu_seqlens):
-    """Invert the chunk-local inclusive prefix sum (differences inside each 64-token chunk)."""
-    g = cumulative_gate.float()
-    tokens = g.shape[1]
-    pos = torch.arange(tokens, device=g.device)
-    if cu_seqlens is not None:
-        start = cu_seqlens.long()
-        seq = torch.searchsorted(start, pos, right=True) - 1
-        pos = pos - start[seq.clamp(max=start.numel() - 2)]
-    first = (pos % 64 == 0)
-    prev = torch.cat((torch.zeros_like(g[:, :1]), g[:, :-1]), 1)
-    return torch.where(first[None, :, None, None], g, g - prev)
 
 
 def chunk_kda(q, k, v, cumulative_gate, beta, initial_state=None, *, cu_seqlens=None,
@@ -92,10 +79,10 @@ def chunk_kda(q, k, v, cumulative_gate, beta, initial_state=None, *, cu_seqlens=
                                     normalize_qk=True, norm_eps=norm_eps)
     if (q.dtype == torch.float32 and q.is_cuda and not needs_grad and q.shape[-1] <= 256
             and (exact_fp32 or off_chunk_shape)):
-        # fp32-accurate path: the token scan on the per-token gate
-        gate = _per_token_gate(cumulative_gate, cu_seqlens)
-        return _fused_recurrent_forward(q, k, v, gate, beta, initial_state, cu_seqlens=cu_seqlens,
-                                        output_final_state=output_final_state)
+        # fp32-accurate path: the token scan, which forms the per-token gate from the cumulative one
+        out, state = _chunk_scan_op(q, k, v, cumulative_gate, beta, initial_state, cu_seqlens,
+                                    bool(output_final_state))
+        return out, state if output_final_state else None
     return _fused_chunk_forward(q, k, v, cumulative_gate, beta, initial_state,
                                 cu_seqlens=cu_seqlens, output_final_state=output_final_state,
                                 fastmath=fastmath, autotune=autotune, recompute=recompute)

@@ -112,6 +112,15 @@ _define("kda_decode_prep",
         "-> (Tensor, Tensor, Tensor, Tensor)")
 
 
+# Operators of this package's own making, in a namespace of their own: the one above holds the reference's.
+_NS_OWN = "kda_b200_fused"
+_lib_own = torch.library.Library(_NS_OWN, "DEF")
+
+# The token scan on the cumulative gate of chunk_kda (the fp32-accurate evaluation).
+_lib_own.define("chunk_scan(Tensor q, Tensor k, Tensor v, Tensor cumulative_gate, Tensor beta, "
+                "Tensor? initial_state, Tensor? cu_seqlens, bool want_state) -> (Tensor, Tensor)")
+
+
 def _require_cuda(t: torch.Tensor, what: str):
     if not t.is_cuda:
         raise ValueError(f"{what} requires CUDA tensors")
@@ -506,6 +515,34 @@ def _recurrent_fwd_paged(q, k, v, gate, beta, state_cache, state_indices, cu_seq
     return _recurrent_impl(q, k, v, gate, beta, state_cache, cu_seqlens, state_indices, False)[0]
 
 
+@torch.library.impl(_lib_own, "chunk_scan", "CUDA")
+def _chunk_scan(q, k, v, gate, beta, initial_state, cu_seqlens, want_state):
+    _require_cuda(q, "the fused recurrent scan")
+    batch, tokens, heads, key_dim = q.shape
+    value_dim = v.shape[-1]
+    nseq = batch if cu_seqlens is None else cu_seqlens.shape[0] - 1
+    q, k, v, gate, beta = (t.contiguous() for t in (q, k, v, gate, beta))
+    if initial_state is not None:
+        initial_state = initial_state.float().contiguous()
+    out = (torch.zeros if cu_seqlens is not None else torch.empty)(v.shape, dtype=q.dtype, device=q.device)
+    final = torch.empty((nseq, heads, key_dim, value_dim) if want_state else (0,), dtype=torch.float32,
+                        device=q.device)
+    _cabi.call("kda_chunk_scan_fwd", 1, _cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
+               _cabi.ptr(beta), _cabi.dt(q), _cabi.dt(k), _cabi.dt(v), _cabi.dt(gate), _cabi.dt(beta),
+               _cabi.ptr(initial_state), _cabi.ptr(final) if want_state else None, _cabi.ptr(out),
+               _cabi.dt(out), _cabi.ptr(cu_seqlens), nseq, tokens, heads, key_dim, value_dim,
+               float(key_dim) ** -0.5, _cabi.stream())
+    return out, final
+
+
+@torch.library.register_fake(f"{_NS_OWN}::chunk_scan")
+def _(q, k, v, gate, beta, initial_state, cu_seqlens, want_state):
+    nseq = q.shape[0] if cu_seqlens is None else cu_seqlens.shape[0] - 1
+    state = q.new_empty((nseq, q.shape[2], q.shape[3], v.shape[-1]) if want_state else (0,),
+                        dtype=torch.float32)
+    return torch.empty_like(v, dtype=q.dtype), state
+
+
 @torch.library.register_fake(f"{_NS}::kda_recurrent_fwd")
 def _(q, k, v, gate, beta, initial_state, cu_seqlens, autotune):
     nseq = q.shape[0] if cu_seqlens is None else cu_seqlens.shape[0] - 1
@@ -793,6 +830,7 @@ chunk_fwd_qknorm_op = _ops.kda_chunk_fwd_qknorm.default
 chunk_bwd_qknorm_op = _ops.kda_chunk_bwd_qknorm.default
 chunk_bwd_op = _ops.kda_chunk_bwd.default
 chunk_bwd_with_state_grad_op = _ops.kda_chunk_bwd_with_state_grad.default
+chunk_scan_op = torch.ops.kda_b200_fused.chunk_scan.default
 recurrent_fwd_op = _ops.kda_recurrent_fwd.default
 recurrent_fwd_no_state_op = _ops.kda_recurrent_fwd_no_state.default
 recurrent_fwd_paged_op = _ops.kda_recurrent_fwd_paged.default

@@ -86,6 +86,15 @@ int kda_recurrent_fwd(const void* q, const void* k, const void* v, const void* g
                       int num_slots, int nseq, int tokens_per_row, int heads, int key_dim,
                       int value_dim, float scale, void* stream);
 
+/* The same recurrence on the cumulative gate of chunk_kda (inclusive log2 prefix inside every 64-token
+ * chunk of a sequence): the per-token gate is formed on the fly.  No paged form.  This is the
+ * fp32-accurate evaluation of chunk_kda for any K <= 256 (the reference's fused path has none). */
+int kda_chunk_scan_fwd(const void* q, const void* k, const void* v, const void* cum_gate,
+                       const void* beta, int dt_q, int dt_k, int dt_v, int dt_gate, int dt_beta,
+                       const float* initial_state, float* final_state, void* out, int dt_out,
+                       const int32_t* cu_seqlens, int nseq, int tokens_per_row, int heads,
+                       int key_dim, int value_dim, float scale, void* stream);
+
 /* out = log2(e) * chunk_local_cumsum(lower_bound * sigmoid(exp(A_log[h]) * (raw + dt_bias[h, :]))).
  * raw: [batch, tokens, H, dim] (dtype code), out fp32 of the same shape; dim % 4 == 0.
  * num_chunks = batch * ceil(tokens / chunk_size) for dense input, the chunk capacity for packed
