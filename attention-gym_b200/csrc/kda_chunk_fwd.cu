@@ -482,3 +482,12 @@ extern "C" int kda_chunk_fwd_noalloc(const void* q, const void* k, const void* v
                        cu_seqlens, chunk_offsets, nseq, tokens, heads, key_dim, value_dim,
                        num_chunks, scratch, need, stream);
 }
+
+extern "C" int kda_dense_offsets(void* offsets, int batch, int tokens, void* stream) {
+  if (!offsets || batch < 1 || tokens < 1) return KDA_ERR_ARG;
+  int32_t* cu = reinterpret_cast<int32_t*>(offsets);
+  const int row_chunks = (int)(((int64_t)tokens + kda::kChunk - 1) / kda::kChunk);
+  kda::dense_offsets_kernel<<<(batch + 256) / 256, 256, 0, (cudaStream_t)stream>>>(cu, cu + batch + 1, batch, 1, tokens,
+                                                                                 row_chunks, row_chunks);
+  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}

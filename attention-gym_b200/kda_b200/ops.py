@@ -130,10 +130,13 @@ def _require_cuda(t: torch.Tensor, what: str):
 # chunked forward / backward
 # --------------------------------------------------------------------------------------------
 def _dense_offsets(q):
+    """Offsets of a dense batch as a packed one: (the buffer that owns both, pointers to cu_seqlens and
+    chunk_offsets, chunks), from one launch (arange and two products: 15 us more of host time)."""
     batch, tokens = q.shape[0], q.shape[1]
-    per_row = (tokens + _CHUNK - 1) // _CHUNK
-    steps = torch.arange(batch + 1, dtype=torch.int32, device=q.device)
-    return steps * tokens, steps * per_row, batch * per_row
+    both = torch.empty(2 * (batch + 1), dtype=torch.int32, device=q.device)
+    base = both.data_ptr()
+    _cabi.call("kda_dense_offsets", 1, base, batch, tokens, _cabi.stream())
+    return both, base, base + 4 * (batch + 1), batch * ((tokens + _CHUNK - 1) // _CHUNK)
 
 
 def _fwd_workspace_bytes(batch, tokens, heads, packed_nseq, keep):
@@ -220,14 +223,14 @@ def _chunk_fwd_ragged_with_state(q, k, v, gate, beta, initial_state, cu_seqlens,
 def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_output,
                     d_final_state, initial_state, want_state_grad, saved=None, rstd=None):
     batch, tokens, heads, _ = q.shape
-    if cu_seqlens is None:
-        cu_seqlens, chunk_offsets, capacity = _dense_offsets(q)
-        nseq = batch
-        packed = False
-    else:
+    packed = cu_seqlens is not None
+    if packed:
         nseq = cu_seqlens.shape[0] - 1
         capacity = chunk_capacity(tokens, nseq, _CHUNK)
-        packed = True
+        cu_ptr, chunks_ptr = _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets)
+    else:
+        nseq = batch
+        offsets, cu_ptr, chunks_ptr, capacity = _dense_offsets(q)
     total = batch * tokens
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     gate = gate.float().contiguous()
@@ -254,8 +257,8 @@ def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_
     head = (_cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
             _cabi.ptr(beta), _cabi.ptr(aqk), _cabi.ptr(akk), _cabi.ptr(initial_state),
             _cabi.ptr(d_output), _cabi.ptr(d_final_state), _cabi.ptr(dq), _cabi.ptr(dk),
-            _cabi.ptr(dv), _cabi.ptr(dg), _cabi.ptr(db), _cabi.ptr(dh0), _cabi.ptr(cu_seqlens),
-            _cabi.ptr(chunk_offsets), nseq, total, heads, 128, 128, capacity)
+            _cabi.ptr(dv), _cabi.ptr(dg), _cabi.ptr(db), _cabi.ptr(dh0), cu_ptr,
+            chunks_ptr, nseq, total, heads, 128, 128, capacity)
     if rstd is not None:
         _cabi.call("kda_chunk_bwd_qknorm_saved", 2, *head, _cabi.ptr(rstd[0]), _cabi.ptr(rstd[1]),
                    _cabi.ptr(workspace), ws_bytes, _cabi.stream())
@@ -306,11 +309,12 @@ def _chunk_bwd_state_saved(gate, aqk, saved, cu_seqlens, chunk_offsets, d_output
     if dim != 128 or gate.shape[-1] != 128:
         raise ValueError("the fused KDA core requires K=V=128")
     if cu_seqlens is None:
-        cu_seqlens, chunk_offsets, capacity = _dense_offsets(d_output)
+        offsets, cu_ptr, chunks_ptr, capacity = _dense_offsets(d_output)
         nseq = batch
     else:
         nseq = cu_seqlens.shape[0] - 1
         capacity = chunk_capacity(tokens, nseq, _CHUNK)
+        cu_ptr, chunks_ptr = _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets)
     total = batch * tokens
     ws_bytes = _cabi.lib().kda_chunk_bwd_workspace_bytes(total, heads, capacity)
     if saved.numel() < ws_bytes or saved.dtype != torch.uint8 or not saved.is_cuda:
@@ -321,8 +325,8 @@ def _chunk_bwd_state_saved(gate, aqk, saved, cu_seqlens, chunk_offsets, d_output
         d_final_state = d_final_state.float().contiguous()
     dh0 = torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=d_output.device)
     _cabi.call("kda_chunk_bwd_state_saved", 1, _cabi.ptr(gate), _cabi.ptr(aqk.contiguous()),
-               _cabi.ptr(d_output), _cabi.ptr(d_final_state), _cabi.ptr(dh0), _cabi.ptr(cu_seqlens),
-               _cabi.ptr(chunk_offsets), nseq, total, heads, 128, 128, capacity, _cabi.ptr(saved),
+               _cabi.ptr(d_output), _cabi.ptr(d_final_state), _cabi.ptr(dh0), cu_ptr,
+               chunks_ptr, nseq, total, heads, 128, 128, capacity, _cabi.ptr(saved),
                saved.numel(), _cabi.stream())
     return dh0
 
@@ -338,13 +342,14 @@ def _chunk_fwd_qknorm(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offs
     batch, tokens, heads, _ = q.shape
     packed = cu_seqlens is not None
     if not packed:
-        cu_seqlens, chunk_offsets, capacity = _dense_offsets(q)
+        offsets, cu_ptr, chunks_ptr, capacity = _dense_offsets(q)
         nseq = batch
     else:
         if batch != 1:
             raise ValueError("packed cu_seqlens require batch size one")
         nseq = cu_seqlens.shape[0] - 1
         capacity = chunk_capacity(tokens, nseq, _CHUNK)
+        cu_ptr, chunks_ptr = _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets)
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     gate, beta = gate.float().contiguous(), beta.float().contiguous()
     if initial_state is not None:
@@ -363,7 +368,7 @@ def _chunk_fwd_qknorm(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offs
     _cabi.call("kda_chunk_fwd_qknorm", 3, _cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
                _cabi.ptr(beta), _cabi.ptr(initial_state), _cabi.ptr(state) if want_state else None,
                _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk), _cabi.ptr(rstd_q), _cabi.ptr(rstd_k),
-               float(eps), _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets), nseq, total, heads, 128, 128,
+               float(eps), cu_ptr, chunks_ptr, nseq, total, heads, 128, 128,
                capacity, _cabi.ptr(workspace), ws_bytes, int(keep), _cabi.stream())
     return out, state, aqk, akk, workspace, rstd_q, rstd_k
 

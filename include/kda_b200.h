@@ -279,6 +279,10 @@ int kda_chunk_bwd_qknorm_saved(const void* q, const void* k, const void* v, cons
                                int key_dim, int value_dim, int num_chunks, const float* rstd_q,
                                const float* rstd_k, void* saved, int64_t saved_bytes, void* stream);
 
+/* The packed description of a dense [batch, tokens] input: cu_seqlens [batch + 1] and, right behind it,
+ * chunk_offsets [batch + 1] (int32, on the device). */
+int kda_dense_offsets(void* offsets, int batch, int tokens, void* stream);
+
 /* The two halves of kda_chunk_fwd: `prepare` = the chunk-parallel part (fills aqk, akk and the
  * workspace), `state` = the serial state recurrence over the workspace (writes out and final_state,
  * either may be NULL).  use_u == 0 runs the homogeneous recurrence: with identity matrices as
