@@ -1,0 +1,47 @@
+"""The state walks of packed batches in the order of their lengths.
+The order of the chains must not touch a bit: every sequence is compared with the same sequence run alone."""
+
+import pytest
+import torch
+
+import kda_b200
+from oracle import kda_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(inp, spans=None, normalize=False, grad=True):
+    leaves = [inp[n].bfloat16().cuda() for n in ("q", "k", "v")] + [inp["cum_gate"].cuda(), inp["beta"].cuda(),
+                                                                   inp["h0"].cuda()]
+    do = torch.randn(inp["v"].shape, generator=torch.Generator().manual_seed(61)).bfloat16().cuda()
+    if spans is not None:
+        a, b, i = spans
+        leaves = [x[:, a:b].contiguous() for x in leaves[:5]] + [leaves[5][i:i + 1].contiguous()]
+        do = do[:, a:b].contiguous()
+    leaves = [x.requires_grad_(grad) for x in leaves]
+    cu = None if spans is not None or inp["cu_seqlens"] is None else inp["cu_seqlens"].cuda()
+    o, st = kda_b200.chunk_kda(*leaves, cu_seqlens=cu, output_final_state=True, normalize_qk=normalize)
+    if not grad:
+        return [o, st]
+    return [o, st, *torch.autograd.grad([o, st], leaves, [do, 0.1 * torch.ones_like(st)])]
+
+
+@pytest.mark.parametrize("sequences", [2, 5, 128, 129])      # 129: more than the kernels rank
+def test_order_of_the_chains_does_not_touch_the_results(sequences):
+    heads = 80 if sequences == 2 else (31 if sequences == 5 else 2)       # more chains than SMs
+    lengths = [1 + (37 * i * i + 11 * i) % 331 for i in range(sequences)]
+    lengths[-1] = 400                                        # the longest comes last
+    if sequences > 2:
+        lengths[1] = 0
+        lengths[2] = lengths[-1]                             # a tie
+    inp = orc.make_inputs(1, sum(lengths), heads, 128, 128, seed=62, with_state=True, lengths=lengths)
+    whole = _run(inp)
+    marks = inp["cu_seqlens"].tolist()
+    for i in {0, 2 % sequences, sequences // 2, sequences - 1}:
+        a, b = marks[i], marks[i + 1]
+        if a == b:
+            continue
+        alone = _run(inp, (a, b, i))
+        for n, (x, y) in enumerate(zip(whole, alone)):
+            part = x[i:i + 1] if n in (1, 7) else x[:, a:b]
+            assert torch.equal(part, y), (i, n)
