@@ -38,6 +38,7 @@ __device__ __forceinline__ float block_sum128(float v, float* scratch, int tid) 
 
 __global__ void __launch_bounds__(128) kda_decode_prep_kernel(const PrepDecodeParams p) {
   __shared__ float scratch[4];
+  grid_dependency_trigger();
   const int tid = threadIdx.x, head = blockIdx.x % p.H, seq = blockIdx.x / p.H;
   const int HD = p.H * 128, C = 3 * HD, W = p.W;
   const int64_t orow = ((int64_t)seq * p.H + head) * 128 + tid;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(128) kda_decode_prep_kernel(const PrepDecodePa
 // eight (head, channel) pairs.
 template <int W>
 __global__ void __launch_bounds__(256) kda_decode_prep_vec_kernel(const PrepDecodeParams p) {
+  grid_dependency_trigger();       // the state update may start fetching states
   const int seq = blockIdx.y, vec = blockIdx.x * 256 + threadIdx.x;
   const int HD = p.H * 128, C = 3 * HD, nvec = C / 8;
   const bool in_range = vec < nvec;

@@ -568,6 +568,7 @@ kda_decode_kernel(const ScanParams p, const __grid_constant__ DecodeMaps maps, i
   };
 
   Ops f0{}, f1{}, f2{};                   // set (item counter mod 3)
+  grid_dependency_wait();                 // q, k, v and the gate may still be on their way (see launch_decode)
   fetch(blockIdx.x, f0);
   publish(0, f0);
   fetch(blockIdx.x + stride, f1);
@@ -587,7 +588,10 @@ kda_decode_kernel(const ScanParams p, const __grid_constant__ DecodeMaps maps, i
 
 static __device__ int g_decode_error = 0;
 
-static int launch_decode(const ScanParams& p, cudaStream_t stream) {
+// overlap: the kernel before this one in the stream is the preprocessing of the same step and everything
+// before that one has finished (it is an ordinary launch), so the states, which the preprocessing neither
+// reads nor writes, are fetched while it drains; only the token operands wait for it.
+static int launch_decode(const ScanParams& p, bool overlap, cudaStream_t stream) {
   const int64_t items = (int64_t)p.nseq * p.H;
   if (items <= 0) return KDA_OK;
   const bool paged = p.state_indices != nullptr;
@@ -605,9 +609,29 @@ static int launch_decode(const ScanParams& p, cudaStream_t stream) {
                            kDecSmemBytes + 1024) != cudaSuccess)
     return KDA_ERR_LAUNCH;
   StageScope timing(kStageRecurrent, stream);
-  kda_decode_kernel<<<(unsigned)(items < sms ? items : sms), kDecConsumers + 128, kDecSmemBytes + 1024, stream>>>(
-      p, maps, error, debug_profile_buffer());
-  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)(items < sms ? items : sms));
+  config.blockDim = dim3(kDecConsumers + 128);
+  config.dynamicSmemBytes = kDecSmemBytes + 1024;
+  config.stream = stream;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&config, kda_decode_kernel, p, maps, error, debug_profile_buffer()) == cudaSuccess
+             ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
+static int launch_recurrent(const ScanParams& p, bool overlap, cudaStream_t s) {
+  // the decode step proper: one token per sequence, K = V = 128, state in and out
+  const bool decode = p.T == 1 && !p.cu_seqlens && p.K == 128 && p.V == 128 &&
+                      p.h0 && (p.state_indices || p.ht) && p.nseq * (int64_t)p.H < (1 << 24) &&
+                      ((uintptr_t)p.h0 & 15) == 0 && ((uintptr_t)p.ht & 15) == 0 &&
+                      (!p.state_indices || (p.slot_stride % 128 == 0 && p.slot_stride >= (int64_t)p.H * 16384 &&
+                                            (int64_t)p.num_slots * (p.slot_stride / 128) < (1LL << 31)));
+  if (decode) return launch_decode(p, overlap, s);
+  return launch_scan_any(p, false, s);
 }
 
 }  // namespace kda
@@ -632,15 +656,41 @@ extern "C" int kda_recurrent_fwd(const void* q, const void* k, const void* v, co
   p.slot_stride = slot_stride; p.num_slots = num_slots;
   p.nseq = nseq; p.T = tokens_per_row; p.H = heads; p.K = key_dim; p.V = value_dim;
   p.scale = scale;
-  cudaStream_t s = (cudaStream_t)stream;
-  // the decode step proper: one token per sequence, K = V = 128, state in and out
-  const bool decode = tokens_per_row == 1 && !cu_seqlens && key_dim == 128 && value_dim == 128 &&
-                      initial_state && (state_indices || final_state) && nseq * (int64_t)heads < (1 << 24) &&
-                      ((uintptr_t)initial_state & 15) == 0 && ((uintptr_t)final_state & 15) == 0 &&
-                      (!state_indices || (slot_stride % 128 == 0 && slot_stride >= (int64_t)heads * 16384 &&
-                                          (int64_t)num_slots * (slot_stride / 128) < (1LL << 31)));
-  if (decode) return launch_decode(p, s);
-  return launch_scan_any(p, false, s);
+  return launch_recurrent(p, false, (cudaStream_t)stream);
+}
+
+// One decode step: preprocessing and state update in one call.  scratch holds q, k, v (dtype) and the gate
+// (fp32), [nseq, heads, 128] each, between the two launches.
+extern "C" int kda_decode_step(const void* x, const void* conv_weight, void* conv_state, const int32_t* state_indices,
+                               const void* raw_gate, int dt_gate, const float* A_log, const float* dt_bias,
+                               const void* beta, int dt_beta, float* state_pool, int64_t slot_stride, void* scratch,
+                               void* out, int dtype, int nseq, int heads, int width, int conv_slots, int state_slots,
+                               int activation, float lower_bound, float eps, void* stream) {
+  using namespace kda;
+  if (!state_indices || !beta || !state_pool || !scratch || !out) return KDA_ERR_ARG;
+  if (nseq < 0 || heads < 1) return KDA_ERR_ARG;
+  const int64_t elems = (int64_t)nseq * heads * 128;
+  unsigned char* q = reinterpret_cast<unsigned char*>(scratch);
+  unsigned char* k = q + elems * dtype_size(dtype);
+  unsigned char* v = k + elems * dtype_size(dtype);
+  float* gate = reinterpret_cast<float*>(v + elems * dtype_size(dtype));
+  const int rc = kda_decode_prep(x, conv_weight, conv_state, state_indices, raw_gate, dt_gate, A_log, dt_bias, q, k, v,
+                                 gate, dtype, nseq, heads, 128, width, conv_slots, activation, lower_bound, eps, stream);
+  if (rc != KDA_OK || nseq == 0) return rc;
+  ScanParams p{};
+  p.q = q; p.k = k; p.v = v; p.g = gate; p.beta = beta;
+  p.dt_q = p.dt_k = p.dt_v = p.dt_out = dtype; p.dt_g = KDA_F32; p.dt_beta = dt_beta;
+  p.h0 = state_pool; p.out = out; p.state_indices = state_indices;
+  p.slot_stride = slot_stride; p.num_slots = state_slots;
+  p.nseq = nseq; p.T = 1; p.H = heads; p.K = p.V = 128;
+  p.scale = 0.08838834764831845f;  // 128^-0.5
+  // The state update overlaps the preprocessing while that is a fraction of a wave; at several waves the early
+  // state loads only slow its last ones down.  H = 32: 37 sequences (222 blocks) 36 us a step overlapped; 256
+  // sequences (1536 blocks) 212.8 overlapped, 208.4 one after the other.
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool overlap = (int64_t)nseq * ((3 * heads * 16 + 255) / 256) <= 2 * sms;
+  return launch_recurrent(p, overlap, (cudaStream_t)stream);
 }
 
 // The recurrence on the cumulative gate of chunk_kda (dense or packed, no paged pool).

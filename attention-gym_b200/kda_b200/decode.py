@@ -1,4 +1,4 @@
-"""The decode step as two launches: fused preprocessing, then the paged state update.
+"""The decode step as one call of two overlapping launches: fused preprocessing, then the paged state update.
 
 ``decode_step`` is what a serving layer runs per generated token: the q | k | v projection goes
 through the short convolution (paged history, advanced in place) and SiLU, q and k are
@@ -6,18 +6,17 @@ L2-normalised, the raw gate projection becomes the bounded per-token log2 gate, 
 state pool is advanced in place.  The reference exposes these as separate operators
 (``causal_conv1d_decode``, ``l2norm``, ``bounded_gate_cumsum(chunk_size=1)``, ``recurrent_kda`` with
 ``state_indices``) and lists "decode preprocessing and scan are separate launches" as a serving
-limitation (attn_gym/linear/kda/api.py:210-212); here the preprocessing is one kernel.
+limitation (attn_gym/linear/kda/api.py:210-212); here the preprocessing is one kernel, and the state update
+starts fetching states while it drains.
 """
 
 from __future__ import annotations
 
 import torch
 
-from . import ops as _opsmod  # noqa: F401  (registers the operators)
-from .api import recurrent_kda
+from .ops import decode_step_op
 from .preops import MAX_GATE_LOWER_BOUND_MAGNITUDE
-
-_ops = torch.ops.kda_b200
+from .validation import SUPPORTED_INPUT_DTYPES
 
 
 def decode_step(x, conv_weight, conv_state, raw_gate, A_log, dt_bias, beta, state_pool,
@@ -59,14 +58,18 @@ def decode_step(x, conv_weight, conv_state, raw_gate, A_log, dt_bias, beta, stat
     if (state_indices.dtype != torch.int32 or tuple(state_indices.shape) != (x.shape[0],)
             or not state_indices.is_contiguous() or state_indices.device != x.device):
         raise ValueError("state_indices must be a contiguous int32 tensor with one entry per sequence")
-    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, conv_weight, raw_gate, beta)):
+    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, conv_weight, raw_gate, beta, state_pool)):
         raise RuntimeError("decode_step is inference-only and has no backward")
-    q, k, v, gate = _ops.kda_decode_prep(x.contiguous(), conv_weight.contiguous(), conv_state,
-                                         state_indices, raw_gate, A_log, dt_bias, heads, activation,
-                                         float(lower_bound), float(eps))
-    out, _ = recurrent_kda(q, k, v, gate, beta.reshape(x.shape[0], 1, heads), state_pool,
-                           state_indices=state_indices)
-    return out.reshape(x.shape[0], heads, 128)
+    if x.shape[0] == 0 or heads == 0:
+        raise ValueError("the decode step requires at least one sequence and one head")
+    if beta.device != x.device:
+        raise ValueError("x and beta must be on the same device")
+    if beta.dtype not in SUPPORTED_INPUT_DTYPES:
+        raise TypeError(f"beta must use one of {', '.join(str(d) for d in SUPPORTED_INPUT_DTYPES)}")
+    if state_pool.stride()[1:] != (128 * 128, 128, 1) or state_pool.stride(0) < heads * 128 * 128:
+        raise TypeError("the state pool must be contiguous within each [H, 128, 128] slot, slots apart")
+    return decode_step_op(x, conv_weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta,
+                          activation, float(lower_bound), float(eps))
 
 
 __all__ = ["decode_step"]

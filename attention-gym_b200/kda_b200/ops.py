@@ -119,6 +119,10 @@ _lib_own = torch.library.Library(_NS_OWN, "DEF")
 # The token scan on the cumulative gate of chunk_kda (the fp32-accurate evaluation).
 _lib_own.define("chunk_scan(Tensor q, Tensor k, Tensor v, Tensor cumulative_gate, Tensor beta, "
                 "Tensor? initial_state, Tensor? cu_seqlens, bool want_state) -> (Tensor, Tensor)")
+# One decode step: preprocessing and paged state update.
+_lib_own.define("decode_step(Tensor x, Tensor weight, Tensor(a!) conv_state, Tensor(b!) state_pool, "
+                "Tensor state_indices, Tensor raw_gate, Tensor A_log, Tensor dt_bias, Tensor beta, "
+                "str? activation, float lower_bound, float eps) -> Tensor")
 
 
 def _require_cuda(t: torch.Tensor, what: str):
@@ -798,6 +802,27 @@ def _decode_prep(x, weight, conv_state, state_indices, raw_gate, A_log, dt_bias,
     return q, k, v, gate
 
 
+@torch.library.impl(_lib_own, "decode_step", "CUDA")
+def _decode_step(x, weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta, activation,
+                 lower_bound, eps):
+    nseq, heads = x.shape[0], state_pool.shape[1]
+    x, weight, raw_gate, beta = x.contiguous(), weight.contiguous(), raw_gate.contiguous(), beta.contiguous()
+    A_log, dt_bias = A_log.float().contiguous(), dt_bias.float().contiguous()
+    out = torch.empty(nseq, heads, 128, dtype=x.dtype, device=x.device)
+    scratch = torch.empty(nseq * heads * 128 * (3 * x.element_size() + 4), dtype=torch.uint8, device=x.device)
+    _cabi.call("kda_decode_step", 2, x.data_ptr(), weight.data_ptr(), conv_state.data_ptr(), state_indices.data_ptr(),
+               raw_gate.data_ptr(), _cabi.dt(raw_gate), A_log.data_ptr(), dt_bias.data_ptr(), beta.data_ptr(),
+               _cabi.dt(beta), state_pool.data_ptr(), state_pool.stride(0), scratch.data_ptr(), out.data_ptr(),
+               _cabi.dt(x), nseq, heads, weight.shape[1], conv_state.shape[0], state_pool.shape[0],
+               _act_code(activation), lower_bound, eps, _cabi.stream())
+    return out
+
+
+@torch.library.register_fake(f"{_NS_OWN}::decode_step")
+def _(x, weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta, activation, lower_bound, eps):
+    return x.new_empty((x.shape[0], state_pool.shape[1], 128))
+
+
 @torch.library.register_fake(f"{_NS}::kda_decode_prep")
 def _(x, weight, conv_state, state_indices, raw_gate, A_log, dt_bias, heads, activation,
       lower_bound, eps):
@@ -836,6 +861,7 @@ chunk_bwd_qknorm_op = _ops.kda_chunk_bwd_qknorm.default
 chunk_bwd_op = _ops.kda_chunk_bwd.default
 chunk_bwd_with_state_grad_op = _ops.kda_chunk_bwd_with_state_grad.default
 chunk_scan_op = torch.ops.kda_b200_fused.chunk_scan.default
+decode_step_op = torch.ops.kda_b200_fused.decode_step.default
 recurrent_fwd_op = _ops.kda_recurrent_fwd.default
 recurrent_fwd_no_state_op = _ops.kda_recurrent_fwd_no_state.default
 recurrent_fwd_paged_op = _ops.kda_recurrent_fwd_paged.default

@@ -374,6 +374,16 @@ int kda_decode_prep(const void* x, const void* conv_weight, void* conv_state,
                     int dtype, int nseq, int heads, int head_dim, int width, int num_slots,
                     int activation, float lower_bound, float eps, void* stream);
 
+/* One decode step: kda_decode_prep and the paged state update of kda_recurrent_fwd (one token per sequence,
+ * K = V = 128) in one call; the state update starts fetching states while the preprocessing drains.
+ * state_indices selects the slot of both pools; scratch: 16-byte aligned, nseq * heads * 128 elements of q, k, v
+ * (dtype) and the gate (fp32) in that order; out [nseq, heads, 128] in `dtype`. */
+int kda_decode_step(const void* x, const void* conv_weight, void* conv_state, const int32_t* state_indices,
+                    const void* raw_gate, int dt_gate, const float* A_log, const float* dt_bias, const void* beta,
+                    int dt_beta, float* state_pool, int64_t slot_stride, void* scratch, void* out, int dtype,
+                    int nseq, int heads, int width, int conv_slots, int state_slots, int activation,
+                    float lower_bound, float eps, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
