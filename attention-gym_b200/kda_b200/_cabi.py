@@ -68,6 +68,8 @@ _SIGNATURES = {
                                     c_int64, c_void_p]),
     "kda_chunk_fwd_dense_save": (c_int, [c_void_p] * 10 + [c_int, c_int64, c_int, c_int, c_int,
                                          c_void_p, c_int64, c_void_p]),
+    "kda_chunk_fwd_dense_qknorm": (c_int, [c_void_p] * 12 + [c_float, c_int, c_int64, c_int, c_int, c_int,
+                                           c_void_p, c_int64, c_int, c_void_p]),
     "kda_set_row_segments": (c_int, [c_int]),
     "kda_chunk_bwd_workspace_bytes": (c_int64, [c_int64, c_int, c_int64]),
     "kda_chunk_bwd": (c_int, [c_void_p] * 18 + [c_int, c_int64, c_int, c_int, c_int, c_int, c_void_p,

@@ -346,14 +346,12 @@ def _chunk_fwd_qknorm(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offs
     batch, tokens, heads, _ = q.shape
     packed = cu_seqlens is not None
     if not packed:
-        offsets, cu_ptr, chunks_ptr, capacity = _dense_offsets(q)
         nseq = batch
     else:
         if batch != 1:
             raise ValueError("packed cu_seqlens require batch size one")
         nseq = cu_seqlens.shape[0] - 1
         capacity = chunk_capacity(tokens, nseq, _CHUNK)
-        cu_ptr, chunks_ptr = _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets)
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     gate, beta = gate.float().contiguous(), beta.float().contiguous()
     if initial_state is not None:
@@ -367,13 +365,17 @@ def _chunk_fwd_qknorm(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offs
     rstd_k = alloc(batch, tokens, heads, dtype=torch.float32, device=q.device)
     state = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=q.device)
              if want_state else q.new_empty((0,), dtype=torch.float32))
-    ws_bytes = _fwd_workspace_bytes(1, total, heads, nseq, keep)
+    ws_bytes = _fwd_workspace_bytes(batch, tokens, heads, nseq if packed else None, keep)
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    _cabi.call("kda_chunk_fwd_qknorm", 3, _cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
-               _cabi.ptr(beta), _cabi.ptr(initial_state), _cabi.ptr(state) if want_state else None,
-               _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk), _cabi.ptr(rstd_q), _cabi.ptr(rstd_k),
-               float(eps), cu_ptr, chunks_ptr, nseq, total, heads, 128, 128,
-               capacity, _cabi.ptr(workspace), ws_bytes, int(keep), _cabi.stream())
+    head = (_cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate), _cabi.ptr(beta), _cabi.ptr(initial_state),
+            _cabi.ptr(state) if want_state else None, _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk),
+            _cabi.ptr(rstd_q), _cabi.ptr(rstd_k), float(eps))
+    if packed:
+        _cabi.call("kda_chunk_fwd_qknorm", 3, *head, _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets), nseq, total,
+                   heads, 128, 128, capacity, _cabi.ptr(workspace), ws_bytes, int(keep), _cabi.stream())
+    else:
+        _cabi.call("kda_chunk_fwd_dense_qknorm", 3, *head, batch, tokens, heads, 128, 128, _cabi.ptr(workspace),
+                   ws_bytes, int(keep), _cabi.stream())
     return out, state, aqk, akk, workspace, rstd_q, rstd_k
 
 
@@ -393,7 +395,7 @@ def _(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state,
     nseq = q.shape[0] if cu_seqlens is None else cu_seqlens.shape[0] - 1
     state = (q.new_empty((nseq, q.shape[2], q.shape[3], v.shape[-1]), dtype=torch.float32)
              if want_state else q.new_empty((0,), dtype=torch.float32))
-    nbytes = _fwd_workspace_bytes(1, q.shape[0] * q.shape[1], q.shape[2], nseq, keep)
+    nbytes = _fwd_workspace_bytes(q.shape[0], q.shape[1], q.shape[2], None if cu_seqlens is None else nseq, keep)
     rstd = q.new_empty(q.shape[:3], dtype=torch.float32)
     return (v.new_empty(v.shape), state, _tape(q), _tape(q), q.new_empty((nbytes,), dtype=torch.uint8),
             rstd, torch.empty_like(rstd))

@@ -180,6 +180,13 @@ int kda_chunk_fwd_dense_save(const void* q, const void* k, const void* v, const 
                              void* out, void* aqk, void* akk, int batch, int64_t tokens_per_row,
                              int heads, int key_dim, int value_dim, void* saved, int64_t saved_bytes,
                              void* stream);
+/* The dense forward for unnormalised q and k: kda_chunk_fwd_qknorm on equal-length rows, long rows of small
+ * batches walked in parallel segments; workspace of kda_chunk_fwd_dense_workspace_bytes(.., keep). */
+int kda_chunk_fwd_dense_qknorm(const void* q, const void* k, const void* v, const float* cum_gate,
+                               const float* beta, const float* initial_state, float* final_state, void* out,
+                               void* aqk, void* akk, float* rstd_q, float* rstd_k, float eps, int batch,
+                               int64_t tokens_per_row, int heads, int key_dim, int value_dim, void* workspace,
+                               int64_t workspace_bytes, int keep, void* stream);
 int kda_set_row_segments(int segments);
 
 /* kda_chunk_fwd for callers that cannot allocate device memory while they run (an inference

@@ -1,11 +1,13 @@
-"""The state walks of packed batches in the order of their lengths.
+"""The state walks of packed batches in the order of their lengths, and of normalised dense rows in segments.
 The order of the chains must not touch a bit: every sequence is compared with the same sequence run alone."""
 
 import pytest
 import torch
 
 import kda_b200
+from kda_b200 import _cabi
 from oracle import kda_oracle as orc
+from helpers import assert_normalised
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +47,22 @@ def test_order_of_the_chains_does_not_touch_the_results(sequences):
         for n, (x, y) in enumerate(zip(whole, alone)):
             part = x[i:i + 1] if n in (1, 7) else x[:, a:b]
             assert torch.equal(part, y), (i, n)
+
+
+@pytest.mark.parametrize("segments", [2, 3])
+@pytest.mark.parametrize("gate_scale", [1.0, 0.02])
+def test_normalised_rows_walked_in_segments(segments, gate_scale):
+    inp = orc.make_inputs(2, 64 * 11 + 17, 2, 128, 128, seed=63, with_state=True)
+    inp["cum_gate"] = inp["cum_gate"] * gate_scale
+    serial = _run(inp, normalize=True)
+    try:
+        assert _cabi.lib().kda_set_row_segments(segments) == 0
+        split = _run(inp, normalize=True)
+        plain = _run(inp, normalize=True, grad=False)
+    finally:
+        _cabi.lib().kda_set_row_segments(0)
+    # as for rows without the normalisation: the serial walk's bits almost everywhere when the gates forget,
+    # else two bf16 evaluations of the boundary states
+    for x, y in zip(split, serial):
+        assert_normalised(x.float(), y.float(), 1e-4 if gate_scale == 1.0 else 1e-2, "segments")
+    assert torch.equal(plain[0], split[0]) and torch.equal(plain[1], split[1])
