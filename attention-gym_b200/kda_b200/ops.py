@@ -551,7 +551,7 @@ def _(q, k, v, gate, beta, initial_state, cu_seqlens, want_state):
     nseq = q.shape[0] if cu_seqlens is None else cu_seqlens.shape[0] - 1
     state = q.new_empty((nseq, q.shape[2], q.shape[3], v.shape[-1]) if want_state else (0,),
                         dtype=torch.float32)
-    return torch.empty_like(v, dtype=q.dtype), state
+    return q.new_empty(v.shape), state           # contiguous, whatever the strides of v
 
 
 @torch.library.register_fake(f"{_NS}::kda_recurrent_fwd")
