@@ -58,7 +58,8 @@ def decode_step(x, conv_weight, conv_state, raw_gate, A_log, dt_bias, beta, stat
     if (state_indices.dtype != torch.int32 or tuple(state_indices.shape) != (x.shape[0],)
             or not state_indices.is_contiguous() or state_indices.device != x.device):
         raise ValueError("state_indices must be a contiguous int32 tensor with one entry per sequence")
-    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, conv_weight, raw_gate, beta, state_pool)):
+    if torch.is_grad_enabled() and any(t.requires_grad for t in (x, conv_weight, conv_state, raw_gate, A_log, dt_bias,
+                                                                 beta, state_pool)):
         raise RuntimeError("decode_step is inference-only and has no backward")
     if x.shape[0] == 0 or heads == 0:
         raise ValueError("the decode step requires at least one sequence and one head")

@@ -20,3 +20,25 @@ def test_scan_result_is_contiguous_whatever_the_layout_of_v(layout):
         out, state = kda_b200.chunk_kda(q, k, v, g, beta, output_final_state=True)
         assert out.shape == v.shape and out.is_contiguous()
         assert tuple(state.shape) == (batch, heads, kd, vd) and state.is_contiguous()
+
+
+def _decode_args(slots=3, heads=2, seqs=2):
+    def e(*shape, dtype=torch.bfloat16):
+        return torch.empty(*shape, dtype=dtype, device="cuda")
+    f32 = torch.float32
+    return dict(x=e(seqs, 384 * heads), conv_weight=e(384 * heads, 4), conv_state=e(slots, 3, 384 * heads),
+                raw_gate=e(seqs, heads, 128), A_log=e(heads, dtype=f32), dt_bias=e(heads, 128, dtype=f32),
+                beta=e(seqs, heads, dtype=f32), state_pool=e(slots, heads, 128, 128, dtype=f32),
+                state_indices=e(seqs, dtype=torch.int32))
+
+
+@pytest.mark.parametrize("name", ["x", "conv_weight", "conv_state", "raw_gate", "A_log", "dt_bias", "beta", "state_pool"])
+def test_decode_step_refuses_tensors_that_ask_for_gradients(name):
+    with FakeTensorMode():
+        args = _decode_args()
+        args[name].requires_grad_()
+        with pytest.raises(RuntimeError, match="inference-only"):
+            kda_b200.decode_step(**args)
+        with torch.no_grad():
+            out = kda_b200.decode_step(**args)
+        assert tuple(out.shape) == (2, 2, 128) and out.dtype == torch.bfloat16 and not out.requires_grad
