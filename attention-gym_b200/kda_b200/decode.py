@@ -67,8 +67,11 @@ def decode_step(x, conv_weight, conv_state, raw_gate, A_log, dt_bias, beta, stat
         raise ValueError("x and beta must be on the same device")
     if beta.dtype not in SUPPORTED_INPUT_DTYPES:
         raise TypeError(f"beta must use one of {', '.join(str(d) for d in SUPPORTED_INPUT_DTYPES)}")
-    if state_pool.stride()[1:] != (128 * 128, 128, 1) or state_pool.stride(0) < heads * 128 * 128:
-        raise TypeError("the state pool must be contiguous within each [H, 128, 128] slot, slots apart")
+    # (an axis of length one may have any stride in a contiguous tensor)
+    if tuple(state_pool.stride()[1:]) != (128 * 128, 128, 1):
+        raise TypeError("the state pool must be contiguous within each [H, 128, 128] slot")
+    if state_pool.stride(0) < heads * 128 * 128:
+        raise ValueError("state pool slots must not overlap")
     return decode_step_op(x, conv_weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta,
                           activation, float(lower_bound), float(eps))
 

@@ -42,3 +42,15 @@ def test_decode_step_refuses_tensors_that_ask_for_gradients(name):
         with torch.no_grad():
             out = kda_b200.decode_step(**args)
         assert tuple(out.shape) == (2, 2, 128) and out.dtype == torch.bfloat16 and not out.requires_grad
+
+
+def test_decode_step_refuses_pools_whose_strides_recurrent_kda_refuses():
+    with FakeTensorMode(), torch.no_grad():
+        args = _decode_args(slots=1)              # an axis of length one may have any stride and count as contiguous
+        args["state_pool"] = args["state_pool"].as_strided((1, 2, 128, 128), (16384, 16384, 128, 1))
+        with pytest.raises(ValueError, match="overlap"):
+            kda_b200.decode_step(**args)
+        args = _decode_args(heads=1)
+        args["state_pool"] = args["state_pool"].as_strided((3, 1, 128, 128), (16384, 7, 128, 1))
+        with pytest.raises(TypeError, match="within each"):
+            kda_b200.decode_step(**args)
