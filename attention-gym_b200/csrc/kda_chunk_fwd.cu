@@ -300,20 +300,33 @@ __global__ void dense_offsets_kernel(int32_t* cu, int32_t* co, int count, int se
 
 static int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
 
-struct DenseScratch {   // byte offsets from the start of the scratch region
-  int64_t cu, co, limit, b, trans, hin, total;
+struct DenseScratch {   // byte offsets from the start of the workspace
+  int64_t cu, co, limit, b, trans, hin, end;      // end: the bytes the workspace needs
 };
-static DenseScratch dense_scratch(int64_t count, int heads) {
-  DenseScratch d;
+// What the dense forward keeps beside w, u, kg, qg: the offsets, and for rows in segments three fp32 states per
+// (segment, head).  A forward that keeps its intermediates puts it where the backward pass will write dh[c], which
+// the forward leaves alone, so the kept buffer does not grow: 32 KiB per (chunk, head) there against 192 KiB per
+// segment of at least 64 chunks.  Otherwise (no kept buffer, or segments forced to be shorter) it is appended.
+static DenseScratch dense_scratch(bool keep, int batch, int64_t tokens_per_row, int heads, const DensePlan& pl) {
+  DenseScratch d{};
+  const int64_t total = (int64_t)batch * tokens_per_row, chunks = (int64_t)batch * pl.row_chunks;
+  const int64_t base = keep ? kda_chunk_bwd_workspace_bytes(total, heads, chunks)
+                            : kda_chunk_fwd_workspace_bytes(total, heads);
   int64_t at = 0;
-  d.cu = at; at = align256(at + (count + 1) * 4);
-  d.co = at; at = align256(at + (count + 1) * 4);
-  d.limit = at; at = align256(at + count * heads * 4);
-  const int64_t states = count * heads * (int64_t)D * D * 4;
-  d.b = at; at += states;
-  d.trans = at; at += states;
-  d.hin = at; at += states;
-  d.total = at;
+  d.cu = at; at = align256(at + (pl.count + 1) * 4);
+  d.co = at; at = align256(at + (pl.count + 1) * 4);
+  if (pl.segs > 1) {
+    const int64_t states = pl.count * heads * (int64_t)D * D * 4;
+    d.limit = at; at = align256(at + pl.count * heads * 4);
+    d.b = at; at += states;
+    d.trans = at; at += states;
+    d.hin = at; at += states;
+  }
+  const int64_t hs = chunks * heads * (int64_t)D * D * 2;      // bytes of h[c], and of dh[c] behind it
+  const bool inside = keep && at <= hs;
+  const int64_t start = inside ? 6 * total * heads * (int64_t)D * 2 + hs : align256(base);
+  for (int64_t* x : {&d.cu, &d.co, &d.limit, &d.b, &d.trans, &d.hin}) *x += start;
+  d.end = inside ? base : start + at;
   return d;
 }
 
@@ -328,14 +341,7 @@ extern "C" int kda_set_row_segments(int segments) {
 extern "C" int64_t kda_chunk_fwd_dense_workspace_bytes(int batch, int64_t tokens_per_row, int heads,
                                                        int keep) {
   if (batch < 1 || tokens_per_row < 1 || heads < 1) return 0;
-  const int64_t total = (int64_t)batch * tokens_per_row;
-  const kda::DensePlan pl = kda::plan_dense(batch, tokens_per_row, heads);
-  const int64_t base = keep ? kda_chunk_bwd_workspace_bytes(total, heads, (int64_t)batch * pl.row_chunks)
-                            : kda_chunk_fwd_workspace_bytes(total, heads);
-  // the plan may change with kda_set_row_segments between this call and the launch: size for the
-  // largest scratch either can ask for (segments only matter through count = batch * segs)
-  const int64_t worst = (int64_t)batch * (pl.segs > 8 ? pl.segs : 8);
-  return kda::align256(base) + kda::dense_scratch(worst, heads).total;
+  return kda::dense_scratch(keep != 0, batch, tokens_per_row, heads, kda::plan_dense(batch, tokens_per_row, heads)).end;
 }
 
 static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float eps, const void* q, const void* k, const void* v,
@@ -351,11 +357,9 @@ static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float e
   const kda::DensePlan pl = kda::plan_dense(batch, tokens_per_row, heads);
   if (pl.count * heads * 8 > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
   const int chunks = batch * pl.row_chunks;
-  const int64_t base = kda::align256(keep ? kda_chunk_bwd_workspace_bytes(total, heads, chunks)
-                                          : kda_chunk_fwd_workspace_bytes(total, heads));
-  const kda::DenseScratch sc = kda::dense_scratch(pl.count, heads);
-  if (workspace_bytes < base + sc.total || ((uintptr_t)workspace & 15) != 0) return KDA_ERR_ARG;
-  unsigned char* scratch = reinterpret_cast<unsigned char*>(workspace) + base;
+  const kda::DenseScratch sc = kda::dense_scratch(keep, batch, tokens_per_row, heads, pl);
+  if (workspace_bytes < sc.end || ((uintptr_t)workspace & 15) != 0) return KDA_ERR_ARG;
+  unsigned char* scratch = reinterpret_cast<unsigned char*>(workspace);
   int32_t* cu = reinterpret_cast<int32_t*>(scratch + sc.cu);
   int32_t* co = reinterpret_cast<int32_t*>(scratch + sc.co);
   cudaStream_t s = (cudaStream_t)stream;

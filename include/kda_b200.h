@@ -166,7 +166,8 @@ int kda_chunk_fwd(const void* q, const void* k, const void* v, const float* cum_
  * zero in fp32; all of them when the gates never forget).  Results equal the unsegmented walk to
  * fp32 resolution of the state.  workspace: kda_chunk_fwd_dense_workspace_bytes(.., keep) bytes with
  * keep = 1 for the _save form, whose buffer kda_chunk_bwd_saved accepts as `saved`.
- * kda_set_row_segments forces the number of segments per row (0 = choose; for tests and tuning).
+ * kda_set_row_segments forces the number of segments per row (0 = choose; for tests and tuning; the size is
+ * that of the plan in force, so it is not to be changed between the sizing and the call).
  * Replaces attn_gym::kda_chunk_fwd / _with_state (kda/ops.py:18-29); the reference lowers dense
  * batches to the packed form too (kda/impl/fused.py:175-182) and walks every row serially. */
 int64_t kda_chunk_fwd_dense_workspace_bytes(int batch, int64_t tokens_per_row, int heads, int keep);

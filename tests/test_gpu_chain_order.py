@@ -66,3 +66,18 @@ def test_normalised_rows_walked_in_segments(segments, gate_scale):
     for x, y in zip(split, serial):
         assert_normalised(x.float(), y.float(), 1e-4 if gate_scale == 1.0 else 1e-2, "segments")
     assert torch.equal(plain[0], split[0]) and torch.equal(plain[1], split[1])
+
+
+@pytest.mark.parametrize("normalize", [False, True])
+def test_kept_forward_of_a_long_row_and_its_gradients(normalize):
+    """Two segments by the library's own choice (128 chunks, few chains): their states lie in the part of the kept
+    buffer that the backward pass overwrites.  Against one segment per row, as above."""
+    inp = orc.make_inputs(1, 64 * 128 + 17, 2, 128, 128, seed=64, with_state=True)
+    split = _run(inp, normalize=normalize)
+    try:
+        assert _cabi.lib().kda_set_row_segments(1) == 0
+        serial = _run(inp, normalize=normalize)
+    finally:
+        _cabi.lib().kda_set_row_segments(0)
+    for x, y in zip(split, serial):
+        assert_normalised(x.float(), y.float(), 1e-4, "segments")
