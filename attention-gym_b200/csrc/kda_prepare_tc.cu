@@ -15,8 +15,8 @@
 //            kg, qg (straight from registers to memory).  Three exponentials per element; everything
 //            else comes from small per-(block, channel) tables.
 //   phase 2  UMMA, M = 64 (the Qr, Kr rows of a pair of row blocks), N = 16 (r + 1) columns of Kn_r
-//   phase 3  epilogue: masked, scaled Aqk tile (bf16); L in fp32; A = (I + L)^-1 by 16 x 16 blocks in
-//            fp32 (diagonal blocks) and split tf32 (the rest); A as a bf16 operand tile and to memory (the tape)
+//   phase 3  epilogue: masked, scaled Aqk tile (bf16); L in fp32; A = (I + L)^-1 by 16 x 16 blocks on
+//            the CUDA cores in fp32; A as a bf16 operand tile and to memory (the tape)
 //   phase 4  UMMA M = 64, N = 128:  w = A (beta k 2^G),  u = A (beta v);  epilogue; TMA stores.
 //
 // Two CTAs of 256 threads per SM, 113 KiB of shared memory and 256 tensor-memory columns each.  An item
@@ -25,10 +25,10 @@
 // comes from the lifetimes: the gates move to registers and their tile becomes the Qr / Kr operand, v is
 // fetched into the q tile when q is spent, and the solve, its operand tile and the result staging share
 // the column-operand tiles.
-// B = 8, T = 4096, H = 32: 0.597 ms = 4.5 TB/s of its 2564 B per unit, against 0.850 ms with one CTA of 512
-// threads per SM and 230 KiB; one sequence of 1000 tokens, H = 32: 33 against 44 us.  (Two CTAs of 512
+// B = 8, T = 4096, H = 32: 0.622 ms = 4.3 TB/s of its 2564 B per unit, against 0.848 ms with one CTA of 512
+// threads per SM and 230 KiB; one sequence of 1000 tokens, H = 32: 34 against 43 us.  (Two CTAs of 512
 // threads with 64 registers: 0.75 ms, 30 % more instructions and more waiting at barriers.)  Issue slots and the
-// shared-memory port are each half busy now; the rest is the latency of the chain at four warps per scheduler.
+// shared-memory port are each half busy; the rest is the latency of the chain at four warps per scheduler.
 //
 // Gate rebasing and its range contract are those of the reference (fwd/triton/gate_fwd.py:619-631):
 // exponents are clamped at 126, so masked entries cannot produce NaN.
@@ -77,8 +77,7 @@ constexpr int K = 49152;                   // k, then beta k 2^G in place
 constexpr int KN = 65536;                  // column operands Kn_0 .. Kn_3; once multiplied:
 constexpr int AQK = KN;                    //   Aqk tile
 constexpr int LF = KN + 8192;              //   L blocks (fp32)
-constexpr int AD = LF + 12800;             //   diagonal blocks of A (fp32), and their transposes
-constexpr int ADT = AD + 5120;
+constexpr int AD = LF + 12800;             //   diagonal blocks of A (fp32)
 constexpr int AT = KN + 32768;             //   A as a bf16 operand tile
 constexpr int W = KN, U = KN + 16384;      //   after the last product: staging of w, u
 constexpr int TAB = KN + 40960;            // per-channel tables of phase 1; then the blocks A[r][r] L[r][m]
@@ -87,7 +86,7 @@ constexpr int BETA = TAB + 7680, MISC = BETA + 512, OFFS = MISC + 128;      // b
 constexpr int kOffCache = 112;             // cu_seqlens / chunk_offsets entries kept in shared memory
 constexpr int TOTAL = OFFS + 2 * 4 * kOffCache;
 constexpr int BP = 20, BLK = 16 * BP;      // pitch and size of a 16 x 16 fp32 block (floats)
-static_assert(ADT + 4 * 4 * BLK <= AT && 6 * 4 * BLK <= BETA - BF && TOTAL <= 115712, "two CTAs per SM");
+static_assert(AD + 4 * 4 * BLK <= AT && 6 * 4 * BLK <= BETA - BF && TOTAL <= 115712, "two CTAs per SM");
 }  // namespace pl
 namespace pt {  // tensor-memory columns
 constexpr int kCols = 256;
@@ -145,27 +144,6 @@ __device__ __forceinline__ f32x2 unpack_pair(uint32_t u) {
   return pack2(f.x, f.y);
 }
 
-// An fp32 value as the sum of two tf32 values (to 2^-22 of it), and D += A B on 16 x 8 x 8 fragments.  Which
-// column of A meets which row of B is free: slots t and t + 4 of a step stand for columns 2 t and 2 t + 1, so
-// fragments are 8-byte loads and the result fragment of one product is the left fragment of the next.
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  // round to nearest by an integer add on the 13 dropped bits (cvt.rna runs on the slow conversion pipe); the
-  // tensor cores ignore the dropped bits of an operand, so only the value that is subtracted is masked
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
-}
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// step `s` (8 columns) of a 16 x 16 row-major block as a left fragment, split
-__device__ __forceinline__ void ld_left(const float* blk, int s, int lid, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-  const float* x = blk + (lid >> 2) * pl::BP + 8 * s + 2 * (lid & 3);
-  const float2 u = *reinterpret_cast<const float2*>(x), v = *reinterpret_cast<const float2*>(x + 8 * pl::BP);
-  split_tf32(u.x, hi[0], lo[0]); split_tf32(v.x, hi[1], lo[1]);
-  split_tf32(u.y, hi[2], lo[2]); split_tf32(v.y, hi[3], lo[3]);
-}
-
 // NORM: q and k arrive unnormalised; every row is scaled to unit L2 norm (and rounded to bf16, as a
 // separate l2norm launch would leave it) while its pieces pass through the registers of phase 1,
 // and the two reciprocal norms are kept for the backward pass
@@ -188,7 +166,6 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   int* s_next = reinterpret_cast<int*>(sm + pl::MISC + 96);                // next item: token0 (two words), valid
   float* Lf = reinterpret_cast<float*>(sm + pl::LF);
   float* Ad = reinterpret_cast<float*>(sm + pl::AD);
-  float* Adt = reinterpret_cast<float*>(sm + pl::ADT);
   float* Bf = reinterpret_cast<float*>(sm + pl::BF);
   // rows: 0..3 R_b, 4..7 2^{R_b}, 8..13 2^{R_r - R_b} for (r, b) = (1,0) (2,0) (3,0) (2,1) (3,1) (3,2), 14 G_last
   float* tab = reinterpret_cast<float*>(sm + pl::TAB);
@@ -502,11 +479,8 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
         for (int i = j + 4; i < 16; ++i) x[i] = fmaf(-l[i].w, x[j + 3], x[i]);
       }
       float* dst = Ad + b * pl::BLK + c;
-      float4* dt = reinterpret_cast<float4*>(Adt + b * pl::BLK + c * pl::BP);
 #pragma unroll
       for (int i = 0; i < 16; ++i) dst[i * pl::BP] = x[i];
-#pragma unroll
-      for (int i = 0; i < 16; i += 4) dt[i >> 2] = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
     } else {         // meanwhile the Aqk tile leaves and v becomes beta v
       for (int idx = tid - 64; idx < valid * 8; idx += NT - 64) {
         const int r = idx >> 3, c = idx & 7;
@@ -533,38 +507,32 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   pr_mark(p, it, 6);
   {
     const int tid = fresh_tid(), warp = tid >> 5, lid = tid & 31;
-    // B[r][m] = A[r][r] L[r][m] for the six blocks below the diagonal, one warp each.  With them every block of
-    // the inverse is ONE product, A[r][c] = -sum_{c <= m < r} B[r][m] A[m][c], and a column of blocks needs no
-    // other column: one warp walks down each.  The products run on the tensor cores with both operands split
-    // in two (hi hi + hi lo + lo hi, fp32 accumulators): 16 x 16 fragments are read once per warp, where scalar
-    // products read every element 4 to 8 times through the shared-memory port, this kernel's busiest unit.
-    // (0.597 ms with these, 0.620 ms with fp32 fused multiply-adds for the same products; the distance of every
-  // output and gradient from a 64-bit evaluation is the same to four digits.)
+    // B[r][m] = A[r][r] L[r][m] for the six blocks below the diagonal, one warp each and a 2 x 4 tile per lane.
+    // With them every block of the inverse is ONE product, A[r][c] = -sum_{c <= m < r} B[r][m] A[m][c], so the
+    // blocks at distance 1, 2, 3 from the diagonal cost one barrier each.  (The same products on the tensor cores,
+    // operands split in two tf32 halves: 0.596 instead of 0.622 ms, but 22 instead of 24 operand bits, which is three
+    // times the rounding error of the inverse, and a split loses NaN.)
     if (warp < 6) {
       const int r = warp < 1 ? 1 : (warp < 3 ? 2 : 3), m = warp < 1 ? 0 : (warp < 3 ? warp - 1 : warp - 3);
-      const int gr = lid >> 2, t2 = 2 * (lid & 3);
-      const float* l = Lf + blk_off(r, m) + t2 * pl::BP + gr;         // L[r][m], rows 2 t, 2 t + 1 (+ 8 s), column gr (+ 8 nb)
-      float d0[2][4] = {}, d1[2][4] = {};
+      const int i = 2 * (lid >> 2), j = 4 * (lid & 3);
+      const float* a = Ad + r * pl::BLK + i * pl::BP;                // A[r][r], rows i, i + 1
+      const float* l = Lf + blk_off(r, m) + j;                       // L[r][m], columns j .. j + 3
+      f32x2 s0[2] = {0, 0}, s1[2] = {0, 0};                          // (zero bits: +0, +0)
 #pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        uint32_t ah[4], al[4];
-        ld_left(Ad + r * pl::BLK, st, lid, ah, al);
+      for (int k = 0; k < 16; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4*>(a + k), a1 = *reinterpret_cast<const float4*>(a + pl::BP + k);
+        const float av0[4] = {a0.x, a0.y, a0.z, a0.w}, av1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          uint32_t h0, l0, h1, l1;
-          split_tf32(l[8 * st * pl::BP + 8 * nb], h0, l0);
-          split_tf32(l[(8 * st + 1) * pl::BP + 8 * nb], h1, l1);
-          mma_tf32(d0[nb], ah, h0, h1);
-          mma_tf32(d1[nb], ah, l0, l1);
-          mma_tf32(d1[nb], al, h0, h1);
+        for (int e = 0; e < 4; ++e) {
+          const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(l + (k + e) * pl::BP);
+          const f32x2 y0 = pack2(av0[e], av0[e]), y1 = pack2(av1[e], av1[e]);
+          s0[0] = fma2(y0, x.x, s0[0]); s0[1] = fma2(y0, x.y, s0[1]);
+          s1[0] = fma2(y1, x.x, s1[0]); s1[1] = fma2(y1, x.y, s1[1]);
         }
       }
-      float* dst = Bf + warp * pl::BLK + gr * pl::BP + t2;
-#pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        *reinterpret_cast<float2*>(dst + 8 * nb) = make_float2(d0[nb][0] + d1[nb][0], d0[nb][1] + d1[nb][1]);
-        *reinterpret_cast<float2*>(dst + 8 * pl::BP + 8 * nb) = make_float2(d0[nb][2] + d1[nb][2], d0[nb][3] + d1[nb][3]);
-      }
+      float* dst = Bf + warp * pl::BLK + i * pl::BP + j;
+      *reinterpret_cast<ulonglong2*>(dst) = make_ulonglong2(s0[0], s0[1]);
+      *reinterpret_cast<ulonglong2*>(dst + pl::BP) = make_ulonglong2(s1[0], s1[1]);
     } else {      // meanwhile the diagonal blocks, and zeros to their right, go into the operand tile: a row per thread
       const int r = tid - 192, b = r >> 4;
       const float4* src = reinterpret_cast<const float4*>(Ad + b * pl::BLK + (r & 15) * pl::BP);
@@ -579,61 +547,43 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   }
   __syncthreads();
   pr_mark(p, it, 7);
-  {
-    const int tid = fresh_tid(), warp = tid >> 5, lid = tid & 31;
-    if (warp < 3) {
-      // transposed, A[r][c]^T = -sum_m A[m][c]^T B[r][m]^T: a result is a left operand of the next products,
-      // and a lane reads back exactly what it wrote (over the L blocks)
-      const int c = warp, gr = lid >> 2, t2 = 2 * (lid & 3), at = gr * pl::BP + t2;
-      float* xt = Lf + 2 * c * pl::BLK + at;               // A[c + 1][c]^T, A[c + 2][c]^T
-      const float* x = Adt + c * pl::BLK + at;
-#pragma unroll 1
-      for (int r = c + 1; r < 4; ++r) {
-        float d0[2][4] = {}, d1[2][4] = {};
-        const float* brow = Bf + (r * (r - 1) / 2 + c) * pl::BLK + at;      // B[r][c ..], row gr (+ 8 nb)
-#pragma unroll 1
-        for (int m = c; m < r; ++m, brow += pl::BLK) {
-          const float* xm = m == c ? x : xt + (m - c - 1) * pl::BLK;
+  // The blocks at distance DIST from the diagonal, over the L blocks (B holds what is still needed of them) and
+  // straight into the operand tile.  A pair of adjacent lanes owns a 2 x 2 tile of a block and splits the inner
+  // dimension between its lanes in interleaved groups of four; one shuffle per accumulator joins the halves
+  // and each lane then stores one row of the tile.
+  auto blocks_at = [&](auto distance) {
+    constexpr int DIST = decltype(distance)::value;
+    for (int t = fresh_tid(); t < (4 - DIST) * 128; t += NT) {       // whole warps
+      const int ks = t & 1, rest = t >> 1, c = rest >> 6, r = c + DIST, i = 2 * ((rest >> 3) & 7), j = 2 * (rest & 7);
+      const float* b = Bf + (r * (r - 1) / 2 + c) * pl::BLK + i * pl::BP;      // B[r][c ..], rows i, i + 1
+      f32x2 s0 = 0, s1 = 0;
 #pragma unroll
-          for (int st = 0; st < 2; ++st) {
-            const float2 u = *reinterpret_cast<const float2*>(xm + 8 * st), v = *reinterpret_cast<const float2*>(xm + 8 * pl::BP + 8 * st);
-            uint32_t ah[4], al[4];
-            split_tf32(u.x, ah[0], al[0]); split_tf32(v.x, ah[1], al[1]);
-            split_tf32(u.y, ah[2], al[2]); split_tf32(v.y, ah[3], al[3]);
+      for (int m = 0; m < 2 * DIST; ++m) {
+        const int blk = m >> 1, k = 4 * ((ks + 2 * m) & 3);
+        const float4 b0 = *reinterpret_cast<const float4*>(b + blk * pl::BLK + k);
+        const float4 b1 = *reinterpret_cast<const float4*>(b + blk * pl::BLK + pl::BP + k);
+        const float bv0[4] = {b0.x, b0.y, b0.z, b0.w}, bv1[4] = {b1.x, b1.y, b1.z, b1.w};
+        const float* a = (blk == 0 ? Ad + c * pl::BLK : Lf + blk_off(c + blk, c)) + k * pl::BP + j;   // A[c + blk][c], columns j, j + 1
 #pragma unroll
-            for (int nb = 0; nb < 2; ++nb) {
-              const float2 f = *reinterpret_cast<const float2*>(brow + 8 * nb * pl::BP + 8 * st);
-              uint32_t h0, l0, h1, l1;
-              split_tf32(f.x, h0, l0);
-              split_tf32(f.y, h1, l1);
-              mma_tf32(d0[nb], ah, h0, h1);
-              mma_tf32(d1[nb], ah, l0, l1);
-              mma_tf32(d1[nb], al, h0, h1);
-            }
-          }
+        for (int e = 0; e < 4; ++e) {
+          const f32x2 x = *reinterpret_cast<const f32x2*>(a + e * pl::BP);
+          s0 = fma2(pack2(bv0[e], bv0[e]), x, s0);
+          s1 = fma2(pack2(bv1[e], bv1[e]), x, s1);
         }
-        uint32_t w[4];
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          float y[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] = -(d0[nb][e] + d1[nb][e]);
-          w[2 * nb] = pack_bf16(y[0], y[1]);
-          w[2 * nb + 1] = pack_bf16(y[2], y[3]);
-          if (r < 3) {
-            float* dst = xt + (r - c - 1) * pl::BLK + 8 * nb;
-            *reinterpret_cast<float2*>(dst) = make_float2(y[0], y[1]);
-            *reinterpret_cast<float2*>(dst + 8 * pl::BP) = make_float2(y[2], y[3]);
-          }
-        }
-        // four 8 x 8 tiles: rows 16 r + 8 nb .. of the operand tile, 16-byte chunk 2 c + (upper half of the columns)
-        const int row = 16 * r + 8 * (lid >> 4) + (lid & 7);
-        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
-                     ::"r"(saddr(sm + pl::AT + sw128_chunk(row, 2 * c + ((lid >> 3) & 1)))), "r"(w[0]), "r"(w[1]),
-                       "r"(w[2]), "r"(w[3]) : "memory");
       }
+      float2 x0 = unpack2(s0), x1 = unpack2(s1);
+      x0.x += __shfl_xor_sync(0xffffffffu, x0.x, 1); x0.y += __shfl_xor_sync(0xffffffffu, x0.y, 1);
+      x1.x += __shfl_xor_sync(0xffffffffu, x1.x, 1); x1.y += __shfl_xor_sync(0xffffffffu, x1.y, 1);
+      const float2 y = ks ? make_float2(-x1.x, -x1.y) : make_float2(-x0.x, -x0.y);
+      if (r < 3) *reinterpret_cast<float2*>(Lf + blk_off(r, c) + (i + ks) * pl::BP + j) = y;
+      *reinterpret_cast<uint32_t*>(sm + pl::AT + sw128_chunk(16 * r + i + ks, 2 * c + (j >> 3)) + 2 * (j & 7)) = pack_bf16(y.x, y.y);
     }
-  }
+  };
+  blocks_at(std::integral_constant<int, 1>{});
+  __syncthreads();
+  blocks_at(std::integral_constant<int, 2>{});
+  __syncthreads();
+  blocks_at(std::integral_constant<int, 3>{});
   fence_async_smem();
   tc_fence_before();
   __syncthreads();

@@ -61,3 +61,63 @@ def test_nearly_equal_keys():
     # the rows of the inverse nearly cancel, and with them the bf16 operands' roundings weigh more than 2e-2
     # of the result: judged by what bf16 operands do to the oracle
     _check(inp, budget=True)
+
+
+def _tape(k, beta=1.0):
+    """(I + L)^-1 of every chunk as the forward pass stores it, for gates of zero: [chunks, H, 64, 64]."""
+    tokens, heads = k.shape[1:3]
+    gen = torch.Generator().manual_seed(45)
+    q, v = (torch.randn(k.shape, generator=gen).bfloat16().cuda() for _ in range(2))
+    akk = torch.ops.kda_b200.kda_chunk_fwd(q, k.bfloat16().cuda(), v, torch.zeros(k.shape, device="cuda"),
+                                           torch.full(k.shape[:3], beta, device="cuda"), None, True)[2]
+    return akk[0].reshape(tokens // 64, 64, heads, 64).transpose(1, 2).double().cpu()
+
+
+def _inverse_by_blocks(L):
+    """(I + L)^-1 by 16 x 16 blocks in the dtype of L: diagonal blocks by substitution, every other block as one
+    product, summed in two halves of interleaved groups of four."""
+    eye = torch.eye(16, dtype=L.dtype)
+    blk = lambda M, r, c: M[..., 16 * r:16 * r + 16, 16 * c:16 * c + 16]
+    A = torch.zeros_like(L)
+    for b in range(4):
+        blk(A, b, b)[:] = torch.linalg.solve_triangular(eye + blk(L, b, b), eye.expand_as(blk(L, b, b)), upper=False)
+    for d in range(1, 4):
+        half = torch.arange(16 * d) % 8 < 4
+        for c in range(4 - d):
+            r = c + d
+            left = torch.cat([blk(A, r, r) @ blk(L, r, m) for m in range(c, r)], -1)
+            right = torch.cat([blk(A, m, c) for m in range(c, r)], -2)
+            blk(A, r, c)[:] = -(left[..., half] @ right[..., half, :] + left[..., ~half] @ right[..., ~half, :])
+    return A
+
+
+def test_inverse_keeps_fp32_operands():
+    """Equal rows k in a chunk make L = c ones below the diagonal, exact in fp32 (c: a sum of 16-bit squares), and an
+    inverse whose entries -c (1 - c)^(d - 1) die out with the distance d: what is stored there is the rounding
+    error of the solve, not hidden by the bf16 of the tape.  It is that of fp32 operands, 5.6e-9 (root mean square), up
+    to the order of sums of 8 terms (factor 1.2); operands of two tf32 halves give 8.8e-9."""
+    gen = torch.Generator().manual_seed(46)
+    heads, chunks = 8, 8
+    base = torch.randint(1, 32, (chunks, heads, 128), generator=gen) / 256.0
+    base = torch.where((base * base).cumsum(-1) < 0.99, base, 0.0)
+    k = base[:, None].expand(chunks, 64, heads, 128).reshape(1, chunks * 64, heads, 128)
+    c = (base.double() ** 2).sum(-1)[..., None, None]
+    L = c * torch.ones(64, 64, dtype=torch.float64).tril(-1)
+    assert torch.equal(L.float().double(), L) and torch.equal(k.bfloat16().float(), k)
+    want = torch.linalg.inv(torch.eye(64, dtype=torch.float64) + L)
+    below = torch.block_diag(*[torch.ones(16, 16)] * 4) == 0
+    where = below & (want.abs() < 1e-9) & (torch.ones(64, 64).tril() > 0)
+    rms = lambda A: float(((A.double() - want)[where] ** 2).mean().sqrt())
+    assert int(where.sum()) > 20000
+    assert rms(_tape(k)) <= 1.2 * rms(_inverse_by_blocks(L.float()).bfloat16())
+
+
+def test_nan_reaches_every_entry_that_depends_on_it():
+    gen = torch.Generator().manual_seed(47)
+    k = torch.nn.functional.normalize(torch.randn(1, 128, 2, 128, generator=gen), dim=-1)
+    k[0, 5, 1, 77] = float("nan")                   # chunk 0, head 1, row 5
+    A = _tape(k, 0.5)
+    # L has NaN in row 5 and column 5: so has the inverse, in every row below
+    assert torch.isnan(A[0, 1, 6:, 5]).all() and torch.isnan(A[0, 1, 5, :5]).all()
+    assert torch.isnan(A[0, 1, 6:, :5]).all()
+    assert torch.isfinite(A[0, 0]).all() and torch.isfinite(A[1]).all()
