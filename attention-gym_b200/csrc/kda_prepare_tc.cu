@@ -12,8 +12,9 @@
 //   phase 1  every (row, 8 channels) piece once: Qr = q 2^{G - R_b}, Kr = k 2^{G - R_b} (R_b = gate of
 //            the first row of the 16-row block b of the row), the column operands
 //            Kn_r = k 2^{R_r - G} for r >= b, the WY operand beta k 2^G (in place), and the results
-//            kg, qg (straight from registers to memory).  Three exponentials per element; everything
-//            else comes from small per-(block, channel) tables.
+//            kg, qg (straight from registers to memory).  Four exponentials per element; 2^{R_r - R_b}
+//            comes from a small per-(block pair, channel) table.  (2^G as 2^{G - R_b} 2^{R_b} with the
+//            second factor from a table rounds qg and beta k 2^G once more and saves nothing: 0.622 ms.)
 //   phase 2  UMMA, M = 64 (the Qr, Kr rows of a pair of row blocks), N = 16 (r + 1) columns of Kn_r
 //   phase 3  epilogue: masked, scaled Aqk tile (bf16); L in fp32; A = (I + L)^-1 by 16 x 16 blocks on
 //            the CUDA cores in fp32; A as a bf16 operand tile and to memory (the tape)
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   float* Lf = reinterpret_cast<float*>(sm + pl::LF);
   float* Ad = reinterpret_cast<float*>(sm + pl::AD);
   float* Bf = reinterpret_cast<float*>(sm + pl::BF);
-  // rows: 0..3 R_b, 4..7 2^{R_b}, 8..13 2^{R_r - R_b} for (r, b) = (1,0) (2,0) (3,0) (2,1) (3,1) (3,2), 14 G_last
+  // rows: 0..3 R_b, 4..9 2^{R_r - R_b} for (r, b) = (1,0) (2,0) (3,0) (2,1) (3,1) (3,2), 10 G_last
   float* tab = reinterpret_cast<float*>(sm + pl::TAB);
   const unsigned char* sG = sm + pl::G;
 
@@ -280,11 +281,11 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
     const float r0 = gate(0), r1 = gate(16), r2 = gate(32), r3 = gate(48);
     if (tid < 128) {
       t[0] = r0; t[128] = r1; t[256] = r2; t[384] = r3;
-      t[128 * 8] = fexp2(r1 - r0); t[128 * 9] = fexp2(r2 - r0); t[128 * 10] = fexp2(r3 - r0);
-      t[128 * 14] = gate(63);
+      t[128 * 4] = fexp2(r1 - r0);
+      t[128 * 10] = gate(63);
     } else {
-      t[128 * 4] = fexp2(r0); t[128 * 5] = fexp2(r1); t[128 * 6] = fexp2(r2); t[128 * 7] = fexp2(r3);
-      t[128 * 11] = fexp2(r2 - r1); t[128 * 12] = fexp2(r3 - r1); t[128 * 13] = fexp2(r3 - r2);
+      t[128 * 5] = fexp2(r2 - r0); t[128 * 6] = fexp2(r3 - r0);
+      t[128 * 7] = fexp2(r2 - r1); t[128 * 8] = fexp2(r3 - r1); t[128 * 9] = fexp2(r3 - r2);
     }
   }
   if (tid == 0) tma_store_wait_read();       // the w, u staging tiles (over Kn) of the previous item have been read
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   // ---- phase 1: one (row, 8 channels) piece of every row block per thread ---------------------------------
   {
     f32x2 gl[4];
-    ld_tab8(tab + 128 * 14, c16, gl);
+    ld_tab8(tab + 128 * 10, c16, gl);
     const int64_t out0 = ((cw.token0 + il) * H + head) * 128 + 8 * c16;
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -342,22 +343,21 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
         pack8v(kk, kw);
       }
       const uint32_t qu[4] = {qw.x, qw.y, qw.z, qw.w}, ku[4] = {kw.x, kw.y, kw.z, kw.w};
-      f32x2 R[4], P[4], kk[4], ei[4];
+      f32x2 R[4], kk[4], ei[4];
       uint32_t qr[4], kr[4], qg[4], kt[4], kg[4], kn[4];
       const f32x2 bt2 = pack2(s_beta[i], s_beta[i]);
       ld_tab8(tab + 128 * n, c16, R);
-      ld_tab8(tab + 128 * (4 + n), c16, P);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 d = unpack2(fma2(R[e], neg1, g[n][e])), l = unpack2(fma2(g[n][e], neg1, gl[e]));
+        const float2 f = unpack2(g[n][e]), d = unpack2(fma2(R[e], neg1, g[n][e])), l = unpack2(fma2(g[n][e], neg1, gl[e]));
+        const f32x2 eg = pack2(fexp2(f.x), fexp2(f.y)), qq = unpack_pair(qu[e]);      // 2^{G_i}
         const f32x2 er = pack2(fexp2(d.x), fexp2(d.y));                               // 2^{G_i - R_b} <= 1
         ei[e] = pack2(fexp2(fminf(-d.x, 126.f)), fexp2(fminf(-d.y, 126.f)));          // 2^{R_b - G_i}
         kk[e] = unpack_pair(ku[e]);
-        const f32x2 a = mul2(unpack_pair(qu[e]), er), b = mul2(kk[e], er);
-        qr[e] = pack_pair(a);
-        kr[e] = pack_pair(b);
-        qg[e] = pack_pair(mul2(mul2(a, P[e]), scale2));                               // scale q 2^G
-        kt[e] = pack_pair(mul2(mul2(b, P[e]), bt2));                                  // beta k 2^G
+        qr[e] = pack_pair(mul2(qq, er));
+        kr[e] = pack_pair(mul2(kk[e], er));
+        qg[e] = pack_pair(mul2(mul2(qq, eg), scale2));                                // scale q 2^G
+        kt[e] = pack_pair(mul2(mul2(kk[e], eg), bt2));                                // beta k 2^G
         kg[e] = pack_pair(mul2(kk[e], pack2(fexp2(l.x), fexp2(l.y))));                // k 2^{G_last - G}
         kn[e] = pack_pair(mul2(kk[e], ei[e]));
       }
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
       for (int rr = n; rr < 4; ++rr) {
         if (rr > n) {
           f32x2 T[4];                                                                 // 2^{R_r - R_b} <= 1
-          ld_tab8(tab + 128 * (n == 0 ? 7 + rr : (n == 1 ? 9 + rr : 13)), c16, T);
+          ld_tab8(tab + 128 * (n == 0 ? 3 + rr : (n == 1 ? 5 + rr : 9)), c16, T);
 #pragma unroll
           for (int e = 0; e < 4; ++e) kn[e] = pack_pair(mul2(kk[e], mul2(ei[e], T[e])));
         }

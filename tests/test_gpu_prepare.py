@@ -121,3 +121,19 @@ def test_nan_reaches_every_entry_that_depends_on_it():
     assert torch.isnan(A[0, 1, 6:, 5]).all() and torch.isnan(A[0, 1, 5, :5]).all()
     assert torch.isnan(A[0, 1, 6:, :5]).all()
     assert torch.isfinite(A[0, 0]).all() and torch.isfinite(A[1]).all()
+
+
+def test_gated_query_is_rounded_once():
+    """scale q 2^G from one exponential and two fp32 products, bit for bit (torch evaluates the same exp2 in fp32 on
+    the device); 2^G as a product of two exponentials differs in one value out of 10^5."""
+    tokens, heads = 4096, 8
+    gen = torch.Generator(device="cuda").manual_seed(48)
+    q, k, v = (torch.randn(1, tokens, heads, 128, generator=gen, device="cuda").bfloat16() for _ in range(3))
+    gate = -0.5 * torch.rand(1, tokens, heads, 128, generator=gen, device="cuda")
+    gate = gate.unflatten(1, (-1, 64)).cumsum(2).flatten(1, 2)
+    beta = torch.full((1, tokens, heads), 0.5, device="cuda")
+    saved = torch.ops.kda_b200.kda_chunk_fwd_saved(q, k, v, gate, beta, None, None, None, False)[4]
+    n = tokens * heads * 128
+    qg = saved[:8 * n].view(torch.bfloat16)[3 * n:].view(q.shape)
+    scale = float(torch.tensor(128.0, dtype=torch.float64).rsqrt().float())
+    assert torch.equal(qg, (q.float() * torch.exp2(gate) * scale).bfloat16())
