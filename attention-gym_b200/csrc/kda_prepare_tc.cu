@@ -78,16 +78,16 @@ constexpr int K = 49152;                   // k, then beta k 2^G in place
 constexpr int KN = 65536;                  // column operands Kn_0 .. Kn_3; once multiplied:
 constexpr int AQK = KN;                    //   Aqk tile
 constexpr int LF = KN + 8192;              //   L blocks (fp32)
-constexpr int AD = LF + 12800;             //   diagonal blocks of A (fp32)
+constexpr int BF = LF + 12800;             //   the blocks A[r][r] L[r][m] (fp32)
 constexpr int AT = KN + 32768;             //   A as a bf16 operand tile
 constexpr int W = KN, U = KN + 16384;      //   after the last product: staging of w, u
-constexpr int TAB = KN + 40960;            // per-channel tables of phase 1; then the blocks A[r][r] L[r][m]
-constexpr int BF = TAB;
-constexpr int BETA = TAB + 7680, MISC = BETA + 512, OFFS = MISC + 128;      // beta: one copy per item parity
-constexpr int kOffCache = 112;             // cu_seqlens / chunk_offsets entries kept in shared memory
+constexpr int TAB = KN + 40960;            // per-channel tables of phase 1; then the diagonal blocks of A (fp32)
+constexpr int AD = TAB;
+constexpr int BETA = TAB + 5632, MISC = BETA + 512, OFFS = MISC + 128;      // beta: one copy per item parity
+constexpr int kOffCache = 368;             // cu_seqlens / chunk_offsets entries kept in shared memory
 constexpr int TOTAL = OFFS + 2 * 4 * kOffCache;
 constexpr int BP = 20, BLK = 16 * BP;      // pitch and size of a 16 x 16 fp32 block (floats)
-static_assert(AD + 4 * 4 * BLK <= AT && 6 * 4 * BLK <= BETA - BF && TOTAL <= 115712, "two CTAs per SM");
+static_assert(BF + 6 * 4 * BLK <= AT && 4 * 4 * BLK <= BETA - AD && TOTAL <= 115712, "two CTAs per SM");
 }  // namespace pl
 namespace pt {  // tensor-memory columns
 constexpr int kCols = 256;

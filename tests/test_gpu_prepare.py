@@ -41,7 +41,7 @@ def test_lengths_around_row_blocks_and_chunks(normalize):
     _check(orc.make_inputs(1, sum(EDGES), 2, 128, 128, seed=41, with_state=True, lengths=EDGES), normalize)
 
 
-@pytest.mark.parametrize("sequences", [111, 112, 113])
+@pytest.mark.parametrize("sequences", [111, 112, 113, 366, 367, 368])
 def test_sequence_counts_around_the_offset_cache(sequences):
     lengths = [1 + (7 * i) % 23 for i in range(sequences)]
     lengths[sequences // 2] = 0
