@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
   constexpr int NE = TT * KP / NT;                 // operand elements per thread, array and tile
   constexpr int NV = (TT * CT + NT - 1) / NT;      // value and output elements per thread and tile
   constexpr int NR = KR / 4;
-  constexpr bool kPrefetch = VC == 1 && KR <= 16;
+  constexpr bool kPrefetch = VC == 1 && KR <= 16 && NP > 0;
   static_assert(TT * KP % NT == 0 && TT <= 32, "tile split");
   __shared__ __align__(16) float s_q[2][TT][KP], s_k[2][TT][KP], s_d[2][TT][KP];
   __shared__ float s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
@@ -302,6 +302,105 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Token scan of a few tokens: bound by the state traffic and by the length of the prologue, so nothing is
+// fetched ahead.  A CTA owns 32 state columns in registers: warp w holds the key rows w, w + 8, .., a lane one
+// column, so that every row access is one 128-byte line whatever V is.  The two K-reductions cross the
+// warps through shared memory, one CTA barrier before and one after.
+// ------------------------------------------------------------------------------------------------
+template <int KR>
+__global__ void __launch_bounds__(256) kda_short_scan_kernel(const ScanParams p) {
+  constexpr int NW = 8;
+  __shared__ float s_q[2][8 * KR], s_k[2][8 * KR], s_d[2][8 * KR];
+  __shared__ float s_red[2][2][NW][32], s_qk[2][NW], s_beta[2];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int K = p.K, V = p.V, H = p.H, vtiles = (V + 31) / 32;
+  const int vt = blockIdx.x % vtiles, sh = blockIdx.x / vtiles;
+  const int head = sh % H, seq = sh / H, c = 32 * vt + lane;
+  int64_t bos, eos;
+  if (p.cu_seqlens) { bos = p.cu_seqlens[seq]; eos = p.cu_seqlens[seq + 1]; }
+  else { bos = (int64_t)seq * p.T; eos = bos + p.T; }
+  const bool paged = p.state_indices != nullptr;
+  const int64_t slot = paged ? p.state_indices[seq] : seq;
+  if (paged && (slot <= 0 || slot >= p.num_slots)) {   // padding: zero output, the pool untouched
+    if (warp == 0 && c < V)
+      for (int64_t t = bos; t < eos; ++t) store_from_float(p.out, p.dt_out, (t * H + head) * V + c, 0.f);
+    return;
+  }
+  const float* sin = p.h0 ? p.h0 + (paged ? slot * p.slot_stride : slot * H * K * V) + (int64_t)head * K * V : nullptr;
+  float* sout = paged ? const_cast<float*>(sin) : (p.ht ? p.ht + (slot * H + head) * K * V : nullptr);
+
+  float S[KR];
+#pragma unroll
+  for (int i = 0; i < KR; ++i) {
+    const int r = i * NW + warp;
+    S[i] = (sin && r < K && c < V) ? sin[(int64_t)r * V + c] : 0.f;
+  }
+  auto stage = [&](int64_t t, int b) {      // a token's operands: q scaled, k, 2^g, beta
+    const int64_t base = (t * H + head) * K;
+    for (int r = tid; r < K; r += 256) {
+      s_q[b][r] = load_as_float(p.q, p.dt_q, base + r) * p.scale;
+      s_k[b][r] = load_as_float(p.k, p.dt_k, base + r);
+      s_d[b][r] = exp2f(load_as_float(p.g, p.dt_g, base + r));
+    }
+    if (tid == 0) s_beta[b] = load_as_float(p.beta, p.dt_beta, t * H + head);
+  };
+  if (bos < eos) stage(bos, 0);
+  for (int64_t t = bos; t < eos; ++t) {
+    const int b = (int)((t - bos) & 1);
+    const float v = c < V ? load_as_float(p.v, p.dt_v, (t * H + head) * V + c) : 0.f;
+    __syncthreads();                        // the token is staged; the step before has been read
+    float pk = 0.f, pq = 0.f, pqk = 0.f;
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+      const int r = i * NW + warp;
+      if (r < K) {
+        S[i] *= s_d[b][r];
+        pqk = fmaf(s_q[b][r], s_k[b][r], pqk);
+        pk = fmaf(s_k[b][r], S[i], pk);
+        pq = fmaf(s_q[b][r], S[i], pq);
+      }
+    }
+    s_red[b][0][warp][lane] = pk;
+    s_red[b][1][warp][lane] = pq;
+    if (lane == 0) s_qk[b][warp] = pqk;
+    if (t + 1 < eos) stage(t + 1, b ^ 1);   // overlaps the exchange
+    __syncthreads();
+    float qk = 0.f, a = 0.f, o = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      qk += s_qk[b][w];
+      a += s_red[b][0][w][lane];
+      o += s_red[b][1][w][lane];
+    }
+    const float delta = s_beta[b] * (v - a);
+    if (warp == 0 && c < V) store_from_float(p.out, p.dt_out, (t * H + head) * V + c, fmaf(qk, delta, o));
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+      const int r = i * NW + warp;
+      if (r < K) S[i] = fmaf(s_k[b][r], delta, S[i]);
+    }
+  }
+  if (sout && c < V) {
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+      const int r = i * NW + warp;
+      if (r < K) sout[(int64_t)r * V + c] = S[i];
+    }
+  }
+}
+
+template <int KR>
+static int launch_short_scan(const ScanParams& p, cudaStream_t stream) {
+  const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + 31) / 32);
+  if (blocks <= 0) return KDA_OK;
+  if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
+  StageScope timing(kStageRecurrent, stream);
+  kda_short_scan_kernel<KR><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
 static int device_sms() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
@@ -323,18 +422,47 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
-// Columns per lane: one (16 columns per CTA, the shortest chain from token to token) while those CTAs take
-// at most two turns on the SMs, else four (128 columns per CTA, 16-byte state accesses).  K = V = 128, us for
-// one / four columns per lane: 32 chains 13.8 / 12.7 at 2 tokens, 28 / 33 at 32, 128 / 187 at 256;
-// 64 chains 19.5 / 13.3, 46 / 34, 249 / 188; 256 chains 48 / 14, 141 / 50, 961 / 325.
+// Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length.
+// Figures in us, both sides of each line.
+// * wide: four columns per lane, 128 per CTA, 16-byte state accesses, once the slices take more than two turns on the
+//   SMs; one column per lane (16 per CTA, operands brought by warps of their own: the shortest chain from token to
+//   token) below.  K = V = 128, one / four columns per lane: 64 chains (512 slices) 17.3 / 10.8 at 2 tokens, 46 / 34 at
+//   32; 32 chains 28 / 33 at 32, 128 / 187 at 256.  For 3 to 6 tokens from one turn on: 32 chains (256 slices) 13.3 / 11.1
+//   at 4; K = 128, V = 64, 48 chains 13.5 / 12.3 at 6, 16 chains (64 slices) 9.0 / 10.4.
+// * many: state rows that are not 16-byte aligned, more than two turns: one column per lane, but 32 per CTA and two CTAs
+//   per SM.  K = 128, V = 130, 16 / 32 columns: 48 chains (432 slices) 15.8 / 10.1 at 3 tokens, 56 / 44 at 64; 2048 chains
+//   414 / 157 at 3, 2305 / 1262 at 64.
+// * the short scan for one token, and for two where the form above loses to it.  K = 128, V = 64, short / else: 48 chains
+//   (192 slices) 9.0 / 11.3 at 1 token, 10.1 / 11.7 at 2; 16 chains 11.8 / 10.4 at 2.  V = 130, 2048 chains 117 / 130 at 1,
+//   184 / 142 at 2.  K = 256, V = 128: 128 chains 14.7 / 21.3 at 1, 19.2 / 23.2 at 2; 16 chains (128 slices) 11.2 / 9.1 at 2.
 static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s) {
   const int sms = device_sms();
+  const int64_t slices = (int64_t)p.nseq * p.H * ((p.V + 15) / 16);
+  const int64_t tokens = p.cu_seqlens && p.nseq > 0 ? p.T / p.nseq : p.T;      // per sequence, on average
   const bool aligned = (((uintptr_t)p.h0 | (uintptr_t)p.ht) & 15) == 0 && p.V % 4 == 0 && p.slot_stride % 4 == 0;
-  const bool wide = aligned && (int64_t)p.nseq * p.H * ((p.V + 15) / 16) > 2 * sms;
-  if (p.K <= 32) return wide ? launch_scan<4, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<4, 1, 4, 4, 1>(p, cumulative, s);
-  if (p.K <= 64) return wide ? launch_scan<8, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<8, 1, 4, 4, 1>(p, cumulative, s);
-  if (p.K <= 128) return wide ? launch_scan<16, 4, 8, 0, 2>(p, cumulative, s) : launch_scan<16, 1, 4, 4, 1>(p, cumulative, s);
-  return launch_scan<32, 1, 4, 4, 2>(p, cumulative, s);
+  const bool wide = aligned && p.K <= 128 && slices > (tokens >= 3 && tokens <= 6 ? sms : 2 * sms);
+  const bool many = !aligned && p.K <= 128 && slices > 2 * sms;
+  const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || p.K <= 32 || slices <= sms ? 1 : 2);
+  if (!wide && !cumulative && tokens <= few) {
+    if (p.K <= 32) return launch_short_scan<4>(p, s);
+    if (p.K <= 64) return launch_short_scan<8>(p, s);
+    if (p.K <= 128) return launch_short_scan<16>(p, s);
+    return launch_short_scan<32>(p, s);
+  }
+  if (p.K > 128) return launch_scan<32, 1, 4, 4, 2>(p, cumulative, s);
+  if (wide) {
+    if (p.K <= 32) return launch_scan<4, 4, 8, 0, 2>(p, cumulative, s);
+    if (p.K <= 64) return launch_scan<8, 4, 8, 0, 2>(p, cumulative, s);
+    return launch_scan<16, 4, 8, 0, 2>(p, cumulative, s);
+  }
+  if (many) {
+    if (p.K <= 32) return launch_scan<4, 1, 8, 0, 2>(p, cumulative, s);
+    if (p.K <= 64) return launch_scan<8, 1, 8, 0, 2>(p, cumulative, s);
+    return launch_scan<16, 1, 8, 0, 2>(p, cumulative, s);
+  }
+  if (p.K <= 32) return launch_scan<4, 1, 4, 4, 1>(p, cumulative, s);
+  if (p.K <= 64) return launch_scan<8, 1, 4, 4, 1>(p, cumulative, s);
+  return launch_scan<16, 1, 4, 4, 1>(p, cumulative, s);
 }
 
 // ------------------------------------------------------------------------------------------------
