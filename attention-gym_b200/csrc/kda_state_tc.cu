@@ -39,7 +39,6 @@ struct StateTcParams {
   int nseq, H;
   int64_t tokens;            // rows of the packed buffers
   int use_u, use_o;
-  int ranked;                // the chains are walked in the order of their lengths
   long long* prof;      // debugging aid: phase timestamps of chunk 10 of the first 64 CTAs (rows 32..63)
 };
 
@@ -94,28 +93,48 @@ __device__ __forceinline__ int tile_off(int r, int c, int box_bytes) {
 // Chains of a packed batch in the order of their lengths: a CTA of rank r walks the sequence with the r-th most
 // chunks (ties by index), so that the long chains start first and the last turn on the SMs is made of short
 // ones.  With more chains than SMs and lengths up to 64 to 1 the order of arrival left up to one longest chain of
-// idle SMs at the end: 16 sequences of 40003 tokens, H = 32: 449 -> 376 us forward; 64 of 279046 tokens: 3.21 ->
-// 3.11 ms forward, 2.78 -> 2.70 ms backward.
-// Every CTA ranks the sequences itself (nseq^2 comparisons over its threads, at most 64 per thread); `scratch`
-// takes nseq + 1 ints.
+// idle SMs at the end.  Every CTA ranks the sequences itself: nseq^2 comparisons of one key each, two threads a
+// sequence and four keys a load (at most 64 comparisons per thread).  `scratch` takes kRankedSequences + 1 ints,
+// 16-byte aligned.
 constexpr int kRankedSequences = 128;
-__device__ __forceinline__ int sequence_of_rank(const int32_t* chunk_offsets, int nseq, int rank, int* scratch, int tid) {
-  for (int j = tid; j < nseq; j += kStateThreads) scratch[j] = chunk_offsets[j + 1] - chunk_offsets[j];
-  __syncthreads();
-  for (int j = tid; j < nseq; j += kStateThreads) {
-    const int n = scratch[j];
-    int before = 0;
-    for (int i = 0; i < nseq; ++i) before += scratch[i] > n || (scratch[i] == n && i < j);
-    if (before == rank) scratch[nseq] = j;
+static_assert(2 * kRankedSequences == kStateThreads, "two threads per sequence");
+__device__ __forceinline__ int sequence_of_rank(const int32_t* chunk_offsets, const int32_t* cu_seqlens, int nseq, int rank, int* scratch, int tid) {
+  // one key per sequence, all different: chunks, then the lower index; -1 behind the last sequence
+  if (tid < kRankedSequences) {
+    int key = -1;
+    if (tid < nseq) {
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(cu_seqlens + tid));      // the winner's entry is read next
+      const int chunks = chunk_offsets[tid + 1] - chunk_offsets[tid];
+      key = min(max(chunks, 0), (1 << 24) - 1) * kRankedSequences + (kRankedSequences - 1 - tid);
+    }
+    scratch[tid] = key;
   }
   __syncthreads();
-  return scratch[nseq];
+  const int j = tid >> 1, mine = scratch[j];
+  int before = 0;
+#pragma unroll 4
+  for (int i = 0; i < kRankedSequences / 8; ++i) {
+    const int4 other = reinterpret_cast<const int4*>(scratch)[2 * i + (tid & 1)];
+    before += (other.x > mine) + (other.y > mine) + (other.z > mine) + (other.w > mine);
+  }
+  before += __shfl_xor_sync(0xffffffffu, before, 1);
+  if (j < nseq && before == rank) scratch[kRankedSequences] = j;
+  __syncthreads();
+  return scratch[kRankedSequences];
 }
-// worth it only when the chains take turns on the SMs
-static bool rank_by_length(int nseq, int64_t ctas) {
+// Worth it only where the chains take turns on the SMs and a turn is long beside the ranking, which takes each
+// CTA about 1 us and a little more with the number of sequences: from 4 + nseq / 8 chunks a sequence on.  H = 32, us of
+// the forward walk in the order of arrival / ranked, lengths up to 64 to 1: 16 sequences of 256 tokens on average
+// 69.4 / 70.6, of 500 112 / 105, of 1000 211 / 193, of 2500 513 / 457; 64 of 500 376 / 386, of 1000 724 / 720, of 2500 1794 /
+// 1751; 128 of 1000 1421 / 1427.  Equal rows gain nothing and lose 0.5 to 3 %: a batch whose token and chunk counts are
+// those of equal rows is taken as one.  (The kernels are compiled without the ranking too: with it as a branch the
+// walks of one or two chunks were 2 to 3 % slower in either order.)
+static bool rank_by_length(int nseq, int64_t ctas, int64_t tokens, int chunks) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return nseq > 1 && nseq <= kRankedSequences && ctas > sms;
+  if (nseq < 2 || nseq > kRankedSequences || ctas <= sms) return false;
+  if (tokens % nseq == 0 && chunks == nseq * ((tokens / nseq + 63) / 64)) return false;
+  return tokens >= 64 * (int64_t)nseq * (4 + nseq / 8);
 }
 
 // NS = number of CTAs that share one (sequence, head) chain; each owns N = 128 / NS value columns of
@@ -127,7 +146,7 @@ static bool rank_by_length(int nseq, int64_t ctas) {
 // reports how many chunks that took (limit_out): past them an entering state cannot change any
 // output or state bit that fp32 can hold, so the corrective pass with the true entering state
 // (limit_in) only needs those leading chunks.  This is measured on the data, never assumed.
-template <int NS>
+template <int NS, bool RANKED>
 __global__ void __launch_bounds__(kStateThreads) kda_state_fwd_tc_kernel(const __grid_constant__ StateTcParams p) {
   constexpr int N = D / NS;            // state columns of this CTA
   constexpr int NC = N / 2;            // columns per thread (two warps share a lane quadrant)
@@ -153,8 +172,8 @@ __global__ void __launch_bounds__(kStateThreads) kda_state_fwd_tc_kernel(const _
   if (trans) item -= chains;
   const int head = item % H;
   int seq = item / H;
-  if (p.ranked) {
-    seq = sequence_of_rank(p.chunk_offsets, p.nseq, seq, reinterpret_cast<int*>(smem + StateTcLayout::BAR + 128), tid);
+  if constexpr (RANKED) {
+    seq = sequence_of_rank(p.chunk_offsets, p.cu_seqlens, p.nseq, seq, reinterpret_cast<int*>(smem + StateTcLayout::BAR + 128), tid);
     item = seq * H + head;
   }
   const int v0 = slice * N;                        // first value column of the slice
@@ -457,14 +476,14 @@ __global__ void __launch_bounds__(kStateThreads) kda_state_fwd_tc_kernel(const _
 
 static __device__ int g_state_tc_error = 0;
 
-template <int NS>
+template <int NS, bool RANKED = false>
 static int launch_state_fwd_split(const StateTcParams& p, int64_t ctas, cudaStream_t s) {
   const int smem = StateTcLayout::TOTAL + 1024;
-  if (cudaFuncSetAttribute(kda_state_fwd_tc_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+  if (cudaFuncSetAttribute(kda_state_fwd_tc_kernel<NS, RANKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return KDA_ERR_LAUNCH;
   StageScope timing(kStageStateFwd, s);
-  kda_state_fwd_tc_kernel<NS><<<(unsigned)(ctas * NS), kStateThreads, smem, s>>>(p);
+  kda_state_fwd_tc_kernel<NS, RANKED><<<(unsigned)(ctas * NS), kStateThreads, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
@@ -500,11 +519,11 @@ int launch_state_fwd_tc(const bf16* w, const bf16* u, const bf16* kg, const bf16
   p.use_u = u != nullptr; p.use_o = o != nullptr;
   p.prof = debug_profile_buffer();
   const int64_t ctas = (int64_t)nseq * H * (trans_out ? 2 : 1);
-  p.ranked = !trans_out && rank_by_length(nseq, ctas);
+  const bool ranked = !trans_out && rank_by_length(nseq, ctas, tokens, chunks);
   switch (pick_value_split(ctas)) {
     case 4: return launch_state_fwd_split<4>(p, ctas, s);
     case 2: return launch_state_fwd_split<2>(p, ctas, s);
-    default: return launch_state_fwd_split<1>(p, ctas, s);
+    default: return ranked ? launch_state_fwd_split<1, true>(p, ctas, s) : launch_state_fwd_split<1>(p, ctas, s);
   }
 }
 
@@ -525,7 +544,6 @@ struct StateBwdTcParams {
   int* error;
   int nseq, H;
   int64_t tokens;            // rows of the packed buffers
-  int ranked;                // the chains are walked in the order of their lengths
 };
 
 constexpr int kBStageBytes = 4 * 16384 + 8192;   // KG, W, QG, DO, AQK
@@ -538,7 +556,7 @@ struct StateBwdLayout {
 };
 
 // NS CTAs share a chain, each owning N = 128 / NS value columns of dh, dO and dv2 (see the forward kernel).
-template <int NS>
+template <int NS, bool RANKED>
 __global__ void __launch_bounds__(kStateThreads) kda_state_bwd_tc_kernel(const __grid_constant__ StateBwdTcParams p) {
   constexpr int N = D / NS;
   constexpr int NC = N / 2;
@@ -558,9 +576,9 @@ __global__ void __launch_bounds__(kStateThreads) kda_state_bwd_tc_kernel(const _
   const int H = p.H;
   const int item = blockIdx.x / NS, slice = blockIdx.x % NS;
   const int head = item % H;
-  const int seq = p.ranked ? sequence_of_rank(p.chunk_offsets, p.nseq, item / H,
-                                              reinterpret_cast<int*>(smem + StateBwdLayout::BAR + 128), tid)
-                           : item / H;
+  int seq = item / H;
+  if constexpr (RANKED)
+    seq = sequence_of_rank(p.chunk_offsets, p.cu_seqlens, p.nseq, seq, reinterpret_cast<int*>(smem + StateBwdLayout::BAR + 128), tid);
   const int v0 = slice * N, col0 = sub * NC;
   const int dcol0 = N < 64 ? (v0 & 63) : 0;        // where the slice starts inside the loaded dO box
   const int64_t bos = p.cu_seqlens[seq], eos = p.cu_seqlens[seq + 1];
@@ -770,14 +788,14 @@ __global__ void __launch_bounds__(kStateThreads) kda_state_bwd_tc_kernel(const _
   if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
-template <int NS>
+template <int NS, bool RANKED = false>
 static int launch_state_bwd_split(const StateBwdTcParams& p, int64_t chains, cudaStream_t s) {
   const int smem = StateBwdLayout::TOTAL + 1024;
-  if (cudaFuncSetAttribute(kda_state_bwd_tc_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+  if (cudaFuncSetAttribute(kda_state_bwd_tc_kernel<NS, RANKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
       cudaSuccess)
     return KDA_ERR_LAUNCH;
   StageScope timing(kStageStateBwd, s);
-  kda_state_bwd_tc_kernel<NS><<<(unsigned)(chains * NS), kStateThreads, smem, s>>>(p);
+  kda_state_bwd_tc_kernel<NS, RANKED><<<(unsigned)(chains * NS), kStateThreads, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
@@ -800,11 +818,11 @@ int launch_state_bwd_tc(const bf16* w, const bf16* kg, const bf16* qg, const bf1
   if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p.error), g_state_tc_error) != cudaSuccess)
     return KDA_ERR_LAUNCH;
   const int64_t chains = (int64_t)nseq * H;
-  p.ranked = rank_by_length(nseq, chains);
+  const bool ranked = rank_by_length(nseq, chains, tokens, chunks);
   switch (pick_value_split(chains)) {
     case 4: return launch_state_bwd_split<4>(p, chains, s);
     case 2: return launch_state_bwd_split<2>(p, chains, s);
-    default: return launch_state_bwd_split<1>(p, chains, s);
+    default: return ranked ? launch_state_bwd_split<1, true>(p, chains, s) : launch_state_bwd_split<1>(p, chains, s);
   }
 }
 

@@ -81,3 +81,39 @@ def test_kept_forward_of_a_long_row_and_its_gradients(normalize):
         _cabi.lib().kda_set_row_segments(0)
     for x, y in zip(split, serial):
         assert_normalised(x.float(), y.float(), 1e-4, "segments")
+
+
+@pytest.mark.parametrize("sequences,heads", [(2, 80), (5, 31), (17, 9), (128, 2)])
+def test_long_chains_first_does_not_touch_the_results(sequences, heads):
+    """Sequences long enough (4 + sequences / 8 chunks on average) for more chains than SMs to be ranked, with an empty
+    one, a tie and the longest last."""
+    mean = 64 * (4 + sequences // 8) + 40
+    lengths = [1 + (37 * i * i + 11 * i) % (2 * mean) for i in range(sequences)]
+    if sequences > 2:
+        lengths[1], lengths[2] = 0, max(lengths)
+    lengths[-1] = max(lengths) + (0 if sequences > 5 else mean)
+    lengths[0] += max(0, mean * sequences - sum(lengths))
+    gen = torch.Generator(device="cuda").manual_seed(65)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    tokens = sum(lengths)
+    q, k = (torch.nn.functional.normalize(r(1, tokens, heads, 128), dim=-1).bfloat16() for _ in range(2))
+    v, do = r(1, tokens, heads, 128).bfloat16(), r(1, tokens, heads, 128).bfloat16()
+    gate, beta, h0 = -0.02 * torch.rand(1, tokens, heads, 128, generator=gen, device="cuda"), r(1, tokens, heads).sigmoid(), 0.02 * r(sequences, heads, 128, 128)
+    marks = [0]
+    for n in lengths:
+        marks.append(marks[-1] + n)
+
+    def run(args, cot, cu):
+        leaves = [x.detach().contiguous().requires_grad_() for x in args]
+        o, st = kda_b200.chunk_kda(*leaves, cu_seqlens=torch.tensor(cu, dtype=torch.int32, device="cuda"), output_final_state=True)
+        return [o, st, *torch.autograd.grad([o, st], leaves, [cot, 0.1 * torch.ones_like(st)])]
+
+    args = (q, k, v, gate, beta, h0)
+    whole = run(args, do, marks)
+    for i in sorted({0, 2 % sequences, sequences // 2, sequences - 1}):
+        a, b = marks[i], marks[i + 1]
+        if a == b:
+            continue
+        alone = run([x[:, a:b] for x in args[:5]] + [h0[i:i + 1]], do[:, a:b].contiguous(), [0, b - a])
+        for n, (x, y) in enumerate(zip(whole, alone)):
+            assert torch.equal(x[i:i + 1] if n in (1, 7) else x[:, a:b], y), (i, n)
