@@ -813,11 +813,10 @@ extern "C" int kda_decode_step(const void* x, const void* conv_weight, void* con
   p.nseq = nseq; p.T = 1; p.H = heads; p.K = p.V = 128;
   p.scale = 0.08838834764831845f;  // 128^-0.5
   // The state update overlaps the preprocessing while that is a fraction of a wave; at several waves the early
-  // state loads only slow its last ones down.  H = 32: 37 sequences (222 blocks) 36 us a step overlapped; 256
-  // sequences (1536 blocks) 212.8 overlapped, 208.4 one after the other.
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool overlap = (int64_t)nseq * ((3 * heads * 16 + 255) / 256) <= 2 * sms;
+  // state loads only slow its last ones down.  us per step of a captured graph, overlapped / one after the other, H = 32:
+  // 8.9 / 9.4 at 1 sequence, 21.3 / 22.0 at 24, 40.0 / 40.4 at 49 (294 blocks), 48.2 / 48.1 at 56, 54.2 / 55.3 at 64, 68.4 / 66.7 at
+  // 80, 206.9 / 204.4 at 256; H = 8: 24.2 / 25.0 at 128 (256 blocks), 31.0 / 31.0 at 160, 39.4 / 39.0 at 192.
+  const bool overlap = (int64_t)nseq * ((3 * heads * 16 + 255) / 256) <= 2 * device_sms();
   return launch_recurrent(p, overlap, (cudaStream_t)stream);
 }
 

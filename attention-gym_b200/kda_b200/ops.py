@@ -112,7 +112,8 @@ _define("kda_decode_prep",
         "-> (Tensor, Tensor, Tensor, Tensor)")
 
 
-# Operators of this package's own making, in a namespace of their own: the one above holds the reference's.
+# Operators behind one public call each, without a counterpart among the reference's; in a namespace of their own, so
+# that the list of kda_b200 operators stays what its users bind to.
 _NS_OWN = "kda_b200_fused"
 _lib_own = torch.library.Library(_NS_OWN, "DEF")
 
