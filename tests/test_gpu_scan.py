@@ -73,6 +73,10 @@ def test_every_form_of_the_scan(kd, vd, heads, lengths, paged):
     args = (dev["q"], dev["k"], dev["v"], dev["gate_log2"], dev["beta"])
     n = len(lengths)
     if not paged:
+        o, s = kda_b200.chunk_kda(*args[:3], dev["cum_gate"], dev["beta"], dev["h0"], cu_seqlens=dev["cu_seqlens"],
+                                  output_final_state=True, exact_fp32=True)        # the same from the cumulative gate
+        _close(o, want_o, "output (cumulative gate)")
+        _close(s, want_s, "state (cumulative gate)")
         o, s = kda_b200.recurrent_kda(*args, dev["h0"], cu_seqlens=dev["cu_seqlens"], output_final_state=True)
     else:                                       # slots in reverse order behind an unused one; the last sequence is padding
         slots = torch.arange(n, 0, -1, dtype=torch.int32)
