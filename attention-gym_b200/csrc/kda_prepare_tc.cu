@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
     // B[r][m] = A[r][r] L[r][m] for the six blocks below the diagonal, one warp each and a 2 x 4 tile per lane.
     // With them every block of the inverse is ONE product, A[r][c] = -sum_{c <= m < r} B[r][m] A[m][c], so the
     // blocks at distance 1, 2, 3 from the diagonal cost one barrier each.  (The same products on the tensor cores,
-    // operands split in two tf32 halves: 0.596 instead of 0.622 ms, but 22 instead of 24 operand bits, which is three
+    // operands split in two tf32 halves: 0.596 instead of 0.622 ms, but 22 instead of 24 operand bits, which is 1.6
     // times the rounding error of the inverse, and a split loses NaN.)
     if (warp < 6) {
       const int r = warp < 1 ? 1 : (warp < 3 ? 2 : 3), m = warp < 1 ? 0 : (warp < 3 ? warp - 1 : warp - 3);
