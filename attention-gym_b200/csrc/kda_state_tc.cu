@@ -123,18 +123,19 @@ __device__ __forceinline__ int sequence_of_rank(const int32_t* chunk_offsets, co
   return scratch[kRankedSequences];
 }
 // Worth it only where the chains take turns on the SMs and a turn is long beside the ranking, which takes each
-// CTA about 1 us and a little more with the number of sequences: from 4 + nseq / 8 chunks a sequence on.  H = 32, us of
-// the forward walk in the order of arrival / ranked, lengths up to 64 to 1: 16 sequences of 256 tokens on average
-// 69.4 / 70.6, of 500 112 / 105, of 1000 211 / 193, of 2500 513 / 457; 64 of 500 376 / 386, of 1000 724 / 720, of 2500 1794 /
-// 1751; 128 of 1000 1421 / 1427.  Equal rows gain nothing and lose 0.5 to 3 %: a batch whose token and chunk counts are
-// those of equal rows is taken as one.  (The kernels are compiled without the ranking too: with it as a branch the
+// CTA about 1 us and a little more with the number of sequences: from 4 + nseq / 8 chunks a sequence on, with at most
+// three turns, where the last one weighs most, from 224 tokens on.  H = 32, us of the forward walk in the order of
+// arrival / ranked, lengths up to 64 to 1: 10 sequences of 150 tokens on average 33.2 / 33.3, of 256 47.5 / 42.5, of 300
+// 57.3 / 47.6; 16 of 256 63.9 / 65.9, of 500 112 / 105, of 1000 211 / 193, of 2500 513 / 457; 64 of 500 376 / 386, of 1000 724 /
+// 720, of 2500 1794 / 1751; 128 of 1000 1421 / 1427.  Equal rows gain nothing and lose 0.5 to 3 %: a batch whose token and
+// chunk counts are those of equal rows is taken as one.  (The kernels are compiled without the ranking too: with it as a branch the
 // walks of one or two chunks were 2 to 3 % slower in either order.)
 static bool rank_by_length(int nseq, int64_t ctas, int64_t tokens, int chunks) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (nseq < 2 || nseq > kRankedSequences || ctas <= sms) return false;
   if (tokens % nseq == 0 && chunks == nseq * ((tokens / nseq + 63) / 64)) return false;
-  return tokens >= 64 * (int64_t)nseq * (4 + nseq / 8);
+  return tokens >= (int64_t)nseq * (ctas <= 3 * sms ? 224 : 64 * (4 + nseq / 8));
 }
 
 // NS = number of CTAs that share one (sequence, head) chain; each owns N = 128 / NS value columns of
