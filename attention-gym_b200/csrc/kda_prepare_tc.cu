@@ -26,7 +26,7 @@
 // comes from the lifetimes: the gates move to registers and their tile becomes the Qr / Kr operand, v is
 // fetched into the q tile when q is spent, and the solve, its operand tile and the result staging share
 // the column-operand tiles.
-// B = 8, T = 4096, H = 32: 0.622 ms = 4.3 TB/s of its 2564 B per unit, against 0.848 ms with one CTA of 512
+// B = 8, T = 4096, H = 32: 0.602 ms = 4.5 TB/s of its 2564 B per unit, against 0.848 ms with one CTA of 512
 // threads per SM and 230 KiB; one sequence of 1000 tokens, H = 32: 34 against 43 us.  (Two CTAs of 512
 // threads with 64 registers: 0.75 ms, 30 % more instructions and more waiting at barriers.)  Issue slots and the
 // shared-memory port are each half busy; the rest is the latency of the chain at four warps per scheduler.
@@ -78,7 +78,7 @@ constexpr int K = 49152;                   // k, then beta k 2^G in place
 constexpr int KN = 65536;                  // column operands Kn_0 .. Kn_3; once multiplied:
 constexpr int AQK = KN;                    //   Aqk tile
 constexpr int LF = KN + 8192;              //   L blocks (fp32)
-constexpr int BF = LF + 12800;             //   the blocks A[r][r] L[r][m] (fp32)
+constexpr int XT = LF + 12800;             //   columns of A by block column, inner index contiguous (fp32)
 constexpr int AT = KN + 32768;             //   A as a bf16 operand tile
 constexpr int W = KN, U = KN + 16384;      //   after the last product: staging of w, u
 constexpr int TAB = KN + 40960;            // per-channel tables of phase 1; then the diagonal blocks of A (fp32)
@@ -87,7 +87,8 @@ constexpr int BETA = TAB + 5632, MISC = BETA + 512, OFFS = MISC + 128;      // b
 constexpr int kOffCache = 368;             // cu_seqlens / chunk_offsets entries kept in shared memory
 constexpr int TOTAL = OFFS + 2 * 4 * kOffCache;
 constexpr int BP = 20, BLK = 16 * BP;      // pitch and size of a 16 x 16 fp32 block (floats)
-static_assert(BF + 6 * 4 * BLK <= AT && 4 * 4 * BLK <= BETA - AD && TOTAL <= 115712, "two CTAs per SM");
+constexpr int TT = XT + 4 * 16 * (52 + 36 + 20);        //   columns of the right-hand sides, 48 x 20 floats
+static_assert(TT + 4 * 48 * 20 <= AT && 4 * 4 * BLK <= BETA - AD && TOTAL <= 115712, "two CTAs per SM");
 }  // namespace pl
 namespace pt {  // tensor-memory columns
 constexpr int kCols = 256;
@@ -145,6 +146,74 @@ __device__ __forceinline__ f32x2 unpack_pair(uint32_t u) {
   return pack2(f.x, f.y);
 }
 
+// columns of block column c of A: floats from one to the next, and the byte offset of the first
+__host__ __device__ constexpr int xt_pitch(int c) { return 52 - 16 * c; }
+__host__ __device__ constexpr int xt_off(int c) { return pl::XT + 64 * (c > 0 ? 52 : 0) + 64 * (c > 1 ? 36 : 0); }
+
+// Inner index k of a row or column of the solve lies at position 2 (k mod 8) + k / 8: a 16-byte vector holds two pairs
+// (k, k + 8) for the packed arithmetic, which then sums the two halves of the inner index side by side.
+__host__ __device__ constexpr int inner_pos(int k) { return 2 * (k & 7) + (k >> 3); }
+
+// NC columns per lane of block column C of A = (I + L)^-1, from its diagonal block down: lane (i = lid / 2, lid & 1) holds
+// row i of every block and NC adjacent columns; `part` is the warp's share of the block's columns.
+template <int C, int NC>
+__device__ __forceinline__ void solve_columns(unsigned char* sm, int part, int lid) {
+  const float* Lf = reinterpret_cast<const float*>(sm + pl::LF);
+  const float* Ad = reinterpret_cast<const float*>(sm + pl::AD);
+  const int i = lid >> 1, pos = inner_pos(i), col0 = 2 * NC * part + NC * (lid & 1);
+  float* x = reinterpret_cast<float*>(sm + xt_off(C)) + col0 * xt_pitch(C);     // [column][row - 16 C]
+  float* t = reinterpret_cast<float*>(sm + pl::TT) + (16 * C + col0) * 20;      // [column][row of the block]
+  auto dot = [&](const float* row, const float* cols, int pitch, f32x2 (&d)[NC]) {     // row . column, 16 inner indices, in halves
+    ulonglong2 a[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = *reinterpret_cast<const ulonglong2*>(row + 4 * k);
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      f32x2 s = 0;             // (zero bits: +0, +0)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(cols + j * pitch + 4 * k);
+        s = fma2(a[k].x, b.x, s);
+        s = fma2(a[k].y, b.y, s);
+      }
+      d[j] = s;
+    }
+  };
+  f32x2 acc[4][NC];            // right-hand sides of the block rows below (only r > C are used)
+#pragma unroll
+  for (int m = C; m < 3; ++m) {            // X_m is known: its share of every right-hand side, then X_{m + 1}
+    const float* xm = x + 16 * (m - C);
+    f32x2 d[NC];
+#pragma unroll
+    for (int r = m + 1; r < 4; ++r) {
+      dot(Lf + blk_off(r, m) + i * pl::BP, xm, xt_pitch(C), d);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) acc[r][j] = m == C ? d[j] : add2(acc[r][j], d[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      const float2 h = unpack2(acc[m + 1][j]);
+      t[j * 20 + pos] = h.x + h.y;
+    }
+    __syncwarp();
+    float out[NC];
+    dot(Ad + (m + 1) * pl::BLK + i * pl::BP, t, 20, d);
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      const float2 h = unpack2(d[j]);
+      out[j] = -(h.x + h.y);
+      if (m + 1 < 3) x[j * xt_pitch(C) + 16 * (m + 1 - C) + pos] = out[j];
+    }
+#pragma unroll
+    for (int j = 0; j < NC; j += 2) {
+      const int c = col0 + j;
+      *reinterpret_cast<uint32_t*>(sm + pl::AT + sw128_chunk(16 * (m + 1) + i, 2 * C + (c >> 3)) + 2 * (c & 7)) =
+          pack_bf16(out[j], out[j + 1]);
+    }
+    __syncwarp();              // the column's next 16 rows are complete; the right-hand side has been read
+  }
+}
+
 // NORM: q and k arrive unnormalised; every row is scaled to unit L2 norm (and rounded to bf16, as a
 // separate l2norm launch would leave it) while its pieces pass through the registers of phase 1,
 // and the two reciprocal norms are kept for the backward pass
@@ -167,7 +236,6 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   int* s_next = reinterpret_cast<int*>(sm + pl::MISC + 96);                // next item: token0 (two words), valid
   float* Lf = reinterpret_cast<float*>(sm + pl::LF);
   float* Ad = reinterpret_cast<float*>(sm + pl::AD);
-  float* Bf = reinterpret_cast<float*>(sm + pl::BF);
   // rows: 0..3 R_b, 4..9 2^{R_r - R_b} for (r, b) = (1,0) (2,0) (3,0) (2,1) (3,1) (3,2), 10 G_last
   float* tab = reinterpret_cast<float*>(sm + pl::TAB);
   const unsigned char* sG = sm + pl::G;
@@ -224,9 +292,10 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   int rc = 0, it = 0;
   bool pre = false;              // this item's loads were issued by the previous item
   ChunkWork cw_next{};
+  int head_n = 0;
   for (int wi = blockIdx.x; wi < p.total; wi += gridDim.x) {
-  const int chunk = wi / H, head = wi - chunk * H;
-  const ChunkWork cw = pre ? cw_next : locate_chunk(cu_off, ch_off, p.nseq, chunk);
+  const int head = pre ? head_n : wi % H;
+  const ChunkWork cw = pre ? cw_next : locate_chunk(cu_off, ch_off, p.nseq, wi / H);
   if (cw.valid == 0) continue;               // capacity slot past the last active chunk
   if (!pre && !chunk_in_range(cw, p.tokens)) {     // (with pre the previous item checked it)
     if (tid == 0 && p.error) atomicExch(p.error, kOffsetsOutOfRange);
@@ -244,7 +313,6 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   }
   // the next item is located by one thread while this item's tiles arrive (the search is a chain of
   // dependent loads); everybody reads the result after the barrier that ends the table step
-  int head_n = 0;
   bool next_ok = false;
   if (tid == 160) {
     const int wn = wi + (int)gridDim.x;
@@ -256,6 +324,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
     s_next[0] = (int)(nx.token0 & 0xffffffffLL);
     s_next[1] = (int)(nx.token0 >> 32);
     s_next[2] = nx.valid;
+    s_next[3] = wn % H;
   }
   auto body = [&]() -> int {
   const int tid = fresh_tid();
@@ -288,13 +357,12 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
       t[128 * 7] = fexp2(r2 - r1); t[128 * 8] = fexp2(r3 - r1); t[128 * 9] = fexp2(r3 - r2);
     }
   }
-  if (tid == 0) tma_store_wait_read();       // the w, u staging tiles (over Kn) of the previous item have been read
+  if (tid == 192) tma_store_wait_read();     // the w, u staging tiles (over Kn) of the previous item have been read
   __syncthreads();
   pr_mark(p, it, 2);
   if (*s_abort) return 2;
   {   // the next item; its beta values travel straight to shared memory
-    const int wn = wi + (int)gridDim.x;
-    head_n = wn - (wn / H) * H;
+    head_n = s_next[3];
     cw_next.token0 = (int64_t)(((uint64_t)(uint32_t)s_next[1] << 32) | (uint32_t)s_next[0]);
     cw_next.valid = s_next[2];
     next_ok = cw_next.valid > 0;        // 0 also when there is no further item
@@ -415,7 +483,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
     if (!mbar_wait(&bar[3], ph)) *s_abort = 1;
     tc_fence_after();
     pr_mark(p, it, 4);
-    if (tid == 0 && next_ok) load_gates(head_n, cw_next.token0);       // over the Qr / Kr tile
+    if (tid == 160 && next_ok) load_gates(head_n, cw_next.token0);     // over the Qr / Kr tile
 
   }
   {
@@ -434,10 +502,15 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
           if (quad & 1) {
             const float bt = s_beta[i];
             float4* dst = reinterpret_cast<float4*>(Lf + blk_off(r, c) + lid * pl::BP);
+            if (r == c) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 4)
-              dst[j >> 2] = make_float4(j < below ? a[j] * bt : 0.f, j + 1 < below ? a[j + 1] * bt : 0.f,
-                                        j + 2 < below ? a[j + 2] * bt : 0.f, j + 3 < below ? a[j + 3] * bt : 0.f);
+              for (int j = 0; j < 16; j += 4)
+                dst[j >> 2] = make_float4(j < lid ? a[j] * bt : 0.f, j + 1 < lid ? a[j + 1] * bt : 0.f,
+                                          j + 2 < lid ? a[j + 2] * bt : 0.f, j + 3 < lid ? a[j + 3] * bt : 0.f);
+            } else {               // (every column is in the row's past) the inner order of the solve
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) dst[j >> 1] = make_float4(a[j] * bt, a[j + 8] * bt, a[j + 1] * bt, a[j + 9] * bt);
+            }
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) a[j] = (j <= below && i < valid) ? a[j] * p.scale : 0.f;
@@ -478,9 +551,14 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
 #pragma unroll
         for (int i = j + 4; i < 16; ++i) x[i] = fmaf(-l[i].w, x[j + 3], x[i]);
       }
-      float* dst = Ad + b * pl::BLK + c;
+      float* dst = Ad + b * pl::BLK + inner_pos(c);
 #pragma unroll
       for (int i = 0; i < 16; ++i) dst[i * pl::BP] = x[i];
+      if (b < 3) {
+        float4* col = reinterpret_cast<float4*>(reinterpret_cast<float*>(sm + xt_off(b)) + c * xt_pitch(b));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) col[i] = make_float4(x[2 * i], x[2 * i + 8], x[2 * i + 1], x[2 * i + 9]);
+      }
     } else {         // meanwhile the Aqk tile leaves and v becomes beta v
       for (int idx = tid - 64; idx < valid * 8; idx += NT - 64) {
         const int r = idx >> 3, c = idx & 7;
@@ -507,83 +585,32 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   pr_mark(p, it, 6);
   {
     const int tid = fresh_tid(), warp = tid >> 5, lid = tid & 31;
-    // B[r][m] = A[r][r] L[r][m] for the six blocks below the diagonal, one warp each and a 2 x 4 tile per lane.
-    // With them every block of the inverse is ONE product, A[r][c] = -sum_{c <= m < r} B[r][m] A[m][c], so the
-    // blocks at distance 1, 2, 3 from the diagonal cost one barrier each.  (The same products on the tensor cores,
-    // operands split in two tf32 halves: 0.596 instead of 0.622 ms, but 22 instead of 24 operand bits, which is 1.6
-    // times the rounding error of the inverse, and a split loses NaN.)
-    if (warp < 6) {
-      const int r = warp < 1 ? 1 : (warp < 3 ? 2 : 3), m = warp < 1 ? 0 : (warp < 3 ? warp - 1 : warp - 3);
-      const int i = 2 * (lid >> 2), j = 4 * (lid & 3);
-      const float* a = Ad + r * pl::BLK + i * pl::BP;                // A[r][r], rows i, i + 1
-      const float* l = Lf + blk_off(r, m) + j;                       // L[r][m], columns j .. j + 3
-      f32x2 s0[2] = {0, 0}, s1[2] = {0, 0};                          // (zero bits: +0, +0)
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) {
-        const float4 a0 = *reinterpret_cast<const float4*>(a + k), a1 = *reinterpret_cast<const float4*>(a + pl::BP + k);
-        const float av0[4] = {a0.x, a0.y, a0.z, a0.w}, av1[4] = {a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(l + (k + e) * pl::BP);
-          const f32x2 y0 = pack2(av0[e], av0[e]), y1 = pack2(av1[e], av1[e]);
-          s0[0] = fma2(y0, x.x, s0[0]); s0[1] = fma2(y0, x.y, s0[1]);
-          s1[0] = fma2(y1, x.x, s1[0]); s1[1] = fma2(y1, x.y, s1[1]);
-        }
+    // The blocks below the diagonal, column block by column block and without a CTA barrier: a warp takes its columns
+    // of block column c through the block rows r > c,  T_r = sum_{c <= m < r} L[r][m] X_m,  X_r = -A[r][r] T_r.
+    // Block column 0 is shared by four warps, 1 by two, 2 belongs to one: 9, 5 and 2 products of 16 x 16 by 4, 8 and 16
+    // columns are about the same work.  Columns lie in shared memory with their inner index contiguous, as the rows of
+    // L and A do, so both operands arrive as 16-byte vectors of pairs for the packed arithmetic.  The pairs are (k, k + 8):
+    // measured against 64 bits (gates x 1, .02, .001 and nearly equal keys), the two halves side by side and the products
+    // L[r][m] X_m added block by block have 0.77 to 0.99 of the rounding error of the products by distance; with pairs
+    // (k, k + 1) it was up to 2.4 times that error, because between nearly equal keys neighbouring terms cancel.
+    // (All six A[r][r] L[r][m] first and then the blocks by their distance from the diagonal: four more CTA
+    // barriers; 0.622 ms for the whole kernel.)
+    if (warp < 4) solve_columns<0, 2>(sm, warp, lid);
+    else if (warp < 6) solve_columns<1, 4>(sm, warp - 4, lid);
+    else if (warp == 6) solve_columns<2, 8>(sm, 0, lid);
+    else {        // meanwhile the diagonal blocks, and zeros to their right, go into the operand tile: two rows per lane
+      for (int r = lid; r < 64; r += 32) {
+        const int b = r >> 4;
+        const float4* src = reinterpret_cast<const float4*>(Ad + b * pl::BLK + (r & 15) * pl::BP);
+        const float4 f0 = src[0], f1 = src[1], f2 = src[2], f3 = src[3];        // pairs (k, k + 8)
+        *reinterpret_cast<uint4*>(sm + pl::AT + sw128_chunk(r, 2 * b)) =
+            make_uint4(pack_bf16(f0.x, f0.z), pack_bf16(f1.x, f1.z), pack_bf16(f2.x, f2.z), pack_bf16(f3.x, f3.z));
+        *reinterpret_cast<uint4*>(sm + pl::AT + sw128_chunk(r, 2 * b + 1)) =
+            make_uint4(pack_bf16(f0.y, f0.w), pack_bf16(f1.y, f1.w), pack_bf16(f2.y, f2.w), pack_bf16(f3.y, f3.w));
+        for (int c = 2 * b + 2; c < 8; ++c) *reinterpret_cast<uint4*>(sm + pl::AT + sw128_chunk(r, c)) = make_uint4(0, 0, 0, 0);
       }
-      float* dst = Bf + warp * pl::BLK + i * pl::BP + j;
-      *reinterpret_cast<ulonglong2*>(dst) = make_ulonglong2(s0[0], s0[1]);
-      *reinterpret_cast<ulonglong2*>(dst + pl::BP) = make_ulonglong2(s1[0], s1[1]);
-    } else {      // meanwhile the diagonal blocks, and zeros to their right, go into the operand tile: a row per thread
-      const int r = tid - 192, b = r >> 4;
-      const float4* src = reinterpret_cast<const float4*>(Ad + b * pl::BLK + (r & 15) * pl::BP);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float4 lo = src[2 * h], hi = src[2 * h + 1];
-        *reinterpret_cast<uint4*>(sm + pl::AT + sw128_chunk(r, 2 * b + h)) =
-            make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w), pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
-      }
-      for (int c = 2 * b + 2; c < 8; ++c) *reinterpret_cast<uint4*>(sm + pl::AT + sw128_chunk(r, c)) = make_uint4(0, 0, 0, 0);
     }
   }
-  __syncthreads();
-  pr_mark(p, it, 7);
-  // The blocks at distance DIST from the diagonal, over the L blocks (B holds what is still needed of them) and
-  // straight into the operand tile.  A pair of adjacent lanes owns a 2 x 2 tile of a block and splits the inner
-  // dimension between its lanes in interleaved groups of four; one shuffle per accumulator joins the halves
-  // and each lane then stores one row of the tile.
-  auto blocks_at = [&](auto distance) {
-    constexpr int DIST = decltype(distance)::value;
-    for (int t = fresh_tid(); t < (4 - DIST) * 128; t += NT) {       // whole warps
-      const int ks = t & 1, rest = t >> 1, c = rest >> 6, r = c + DIST, i = 2 * ((rest >> 3) & 7), j = 2 * (rest & 7);
-      const float* b = Bf + (r * (r - 1) / 2 + c) * pl::BLK + i * pl::BP;      // B[r][c ..], rows i, i + 1
-      f32x2 s0 = 0, s1 = 0;
-#pragma unroll
-      for (int m = 0; m < 2 * DIST; ++m) {
-        const int blk = m >> 1, k = 4 * ((ks + 2 * m) & 3);
-        const float4 b0 = *reinterpret_cast<const float4*>(b + blk * pl::BLK + k);
-        const float4 b1 = *reinterpret_cast<const float4*>(b + blk * pl::BLK + pl::BP + k);
-        const float bv0[4] = {b0.x, b0.y, b0.z, b0.w}, bv1[4] = {b1.x, b1.y, b1.z, b1.w};
-        const float* a = (blk == 0 ? Ad + c * pl::BLK : Lf + blk_off(c + blk, c)) + k * pl::BP + j;   // A[c + blk][c], columns j, j + 1
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const f32x2 x = *reinterpret_cast<const f32x2*>(a + e * pl::BP);
-          s0 = fma2(pack2(bv0[e], bv0[e]), x, s0);
-          s1 = fma2(pack2(bv1[e], bv1[e]), x, s1);
-        }
-      }
-      float2 x0 = unpack2(s0), x1 = unpack2(s1);
-      x0.x += __shfl_xor_sync(0xffffffffu, x0.x, 1); x0.y += __shfl_xor_sync(0xffffffffu, x0.y, 1);
-      x1.x += __shfl_xor_sync(0xffffffffu, x1.x, 1); x1.y += __shfl_xor_sync(0xffffffffu, x1.y, 1);
-      const float2 y = ks ? make_float2(-x1.x, -x1.y) : make_float2(-x0.x, -x0.y);
-      if (r < 3) *reinterpret_cast<float2*>(Lf + blk_off(r, c) + (i + ks) * pl::BP + j) = y;
-      *reinterpret_cast<uint32_t*>(sm + pl::AT + sw128_chunk(16 * r + i + ks, 2 * c + (j >> 3)) + 2 * (j & 7)) = pack_bf16(y.x, y.y);
-    }
-  };
-  blocks_at(std::integral_constant<int, 1>{});
-  __syncthreads();
-  blocks_at(std::integral_constant<int, 2>{});
-  __syncthreads();
-  blocks_at(std::integral_constant<int, 3>{});
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -644,7 +671,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   {
     const int tid = fresh_tid();
     if (valid == 64) {
-      if (tid == 0) {
+      if (tid == 192) {
         for (int b = 0; b < 2; ++b) {
           tma_store_2d(&p.tm_w, sm + pl::W + b * 8192, tx + 64 * b, ty);
           tma_store_2d(&p.tm_u, sm + pl::U + b * 8192, tx + 64 * b, ty);
@@ -670,7 +697,7 @@ __global__ void __launch_bounds__(NT, 2) kda_prepare_tc_kernel(const __grid_cons
   ph ^= 1;
   ++it;
   }  // work items
-  if (tid == 0) tma_store_wait_read();      // staged tiles must outlive the bulk stores' reads
+  if (tid == 192) tma_store_wait_read();    // staged tiles must outlive the bulk stores' reads
   if (rc && tid == 0 && p.error) atomicExch(p.error, 32 + rc);
   tc_fence_before();
   __syncthreads();
