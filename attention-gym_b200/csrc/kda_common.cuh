@@ -57,12 +57,6 @@ __device__ __forceinline__ float fexp2(float x) {
   return y;
 }
 
-// Programmatic dependent launch: the first lets a kernel that was launched as this one's dependent start while
-// this one still runs, the second holds such a dependent until every kernel it depends on has finished and
-// its writes are visible (both do nothing between ordinary launches).
-__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Two fp32 values in a 64-bit register pair and the packed arithmetic of sm_100 on them (one issue
 // slot for two IEEE operations; the same results as the scalar forms).  A float4 from memory is two
 // pairs without any move.

@@ -7,24 +7,16 @@
 // l2norm twice (fwd/triton/l2norm_fwd.py:231) and the bounded gate with chunk size 1
 // (fwd/triton/gate_fwd.py:716) -- and names "decode preprocessing and scan are separate launches"
 // as a serving limitation (kda/api.py:210-212).  Here the preprocessing is one kernel and the
-// state update (kda_recurrent_fwd) the second.
+// state update (kda_recurrent_fwd) the second; 16-bit decode steps do both in one launch (kda_stream.cu),
+// with the functions of kda_recurrent.cuh.
 //
 // x and the history are [.., 3 * H * 128] with the q channels first, then k, then v.  Two kernels:
 // the vector kernel further down for 16-bit tensors, and this scalar one (any dtype, W <= 8): one
 // block of 128 threads per (sequence, head), thread c owns channel c of the head's q, k and v blocks.
-#include "kda_common.cuh"
+#include "kda_recurrent.cuh"
 #include "kda_timing.cuh"
 
 namespace kda {
-
-struct PrepDecodeParams {
-  const void* x; const void* w; void* conv_state;          // [N, 3HD], [3HD, W], [slots, W-1, 3HD]
-  const void* raw_gate; const float* A_log; const float* dt_bias;   // [N, H, D], [H], [H, D]
-  void* q; void* k; void* v; float* g;                     // [N, H, D] each (q, k, v in the dtype of x)
-  const int32_t* state_indices;                            // conv pool slots or NULL (slot = sequence)
-  int dt, dt_gate, nseq, H, W, num_slots, act;
-  float lower_bound, eps;
-};
 
 __device__ __forceinline__ float block_sum128(float v, float* scratch, int tid) {
 #pragma unroll
@@ -38,7 +30,6 @@ __device__ __forceinline__ float block_sum128(float v, float* scratch, int tid) 
 
 __global__ void __launch_bounds__(128) kda_decode_prep_kernel(const PrepDecodeParams p) {
   __shared__ float scratch[4];
-  grid_dependency_trigger();
   const int tid = threadIdx.x, head = blockIdx.x % p.H, seq = blockIdx.x / p.H;
   const int HD = p.H * 128, C = 3 * HD, W = p.W;
   const int64_t orow = ((int64_t)seq * p.H + head) * 128 + tid;
@@ -76,8 +67,8 @@ __global__ void __launch_bounds__(128) kda_decode_prep_kernel(const PrepDecodePa
   store_from_float(p.q, p.dt, orow, y[0] * rq);
   store_from_float(p.k, p.dt, orow, y[1] * rk);
   store_from_float(p.v, p.dt, orow, y[2]);
-  const float z = expf(p.A_log[head]) * (load_as_float(p.raw_gate, p.dt_gate, orow) + p.dt_bias[head * 128 + tid]);
-  p.g[orow] = p.lower_bound / (1.f + expf(-z)) * kLog2e;
+  p.g[orow] = decode_gate(expf(p.A_log[head]), load_as_float(p.raw_gate, p.dt_gate, orow), p.dt_bias[head * 128 + tid],
+                          p.lower_bound);
 }
 
 // 16-bit tensors: a thread owns one 16-byte vector of 8 adjacent channels.  Vector v covers channels
@@ -87,7 +78,6 @@ __global__ void __launch_bounds__(128) kda_decode_prep_kernel(const PrepDecodePa
 // eight (head, channel) pairs.
 template <int W>
 __global__ void __launch_bounds__(256) kda_decode_prep_vec_kernel(const PrepDecodeParams p) {
-  grid_dependency_trigger();       // the state update may start fetching states
   const int seq = blockIdx.y, vec = blockIdx.x * 256 + threadIdx.x;
   const int HD = p.H * 128, C = 3 * HD, nvec = C / 8;
   const bool in_range = vec < nvec;
@@ -114,30 +104,14 @@ __global__ void __launch_bounds__(256) kda_decode_prep_vec_kernel(const PrepDeco
     uint4 wraw[W];                                 // 8 W weights = W vectors; element i * W + j
 #pragma unroll
     for (int j = 0; j < W; ++j) wraw[j] = wv[j];
-    const unsigned short* wh = reinterpret_cast<const unsigned short*>(wraw);
-#pragma unroll
-    for (int j = 0; j < W; ++j) {
-      float f[8];
-      raw8_to_float(raw[j], dt, f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = fmaf(raw_to_float(wh[i * W + j], dt), f[i], y[i]);
-    }
+    conv8<W>(raw, wraw, dt, p.act, y);
 #pragma unroll
     for (int j = 0; j < W - 1; ++j) hist[(int64_t)j * nvec] = raw[j + 1];      // shift left, append x
-    if (p.act) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = y[i] / (1.f + expf(-y[i]));
-    }
   }
   // q, k: L2 norm over the 128 channels of the head = 16 adjacent lanes (all lanes take part)
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) ss = fmaf(y[i], y[i], ss);
-#pragma unroll
-  for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  const float r = row_rnorm(y, p.eps);
   if (!in_range) return;
   if (part < 2) {
-    const float r = rsqrtf(ss + p.eps);
 #pragma unroll
     for (int i = 0; i < 8; ++i) y[i] *= r;
   }
@@ -151,11 +125,9 @@ __global__ void __launch_bounds__(256) kda_decode_prep_vec_kernel(const PrepDeco
     if (active) {
       const float a = expf(p.A_log[head]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float z = a * (load_as_float(p.raw_gate, p.dt_gate, ((int64_t)seq * p.H + head) * 128 + c0 + i) +
-                             p.dt_bias[head * 128 + c0 + i]);
-        g[i] = p.lower_bound / (1.f + expf(-z)) * kLog2e;
-      }
+      for (int i = 0; i < 8; ++i)
+        g[i] = decode_gate(a, load_as_float(p.raw_gate, p.dt_gate, ((int64_t)seq * p.H + head) * 128 + c0 + i),
+                           p.dt_bias[head * 128 + c0 + i], p.lower_bound);
     }
     float4* go = reinterpret_cast<float4*>(p.g + ((int64_t)seq * p.H + head) * 128 + c0);
     go[0] = make_float4(g[0], g[1], g[2], g[3]);

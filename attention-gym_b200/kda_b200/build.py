@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(HERE, "libkda_b200.so")
 SOURCES = [
     "kda_cabi.cu",
     "kda_recurrent.cu",
+    "kda_stream.cu",
     "kda_preops.cu",
     "kda_conv.cu",
     "kda_chunk_fwd.cu",

@@ -1,4 +1,4 @@
-"""The decode step as one call of two overlapping launches: fused preprocessing, then the paged state update.
+"""The decode step as one call and, for 16-bit tensors, one launch: preprocessing and paged state update.
 
 ``decode_step`` is what a serving layer runs per generated token: the q | k | v projection goes
 through the short convolution (paged history, advanced in place) and SiLU, q and k are
@@ -6,8 +6,8 @@ L2-normalised, the raw gate projection becomes the bounded per-token log2 gate, 
 state pool is advanced in place.  The reference exposes these as separate operators
 (``causal_conv1d_decode``, ``l2norm``, ``bounded_gate_cumsum(chunk_size=1)``, ``recurrent_kda`` with
 ``state_indices``) and lists "decode preprocessing and scan are separate launches" as a serving
-limitation (attn_gym/linear/kda/api.py:210-212); here the preprocessing is one kernel, and the state update
-starts fetching states while it drains.
+limitation (attn_gym/linear/kda/api.py:210-212); here warps of the state-streaming kernel compute the operands of
+the states that are still on their way (fp32 tensors and widths above 4: a preprocessing kernel before it).
 """
 
 from __future__ import annotations

@@ -812,12 +812,16 @@ def _decode_step(x, weight, conv_state, state_pool, state_indices, raw_gate, A_l
     x, weight, raw_gate, beta = x.contiguous(), weight.contiguous(), raw_gate.contiguous(), beta.contiguous()
     A_log, dt_bias = A_log.float().contiguous(), dt_bias.float().contiguous()
     out = torch.empty(nseq, heads, 128, dtype=x.dtype, device=x.device)
-    scratch = torch.empty(nseq * heads * 128 * (3 * x.element_size() + 4), dtype=torch.uint8, device=x.device)
-    _cabi.call("kda_decode_step", 2, x.data_ptr(), weight.data_ptr(), conv_state.data_ptr(), state_indices.data_ptr(),
-               raw_gate.data_ptr(), _cabi.dt(raw_gate), A_log.data_ptr(), dt_bias.data_ptr(), beta.data_ptr(),
-               _cabi.dt(beta), state_pool.data_ptr(), state_pool.stride(0), scratch.data_ptr(), out.data_ptr(),
-               _cabi.dt(x), nseq, heads, weight.shape[1], conv_state.shape[0], state_pool.shape[0],
-               _act_code(activation), lower_bound, eps, _cabi.stream())
+    xp, wp, cp, bp = x.data_ptr(), weight.data_ptr(), conv_state.data_ptr(), dt_bias.data_ptr()
+    pool, width, dtype = state_pool.data_ptr(), weight.shape[1], _cabi.dt(x)
+    # 0: the whole step is one launch
+    need = _cabi.lib().kda_decode_step_scratch_bytes(xp | wp | cp | bp | pool | 4 * state_pool.stride(0), dtype, nseq,
+                                                     heads, width)
+    scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+    _cabi.call("kda_decode_step", 2 if need else 1, xp, wp, cp, state_indices.data_ptr(), raw_gate.data_ptr(),
+               _cabi.dt(raw_gate), A_log.data_ptr(), bp, beta.data_ptr(), _cabi.dt(beta), pool, state_pool.stride(0),
+               _cabi.ptr(scratch), out.data_ptr(), dtype, nseq, heads, width, conv_state.shape[0],
+               state_pool.shape[0], _act_code(activation), lower_bound, eps, _cabi.stream())
     return out
 
 

@@ -382,10 +382,13 @@ int kda_decode_prep(const void* x, const void* conv_weight, void* conv_state,
                     int dtype, int nseq, int heads, int head_dim, int width, int num_slots,
                     int activation, float lower_bound, float eps, void* stream);
 
-/* One decode step: kda_decode_prep and the paged state update of kda_recurrent_fwd (one token per sequence,
- * K = V = 128) in one call; the state update starts fetching states while the preprocessing drains.
- * state_indices selects the slot of both pools; scratch: 16-byte aligned, nseq * heads * 128 elements of q, k, v
- * (dtype) and the gate (fp32) in that order; out [nseq, heads, 128] in `dtype`. */
+/* One decode step: what kda_decode_prep and the paged state update of kda_recurrent_fwd (one token per sequence,
+ * K = V = 128) do one after the other, with the same bits.  One launch for 16-bit tensors, widths 2 to 4 and 16-byte
+ * aligned addresses and slots: kda_decode_step_scratch_bytes is 0 then and scratch may be NULL (address_bits: x,
+ * conv_weight, conv_state, dt_bias, state_pool and the slot stride in bytes, or-ed together).  Else scratch: 16-byte
+ * aligned, nseq * heads * 128 elements of q, k, v (dtype) and the gate (fp32) in that order.
+ * state_indices selects the slot of both pools; out [nseq, heads, 128] in `dtype`. */
+int64_t kda_decode_step_scratch_bytes(int64_t address_bits, int dtype, int nseq, int heads, int width);
 int kda_decode_step(const void* x, const void* conv_weight, void* conv_state, const int32_t* state_indices,
                     const void* raw_gate, int dt_gate, const float* A_log, const float* dt_bias, const void* beta,
                     int dt_beta, float* state_pool, int64_t slot_stride, void* scratch, void* out, int dtype,
