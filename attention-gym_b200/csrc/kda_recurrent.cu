@@ -19,12 +19,8 @@ namespace kda {
 // operands are fetched TT tokens at a time, one tile ahead of their use (raw bits in registers), and
 // published to shared memory as fp32 (q scaled, 2^g) with one barrier per tile.
 //
-// A long scan of few sequences is bound by the latency of one token: the dependent chain of decay,
-// reduction, three shuffles and update, 0.15 us of a warp that issues nothing else.  So NP warps of
-// their own fetch, publish and store (NP = 0: the computing warps do it), and the next token's operands
-// are read from shared memory before the shuffles.  T = 512, H = 4, K = V = 64: 726 us with eight warps
-// sharing a column slab, two CTA barriers and a shared-memory exchange per token; 135 us in this split
-// with scalar arithmetic and no moving warps, 114 us with packed arithmetic, 79 us with moving warps.
+// K > 128: bound by the latency of one token, the dependent chain of decay, reduction, three shuffles and update, so that NP
+// warps of their own fetch, publish and store (NP = 0: the computing warps do it).
 // A short scan of many sequences is bound by the state traffic and by how much of it two CTAs per SM
 // can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 141 us before, 60 us
 // now.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
@@ -37,8 +33,6 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
   constexpr int KP = 8 * KR, CT = 4 * VC * NW;
   constexpr int NE = TT * KP / NT;                 // operand elements per thread, array and tile
   constexpr int NV = (TT * CT + NT - 1) / NT;      // value and output elements per thread and tile
-  constexpr int NR = KR / 4;
-  constexpr bool kPrefetch = VC == 1 && KR <= 16 && NP > 0;
   static_assert(TT * KP % NT == 0 && TT <= 32, "tile split");
   __shared__ __align__(16) float s_q[2][TT][KP], s_k[2][TT][KP], s_d[2][TT][KP];
   __shared__ float s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
@@ -175,31 +169,16 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
     if (moves && more) fetch(t0 + TT);
     if (NP && moves && t0 > bos) flush(t0 - TT, b ^ 1, TT);
     if (computes) {
-    // The operands of a long scan's next token are read from shared memory between the two halves of
-    // a step, where their latency hides behind the shuffles.
-    f32x2 q[KR / 2], k[KR / 2], d[KR / 2];
-    auto read = [&](int tok, f32x2 (&qd)[KR / 2], f32x2 (&kd)[KR / 2], f32x2 (&dd)[KR / 2]) {
-      const ulonglong2* qs = reinterpret_cast<const ulonglong2*>(s_q[b][tok]) + lk;
-      const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
-      const ulonglong2* ds = reinterpret_cast<const ulonglong2*>(s_d[b][tok]) + lk;
-#pragma unroll
-      for (int i = 0; i < NR; ++i) {
-        const ulonglong2 a = qs[8 * i], c = ks[8 * i], e = ds[8 * i];
-        qd[2 * i] = a.x; qd[2 * i + 1] = a.y;
-        kd[2 * i] = c.x; kd[2 * i + 1] = c.y;
-        dd[2 * i] = e.x; dd[2 * i + 1] = e.y;
-      }
-    };
-    if (kPrefetch) read(0, q, k, d);
-#pragma unroll(kPrefetch ? 2 : 1)
+#pragma unroll 1
     for (int tok = 0; tok < ntok; ++tok) {
       f32x2 pk[VC], pq[VC], pqk = 0;       // (zero bits: +0, +0) even rows in the low half, odd in the high
 #pragma unroll
       for (int j = 0; j < VC; ++j) pk[j] = pq[j] = 0;
       const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
+      f32x2 q[KR / 2], k[KR / 2], d[KR / 2];
 #pragma unroll
       for (int i = 0; i < KR / 2; ++i) {
-        if (!kPrefetch && i % 2 == 0) {
+        if (i % 2 == 0) {
           const ulonglong2 x = reinterpret_cast<const ulonglong2*>(s_q[b][tok])[lk + 4 * i], y = ks[4 * i],
                            z = reinterpret_cast<const ulonglong2*>(s_d[b][tok])[lk + 4 * i];
           q[i] = x.x; q[i + 1] = x.y; k[i] = y.x; k[i + 1] = y.y; d[i] = z.x; d[i + 1] = z.y;
@@ -221,8 +200,6 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
         a[j] = y.x + y.y;
         o[j] = z.x + z.y;
       }
-      f32x2 qn[KR / 2], kn[KR / 2], dn[KR / 2];
-      if (kPrefetch) read(tok + 1 < TT ? tok + 1 : tok, qn, kn, dn);
 #pragma unroll
       for (int m = 4; m < 32; m <<= 1) {
 #pragma unroll
@@ -244,15 +221,11 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
       }
 #pragma unroll
       for (int i = 0; i < KR / 2; ++i) {
-        if (!kPrefetch && i % 2 == 0) { const ulonglong2 y = ks[4 * i]; k[i] = y.x; k[i + 1] = y.y; }
+        if (i % 2 == 0) { const ulonglong2 y = ks[4 * i]; k[i] = y.x; k[i + 1] = y.y; }      // read again: fewer registers
 #pragma unroll
         for (int j = 0; j < VC; ++j) S[i][j] = fma2(k[i], delta2[j], S[i][j]);
       }
       if (lk < VC) s_o[b][tok][wc + lk] = mine;
-      if (kPrefetch) {
-#pragma unroll
-        for (int i = 0; i < KR / 2; ++i) { q[i] = qn[i]; k[i] = kn[i]; d[i] = dn[i]; }
-      }
     }
     }
     if (moves && more) publish(b ^ 1, (int)min((int64_t)TT, eos - t0 - TT));   // those buffers were last read before the previous barrier
@@ -282,6 +255,273 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
             if (c0 + j < V) sout[(int64_t)r * V + c0 + j] = x[j];
         }
       }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Token scan of few chains: four tokens at a time.  With D_i the product of the decays of a block's tokens 0 .. i and S
+// the state that enters the block,
+//     a_i = (k_i D_i)^T S + sum_{j < i} P_ij d_j,     P_ij = sum_kappa k_i k_j D_i / D_j,     d_i = beta_i (v_i - a_i)
+//     o_i = (q_i D_i)^T S + sum_{j <= i} Q_ij d_j,    Q_ij = sum_kappa q_i k_j D_i / D_j
+//     S  <- D_3 S + sum_j (k_j D_3 / D_j) d_j
+// so the dot products with the state and their shuffles, most of a token's dependent chain, are taken once for
+// four tokens, and what is left token by token are two scalar operations.  Everything that does not depend on the state
+// (the scaled rows, the ten Q and six P, as products of decays: no division, no difference of logarithms) is made by four
+// warps of their own, one tile of blocks ahead, from operands fetched two tiles ahead.  A block that the sequence does not fill has zero rows and unit
+// decays at its end.  The computing warps own four columns each: lane (lk = lane / 4, lane % 4) holds one column and the
+// key rows 4 (lk + 8 i) .. + 3.  Bound by the chain from block to block (two dot products per token, three rounds of
+// shuffles, four corrections, the update).  fp32, 4 chains, 512 tokens from the cumulative gate, us, one token at a time /
+// blocks: K = V = 32 60 / 39, 64 80 / 51, 96 147 / 80, 128 147 / 81.  The error against 64 bits is the same (the state is
+// rounded five times a block instead of eight).
+// ------------------------------------------------------------------------------------------------
+// F32: every operand is fp32.
+template <int KR, bool CUM, bool F32>
+__global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams p) {
+  constexpr int C = 4, KP = 8 * KR, NR = KR / 4, CT = 16;
+  constexpr int TT = KR <= 8 ? 16 : 8, NB = TT / C;         // tokens and blocks of a tile
+  constexpr int SW = KP / 32, SETS = 4 / SW, NBS = NB / SETS;       // moving warps of a block, blocks at a time, blocks per set and tile
+  static_assert(NBS * SETS == NB && SW >= 1, "blocks of a tile");
+  __shared__ __align__(16) float s_kt[2][TT][KP], s_qt[2][TT][KP], s_kn[2][TT][KP], s_dc[2][NB][KP];
+  __shared__ __align__(16) float s_p[2][NB][SW][16], s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cv = lane & 3, lk = lane >> 2;
+  const bool moving = warp >= 4;
+  const int tid = (int)threadIdx.x - 128;                   // index among the moving threads
+  const int K = p.K, V = p.V, H = p.H;
+  const int vtiles = (V + CT - 1) / CT;
+  const int vt = blockIdx.x % vtiles, sh = blockIdx.x / vtiles;
+  const int head = sh % H, seq = sh / H;
+  int64_t bos, eos;
+  if (p.cu_seqlens) { bos = p.cu_seqlens[seq]; eos = p.cu_seqlens[seq + 1]; }
+  else { bos = (int64_t)seq * p.T; eos = bos + p.T; }
+  const int cta0 = vt * CT, wc = 4 * warp + cv, c0 = cta0 + wc;       // this lane's column
+  const bool paged = p.state_indices != nullptr;
+  const int64_t slot = paged ? p.state_indices[seq] : seq;
+  if (paged && (slot <= 0 || slot >= p.num_slots)) {   // padding: zero output, the pool untouched
+    for (int64_t t = bos + (threadIdx.x >> 4); t < eos; t += 16) {
+      const int c = cta0 + (threadIdx.x & 15);
+      if (c < V) store_from_float(p.out, p.dt_out, (t * H + head) * V + c, 0.f);
+    }
+    return;
+  }
+  const float* sin = p.h0 ? p.h0 + (paged ? slot * p.slot_stride : slot * H * K * V) + (int64_t)head * K * V : nullptr;
+  float* sout = paged ? const_cast<float*>(sin) : (p.ht ? p.ht + (slot * H + head) * K * V : nullptr);
+
+  // ---- operand tiles: raw bits in registers, two tiles ahead; a moving thread owns one channel of its set's blocks ----
+  // (one base address per operand and 32-bit offsets from it: with 64-bit index arithmetic and a type test for every
+  // element the moving warps took longer than the computing ones)
+  const int set = tid / KP, ch = tid % KP;       // (moving threads only)
+  uint32_t rq[NBS][C], rk[NBS][C], rg[NBS][C], rp[NBS], rv[TT * CT / 128], rb = 0;
+  auto operand = [&](const void* base, int dt, int64_t at) {
+    return reinterpret_cast<const unsigned char*>(base) + at * (F32 ? 4 : dtype_size(dt));
+  };
+  auto bits = [&](const unsigned char* base, int dt, uint32_t off) -> uint32_t {
+    if (F32 || dt == KDA_F32) return *reinterpret_cast<const uint32_t*>(base + 4 * off);
+    return *reinterpret_cast<const unsigned short*>(base + 2 * off);
+  };
+  auto number = [&](uint32_t raw, int dt) { return F32 ? __uint_as_float(raw) : raw_to_float(raw, dt); };
+  const int64_t kat = (bos * H + head) * K + (ch < K ? ch : 0), vat = (bos * H + head) * V + cta0;
+  const unsigned char *bq = operand(p.q, p.dt_q, kat), *bk = operand(p.k, p.dt_k, kat), *bg = operand(p.g, p.dt_g, kat),
+                      *bv = operand(p.v, p.dt_v, vat), *bb = operand(p.beta, p.dt_beta, bos * H + head);
+  const uint32_t krow = (uint32_t)H * K, vrow = (uint32_t)H * V;      // (a tile of rows is well below 2^31 bytes)
+  auto fetch = [&](int64_t t0) {
+    const int ntok = (int)min((int64_t)TT, eos - t0);
+    const int64_t kt = (t0 - bos) * krow, vt0 = (t0 - bos) * vrow, bt0 = (t0 - bos) * H;
+    const unsigned char *q = bq + kt * (F32 ? 4 : dtype_size(p.dt_q)), *k = bk + kt * (F32 ? 4 : dtype_size(p.dt_k)),
+                        *g = bg + kt * (F32 ? 4 : dtype_size(p.dt_g)), *v = bv + vt0 * (F32 ? 4 : dtype_size(p.dt_v));
+#pragma unroll
+    for (int n = 0; n < NBS; ++n) {
+      const int tok0 = C * (set + n * SETS);
+      rp[n] = 0;
+      // the gate before the block, unless the block starts a chunk (a block never straddles two)
+      if (CUM && ch < K && tok0 < ntok && (((int)(t0 - bos) + tok0) & (kChunk - 1)) != 0)
+        rp[n] = bits(g - (size_t)krow * (F32 ? 4 : dtype_size(p.dt_g)), p.dt_g, tok0 * krow);
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        const bool in = tok0 + i < ntok && ch < K;
+        const uint32_t off = (uint32_t)(tok0 + i) * krow;
+        rq[n][i] = in ? bits(q, p.dt_q, off) : 0;
+        rk[n][i] = in ? bits(k, p.dt_k, off) : 0;
+        rg[n][i] = in ? bits(g, p.dt_g, off) : 0;
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < TT * CT / 128; ++n) {
+      const int e = tid + n * 128, tok = e / CT, c = e % CT;
+      rv[n] = (tok < ntok && cta0 + c < V) ? bits(v, p.dt_v, (uint32_t)tok * vrow + c) : 0;
+    }
+    rb = tid < ntok ? bits(bb + bt0 * (F32 ? 4 : dtype_size(p.dt_beta)), p.dt_beta, (uint32_t)tid * H) : 0;
+  };
+  auto publish = [&](int b, int ntok) {
+#pragma unroll
+    for (int n = 0; n < NBS; ++n) {
+      const int blk = set + n * SETS, tok0 = C * blk;
+      float q[C], k[C], d[C];
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        q[i] = number(rq[n][i], p.dt_q) * p.scale;
+        k[i] = number(rk[n][i], p.dt_k);
+        float g = number(rg[n][i], p.dt_g);
+        if (CUM) g -= number(i == 0 ? rp[n] : rg[n][i - 1 < 0 ? 0 : i - 1], p.dt_g);
+        d[i] = tok0 + i < ntok ? exp2f(g) : 1.f;
+      }
+      const float d01 = d[0] * d[1], d12 = d[1] * d[2], d23 = d[2] * d[3], d123 = d12 * d[3], d012 = d01 * d[2];
+      const float D[C] = {d[0], d01, d012, d01 * d23}, E[C] = {d123, d23, d[3], 1.f};
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        s_kt[b][tok0 + i][ch] = k[i] * D[i];
+        s_qt[b][tok0 + i][ch] = q[i] * D[i];
+        s_kn[b][tok0 + i][ch] = k[i] * E[i];
+      }
+      s_dc[b][blk][ch] = D[3];
+      const float k0d1 = k[0] * d[1], k0d12 = k[0] * d12, k0d123 = k[0] * d123, k1d2 = k[1] * d[2], k1d23 = k[1] * d23,
+                  k2d3 = k[2] * d[3];
+      // P10 P20 P21 P30 P31 P32 | Q00 Q10 Q11 Q20 Q21 Q22 Q30 Q31 Q32 Q33
+      float x[16] = {k[1] * k0d1, k[2] * k0d12, k[2] * k1d2, k[3] * k0d123, k[3] * k1d23, k[3] * k2d3,
+                     q[0] * k[0], q[1] * k0d1, q[1] * k[1], q[2] * k0d12, q[2] * k1d2, q[2] * k[2],
+                     q[3] * k0d123, q[3] * k1d23, q[3] * k2d3, q[3] * k[3]};
+      // over the 32 lanes: afterwards lanes 2 e and 2 e + 1 hold the total of entry e
+#pragma unroll
+      for (int off = 16, m = 8; off >= 2; off >>= 1, m >>= 1) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (j < m) {
+            const bool up = (lane & off) != 0;
+            const float send = up ? x[j] : x[j + m], keep = up ? x[j + m] : x[j];
+            x[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+          }
+        }
+      }
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+      if ((lane & 1) == 0) s_p[b][blk][warp & (SW - 1)][lane >> 1] = x[0];
+    }
+#pragma unroll
+    for (int n = 0; n < TT * CT / 128; ++n) {
+      const int e = tid + n * 128;
+      s_v[b][e / CT][e % CT] = number(rv[n], p.dt_v);
+    }
+    if (tid < TT) s_beta[b][tid] = number(rb, p.dt_beta);
+  };
+  auto flush = [&](int64_t t0, int b, int ntok) {      // the outputs of a tile
+#pragma unroll
+    for (int n = 0; n < TT * CT / 128; ++n) {
+      const int e = tid + n * 128, tok = e / CT, c = e % CT;
+      if (tok < ntok && cta0 + c < V) store_from_float(p.out, p.dt_out, ((t0 + tok) * H + head) * V + cta0 + c, s_o[b][tok][c]);
+    }
+  };
+
+  if (moving) fetch(bos);
+  // ---- state: S[i] holds the rows 2 i, 2 i + 1 of this lane's list, rows 4 (lk + 8 i) .. + 3 ----------------
+  f32x2 S[KR / 2];
+  auto row = [&](int i) { return 4 * (lk + 8 * (i >> 2)) + (i & 3); };
+#pragma unroll
+  for (int i = 0; i < KR; i += 2) {
+    const bool in = !moving && sin && c0 < V;
+    const float x = in && row(i) < K ? sin[(int64_t)row(i) * V + c0] : 0.f;
+    const float y = in && row(i + 1) < K ? sin[(int64_t)row(i + 1) * V + c0] : 0.f;
+    S[i >> 1] = pack2(x, y);
+  }
+  if (moving) {
+    publish(0, (int)min((int64_t)TT, eos - bos));
+    if (bos + TT < eos) fetch(bos + TT);
+  }
+  __syncthreads();
+  int b = 0;
+  for (int64_t t0 = bos; t0 < eos; t0 += TT, b ^= 1) {
+    const bool more = t0 + TT < eos;
+    const int ntok = more ? TT : (int)(eos - t0);
+    if (moving) {
+      if (more) publish(b ^ 1, (int)min((int64_t)TT, eos - t0 - TT));
+      if (t0 + 2 * TT < eos) fetch(t0 + 2 * TT);
+      if (t0 > bos) flush(t0 - TT, b ^ 1, TT);
+    } else {
+      for (int blk = 0; C * blk < ntok; ++blk) {
+        const int tok0 = C * blk;
+        f32x2 pa[C], po[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(s_kt[b][tok0 + i]) + lk;
+          const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(s_qt[b][tok0 + i]) + lk;
+          pa[i] = po[i] = 0;         // (zero bits: +0, +0) even rows in the low half, odd in the high
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            const ulonglong2 x = kt[8 * r], y = qt[8 * r];
+            pa[i] = fma2(x.x, S[2 * r], pa[i]);
+            po[i] = fma2(y.x, S[2 * r], po[i]);
+            pa[i] = fma2(x.y, S[2 * r + 1], pa[i]);
+            po[i] = fma2(y.y, S[2 * r + 1], po[i]);
+          }
+        }
+        float a[C], o[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const float2 x = unpack2(pa[i]), y = unpack2(po[i]);
+          a[i] = x.x + x.y;
+          o[i] = y.x + y.y;
+        }
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            a[i] += __shfl_xor_sync(0xffffffffu, a[i], m);
+            o[i] += __shfl_xor_sync(0xffffffffu, o[i], m);
+          }
+        }
+        float w[16];                 // the pairwise products
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+          float4 x = *reinterpret_cast<const float4*>(&s_p[b][blk][0][e]);
+#pragma unroll
+          for (int u = 1; u < SW; ++u) {
+            const float4 y = *reinterpret_cast<const float4*>(&s_p[b][blk][u][e]);
+            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+          }
+          w[e] = x.x; w[e + 1] = x.y; w[e + 2] = x.z; w[e + 3] = x.w;
+        }
+        const float4 bt = *reinterpret_cast<const float4*>(&s_beta[b][tok0]);
+        const float (*vv)[CT] = &s_v[b][tok0];
+        const float e0 = bt.x * (vv[0][wc] - a[0]);
+        const float e1 = bt.y * (vv[1][wc] - fmaf(w[0], e0, a[1]));
+        const float e2 = bt.z * (vv[2][wc] - fmaf(w[2], e1, fmaf(w[1], e0, a[2])));
+        const float e3 = bt.w * (vv[3][wc] - fmaf(w[5], e2, fmaf(w[4], e1, fmaf(w[3], e0, a[3]))));
+        const float e[C] = {e0, e1, e2, e3};
+        {
+          const ulonglong2* dc = reinterpret_cast<const ulonglong2*>(s_dc[b][blk]) + lk;
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            const ulonglong2 x = dc[8 * r];
+            S[2 * r] = mul2(S[2 * r], x.x);
+            S[2 * r + 1] = mul2(S[2 * r + 1], x.y);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+          const ulonglong2* kn = reinterpret_cast<const ulonglong2*>(s_kn[b][tok0 + j]) + lk;
+          const f32x2 ej = pack2(e[j], e[j]);
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            const ulonglong2 x = kn[8 * r];
+            S[2 * r] = fma2(x.x, ej, S[2 * r]);
+            S[2 * r + 1] = fma2(x.y, ej, S[2 * r + 1]);
+          }
+        }
+        o[0] = fmaf(w[6], e0, o[0]);
+        o[1] = fmaf(w[8], e1, fmaf(w[7], e0, o[1]));
+        o[2] = fmaf(w[11], e2, fmaf(w[10], e1, fmaf(w[9], e0, o[2])));
+        o[3] = fmaf(w[15], e3, fmaf(w[14], e2, fmaf(w[13], e1, fmaf(w[12], e0, o[3]))));
+        if (lk < C) s_o[b][tok0 + lk][wc] = lk == 0 ? o[0] : (lk == 1 ? o[1] : (lk == 2 ? o[2] : o[3]));
+      }
+    }
+    __syncthreads();
+    if (moving && !more) flush(t0, b, ntok);
+  }
+  if (sout && !moving && c0 < V) {
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+      const float2 y = unpack2(S[i >> 1]);
+      if (row(i) < K) sout[(int64_t)row(i) * V + c0] = (i & 1) ? y.y : y.x;
     }
   }
 }
@@ -392,6 +632,20 @@ int device_sms() {
   return sms;
 }
 
+template <int KR>
+static int launch_block_scan(const ScanParams& p, bool cumulative, cudaStream_t stream) {
+  const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + 15) / 16);
+  if (blocks <= 0) return KDA_OK;
+  if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
+  StageScope timing(kStageRecurrent, stream);
+  const bool f32 = p.dt_q == KDA_F32 && p.dt_k == KDA_F32 && p.dt_v == KDA_F32 && p.dt_g == KDA_F32 && p.dt_beta == KDA_F32;
+  if (cumulative && f32) kda_block_scan_kernel<KR, true, true><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else if (cumulative) kda_block_scan_kernel<KR, true, false><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else if (f32) kda_block_scan_kernel<KR, false, true><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else kda_block_scan_kernel<KR, false, false><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
 template <int KR, int VC, int NW, int NP, int MINB>
 static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream) {
   constexpr int CT = 4 * VC * NW, KP = 8 * KR;
@@ -406,27 +660,29 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
-// Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length.
-// Figures in us, both sides of each line.
-// * wide: four columns per lane, 128 per CTA, 16-byte state accesses, once the slices take more than two turns on the
-//   SMs; one column per lane (16 per CTA, operands brought by warps of their own: the shortest chain from token to
-//   token) below.  K = V = 128, one / four columns per lane: 64 chains (512 slices) 17.3 / 10.8 at 2 tokens, 46 / 34 at
-//   32; 32 chains 28 / 33 at 32, 128 / 187 at 256.  For 3 to 6 tokens from one turn on: 32 chains (256 slices) 13.3 / 11.1
-//   at 4; K = 128, V = 64, 48 chains 13.5 / 12.3 at 6, 16 chains (64 slices) 9.0 / 10.4.
+// Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length, a turn as
+// many slices as there are SMs.  Figures in us, both sides of each line (K = V = 128 unless said otherwise).
+// * wide: four columns per lane, 128 per CTA, 16-byte state accesses, two CTAs per SM, from more than two turns on; from more
+//   than one turn on for 2 to 8 tokens.  Below: blocks of four tokens, 16 columns per CTA.  Blocks / wide: 16 chains (128
+//   slices) 5.6 / 6.6 at 2 tokens, 12 / 27 at 32, 68 / 183 at 256; 32 chains 9.2 / 6.5 at 2, 10.1 / 10.0 at 8, 13.9 / 15.4 at 16,
+//   134 / 183 at 256; 48 chains (384) 12.7 / 6.4 at 2, 20 / 15.5 at 16, 56 / 49 at 64.  K = V = 32 up to four turns from 64 tokens
+//   on: 192 chains (384) 11.0 / 11.2 at 16, 25 / 36 at 64; 296 chains (592) 21.3 / 19.5 at 32, 109 / 135 at 256.
 // * many: state rows that are not 16-byte aligned, more than two turns: one column per lane, but 32 per CTA and two CTAs
-//   per SM.  K = 128, V = 130, 16 / 32 columns: 48 chains (432 slices) 15.8 / 10.1 at 3 tokens, 56 / 44 at 64; 2048 chains
-//   414 / 157 at 3, 2305 / 1262 at 64.
-// * the short scan for one token, and for two where the form above loses to it.  K = 128, V = 64, short / else: 48 chains
-//   (192 slices) 9.0 / 11.3 at 1 token, 10.1 / 11.7 at 2; 16 chains 11.8 / 10.4 at 2.  V = 130, 2048 chains 117 / 130 at 1,
-//   184 / 142 at 2.  K = 256, V = 128: 128 chains 14.7 / 21.3 at 1, 19.2 / 23.2 at 2; 16 chains (128 slices) 11.2 / 9.1 at 2.
+//   per SM.  K = 128, V = 130, one token at a time in 16 / 32 columns: 48 chains (432 slices) 15.8 / 10.1 at 3 tokens, 56 / 44 at
+//   64 (blocks of four: 56 at 64 and 384 slices).
+// * the short scan for one token, and where the forms above lose to it.  K = 128, V = 64, short / blocks / wide: 16 chains
+//   4.4 / 5.4 / 4.8 at 1 token, 6.2 / 5.5 / 5.5 at 2; 48 chains (192 slices) 4.6 / 9.0 / 5.1 at 1, 7.9 / 8.9 / 6.1 at 3, 9.9 / 8.9 /
+//   6.8 at 4.  V = 130, 2048 chains, short / many 117 / 130 at 1, 184 / 142 at 2.  K = 256, V = 128, short / one column per
+//   lane: 128 chains 14.7 / 21.3 at 1, 19.2 / 23.2 at 2; 16 chains (128 slices) 11.2 / 9.1 at 2.
 static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s) {
   const int sms = device_sms();
   const int64_t slices = (int64_t)p.nseq * p.H * ((p.V + 15) / 16);
   const int64_t tokens = p.cu_seqlens && p.nseq > 0 ? p.T / p.nseq : p.T;      // per sequence, on average
   const bool aligned = (((uintptr_t)p.h0 | (uintptr_t)p.ht) & 15) == 0 && p.V % 4 == 0 && p.slot_stride % 4 == 0;
-  const bool wide = aligned && p.K <= 128 && slices > (tokens >= 3 && tokens <= 6 ? sms : 2 * sms);
+  const int turns = tokens >= 2 && tokens <= 8 ? 1 : (p.K <= 32 && tokens >= 64 ? 4 : 2);
+  const bool wide = aligned && p.K <= 128 && slices > (int64_t)turns * sms;
   const bool many = !aligned && p.K <= 128 && slices > 2 * sms;
-  const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || p.K <= 32 || slices <= sms ? 1 : 2);
+  const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || slices <= sms ? 1 : (p.K <= 32 ? 2 : 3));
   if (!wide && !cumulative && tokens <= few) {
     if (p.K <= 32) return launch_short_scan<4>(p, s);
     if (p.K <= 64) return launch_short_scan<8>(p, s);
@@ -444,9 +700,9 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
     if (p.K <= 64) return launch_scan<8, 1, 8, 0, 2>(p, cumulative, s);
     return launch_scan<16, 1, 8, 0, 2>(p, cumulative, s);
   }
-  if (p.K <= 32) return launch_scan<4, 1, 4, 4, 1>(p, cumulative, s);
-  if (p.K <= 64) return launch_scan<8, 1, 4, 4, 1>(p, cumulative, s);
-  return launch_scan<16, 1, 4, 4, 1>(p, cumulative, s);
+  if (p.K <= 32) return launch_block_scan<4>(p, cumulative, s);
+  if (p.K <= 64) return launch_block_scan<8>(p, cumulative, s);
+  return launch_block_scan<16>(p, cumulative, s);
 }
 
 static int launch_recurrent(const ScanParams& p, cudaStream_t s) {

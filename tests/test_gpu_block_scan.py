@@ -1,0 +1,54 @@
+"""The scan in blocks of four tokens where its blocks, tiles and moving warps end: token counts around 4, 8, 16 and 32, head
+sizes around its row groups (32, 64, 128) and column slices (16), chunk boundaries of the cumulative gate, mixed dtypes,
+gates that forget at once; against the fp64 recurrence."""
+
+import pytest
+import torch
+
+import kda_b200
+from oracle import kda_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+# fp32 sums of at most 128 terms over at most 200 tokens of a contracting recurrence: 200 * 128 * 2^-24 = 1.5e-3 of the
+# largest value bounds the worst case
+TOL = 1.5e-3
+
+
+def _close(got, want, what):
+    err = float((got.double().cpu() - want).abs().max() / want.abs().max().clamp_min(1e-30))
+    assert err < TOL, (what, err)
+
+
+@pytest.mark.parametrize("kd,vd", [(20, 5), (32, 16), (33, 17), (64, 64), (96, 33), (128, 128)])
+@pytest.mark.parametrize("lengths", [[5, 0, 7, 12, 31, 1], [15, 16, 17, 32, 33], [64, 65, 200]], ids=str)
+def test_block_and_tile_edges(kd, vd, lengths):
+    inp = orc.make_inputs(1, sum(lengths), 2, kd, vd, seed=kd + len(lengths), with_state=True, lengths=lengths)
+    dev = {n: t.cuda() if torch.is_tensor(t) else t for n, t in inp.items()}
+    want_o, want_s = orc.recurrent_kda_ref(*(inp[n].double() for n in ("q", "k", "v", "gate_log2", "beta", "h0")),
+                                           inp["cu_seqlens"])
+    args = (dev["q"], dev["k"], dev["v"])
+    o, s = kda_b200.recurrent_kda(*args, dev["gate_log2"], dev["beta"], dev["h0"], cu_seqlens=dev["cu_seqlens"],
+                                  output_final_state=True)
+    _close(o, want_o, "output")
+    _close(s, want_s, "state")
+    o, s = kda_b200.chunk_kda(*args, dev["cum_gate"], dev["beta"], dev["h0"], cu_seqlens=dev["cu_seqlens"],
+                              output_final_state=True, exact_fp32=True)
+    _close(o, want_o, "output (cumulative gate)")
+    _close(s, want_s, "state (cumulative gate)")
+
+
+def test_mixed_dtypes_and_gates_that_forget():
+    inp = orc.make_inputs(2, 37, 3, 64, 40, seed=9, with_state=True)
+    q, k, v = inp["q"].bfloat16(), inp["k"].half(), inp["v"].bfloat16()
+    gate = inp["gate_log2"].clone()
+    gate[:, 5] = -300.0                    # 2^g is zero in fp32
+    gate[:, 18, :, ::2] = float("-inf")
+    want_o, want_s = orc.recurrent_kda_ref(q.double(), k.double(), v.double(), gate.double(), inp["beta"].double(),
+                                           inp["h0"].double())
+    o, s = kda_b200.recurrent_kda(q.cuda(), k.cuda(), v.cuda(), gate.cuda(), inp["beta"].cuda(), inp["h0"].cuda(),
+                                  output_final_state=True)
+    assert torch.isfinite(o.float()).all() and torch.isfinite(s).all()
+    err = float((o.double().cpu() - want_o).abs().max() / want_o.abs().max())
+    assert err < 2.0 ** -8 + TOL
+    _close(s, want_s, "state")
