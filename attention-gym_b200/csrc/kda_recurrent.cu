@@ -268,20 +268,20 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
 // so the dot products with the state and their shuffles, most of a token's dependent chain, are taken once for
 // four tokens, and what is left token by token are two scalar operations.  Everything that does not depend on the state
 // (the scaled rows, the ten Q and six P, as products of decays: no division, no difference of logarithms) is made by four
-// warps of their own, one tile of blocks ahead, from operands fetched two tiles ahead.  A block that the sequence does not fill has zero rows and unit
-// decays at its end.  The computing warps own four columns each: lane (lk = lane / 4, lane % 4) holds one column and the
+// warps of their own, two channels per thread, one tile of blocks ahead, from operands fetched two tiles ahead.  A block that
+// the sequence does not fill has zero rows and unit decays at its end.  The computing warps own four columns each: lane (lk = lane / 4, lane % 4) holds one column and the
 // key rows 4 (lk + 8 i) .. + 3.  Bound by the chain from block to block (two dot products per token, three rounds of
 // shuffles, four corrections, the update).  fp32, 4 chains, 512 tokens from the cumulative gate, us, one token at a time /
-// blocks: K = V = 32 60 / 39, 64 80 / 51, 96 147 / 80, 128 147 / 81.  The error against 64 bits is the same (the state is
-// rounded five times a block instead of eight).
+// blocks: K = V = 32 60 / 46, 64 80 / 50, 96 147 / 77, 128 147 / 78.  The error against 64 bits is the same; with one channel per
+// thread (its products rounded before the sum) it was 3 to 8 % larger at gates that forget fast.  (The state is
+// rounded five times a block instead of eight.)
 // ------------------------------------------------------------------------------------------------
 // F32: every operand is fp32.
 template <int KR, bool CUM, bool F32>
 __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams p) {
   constexpr int C = 4, KP = 8 * KR, NR = KR / 4, CT = 16;
-  constexpr int TT = KR <= 8 ? 16 : 8, NB = TT / C;         // tokens and blocks of a tile
-  constexpr int SW = KP / 32, SETS = 4 / SW, NBS = NB / SETS;       // moving warps of a block, blocks at a time, blocks per set and tile
-  static_assert(NBS * SETS == NB && SW >= 1, "blocks of a tile");
+  constexpr int LB = KP / 2, SW = (LB + 31) / 32;           // moving threads of a block (two channels each) and their warps
+  constexpr int NB = 128 / LB, TT = C * NB;                 // blocks and tokens of a tile: 32, 16 or 8
   __shared__ __align__(16) float s_kt[2][TT][KP], s_qt[2][TT][KP], s_kn[2][TT][KP], s_dc[2][NB][KP];
   __shared__ __align__(16) float s_p[2][NB][SW][16], s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
 
@@ -309,11 +309,12 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
   const float* sin = p.h0 ? p.h0 + (paged ? slot * p.slot_stride : slot * H * K * V) + (int64_t)head * K * V : nullptr;
   float* sout = paged ? const_cast<float*>(sin) : (p.ht ? p.ht + (slot * H + head) * K * V : nullptr);
 
-  // ---- operand tiles: raw bits in registers, two tiles ahead; a moving thread owns one channel of its set's blocks ----
+  // ---- operand tiles: raw bits in registers, two tiles ahead; a moving thread owns two channels of one block ----
   // (one base address per operand and 32-bit offsets from it: with 64-bit index arithmetic and a type test for every
   // element the moving warps took longer than the computing ones)
-  const int set = tid / KP, ch = tid % KP;       // (moving threads only)
-  uint32_t rq[NBS][C], rk[NBS][C], rg[NBS][C], rp[NBS], rv[TT * CT / 128], rb = 0;
+  const int blk0 = tid / LB, ch = 2 * (tid % LB), tok0 = C * blk0;       // (moving threads only)
+  const bool in0 = ch < K, in1 = ch + 1 < K;
+  uint32_t rq[C][2], rk[C][2], rg[C][2], rp[2], rv[TT * CT / 128], rb = 0;
   auto operand = [&](const void* base, int dt, int64_t at) {
     return reinterpret_cast<const unsigned char*>(base) + at * (F32 ? 4 : dtype_size(dt));
   };
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
     return *reinterpret_cast<const unsigned short*>(base + 2 * off);
   };
   auto number = [&](uint32_t raw, int dt) { return F32 ? __uint_as_float(raw) : raw_to_float(raw, dt); };
-  const int64_t kat = (bos * H + head) * K + (ch < K ? ch : 0), vat = (bos * H + head) * V + cta0;
+  const int64_t kat = (bos * H + head) * K + (in0 ? ch : 0), vat = (bos * H + head) * V + cta0;
   const unsigned char *bq = operand(p.q, p.dt_q, kat), *bk = operand(p.k, p.dt_k, kat), *bg = operand(p.g, p.dt_g, kat),
                       *bv = operand(p.v, p.dt_v, vat), *bb = operand(p.beta, p.dt_beta, bos * H + head);
   const uint32_t krow = (uint32_t)H * K, vrow = (uint32_t)H * V;      // (a tile of rows is well below 2^31 bytes)
@@ -331,20 +332,21 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
     const int64_t kt = (t0 - bos) * krow, vt0 = (t0 - bos) * vrow, bt0 = (t0 - bos) * H;
     const unsigned char *q = bq + kt * (F32 ? 4 : dtype_size(p.dt_q)), *k = bk + kt * (F32 ? 4 : dtype_size(p.dt_k)),
                         *g = bg + kt * (F32 ? 4 : dtype_size(p.dt_g)), *v = bv + vt0 * (F32 ? 4 : dtype_size(p.dt_v));
+    // the gate before the block, unless the block starts a chunk (a block never straddles two)
+    const bool before = CUM && tok0 < ntok && (((int)(t0 - bos) + tok0) & (kChunk - 1)) != 0;
+    const unsigned char* gp = g - (size_t)krow * (F32 ? 4 : dtype_size(p.dt_g));
+    rp[0] = before && in0 ? bits(gp, p.dt_g, tok0 * krow) : 0;
+    rp[1] = before && in1 ? bits(gp, p.dt_g, tok0 * krow + 1) : 0;
 #pragma unroll
-    for (int n = 0; n < NBS; ++n) {
-      const int tok0 = C * (set + n * SETS);
-      rp[n] = 0;
-      // the gate before the block, unless the block starts a chunk (a block never straddles two)
-      if (CUM && ch < K && tok0 < ntok && (((int)(t0 - bos) + tok0) & (kChunk - 1)) != 0)
-        rp[n] = bits(g - (size_t)krow * (F32 ? 4 : dtype_size(p.dt_g)), p.dt_g, tok0 * krow);
+    for (int i = 0; i < C; ++i) {
+      const bool live = tok0 + i < ntok;
+      const uint32_t off = (uint32_t)(tok0 + i) * krow;
 #pragma unroll
-      for (int i = 0; i < C; ++i) {
-        const bool in = tok0 + i < ntok && ch < K;
-        const uint32_t off = (uint32_t)(tok0 + i) * krow;
-        rq[n][i] = in ? bits(q, p.dt_q, off) : 0;
-        rk[n][i] = in ? bits(k, p.dt_k, off) : 0;
-        rg[n][i] = in ? bits(g, p.dt_g, off) : 0;
+      for (int u = 0; u < 2; ++u) {
+        const bool in = live && (u ? in1 : in0);
+        rq[i][u] = in ? bits(q, p.dt_q, off + u) : 0;
+        rk[i][u] = in ? bits(k, p.dt_k, off + u) : 0;
+        rg[i][u] = in ? bits(g, p.dt_g, off + u) : 0;
       }
     }
 #pragma unroll
@@ -355,47 +357,59 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
     rb = tid < ntok ? bits(bb + bt0 * (F32 ? 4 : dtype_size(p.dt_beta)), p.dt_beta, (uint32_t)tid * H) : 0;
   };
   auto publish = [&](int b, int ntok) {
+    float q[C][2], k[C][2], d[C][2], kt[C][2], qt[C][2], kn[C][2], dc[2], x[16];
 #pragma unroll
-    for (int n = 0; n < NBS; ++n) {
-      const int blk = set + n * SETS, tok0 = C * blk;
-      float q[C], k[C], d[C];
-#pragma unroll
-      for (int i = 0; i < C; ++i) {
-        q[i] = number(rq[n][i], p.dt_q) * p.scale;
-        k[i] = number(rk[n][i], p.dt_k);
-        float g = number(rg[n][i], p.dt_g);
-        if (CUM) g -= number(i == 0 ? rp[n] : rg[n][i - 1 < 0 ? 0 : i - 1], p.dt_g);
-        d[i] = tok0 + i < ntok ? exp2f(g) : 1.f;
-      }
-      const float d01 = d[0] * d[1], d12 = d[1] * d[2], d23 = d[2] * d[3], d123 = d12 * d[3], d012 = d01 * d[2];
-      const float D[C] = {d[0], d01, d012, d01 * d23}, E[C] = {d123, d23, d[3], 1.f};
+    for (int u = 0; u < 2; ++u) {
 #pragma unroll
       for (int i = 0; i < C; ++i) {
-        s_kt[b][tok0 + i][ch] = k[i] * D[i];
-        s_qt[b][tok0 + i][ch] = q[i] * D[i];
-        s_kn[b][tok0 + i][ch] = k[i] * E[i];
+        q[i][u] = number(rq[i][u], p.dt_q) * p.scale;
+        k[i][u] = number(rk[i][u], p.dt_k);
+        float g = number(rg[i][u], p.dt_g);
+        if (CUM) g -= number(i == 0 ? rp[u] : rg[i == 0 ? 0 : i - 1][u], p.dt_g);
+        d[i][u] = tok0 + i < ntok ? exp2f(g) : 1.f;
       }
-      s_dc[b][blk][ch] = D[3];
-      const float k0d1 = k[0] * d[1], k0d12 = k[0] * d12, k0d123 = k[0] * d123, k1d2 = k[1] * d[2], k1d23 = k[1] * d23,
-                  k2d3 = k[2] * d[3];
-      // P10 P20 P21 P30 P31 P32 | Q00 Q10 Q11 Q20 Q21 Q22 Q30 Q31 Q32 Q33
-      float x[16] = {k[1] * k0d1, k[2] * k0d12, k[2] * k1d2, k[3] * k0d123, k[3] * k1d23, k[3] * k2d3,
-                     q[0] * k[0], q[1] * k0d1, q[1] * k[1], q[2] * k0d12, q[2] * k1d2, q[2] * k[2],
-                     q[3] * k0d123, q[3] * k1d23, q[3] * k2d3, q[3] * k[3]};
-      // over the 32 lanes: afterwards lanes 2 e and 2 e + 1 hold the total of entry e
+      const float d01 = d[0][u] * d[1][u], d12 = d[1][u] * d[2][u], d23 = d[2][u] * d[3][u], d123 = d12 * d[3][u];
+      const float D[C] = {d[0][u], d01, d01 * d[2][u], d01 * d23}, E[C] = {d123, d23, d[3][u], 1.f};
 #pragma unroll
-      for (int off = 16, m = 8; off >= 2; off >>= 1, m >>= 1) {
+      for (int i = 0; i < C; ++i) {
+        kt[i][u] = k[i][u] * D[i];
+        qt[i][u] = q[i][u] * D[i];
+        kn[i][u] = k[i][u] * E[i];
+      }
+      dc[u] = D[3];
+      const float k0d1 = k[0][u] * d[1][u], k0d12 = k[0][u] * d12, k1d2 = k[1][u] * d[2][u];
+      // P10 P20 P21 P30 P31 P32 | Q00 Q10 Q11 Q20 Q21 Q22 Q30 Q31 Q32 Q33 as (row, column) factors
+      const float f[16] = {k[1][u], k[2][u], k[2][u], k[3][u], k[3][u], k[3][u], q[0][u], q[1][u],
+                           q[1][u], q[2][u], q[2][u], q[2][u], q[3][u], q[3][u], q[3][u], q[3][u]};
+      const float h[16] = {k0d1, k0d12, k1d2, kn[0][u], kn[1][u], kn[2][u], k[0][u], k0d1,
+                           k[1][u], k0d12, k1d2, k[2][u], kn[0][u], kn[1][u], kn[2][u], k[3][u]};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (j < m) {
-            const bool up = (lane & off) != 0;
-            const float send = up ? x[j] : x[j + m], keep = up ? x[j + m] : x[j];
-            x[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-          }
+      for (int e = 0; e < 16; ++e) x[e] = u == 0 ? f[e] * h[e] : fmaf(f[e], h[e], x[e]);
+    }
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      *reinterpret_cast<float2*>(&s_kt[b][tok0 + i][ch]) = make_float2(kt[i][0], kt[i][1]);
+      *reinterpret_cast<float2*>(&s_qt[b][tok0 + i][ch]) = make_float2(qt[i][0], qt[i][1]);
+      *reinterpret_cast<float2*>(&s_kn[b][tok0 + i][ch]) = make_float2(kn[i][0], kn[i][1]);
+    }
+    *reinterpret_cast<float2*>(&s_dc[b][blk0][ch]) = make_float2(dc[0], dc[1]);
+    // sums over the block's lanes: afterwards lane e of 16, or lanes 2 e and 2 e + 1 of a warp, hold the total of entry e
+#pragma unroll
+    for (int off = LB >= 32 ? 16 : 8, m = 8; m >= 1; off >>= 1, m >>= 1) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j < m) {
+          const bool up = (lane & off) != 0;
+          const float send = up ? x[j] : x[j + m], keep = up ? x[j + m] : x[j];
+          x[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
       }
+    }
+    if (LB >= 32) {
       x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
-      if ((lane & 1) == 0) s_p[b][blk][warp & (SW - 1)][lane >> 1] = x[0];
+      if ((lane & 1) == 0) s_p[b][blk0][warp & (SW - 1)][lane >> 1] = x[0];
+    } else {
+      s_p[b][blk0][0][lane & 15] = x[0];
     }
 #pragma unroll
     for (int n = 0; n < TT * CT / 128; ++n) {
