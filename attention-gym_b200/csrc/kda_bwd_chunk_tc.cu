@@ -44,6 +44,7 @@ struct BwdTcParams {
   int* error;
   int nseq, H, total;          // total = chunk capacity x heads work items
   int64_t tokens;              // rows of the packed buffers
+  int64_t pitch;               // elements from one token's row of q, k, v, dq, dk, dv to the next one's
   float scale;
   long long* prof;
 };
@@ -649,7 +650,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
   if (valid < 64) {
     for (int idx = tid; idx < valid * 16; idx += NT) {
       const int r = idx >> 4, ch = idx & 15;
-      *reinterpret_cast<uint4*>(p.dv + ((cw.token0 + r) * H + head) * 128 + ch * 8) =
+      *reinterpret_cast<uint4*>(p.dv + (cw.token0 + r) * p.pitch + head * 128 + ch * 8) =
           *reinterpret_cast<const uint4*>(sm + bl::DVO + (ch >> 3) * 8192 + sw128_chunk(r, ch & 7));
     }
   }
@@ -843,7 +844,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
       const int i = (tid >> 4) + 32 * n;
       raw_q[n] = raw_k[n] = make_uint4(0, 0, 0, 0);
       if (i < valid) {
-        const int64_t at = ((cw.token0 + i) * H + head) * 128 + 8 * (tid & 15);
+        const int64_t at = (cw.token0 + i) * p.pitch + head * 128 + 8 * (tid & 15);
         raw_q[n] = *reinterpret_cast<const uint4*>(p.q + at);
         raw_k[n] = *reinterpret_cast<const uint4*>(p.k + at);
       }
@@ -978,7 +979,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
   } else {
     for (int idx = tid; idx < valid * 16; idx += NT) {
       const int r = idx >> 4, ch = idx & 15;
-      const int64_t gi = ((cw.token0 + r) * H + head) * 128 + ch * 8;
+      const int64_t gi = (cw.token0 + r) * p.pitch + head * 128 + ch * 8;
       const int so = (ch >> 3) * 8192 + sw128_chunk(r, ch & 7);
       *reinterpret_cast<uint4*>(p.dq + gi) = *reinterpret_cast<const uint4*>(sm + bl::Q + so);
       *reinterpret_cast<uint4*>(p.dk + gi) = *reinterpret_cast<const uint4*>(sm + bl::K + so);
@@ -1015,7 +1016,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
 
 static __device__ int g_bwd_tc_error = 0;
 
-int launch_bwd_chunk_tc(const bf16* q, const bf16* k, const bf16* v, const float* g, const float* beta,
+int launch_bwd_chunk_tc(const bf16* q, const bf16* k, const bf16* v, int64_t pitch, const float* g, const float* beta,
                         const bf16* akk, const bf16* h, const bf16* dh, const bf16* vnew,
                         const bf16* dv2, const bf16* dout, bf16* dq, bf16* dk, bf16* dv, float* dg,
                         float* db, const float* rstd_q, const float* rstd_k, const int32_t* cu,
@@ -1025,16 +1026,19 @@ int launch_bwd_chunk_tc(const bf16* q, const bf16* k, const bf16* v, const float
   if ((rstd_q == nullptr) != (rstd_k == nullptr)) return KDA_ERR_ARG;
   BwdTcParams p;
   p.prof = prof;
+  p.pitch = pitch;
   p.q = q; p.k = k; p.rstd_q = rstd_q; p.rstd_k = rstd_k;
   const int64_t cols = (int64_t)H * 128, hrows = (int64_t)chunks * H * 128;
   bool ok = make_tensor_map(&p.tm_h, h, hrows, 128, 128) && make_tensor_map(&p.tm_dh, dh, hrows, 128, 128) &&
             make_tensor_map(&p.tm_do, dout, tokens, cols, 64) && make_tensor_map(&p.tm_vn, vnew, tokens, cols, 64) &&
-            make_tensor_map(&p.tm_dv2, dv2, tokens, cols, 64) && make_tensor_map(&p.tm_v, v, tokens, cols, 64) &&
-            make_tensor_map(&p.tm_k, k, tokens, cols, 64) && make_tensor_map(&p.tm_q, q, tokens, cols, 64) &&
+            make_tensor_map(&p.tm_dv2, dv2, tokens, cols, 64) && make_tensor_map(&p.tm_v, v, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_k, k, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_q, q, tokens, cols, 64, false, pitch) &&
             make_tensor_map(&p.tm_a, akk, tokens, (int64_t)H * 64, 64) &&
             make_tensor_map(&p.tm_g, g, tokens, cols, 64, true) &&
-            make_tensor_map(&p.tm_dq, dq, tokens, cols, 64) && make_tensor_map(&p.tm_dk, dk, tokens, cols, 64) &&
-            make_tensor_map(&p.tm_dv, dv, tokens, cols, 64) && make_tensor_map(&p.tm_dg, dg, tokens, cols, 64, true);
+            make_tensor_map(&p.tm_dq, dq, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_dk, dk, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_dv, dv, tokens, cols, 64, false, pitch) && make_tensor_map(&p.tm_dg, dg, tokens, cols, 64, true);
   if (!ok) return KDA_ERR_LAUNCH;
   p.beta = beta; p.dq = dq; p.dk = dk; p.dv = dv; p.dg = dg; p.db = db;
   p.cu_seqlens = cu; p.chunk_offsets = co; p.nseq = nseq; p.H = H;

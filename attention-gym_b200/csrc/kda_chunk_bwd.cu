@@ -17,7 +17,7 @@ int launch_state_bwd_tc(const bf16* w, const bf16* kg, const bf16* qg, const bf1
                         const float* g, const float* dht, float* dh0, bf16* dh_out, bf16* dv2_out,
                         const int32_t* cu, const int32_t* co, int nseq, int H, int64_t tokens,
                         int chunks, cudaStream_t s);
-int launch_bwd_chunk_tc(const bf16* q, const bf16* k, const bf16* v, const float* g, const float* beta,
+int launch_bwd_chunk_tc(const bf16* q, const bf16* k, const bf16* v, int64_t pitch, const float* g, const float* beta,
                         const bf16* akk, const bf16* h, const bf16* dh, const bf16* vnew,
                         const bf16* dv2, const bf16* dout, bf16* dq, bf16* dk, bf16* dv, float* dg,
                         float* db, const float* rstd_q, const float* rstd_k, const int32_t* cu,
@@ -51,7 +51,9 @@ extern "C" int64_t kda_chunk_bwd_workspace_bytes(int64_t tokens, int heads, int6
   return (6 * nd + 2 * hs + nd) * 2 + 256;
 }
 
-static int chunk_bwd_impl(bool saved, const float* rstd_q, const float* rstd_k, const void* q, const void* k, const void* v, const float* cum_gate,
+// pitch: elements from one token's row of q, k, v and of their gradients to the next one's (with saved only)
+static int chunk_bwd_impl(bool saved, const float* rstd_q, const float* rstd_k, int64_t pitch, const void* q, const void* k,
+                          const void* v, const float* cum_gate,
                           const float* beta, const void* aqk, const void* akk,
                           const float* initial_state, const void* d_out,
                           const float* d_final_state, void* dq, void* dk, void* dv, float* dg,
@@ -85,7 +87,7 @@ static int chunk_bwd_impl(bool saved, const float* rstd_q, const float* rstd_k, 
                                 d_final_state, d_initial_state, dhbuf, dv2, cu_seqlens, chunk_offsets,
                                 nseq, heads, tokens, num_chunks, s);
   if (rc) return rc;
-  return kda::launch_bwd_chunk_tc(qb, kb, vb, cum_gate, beta, (const bf16*)akk, hbuf, dhbuf, vnew, dv2,
+  return kda::launch_bwd_chunk_tc(qb, kb, vb, pitch, cum_gate, beta, (const bf16*)akk, hbuf, dhbuf, vnew, dv2,
                                   (const bf16*)d_out, (bf16*)dq, (bf16*)dk, (bf16*)dv, dg, dbeta,
                                   rstd_q, rstd_k, cu_seqlens, chunk_offsets, nseq, heads, tokens,
                                   num_chunks, g_prof_buffer, s);
@@ -102,7 +104,7 @@ static int chunk_bwd_impl(bool saved, const float* rstd_q, const float* rstd_k, 
       d_initial_state, cu_seqlens, chunk_offsets, nseq, tokens, heads, key_dim, value_dim, num_chunks
 
 extern "C" int kda_chunk_bwd(KDA_BWD_ARGS, void* workspace, int64_t workspace_bytes, void* stream) {
-  return chunk_bwd_impl(false, nullptr, nullptr, KDA_BWD_PASS, workspace, workspace_bytes, stream);
+  return chunk_bwd_impl(false, nullptr, nullptr, (int64_t)heads * 128, KDA_BWD_PASS, workspace, workspace_bytes, stream);
 }
 
 // The state-gradient walk of kda_chunk_bwd_saved alone: d_initial_state for the cotangents
@@ -130,7 +132,7 @@ extern "C" int kda_chunk_bwd_state_saved(const float* cum_gate, const void* aqk,
 }
 
 extern "C" int kda_chunk_bwd_saved(KDA_BWD_ARGS, void* saved, int64_t saved_bytes, void* stream) {
-  return chunk_bwd_impl(true, nullptr, nullptr, KDA_BWD_PASS, saved, saved_bytes, stream);
+  return chunk_bwd_impl(true, nullptr, nullptr, (int64_t)heads * 128, KDA_BWD_PASS, saved, saved_bytes, stream);
 }
 
 // Backward of kda_chunk_fwd_qknorm(keep = 1): q and k are the unnormalised rows, rstd_q / rstd_k the
@@ -138,5 +140,21 @@ extern "C" int kda_chunk_bwd_saved(KDA_BWD_ARGS, void* saved, int64_t saved_byte
 extern "C" int kda_chunk_bwd_qknorm_saved(KDA_BWD_ARGS, const float* rstd_q, const float* rstd_k,
                                           void* saved, int64_t saved_bytes, void* stream) {
   if (!rstd_q || !rstd_k) return KDA_ERR_ARG;
-  return chunk_bwd_impl(true, rstd_q, rstd_k, KDA_BWD_PASS, saved, saved_bytes, stream);
+  return chunk_bwd_impl(true, rstd_q, rstd_k, (int64_t)heads * 128, KDA_BWD_PASS, saved, saved_bytes, stream);
+}
+
+// Backward of kda_chunk_fwd_qkv(keep = 1): dqkv takes the gradients in the layout of qkv.
+extern "C" int kda_chunk_bwd_qkv_saved(const void* qkv, const float* cum_gate, const float* beta, const void* aqk,
+                                       const void* akk, const float* initial_state, const void* d_out,
+                                       const float* d_final_state, void* dqkv, float* dg, float* dbeta,
+                                       float* d_initial_state, const float* rstd_q, const float* rstd_k,
+                                       const int32_t* cu_seqlens, const int32_t* chunk_offsets, int nseq, int64_t tokens,
+                                       int heads, int num_chunks, void* saved, int64_t saved_bytes, void* stream) {
+  if (!qkv || !dqkv || !rstd_q || !rstd_k || heads < 1) return KDA_ERR_ARG;
+  const int64_t width = (int64_t)heads * 128;
+  const bf16* q = (const bf16*)qkv;
+  bf16* dq = (bf16*)dqkv;
+  return chunk_bwd_impl(true, rstd_q, rstd_k, 3 * width, q, q + width, q + 2 * width, cum_gate, beta, aqk, akk, initial_state,
+                        d_out, d_final_state, dq, dq + width, dq + 2 * width, dg, dbeta, d_initial_state, cu_seqlens,
+                        chunk_offsets, nseq, tokens, heads, 128, 128, num_chunks, saved, saved_bytes, stream);
 }

@@ -21,6 +21,7 @@ namespace kda {
 constexpr int D = 128;     // K = V
 struct ChunkParams {
   const bf16* q; const bf16* k; const bf16* v; const float* g; const float* beta;
+  int64_t pitch;                        // elements from one token's row of q, k, v to the next one's
   bf16* aqk; bf16* akk;                 // tape [N, H, 64]
   bf16* w; bf16* u; bf16* kg; bf16* qg;  // [N, H, 128]
   float* rstd_q; float* rstd_k; float eps;   // q / k arrive unnormalised when these are set
@@ -35,7 +36,7 @@ struct ChunkParams {
   int chunks;       // chunk capacity: h_out holds chunks * H states (needed only with h_out)
 };
 
-int launch_prepare_tc(const bf16* q, const bf16* k, const bf16* v, const float* g, const float* beta,
+int launch_prepare_tc(const bf16* q, const bf16* k, const bf16* v, int64_t pitch, const float* g, const float* beta,
                       bf16* aqk, bf16* akk, bf16* w, bf16* u, bf16* kg, bf16* qg, float* rstd_q,
                       float* rstd_k, float eps, const int32_t* cu, const int32_t* co, int nseq, int H,
                       int64_t tokens, int chunks, cudaStream_t s);
@@ -47,7 +48,7 @@ int launch_state_fwd_tc(const bf16* w, const bf16* u, const bf16* kg, const bf16
 
 // forward: the whole chunk-parallel part (tape, w, u, kg, qg) in one tcgen05 kernel
 int launch_prepare(const ChunkParams& p, int chunks, cudaStream_t s) {
-  return launch_prepare_tc(p.q, p.k, p.v, p.g, p.beta, p.aqk, p.akk, p.w, p.u, p.kg, p.qg, p.rstd_q,
+  return launch_prepare_tc(p.q, p.k, p.v, p.pitch, p.g, p.beta, p.aqk, p.akk, p.w, p.u, p.kg, p.qg, p.rstd_q,
                            p.rstd_k, p.eps, p.cu_seqlens, p.chunk_offsets, p.nseq, p.H, p.tokens, chunks, s);
 }
 int launch_state_fwd(const ChunkParams& p, cudaStream_t s) {
@@ -63,6 +64,7 @@ int launch_recompute(const void* q, const void* k, const void* v, const float* g
                      int nseq, int H, int chunks, int64_t tokens, cudaStream_t s) {
   ChunkParams p{};
   p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v; p.g = g; p.beta = beta;
+  p.pitch = (int64_t)H * 128;
   p.aqk = (bf16*)aqk; p.akk = (bf16*)akk;
   p.w = (bf16*)w; p.u = (bf16*)u; p.kg = (bf16*)kg; p.qg = (bf16*)qg;
   p.h0 = h0; p.ht = nullptr; p.o = nullptr;
@@ -80,7 +82,8 @@ int launch_recompute(const void* q, const void* k, const void* v, const float* g
 
 using kda::bf16;
 
-static int chunk_fwd_impl(bool keep, float* rstd_q, float* rstd_k, float eps, const void* q, const void* k, const void* v, const float* cum_gate,
+static int chunk_fwd_impl(bool keep, float* rstd_q, float* rstd_k, float eps, int64_t pitch, const void* q, const void* k,
+                             const void* v, const float* cum_gate,
                              const float* beta, const float* initial_state, float* final_state,
                              void* out, void* aqk, void* akk, const int32_t* cu_seqlens,
                              const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
@@ -100,6 +103,7 @@ static int chunk_fwd_impl(bool keep, float* rstd_q, float* rstd_k, float eps, co
   const int64_t nd = tokens * heads * 128;
   bf16* ws = reinterpret_cast<bf16*>(workspace);
   p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v; p.g = cum_gate; p.beta = beta;
+  p.pitch = pitch;
   p.aqk = (bf16*)aqk; p.akk = (bf16*)akk;
   p.w = ws; p.u = ws + nd; p.kg = ws + 2 * nd; p.qg = ws + 3 * nd;
   p.rstd_q = rstd_q; p.rstd_k = rstd_k; p.eps = eps;
@@ -124,7 +128,7 @@ extern "C" int kda_chunk_fwd(const void* q, const void* k, const void* v, const 
                              const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
                              int key_dim, int value_dim, int num_chunks, void* workspace,
                              int64_t workspace_bytes, void* stream) {
-  return chunk_fwd_impl(false, nullptr, nullptr, 0.f, q, k, v, cum_gate, beta, initial_state, final_state,
+  return chunk_fwd_impl(false, nullptr, nullptr, 0.f, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state, final_state,
                         out, aqk, akk, cu_seqlens, chunk_offsets, nseq, tokens, heads, key_dim, value_dim,
                         num_chunks, workspace, workspace_bytes, stream);
 }
@@ -140,7 +144,7 @@ extern "C" int kda_chunk_fwd_qknorm(const void* q, const void* k, const void* v,
                                     int num_chunks, void* workspace, int64_t workspace_bytes, int keep,
                                     void* stream) {
   if (!rstd_q || !rstd_k || !(eps >= 0.f)) return KDA_ERR_ARG;
-  return chunk_fwd_impl(keep != 0, rstd_q, rstd_k, eps, q, k, v, cum_gate, beta, initial_state,
+  return chunk_fwd_impl(keep != 0, rstd_q, rstd_k, eps, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state,
                         final_state, out, aqk, akk, cu_seqlens, chunk_offsets, nseq, tokens, heads,
                         key_dim, value_dim, num_chunks, workspace, workspace_bytes, stream);
 }
@@ -151,7 +155,7 @@ extern "C" int kda_chunk_fwd_save(const void* q, const void* k, const void* v, c
                                   const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
                                   int key_dim, int value_dim, int num_chunks, void* saved,
                                   int64_t saved_bytes, void* stream) {
-  return chunk_fwd_impl(true, nullptr, nullptr, 0.f, q, k, v, cum_gate, beta, initial_state, final_state,
+  return chunk_fwd_impl(true, nullptr, nullptr, 0.f, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state, final_state,
                         out, aqk, akk, cu_seqlens, chunk_offsets, nseq, tokens, heads, key_dim, value_dim,
                         num_chunks, saved, saved_bytes, stream);
 }
@@ -178,6 +182,7 @@ extern "C" int kda_chunk_fwd_prepare(const void* q, const void* k, const void* v
   const int64_t nd = tokens * heads * 128;
   bf16* ws = reinterpret_cast<bf16*>(workspace);
   p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v; p.g = cum_gate; p.beta = beta;
+  p.pitch = (int64_t)heads * 128;
   p.aqk = (bf16*)aqk; p.akk = (bf16*)akk;
   p.w = ws; p.u = ws + nd; p.kg = ws + 2 * nd; p.qg = ws + 3 * nd;
   p.cu_seqlens = cu_seqlens; p.chunk_offsets = chunk_offsets; p.nseq = nseq; p.H = heads;
@@ -344,8 +349,8 @@ extern "C" int64_t kda_chunk_fwd_dense_workspace_bytes(int batch, int64_t tokens
   return kda::dense_scratch(keep != 0, batch, tokens_per_row, heads, kda::plan_dense(batch, tokens_per_row, heads)).end;
 }
 
-static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float eps, const void* q, const void* k, const void* v,
-                                const float* cum_gate, const float* beta, const float* initial_state,
+static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float eps, int64_t pitch, const void* q,
+                                const void* k, const void* v, const float* cum_gate, const float* beta, const float* initial_state,
                                 float* final_state, void* out, void* aqk, void* akk, int batch,
                                 int64_t tokens_per_row, int heads, int key_dim, int value_dim,
                                 void* workspace, int64_t workspace_bytes, void* stream) {
@@ -372,6 +377,7 @@ static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float e
   const int64_t nd = total * heads * 128;
   bf16* ws = reinterpret_cast<bf16*>(workspace);
   p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v; p.g = cum_gate; p.beta = beta;
+  p.pitch = pitch;
   p.aqk = (bf16*)aqk; p.akk = (bf16*)akk;
   p.w = ws; p.u = ws + nd; p.kg = ws + 2 * nd; p.qg = ws + 3 * nd;
   p.rstd_q = rstd_q; p.rstd_k = rstd_k; p.eps = eps;
@@ -427,7 +433,7 @@ extern "C" int kda_chunk_fwd_dense(const void* q, const void* k, const void* v, 
                                    void* out, void* aqk, void* akk, int batch, int64_t tokens_per_row,
                                    int heads, int key_dim, int value_dim, void* workspace,
                                    int64_t workspace_bytes, void* stream) {
-  return chunk_fwd_dense_impl(false, nullptr, nullptr, 0.f, q, k, v, cum_gate, beta, initial_state, final_state, out, aqk, akk,
+  return chunk_fwd_dense_impl(false, nullptr, nullptr, 0.f, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state, final_state, out, aqk, akk,
                               batch, tokens_per_row, heads, key_dim, value_dim, workspace,
                               workspace_bytes, stream);
 }
@@ -438,7 +444,7 @@ extern "C" int kda_chunk_fwd_dense_save(const void* q, const void* k, const void
                                         void* aqk, void* akk, int batch, int64_t tokens_per_row,
                                         int heads, int key_dim, int value_dim, void* saved,
                                         int64_t saved_bytes, void* stream) {
-  return chunk_fwd_dense_impl(true, nullptr, nullptr, 0.f, q, k, v, cum_gate, beta, initial_state, final_state, out, aqk, akk,
+  return chunk_fwd_dense_impl(true, nullptr, nullptr, 0.f, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state, final_state, out, aqk, akk,
                               batch, tokens_per_row, heads, key_dim, value_dim, saved, saved_bytes,
                               stream);
 }
@@ -451,8 +457,28 @@ extern "C" int kda_chunk_fwd_dense_qknorm(const void* q, const void* k, const vo
                                           int batch, int64_t tokens_per_row, int heads, int key_dim, int value_dim,
                                           void* workspace, int64_t workspace_bytes, int keep, void* stream) {
   if (!rstd_q || !rstd_k || !(eps >= 0.f)) return KDA_ERR_ARG;
-  return chunk_fwd_dense_impl(keep != 0, rstd_q, rstd_k, eps, q, k, v, cum_gate, beta, initial_state, final_state,
+  return chunk_fwd_dense_impl(keep != 0, rstd_q, rstd_k, eps, (int64_t)heads * 128, q, k, v, cum_gate, beta, initial_state, final_state,
                               out, aqk, akk, batch, tokens_per_row, heads, key_dim, value_dim, workspace,
+                              workspace_bytes, stream);
+}
+
+// kda_chunk_fwd_qknorm (cu_seqlens given) or kda_chunk_fwd_dense_qknorm (cu_seqlens NULL: nseq rows of tokens / nseq
+// tokens) on rows of [q | k | v], 3 * heads * 128 elements a token, as a projection or a convolution leaves them.
+extern "C" int kda_chunk_fwd_qkv(const void* qkv, const float* cum_gate, const float* beta, const float* initial_state,
+                                 float* final_state, void* out, void* aqk, void* akk, float* rstd_q, float* rstd_k,
+                                 float eps, const int32_t* cu_seqlens, const int32_t* chunk_offsets, int nseq,
+                                 int64_t tokens, int heads, int num_chunks, void* workspace, int64_t workspace_bytes,
+                                 int keep, void* stream) {
+  if (!qkv || !rstd_q || !rstd_k || !(eps >= 0.f) || nseq < 1 || heads < 1 || tokens < 1) return KDA_ERR_ARG;
+  const int64_t width = (int64_t)heads * 128;
+  const bf16 *q = (const bf16*)qkv, *k = q + width, *v = k + width;
+  if (cu_seqlens)
+    return chunk_fwd_impl(keep != 0, rstd_q, rstd_k, eps, 3 * width, q, k, v, cum_gate, beta, initial_state, final_state,
+                          out, aqk, akk, cu_seqlens, chunk_offsets, nseq, tokens, heads, 128, 128, num_chunks, workspace,
+                          workspace_bytes, stream);
+  if (tokens % nseq) return KDA_ERR_ARG;
+  return chunk_fwd_dense_impl(keep != 0, rstd_q, rstd_k, eps, 3 * width, q, k, v, cum_gate, beta, initial_state,
+                              final_state, out, aqk, akk, nseq, tokens / nseq, heads, 128, 128, workspace,
                               workspace_bytes, stream);
 }
 

@@ -710,15 +710,17 @@ static __device__ int g_prepare_error = 0;
 
 long long* debug_profile_buffer();
 
-int launch_prepare_tc(const bf16* q, const bf16* k, const bf16* v, const float* g, const float* beta,
+// pitch: elements from one token's row of q, k, v to the next one's
+int launch_prepare_tc(const bf16* q, const bf16* k, const bf16* v, int64_t pitch, const float* g, const float* beta,
                       bf16* aqk, bf16* akk, bf16* w, bf16* u, bf16* kg, bf16* qg, float* rstd_q,
                       float* rstd_k, float eps, const int32_t* cu, const int32_t* co, int nseq, int H,
                       int64_t tokens, int chunks, cudaStream_t s) {
   if (chunks == 0) return KDA_OK;
   PrepParams p;
   const int64_t cols = (int64_t)H * 128;
-  bool ok = make_tensor_map(&p.tm_q, q, tokens, cols, 64) && make_tensor_map(&p.tm_k, k, tokens, cols, 64) &&
-            make_tensor_map(&p.tm_v, v, tokens, cols, 64) && make_tensor_map(&p.tm_g, g, tokens, cols, 64, true) &&
+  bool ok = make_tensor_map(&p.tm_q, q, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_k, k, tokens, cols, 64, false, pitch) &&
+            make_tensor_map(&p.tm_v, v, tokens, cols, 64, false, pitch) && make_tensor_map(&p.tm_g, g, tokens, cols, 64, true) &&
             make_tensor_map(&p.tm_w, w, tokens, cols, 64) && make_tensor_map(&p.tm_u, u, tokens, cols, 64);
   // the other results are written with plain 16-byte stores
   if (!ok || (((uintptr_t)qg | (uintptr_t)kg | (uintptr_t)aqk | (uintptr_t)akk) & 15) != 0) return KDA_ERR_LAUNCH;

@@ -305,14 +305,15 @@ inline EncodeTiledFn encode_tiled_fn() {
 }
 
 // Row-major [rows x cols] tensor of 2-byte (bf16) or 4-byte (fp32) elements; boxes of
-// [box_rows x 128 bytes] with the 128-byte swizzle; out-of-range rows read as zero.
+// [box_rows x 128 bytes] with the 128-byte swizzle; out-of-range rows read as zero.  pitch: elements from one row
+// to the next (0 = cols).
 inline bool make_tensor_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols,
-                            int box_rows, bool fp32 = false) {
+                            int box_rows, bool fp32 = false, int64_t pitch = 0) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return false;
   const int esz = fp32 ? 4 : 2;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * esz};
+  cuuint64_t strides[1] = {(cuuint64_t)(pitch ? pitch : cols) * esz};
   cuuint32_t box[2] = {(cuuint32_t)(128 / esz), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,

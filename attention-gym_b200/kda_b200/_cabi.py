@@ -59,6 +59,9 @@ _SIGNATURES = {
                                    c_void_p, c_int64, c_void_p]),
     "kda_chunk_fwd_qknorm": (c_int, [c_void_p] * 12 + [c_float, c_void_p, c_void_p, c_int, c_int64, c_int,
                                      c_int, c_int, c_int, c_void_p, c_int64, c_int, c_void_p]),
+    "kda_chunk_fwd_qkv": (c_int, [c_void_p] * 10 + [c_float, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p,
+                                  c_int64, c_int, c_void_p]),
+    "kda_chunk_bwd_qkv_saved": (c_int, [c_void_p] * 16 + [c_int, c_int64, c_int, c_int, c_void_p, c_int64, c_void_p]),
     "kda_chunk_bwd_qknorm_saved": (c_int, [c_void_p] * 18 + [c_int, c_int64, c_int, c_int, c_int, c_int,
                                            c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
     "kda_chunk_fwd_noalloc": (c_int, [c_void_p] * 12 + [c_int, c_int64, c_int, c_int, c_int, c_int,

@@ -106,6 +106,45 @@ class _ChunkKDAQKNorm(torch.autograd.Function):
         return dq, dk, dv, dg, db, (dh0 if initial_state is not None else None), None, None, None, None
 
 
+class _ChunkKDAQKV(torch.autograd.Function):
+    """_ChunkKDAQKNorm on one tensor ``[B, T, 3, H, 128]`` of q, k and v rows."""
+
+    @staticmethod
+    def forward(ctx, qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, output_final_state, eps):
+        keep = any(ctx.needs_input_grad[:4])
+        out, state, aqk, akk, saved, rstd_q, rstd_k = ops.chunk_fwd_qkv_op(
+            qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, output_final_state, keep, eps)
+        ctx.save_for_backward(qkv, gate, beta, aqk, akk, initial_state, cu_seqlens, chunk_offsets, saved,
+                              rstd_q, rstd_k)
+        ctx.set_materialize_grads(False)
+        return (out, state) if output_final_state else out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, d_output, d_final_state=None):
+        (qkv, gate, beta, aqk, akk, initial_state, cu_seqlens, chunk_offsets, saved, rstd_q,
+         rstd_k) = ctx.saved_tensors
+        dqkv, dg, db, dh0 = ops.chunk_bwd_qkv_op(
+            qkv, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_seqlens, chunk_offsets, d_output, d_final_state,
+            initial_state, initial_state is not None)
+        return dqkv, dg, db, (dh0 if initial_state is not None else None), None, None, None, None
+
+
+def chunk_forward_qkv(qkv, cumulative_gate, beta, initial_state=None, *, metadata: RaggedChunkMetadata | None = None,
+                      output_final_state=False, norm_eps=1e-6):
+    """``chunk_forward(normalize_qk=True)`` on the rows ``[B, T, 3, H, 128]`` (bf16) of a fused projection, without
+    copies of q, k and v."""
+    cu = offsets = None
+    if metadata is not None:
+        metadata.validate_chunk_size(_CHUNK)
+        cu, offsets = metadata.cu_seqlens, metadata.chunk_offsets
+    if initial_state is not None:
+        initial_state = initial_state.float().contiguous()
+    res = _ChunkKDAQKV.apply(qkv, cumulative_gate.float().contiguous(), beta.float().contiguous(), initial_state, cu,
+                             offsets, bool(output_final_state), float(norm_eps))
+    return res if output_final_state else (res, None)
+
+
 def chunk_forward(q, k, v, cumulative_gate, beta, initial_state=None, *, cu_seqlens=None,
                   metadata: RaggedChunkMetadata | None = None, output_final_state=False,
                   fastmath=False, autotune=True, recompute=False, normalize_qk=False,
@@ -143,4 +182,4 @@ def chunk_forward(q, k, v, cumulative_gate, beta, initial_state=None, *, cu_seql
     return out.reshape(out_shape).to(out_dtype), state
 
 
-__all__ = ["chunk_forward"]
+__all__ = ["chunk_forward", "chunk_forward_qkv"]

@@ -32,7 +32,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .chunk_schedule import prepare_ragged_chunk_metadata
-from .fused import chunk_forward as _chunk_kda
+from .fused import chunk_forward as _chunk_kda, chunk_forward_qkv as _chunk_kda_qkv
 from .masking import active_token_mask, mask_inactive_token_gradients, mask_inactive_tokens
 from .preops import _bounded_gate_cumsum, causal_conv1d, gated_output_norm, l2norm
 from .reference_impl import reference_kda
@@ -165,24 +165,28 @@ class KDAAttention(nn.Module):
         qkv, final_conv_state = self.short_convolution(qkv, initial_conv_state, cu_seqlens=cu_seqlens,
                                                        return_final_state=return_final_state)
         qkv = mask_inactive_tokens(qkv, mask)
-        q, k, v = qkv.view(batch, tokens, 3, self.num_heads, self.head_dim).unbind(2)
+        qkv = qkv.view(batch, tokens, 3, self.num_heads, self.head_dim)
         raw_gate, beta = self.gate_projections(hidden)
         raw_gate = mask_inactive_token_gradients(raw_gate, mask)
         beta = mask_inactive_token_gradients(beta, mask)
         if self.backend == "reference":
-            out, final_state = self._reference_core(q, k, v, raw_gate, beta, initial_state,
+            out, final_state = self._reference_core(*qkv.unbind(2), raw_gate, beta, initial_state,
                                                     return_final_state)
         else:
-            if not self.fuse_qk_norm:
-                q, k = l2norm(q.contiguous()), l2norm(k.contiguous())
             metadata = (None if cu_seqlens is None
                         else prepare_ragged_chunk_metadata(cu_seqlens, tokens, self.chunk_size))
             gate = _bounded_gate_cumsum(raw_gate, self.A_log, self.dt_bias, chunk_size=self.chunk_size,
                                         lower_bound=self.lower_bound, fastmath=self.fastmath,
                                         metadata=metadata)
-            out, final_state = _chunk_kda(q, k, v.contiguous(), gate, beta, initial_state,
-                                          metadata=metadata, output_final_state=return_final_state,
-                                          fastmath=self.fastmath, normalize_qk=self.fuse_qk_norm)
+            if self.fuse_qk_norm:
+                out, final_state = _chunk_kda_qkv(qkv, gate, beta, initial_state, metadata=metadata,
+                                                  output_final_state=return_final_state)
+            else:
+                q, k, v = qkv.unbind(2)
+                q, k = l2norm(q.contiguous()), l2norm(k.contiguous())
+                out, final_state = _chunk_kda(q, k, v.contiguous(), gate, beta, initial_state,
+                                              metadata=metadata, output_final_state=return_final_state,
+                                              fastmath=self.fastmath)
         out = mask_inactive_tokens(out, mask)
         logits = self._linear(self._linear(hidden, self.g_a_proj), self.g_b_proj).view_as(out)
         if self.backend == "fused":

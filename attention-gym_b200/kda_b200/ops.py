@@ -125,6 +125,17 @@ _lib_own.define("decode_step(Tensor x, Tensor weight, Tensor(a!) conv_state, Ten
                 "Tensor state_indices, Tensor raw_gate, Tensor A_log, Tensor dt_bias, Tensor beta, "
                 "str? activation, float lower_bound, float eps) -> Tensor")
 
+# What KDAAttention needs beside the public calls: the chunked pair with normalisation on rows of q | k | v.
+_NS_LAYER = "kda_b200_layer"
+_lib_layer = torch.library.Library(_NS_LAYER, "DEF")
+_lib_layer.define("chunk_fwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta, Tensor? initial_state, "
+                "Tensor? cu_seqlens, Tensor? chunk_offsets, bool want_state, bool keep, float eps) "
+                "-> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)")
+_lib_layer.define("chunk_bwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta, Tensor Aqk, Tensor Akk, "
+                "Tensor(a!) saved, Tensor rstd_q, Tensor rstd_k, Tensor? cu_seqlens, Tensor? chunk_offsets, "
+                "Tensor? d_output, Tensor? d_final_state, Tensor? initial_state, bool want_state_grad) "
+                "-> (Tensor, Tensor, Tensor, Tensor)")
+
 
 def _require_cuda(t: torch.Tensor, what: str):
     if not t.is_cuda:
@@ -389,6 +400,100 @@ def _chunk_bwd_qknorm(q, k, v, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_s
     if dh0 is None:
         dh0 = torch.empty(0, dtype=torch.float32, device=q.device)
     return dq, dk, dv, dg, db, dh0
+
+
+# The two operators above on one tensor [B, T, 3, H, 128] of q, k and v rows, as the layer's convolution leaves them:
+# no copies of q, k and v, and their gradients come back in one tensor of the same layout.
+@torch.library.impl(_lib_layer, "chunk_fwd_qkv", "CUDA")
+def _chunk_fwd_qkv(qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state, keep, eps):
+    _require_cuda(qkv, "the fused KDA core")
+    if qkv.ndim != 5 or qkv.shape[2] != 3 or qkv.shape[4] != 128:
+        raise ValueError("expected qkv [B, T, 3, H, 128]")
+    if qkv.dtype != torch.bfloat16:
+        raise TypeError("the fused KDA core takes bfloat16 q, k, v")
+    batch, tokens, _, heads, _ = qkv.shape
+    packed = cu_seqlens is not None
+    nseq, capacity = batch, 0
+    if packed:
+        if batch != 1:
+            raise ValueError("packed cu_seqlens require batch size one")
+        nseq = cu_seqlens.shape[0] - 1
+        capacity = chunk_capacity(tokens, nseq, _CHUNK)
+    qkv, gate, beta = qkv.contiguous(), gate.float().contiguous(), beta.float().contiguous()
+    if initial_state is not None:
+        initial_state = initial_state.float().contiguous()
+    alloc = torch.zeros if packed else torch.empty
+    out = alloc(batch, tokens, heads, 128, dtype=qkv.dtype, device=qkv.device)
+    aqk = torch.empty(batch, tokens, heads, _CHUNK, dtype=qkv.dtype, device=qkv.device)
+    akk = torch.empty_like(aqk)
+    rstd_q = alloc(batch, tokens, heads, dtype=torch.float32, device=qkv.device)
+    rstd_k = alloc(batch, tokens, heads, dtype=torch.float32, device=qkv.device)
+    state = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=qkv.device)
+             if want_state else qkv.new_empty((0,), dtype=torch.float32))
+    ws_bytes = _fwd_workspace_bytes(batch, tokens, heads, nseq if packed else None, keep)
+    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=qkv.device)
+    _cabi.call("kda_chunk_fwd_qkv", 3, _cabi.ptr(qkv), _cabi.ptr(gate), _cabi.ptr(beta), _cabi.ptr(initial_state),
+               _cabi.ptr(state) if want_state else None, _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk),
+               _cabi.ptr(rstd_q), _cabi.ptr(rstd_k), float(eps), _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets), nseq,
+               batch * tokens, heads, capacity, _cabi.ptr(workspace), ws_bytes, int(keep), _cabi.stream())
+    return out, state, aqk, akk, workspace, rstd_q, rstd_k
+
+
+@torch.library.impl(_lib_layer, "chunk_bwd_qkv", "CUDA")
+def _chunk_bwd_qkv(qkv, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_seqlens, chunk_offsets, d_output,
+                   d_final_state, initial_state, want_state_grad):
+    batch, tokens, _, heads, _ = qkv.shape
+    packed = cu_seqlens is not None
+    if packed:
+        nseq = cu_seqlens.shape[0] - 1
+        capacity = chunk_capacity(tokens, nseq, _CHUNK)
+        cu_ptr, chunks_ptr = _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets)
+    else:
+        nseq = batch
+        offsets, cu_ptr, chunks_ptr, capacity = _dense_offsets(qkv)
+    total = batch * tokens
+    qkv, gate, beta = qkv.contiguous(), gate.float().contiguous(), beta.float().contiguous()
+    rstd_q, rstd_k = rstd_q.contiguous(), rstd_k.contiguous()
+    if d_output is None:
+        d_output = torch.zeros(batch, tokens, heads, 128, dtype=qkv.dtype, device=qkv.device)
+    d_output = d_output.to(torch.bfloat16).contiguous()
+    if d_final_state is not None:
+        d_final_state = d_final_state.float().contiguous()
+    if initial_state is not None:
+        initial_state = initial_state.float().contiguous()
+    alloc = torch.zeros_like if packed else torch.empty_like
+    dqkv, dg, db = alloc(qkv), alloc(gate), alloc(beta)
+    dh0 = torch.empty((nseq, heads, 128, 128) if want_state_grad else (0,), dtype=torch.float32, device=qkv.device)
+    ws_bytes = _cabi.lib().kda_chunk_bwd_workspace_bytes(total, heads, capacity)
+    if saved.numel() < ws_bytes or saved.dtype != torch.uint8 or not saved.is_cuda:
+        raise ValueError("`saved` is not the buffer chunk_fwd_qkv returned for these shapes")
+    _cabi.call("kda_chunk_bwd_qkv_saved", 2, _cabi.ptr(qkv), _cabi.ptr(gate), _cabi.ptr(beta), _cabi.ptr(aqk),
+               _cabi.ptr(akk), _cabi.ptr(initial_state), _cabi.ptr(d_output), _cabi.ptr(d_final_state), _cabi.ptr(dqkv),
+               _cabi.ptr(dg), _cabi.ptr(db), _cabi.ptr(dh0) if want_state_grad else None, _cabi.ptr(rstd_q),
+               _cabi.ptr(rstd_k), cu_ptr, chunks_ptr, nseq, total, heads, capacity, _cabi.ptr(saved), ws_bytes,
+               _cabi.stream())
+    return dqkv, dg, db, dh0
+
+
+@torch.library.register_fake(f"{_NS_LAYER}::chunk_fwd_qkv")
+def _(qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state, keep, eps):
+    batch, tokens, _, heads, _ = qkv.shape
+    nseq = batch if cu_seqlens is None else cu_seqlens.shape[0] - 1
+    state = qkv.new_empty((nseq, heads, 128, 128) if want_state else (0,), dtype=torch.float32)
+    nbytes = _fwd_workspace_bytes(batch, tokens, heads, None if cu_seqlens is None else nseq, keep)
+    tape = qkv.new_empty((batch, tokens, heads, _CHUNK))
+    rstd = qkv.new_empty((batch, tokens, heads), dtype=torch.float32)
+    return (qkv.new_empty((batch, tokens, heads, 128)), state, tape, torch.empty_like(tape),
+            qkv.new_empty((nbytes,), dtype=torch.uint8), rstd, torch.empty_like(rstd))
+
+
+@torch.library.register_fake(f"{_NS_LAYER}::chunk_bwd_qkv")
+def _(qkv, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_seqlens, chunk_offsets, d_output, d_final_state,
+      initial_state, want_state_grad):
+    nseq = qkv.shape[0] if cu_seqlens is None else cu_seqlens.shape[0] - 1
+    return (qkv.new_empty(qkv.shape), gate.new_empty(gate.shape, dtype=torch.float32),
+            beta.new_empty(beta.shape, dtype=torch.float32),
+            qkv.new_empty((nseq, qkv.shape[3], 128, 128) if want_state_grad else (0,), dtype=torch.float32))
 
 
 @torch.library.register_fake(f"{_NS}::kda_chunk_fwd_qknorm")
@@ -867,6 +972,8 @@ chunk_fwd_qknorm_op = _ops.kda_chunk_fwd_qknorm.default
 chunk_bwd_qknorm_op = _ops.kda_chunk_bwd_qknorm.default
 chunk_bwd_op = _ops.kda_chunk_bwd.default
 chunk_bwd_with_state_grad_op = _ops.kda_chunk_bwd_with_state_grad.default
+chunk_fwd_qkv_op = torch.ops.kda_b200_layer.chunk_fwd_qkv.default
+chunk_bwd_qkv_op = torch.ops.kda_b200_layer.chunk_bwd_qkv.default
 chunk_scan_op = torch.ops.kda_b200_fused.chunk_scan.default
 decode_step_op = torch.ops.kda_b200_fused.decode_step.default
 recurrent_fwd_op = _ops.kda_recurrent_fwd.default

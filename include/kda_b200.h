@@ -287,6 +287,19 @@ int kda_chunk_bwd_qknorm_saved(const void* q, const void* k, const void* v, cons
                                int key_dim, int value_dim, int num_chunks, const float* rstd_q,
                                const float* rstd_k, void* saved, int64_t saved_bytes, void* stream);
 
+/* The same pair on rows of [q | k | v], 3 * heads * 128 elements a token, as a fused projection leaves them; dqkv takes
+ * the gradients in that layout.  cu_seqlens NULL: nseq dense rows of tokens / nseq tokens (forward; the backward pass
+ * takes the offsets of kda_dense_offsets), with the workspace of kda_chunk_fwd_dense. */
+int kda_chunk_fwd_qkv(const void* qkv, const float* cum_gate, const float* beta, const float* initial_state,
+                      float* final_state, void* out, void* aqk, void* akk, float* rstd_q, float* rstd_k, float eps,
+                      const int32_t* cu_seqlens, const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
+                      int num_chunks, void* workspace, int64_t workspace_bytes, int keep, void* stream);
+int kda_chunk_bwd_qkv_saved(const void* qkv, const float* cum_gate, const float* beta, const void* aqk, const void* akk,
+                            const float* initial_state, const void* d_out, const float* d_final_state, void* dqkv,
+                            float* dg, float* dbeta, float* d_initial_state, const float* rstd_q, const float* rstd_k,
+                            const int32_t* cu_seqlens, const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
+                            int num_chunks, void* saved, int64_t saved_bytes, void* stream);
+
 /* The packed description of a dense [batch, tokens] input: cu_seqlens [batch + 1] and, right behind it,
  * chunk_offsets [batch + 1] (int32, on the device). */
 int kda_dense_offsets(void* offsets, int batch, int tokens, void* stream);
