@@ -211,6 +211,23 @@ __global__ void __launch_bounds__(256) out_gate_bwd_kernel(const void* x, const 
   }
 }
 
+// 16-bit values as fp32: the gradient of a weight that was cast down for its GEMM, on the way back to the fp32
+// parameter.  Bound by memory, 6 B per element: four elements per access, so that the 16-byte stores of a warp lie side by
+// side, and eight loads per thread ahead of their stores.
+__global__ void __launch_bounds__(256) widen_kernel(const uint2* __restrict__ x, int dt, float4* __restrict__ y, int64_t n4) {
+  const int64_t i0 = (int64_t)blockIdx.x * 2048 + threadIdx.x;
+  uint2 raw[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (i0 + 256 * j < n4) raw[j] = x[i0 + 256 * j];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (i0 + 256 * j < n4)
+      y[i0 + 256 * j] = make_float4(raw_to_float(raw[j].x & 0xffff, dt), raw_to_float(raw[j].x >> 16, dt),
+                                    raw_to_float(raw[j].y & 0xffff, dt), raw_to_float(raw[j].y >> 16, dt));
+  }
+}
+
 static bool epilogue_vec_ok(int dtype, int dim, const void* a, const void* b, const void* c,
                             const void* d, const void* e) {
   const uintptr_t bits = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e;
@@ -271,5 +288,16 @@ extern "C" int kda_output_gate_bwd(const void* o, const void* gate_logits, const
     kda::out_gate_bwd_kernel<<<blocks, 256, 0, s>>>(o, gate_logits, dy, weight, dtype, d_o, d_logits,
                                                     dw_partial, rows, dim, eps);
   }
+  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
+extern "C" int kda_widen(const void* x, int dtype, float* y, int64_t n, void* stream) {
+  if (!x || !y || n < 0 || dtype == KDA_F32) return KDA_ERR_ARG;
+  if (n % 8 || (((uintptr_t)x | (uintptr_t)y) & 15) != 0) return KDA_ERR_UNSUPPORTED;
+  const int64_t n4 = n / 4, blocks = (n4 + 2047) / 2048;
+  if (n == 0) return KDA_OK;
+  if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
+  kda::widen_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const uint2*>(x), dtype, reinterpret_cast<float4*>(y), n4);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }

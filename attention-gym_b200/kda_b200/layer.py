@@ -34,10 +34,26 @@ import torch.nn.functional as F
 from .chunk_schedule import prepare_ragged_chunk_metadata
 from .fused import chunk_forward as _chunk_kda, chunk_forward_qkv as _chunk_kda_qkv
 from .masking import active_token_mask, mask_inactive_token_gradients, mask_inactive_tokens
+from .ops import widen_op
 from .preops import _bounded_gate_cumsum, causal_conv1d, gated_output_norm, l2norm
 from .reference_impl import reference_kda
 
 _LOG2E = math.log2(math.e)
+
+
+class _CastWeight(torch.autograd.Function):
+    """``weight.to(torch.bfloat16)`` of an fp32 parameter (fused backend); the same values both ways.  The gradient goes
+    back to fp32 in a streaming kernel: 50 M elements take 46 us, the copy kernel behind ``.to`` 138."""
+
+    @staticmethod
+    def forward(ctx, weight):
+        return weight.to(torch.bfloat16)
+
+    @staticmethod
+    def backward(ctx, grad):
+        if torch.is_grad_enabled():            # to be differentiated once more
+            return grad.to(torch.float32)
+        return widen_op(grad)
 
 
 class KDAAttentionOutput(NamedTuple):
@@ -97,7 +113,11 @@ class KDAAttention(nn.Module):
 
     # ---- stages -------------------------------------------------------------------------------
     def _linear(self, x, layer):
-        return F.linear(x, layer.weight.to(self.compute_dtype))
+        weight = layer.weight
+        if (self.backend == "fused" and type(weight) is nn.Parameter and weight.is_cuda and weight.requires_grad
+                and weight.dtype == torch.float32 and torch.is_grad_enabled()):
+            return F.linear(x, _CastWeight.apply(weight))
+        return F.linear(x, weight.to(self.compute_dtype))
 
     def short_convolution(self, qkv, initial_state, *, cu_seqlens=None, return_final_state=False):
         batch, tokens, channels = qkv.shape

@@ -125,7 +125,8 @@ _lib_own.define("decode_step(Tensor x, Tensor weight, Tensor(a!) conv_state, Ten
                 "Tensor state_indices, Tensor raw_gate, Tensor A_log, Tensor dt_bias, Tensor beta, "
                 "str? activation, float lower_bound, float eps) -> Tensor")
 
-# What KDAAttention needs beside the public calls: the chunked pair with normalisation on rows of q | k | v.
+# What KDAAttention needs beside the public calls: the chunked pair with normalisation on rows of q | k | v, and a weight
+# gradient's way back.
 _NS_LAYER = "kda_b200_layer"
 _lib_layer = torch.library.Library(_NS_LAYER, "DEF")
 _lib_layer.define("chunk_fwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta, Tensor? initial_state, "
@@ -135,6 +136,8 @@ _lib_layer.define("chunk_bwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta
                 "Tensor(a!) saved, Tensor rstd_q, Tensor rstd_k, Tensor? cu_seqlens, Tensor? chunk_offsets, "
                 "Tensor? d_output, Tensor? d_final_state, Tensor? initial_state, bool want_state_grad) "
                 "-> (Tensor, Tensor, Tensor, Tensor)")
+# A 16-bit tensor as fp32 (the gradient of a weight that was cast for its GEMM).
+_lib_layer.define("widen(Tensor x) -> Tensor")
 
 
 def _require_cuda(t: torch.Tensor, what: str):
@@ -910,6 +913,21 @@ def _decode_prep(x, weight, conv_state, state_indices, raw_gate, A_log, dt_bias,
     return q, k, v, gate
 
 
+@torch.library.impl(_lib_layer, "widen", "CUDA")
+def _widen(x):
+    x = x.contiguous()
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    if x.dtype == torch.float32 or x.numel() == 0 or x.numel() % 8 or x.data_ptr() % 16:
+        return out.copy_(x)
+    _cabi.call("kda_widen", 1, x.data_ptr(), _cabi.dt(x), out.data_ptr(), x.numel(), _cabi.stream())
+    return out
+
+
+@torch.library.register_fake(f"{_NS_LAYER}::widen")
+def _(x):
+    return x.new_empty(x.shape, dtype=torch.float32)
+
+
 @torch.library.impl(_lib_own, "decode_step", "CUDA")
 def _decode_step(x, weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta, activation,
                  lower_bound, eps):
@@ -974,6 +992,7 @@ chunk_bwd_op = _ops.kda_chunk_bwd.default
 chunk_bwd_with_state_grad_op = _ops.kda_chunk_bwd_with_state_grad.default
 chunk_fwd_qkv_op = torch.ops.kda_b200_layer.chunk_fwd_qkv.default
 chunk_bwd_qkv_op = torch.ops.kda_b200_layer.chunk_bwd_qkv.default
+widen_op = torch.ops.kda_b200_layer.widen.default
 chunk_scan_op = torch.ops.kda_b200_fused.chunk_scan.default
 decode_step_op = torch.ops.kda_b200_fused.decode_step.default
 recurrent_fwd_op = _ops.kda_recurrent_fwd.default

@@ -381,6 +381,9 @@ int kda_conv1d_decode(const void* x, const void* weight, void* state, const int3
                       void* y, int dtype, int nseq, int num_slots, int channels, int width,
                       int activation, void* stream);
 
+/* y = x as fp32, n values of a 16-bit dtype (n a multiple of 8, both addresses 16-byte aligned). */
+int kda_widen(const void* x, int dtype, float* y, int64_t n, void* stream);
+
 /* Decode-step preprocessing in one launch: the q | k | v projection x [N, 3 * H * 128] goes through the
  * depthwise causal convolution over the paged history conv_state [num_slots, W-1, 3 * H * 128] (advanced
  * in place; conv_state_indices as for kda_conv1d_decode, NULL = slot i for sequence i) and the
