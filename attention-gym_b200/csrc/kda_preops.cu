@@ -196,14 +196,17 @@ __global__ void __launch_bounds__(128) gate_cumsum_fwd_kernel(const GateParams p
   }
 }
 
-constexpr int kGateBwdGroup = 4;   // chunks per block of the backward kernel = chunks per partial row
+// Chunks per block of the backward kernel = chunks per partial row: few chunks are spread over more blocks, many cost
+// partial rows and their reduction.  us of both kernels with 1 / 2 / 4 chunks a block: 32 heads, 64 chunks 33 / 41 / 62, 128 chunks
+// 65 / 56 / 71, 256 chunks 110 / 107 / 100; 4 heads, 64 chunks 19 / 27 / 47, 256 34 / 34 / 52, 512 62 / 53 / 67, 1024 122 / 84 / 85.
+static int gate_bwd_group(int64_t num_chunks) { return num_chunks <= 96 ? 1 : (num_chunks <= 192 ? 2 : 4); }
 
-__global__ void __launch_bounds__(128) gate_cumsum_bwd_kernel(const GateParams p, int num_chunks) {
+__global__ void __launch_bounds__(128) gate_cumsum_bwd_kernel(const GateParams p, int num_chunks, int group) {
   const int HK = p.H * p.K;
   const int f0 = (blockIdx.y * 128 + threadIdx.x) * 4;
   if (f0 >= HK) return;
   float pa[4] = {0.f, 0.f, 0.f, 0.f}, pb[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int gc = blockIdx.x * kGateBwdGroup; gc < min(num_chunks, (int)(blockIdx.x + 1) * kGateBwdGroup); ++gc) {
+  for (int gc = blockIdx.x * group; gc < min(num_chunks, (int)(blockIdx.x + 1) * group); ++gc) {
   int64_t token0; int valid;
   if (gate_locate(p, gc, token0, valid)) {
     const float a = expf(p.A_log[f0 / p.K]);
@@ -511,7 +514,8 @@ extern "C" int kda_gate_cumsum_fwd(const void* raw_gate, int dt_raw, const float
 }
 
 extern "C" int64_t kda_gate_bwd_partial_rows(int64_t num_chunks) {
-  return (num_chunks + kda::kGateBwdGroup - 1) / kda::kGateBwdGroup;
+  const int group = kda::gate_bwd_group(num_chunks);
+  return (num_chunks + group - 1) / group;
 }
 
 extern "C" int kda_gate_cumsum_bwd(const void* raw_gate, int dt_raw, const float* A_log,
@@ -533,7 +537,8 @@ extern "C" int kda_gate_cumsum_bwd(const void* raw_gate, int dt_raw, const float
   p.lower_bound = lower_bound;
   dim3 grid((unsigned)kda_gate_bwd_partial_rows(num_chunks), (unsigned)((heads * dim / 4 + 127) / 128));
   kda::StageScope timing(kda::kStageGateBwd, (cudaStream_t)stream);
-  kda::gate_cumsum_bwd_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(p, (int)num_chunks);
+  kda::gate_cumsum_bwd_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(p, (int)num_chunks,
+                                                                        kda::gate_bwd_group(num_chunks));
   return kda::check_launch();
 }
 
