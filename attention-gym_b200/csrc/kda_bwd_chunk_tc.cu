@@ -454,6 +454,27 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
     }
   }
 
+  // A lower triangular [64 x 64] accumulator (M = 64: row r on lane 32 (r / 16) + r % 16) as a bf16 tile, scaled: whole warps
+  // are below the diagonal, on it or above it (only zeros), so that one in four compares columns with rows.
+  auto lower_tile = [&](int col, int tile, bool diagonal, auto scaled) {
+    float y[16];
+    uint4 v[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    const int r = quad * 16 + lid;
+    if (quad >= rq) {
+      tmem_ld16(tl + col + r0, y);
+      scaled(y);
+      if (quad == rq) {
+        const int last = diagonal ? lid : lid - 1;
+#pragma unroll
+        for (int jj = 0; jj < 16; ++jj) y[jj] = jj <= last ? y[jj] : 0.f;
+      }
+      if (r < valid) { pack8v(y, v[0]); pack8v(y + 8, v[1]); }
+    }
+    if (lid < 16) {
+      *reinterpret_cast<uint4*>(sm + tile + sw128_chunk(r, 2 * rq)) = v[0];
+      *reinterpret_cast<uint4*>(sm + tile + sw128_chunk(r, 2 * rq + 1)) = v[1];
+    }
+  };
   // This thread's two (row, 8-channel) pieces -- rows tid / 16 and tid / 16 + 32, channels 8 (tid % 16) --
   // are the same in every pass that builds gated k tiles: their k (raw bf16) and gate values are read
   // once and stay in registers.
@@ -462,9 +483,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
   // ---- phase 1 epilogue: operand tiles for the next products; dq^T and dks^T stay in tensor memory
   {
     float a[16];
-    tmem_ld16(tl + tc::DW + r0, a);      // h dv2: dw^T = -(h dv2)
-#pragma unroll
-    for (int jj = 0; jj < 16; ++jj) a[jj] = -a[jj];
+    tmem_ld16(tl + tc::DW + r0, a);      // h dv2 = -dw^T: the products with this tile negate it
 #pragma unroll
     for (int qd = 0; qd < 2; ++qd) {
       uint4 v;
@@ -484,19 +503,10 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
       st_bf8(sm + bl::KGM, 8192, i, c16, kk);
     }
     // dAqk (M = 64 accumulator: row r lives on lane 32 (r / 16) + r % 16)
-    tmem_ld16(tl + tc::DAQK + r0, a);
-    if (lid < 16) {
-      const int r = quad * 16 + lid;
-      float y[16];
+    lower_tile(tc::DAQK, bl::DA, true, [&](float (&y)[16]) {
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) y[jj] = (r >= r0 + jj && r < valid) ? a[jj] * p.scale : 0.f;
-#pragma unroll
-      for (int qd = 0; qd < 2; ++qd) {
-        uint4 v;
-        pack8v(y + 8 * qd, v);
-        *reinterpret_cast<uint4*>(sm + bl::DA + sw128_chunk(r, 2 * rq + qd)) = v;
-      }
-    }
+      for (int jj = 0; jj < 16; ++jj) y[jj] *= p.scale;
+    });
   }
   fence_async_smem();
   tc_fence_before();
@@ -517,7 +527,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
         umma(tmem + tc::DKG, desc_kmajor(dwt, ks, 0), desc_mnmajor(ak, ks, 0),
-             instr_desc(128, 64, 0, 1), ks > 0);
+             instr_desc(128, 64, 0, 1, 1), ks > 0);
     } else {
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks)
@@ -526,7 +536,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks)
         umma(tmem + tc::X, desc_mnmajor(dwt, ks, 0), desc_kmajor(kgm, ks, 8192),
-             instr_desc(64, 64, 1, 0), 1);
+             instr_desc(64, 64, 1, 0, 1), 1);
     }
     umma_commit(&bar[2]);
   }
@@ -610,22 +620,10 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
       const float tot = warp_transpose_reduce16(pb, lid);
       if ((lid & 1) == 0) s_db[quad * 64 + r0 + (lid >> 1)] = tot;
     }
-    tmem_ld16(tl + tc::X + r0, a);
-    if (lid < 16) {
-      const int t = quad * 16 + lid;
-      float y[16];
+    lower_tile(tc::X, bl::X, false, [&](float (&y)[16]) {
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        const int s = r0 + jj;
-        y[jj] = (t > s && t < valid) ? a[jj] * bt[jj] : 0.f;
-      }
-#pragma unroll
-      for (int qd = 0; qd < 2; ++qd) {
-        uint4 v;
-        pack8v(y + 8 * qd, v);
-        *reinterpret_cast<uint4*>(sm + bl::X + sw128_chunk(t, 2 * rq + qd)) = v;
-      }
-    }
+      for (int jj = 0; jj < 16; ++jj) y[jj] *= bt[jj];
+    });
   }
   fence_async_smem();
   tc_fence_before();
@@ -742,22 +740,7 @@ __global__ void __launch_bounds__(NT, 1) kda_bwd_chunk_tc_kernel(const __grid_co
   tc_mark(p, it, 24);
   if (!mbar_wait(&bar[4], ph)) *s_abort = 1;
   tc_fence_after();
-  {
-    float a[16];
-    tmem_ld16(tl + tc::DL + r0, a);
-    if (lid < 16) {
-      const int r = quad * 16 + lid;
-      float y[16];
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj) y[jj] = (r > r0 + jj && r < valid) ? a[jj] : 0.f;
-#pragma unroll
-      for (int qd = 0; qd < 2; ++qd) {
-        uint4 v;
-        pack8v(y + 8 * qd, v);
-        *reinterpret_cast<uint4*>(sm + bl::DL + sw128_chunk(r, 2 * rq + qd)) = v;
-      }
-    }
-  }
+  lower_tile(tc::DL, bl::DL, false, [](float (&)[16]) {});
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
