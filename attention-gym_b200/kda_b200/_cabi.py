@@ -16,14 +16,15 @@ import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libkda_b200.so")
+TORCH_LIB_PATH = os.path.join(HERE, "libkda_b200_torch.so")
 
 KDA_F32, KDA_BF16, KDA_F16 = 0, 1, 2
 _DTYPES = {torch.float32: KDA_F32, torch.bfloat16: KDA_BF16, torch.float16: KDA_F16}
 _ERRORS = {-1: "invalid argument", -2: "unsupported shape", -3: "CUDA launch failed",
            -4: "problem exceeds the built-in scratch array"}
 
-# kernels launched through this module since import (bench.py reports it as gpu_launches)
-launch_count = 0
+# kernels launched through this module; with those of the C++ operators, `launch_count` (bench.py reports it as gpu_launches)
+_launches = 0
 
 _SIGNATURES = {
     "kda_b200_version": (c_int, []),
@@ -125,6 +126,24 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_torch_lib = None
+
+
+def load_torch_library() -> None:
+    """Register the C++ implementations of the operators, once their library has been built."""
+    global _torch_lib
+    if _torch_lib is None and os.path.exists(TORCH_LIB_PATH):
+        torch.ops.load_library(TORCH_LIB_PATH)
+        _torch_lib = ctypes.CDLL(TORCH_LIB_PATH)
+        _torch_lib.kda_torch_launches.restype = c_int64
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _launches + (_torch_lib.kda_torch_launches() if _torch_lib is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 def exported_symbols():
     return list(_SIGNATURES)
 
@@ -158,7 +177,7 @@ def call(name: str, launches: int, *args):
     """Invoke an entry point that returns a status code; raise on failure.  Under an active torch
     profiler the call is a range named after the entry point; inside it, every kernel launch is an
     NVTX range named after the reference stages it fuses (kda_cabi.cu)."""
-    global launch_count
+    global _launches
     entry = getattr(_lib or lib(), name)
     if torch.autograd.profiler._is_profiler_enabled:
         with profiler_range("kda_b200/" + name):
@@ -167,7 +186,7 @@ def call(name: str, launches: int, *args):
         rc = entry(*args)
     if rc != 0:
         raise RuntimeError(f"{name} failed: {_ERRORS.get(rc, rc)}")
-    launch_count += launches
+    _launches += launches
 
 
 def stage_timing(enable: bool) -> None:

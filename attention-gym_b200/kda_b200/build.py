@@ -13,6 +13,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "csrc")
 LIB_PATH = os.path.join(HERE, "libkda_b200.so")
+TORCH_LIB_PATH = os.path.join(HERE, "libkda_b200_torch.so")      # operators in C++ on top of it
+TORCH_SOURCE = "kda_torch.cpp"
 SOURCES = [
     "kda_cabi.cu",
     "kda_recurrent.cu",
@@ -42,16 +44,17 @@ def _nvcc() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(TORCH_LIB_PATH):
         return True
-    built = os.path.getmtime(LIB_PATH)
+    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(TORCH_LIB_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     deps.append(os.path.join(os.path.dirname(os.path.dirname(HERE)), "include", "kda_b200.h"))
     return any(os.path.getmtime(d) > built for d in deps if os.path.exists(d))
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every kernel for sm_100a into one shared library; returns its path."""
+    """Compile every kernel for sm_100a into one shared library, and the C++ operators into a second one; returns the
+    path of the first."""
     if not force and not needs_build():
         return LIB_PATH
     objs = []
@@ -74,7 +77,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if proc.returncode:
             raise RuntimeError(f"nvcc failed on {src}")
     subprocess.check_call([_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-lcudart", "-ldl"])
+    _build_torch()
+    from . import _cabi
+
+    _cabi.load_torch_library()
     return LIB_PATH
+
+
+def _build_torch() -> None:
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    lib = os.path.join(root, "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include")]
+    subprocess.check_call([
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes),
+        os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_LIB_PATH, f"-L{HERE}", "-l:libkda_b200.so", f"-L{lib}", "-ltorch",
+        "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
 
 
 if __name__ == "__main__":

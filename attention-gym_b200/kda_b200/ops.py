@@ -5,7 +5,9 @@ operators (attn_gym/linear/kda/ops.py:18-136, fwd/triton/gate_fwd.py:379-393,
 fwd/triton/l2norm_fwd.py:84,143, bwd/cute/gate_bwd_fused.py:498-502) under the ``kda_b200``
 namespace, so the reference can be imported beside this package.  Each CUDA implementation
 allocates its outputs and workspace with torch and makes one call into the shared library on
-the current stream: no host synchronisation, no second back end, no CPU implementation.
+the current stream: no host synchronisation, no second back end, no CPU implementation.  The operators
+on the path of small calls (the chunked forward, its backward from kept intermediates, the recurrence, the
+decode step) have that implementation in C++ (csrc/kda_torch.cpp), because their calls are bound by the host.
 """
 
 from __future__ import annotations
@@ -140,6 +142,9 @@ _lib_layer.define("chunk_bwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta
 _lib_layer.define("widen(Tensor x) -> Tensor")
 
 
+_cabi.load_torch_library()
+
+
 def _require_cuda(t: torch.Tensor, what: str):
     if not t.is_cuda:
         raise ValueError(f"{what} requires CUDA tensors")
@@ -170,77 +175,9 @@ def _fwd_workspace_bytes(batch, tokens, heads, packed_nseq, keep):
     return int(lib.kda_chunk_fwd_workspace_bytes(tokens, heads))
 
 
-def _chunk_fwd_impl(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state,
-                    keep=False):
-    _require_cuda(q, "the fused KDA core")
-    if q.shape[-1] != 128 or v.shape[-1] != 128:
-        raise ValueError("the fused KDA core requires K=V=128")
-    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
-        raise TypeError("the fused KDA core takes bfloat16 q, k, v")
-    batch, tokens, heads, _ = q.shape
-    packed = cu_seqlens is not None
-    if not packed:
-        nseq, capacity = batch, None
-    else:
-        if batch != 1:
-            raise ValueError("packed cu_seqlens require batch size one")
-        nseq = cu_seqlens.shape[0] - 1
-        capacity = chunk_capacity(tokens, nseq, _CHUNK)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    gate = gate.float().contiguous()
-    beta = beta.float().contiguous()
-    if initial_state is not None:
-        initial_state = initial_state.float().contiguous()
-    total = batch * tokens
-    out = torch.zeros_like(v) if packed else torch.empty_like(v)
-    aqk = torch.empty(batch, tokens, heads, _CHUNK, dtype=q.dtype, device=q.device)
-    akk = torch.empty_like(aqk)
-    state = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=q.device)
-             if want_state else None)
-    ws_bytes = _fwd_workspace_bytes(batch, tokens, heads, None if not packed else nseq, keep)
-    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    head = (_cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate), _cabi.ptr(beta),
-            _cabi.ptr(initial_state), _cabi.ptr(state), _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk))
-    if packed:
-        _cabi.call("kda_chunk_fwd_save" if keep else "kda_chunk_fwd", 3, *head, _cabi.ptr(cu_seqlens),
-                   _cabi.ptr(chunk_offsets), nseq, total, heads, 128, 128, capacity,
-                   _cabi.ptr(workspace), ws_bytes, _cabi.stream())
-    else:
-        # dense rows: offsets are built on the device, long rows of small batches are walked in
-        # parallel segments
-        _cabi.call("kda_chunk_fwd_dense_save" if keep else "kda_chunk_fwd_dense", 3, *head, batch,
-                   tokens, heads, 128, 128, _cabi.ptr(workspace), ws_bytes, _cabi.stream())
-    if keep:
-        return out, state, aqk, akk, workspace
-    return out, state, aqk, akk
-
-
-@torch.library.impl(_lib, "kda_chunk_fwd", "CUDA")
-def _chunk_fwd(q, k, v, gate, beta, initial_state, autotune):
-    out, _, aqk, akk = _chunk_fwd_impl(q, k, v, gate, beta, initial_state, None, None, False)
-    return out, aqk, akk
-
-
-@torch.library.impl(_lib, "kda_chunk_fwd_with_state", "CUDA")
-def _chunk_fwd_with_state(q, k, v, gate, beta, initial_state, autotune):
-    return _chunk_fwd_impl(q, k, v, gate, beta, initial_state, None, None, True)
-
-
-@torch.library.impl(_lib, "kda_chunk_fwd_ragged", "CUDA")
-def _chunk_fwd_ragged(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, autotune):
-    out, _, aqk, akk = _chunk_fwd_impl(q, k, v, gate, beta, initial_state, cu_seqlens,
-                                       chunk_offsets, False)
-    return out, aqk, akk
-
-
-@torch.library.impl(_lib, "kda_chunk_fwd_ragged_with_state", "CUDA")
-def _chunk_fwd_ragged_with_state(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets,
-                                 autotune):
-    return _chunk_fwd_impl(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, True)
-
-
 def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_output,
-                    d_final_state, initial_state, want_state_grad, saved=None, rstd=None):
+                    d_final_state, initial_state, want_state_grad):
+    """The backward pass that rebuilds the forward intermediates."""
     batch, tokens, heads, _ = q.shape
     packed = cu_seqlens is not None
     if packed:
@@ -267,23 +204,13 @@ def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_
     dh0 = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=q.device)
            if want_state_grad else None)
     ws_bytes = _cabi.lib().kda_chunk_bwd_workspace_bytes(total, heads, capacity)
-    if saved is not None:
-        if saved.numel() < ws_bytes or saved.dtype != torch.uint8 or not saved.is_cuda:
-            raise ValueError("`saved` is not the buffer kda_chunk_fwd_saved returned for these shapes")
-        workspace = saved
-    else:
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
     head = (_cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
             _cabi.ptr(beta), _cabi.ptr(aqk), _cabi.ptr(akk), _cabi.ptr(initial_state),
             _cabi.ptr(d_output), _cabi.ptr(d_final_state), _cabi.ptr(dq), _cabi.ptr(dk),
             _cabi.ptr(dv), _cabi.ptr(dg), _cabi.ptr(db), _cabi.ptr(dh0), cu_ptr,
             chunks_ptr, nseq, total, heads, 128, 128, capacity)
-    if rstd is not None:
-        _cabi.call("kda_chunk_bwd_qknorm_saved", 2, *head, _cabi.ptr(rstd[0]), _cabi.ptr(rstd[1]),
-                   _cabi.ptr(workspace), ws_bytes, _cabi.stream())
-    else:
-        _cabi.call("kda_chunk_bwd_saved" if saved is not None else "kda_chunk_bwd", 5, *head,
-                   _cabi.ptr(workspace), ws_bytes, _cabi.stream())
+    _cabi.call("kda_chunk_bwd", 5, *head, _cabi.ptr(workspace), ws_bytes, _cabi.stream())
     return dq, dk, dv, dg, db, dh0
 
 
@@ -299,26 +226,6 @@ def _chunk_bwd_with_state_grad(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_
                                d_final_state, initial_state, fastmath, autotune):
     return _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_output,
                            d_final_state, initial_state, True)
-
-
-@torch.library.impl(_lib, "kda_chunk_fwd_saved", "CUDA")
-def _chunk_fwd_saved(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state):
-    out, state, aqk, akk, saved = _chunk_fwd_impl(q, k, v, gate, beta, initial_state, cu_seqlens,
-                                                  chunk_offsets, want_state, keep=True)
-    if state is None:
-        state = torch.empty(0, dtype=torch.float32, device=q.device)
-    return out, state, aqk, akk, saved
-
-
-@torch.library.impl(_lib, "kda_chunk_bwd_saved", "CUDA")
-def _chunk_bwd_saved(q, k, v, gate, beta, aqk, akk, saved, cu_seqlens, chunk_offsets, d_output,
-                     d_final_state, initial_state, want_state_grad):
-    dq, dk, dv, dg, db, dh0 = _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens,
-                                              chunk_offsets, d_output, d_final_state, initial_state,
-                                              want_state_grad, saved=saved)
-    if dh0 is None:
-        dh0 = torch.empty(0, dtype=torch.float32, device=q.device)
-    return dq, dk, dv, dg, db, dh0
 
 
 @torch.library.impl(_lib, "kda_chunk_bwd_state_saved", "CUDA")
@@ -350,62 +257,7 @@ def _chunk_bwd_state_saved(gate, aqk, saved, cu_seqlens, chunk_offsets, d_output
     return dh0
 
 
-@torch.library.impl(_lib, "kda_chunk_fwd_qknorm", "CUDA")
-def _chunk_fwd_qknorm(q, k, v, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state, keep,
-                      eps):
-    _require_cuda(q, "the fused KDA core")
-    if q.shape[-1] != 128 or v.shape[-1] != 128:
-        raise ValueError("the fused KDA core requires K=V=128")
-    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
-        raise TypeError("the fused KDA core takes bfloat16 q, k, v")
-    batch, tokens, heads, _ = q.shape
-    packed = cu_seqlens is not None
-    if not packed:
-        nseq = batch
-    else:
-        if batch != 1:
-            raise ValueError("packed cu_seqlens require batch size one")
-        nseq = cu_seqlens.shape[0] - 1
-        capacity = chunk_capacity(tokens, nseq, _CHUNK)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    gate, beta = gate.float().contiguous(), beta.float().contiguous()
-    if initial_state is not None:
-        initial_state = initial_state.float().contiguous()
-    total = batch * tokens
-    out = torch.zeros_like(v) if packed else torch.empty_like(v)
-    aqk = torch.empty(batch, tokens, heads, _CHUNK, dtype=q.dtype, device=q.device)
-    akk = torch.empty_like(aqk)
-    alloc = torch.zeros if packed else torch.empty
-    rstd_q = alloc(batch, tokens, heads, dtype=torch.float32, device=q.device)
-    rstd_k = alloc(batch, tokens, heads, dtype=torch.float32, device=q.device)
-    state = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=q.device)
-             if want_state else q.new_empty((0,), dtype=torch.float32))
-    ws_bytes = _fwd_workspace_bytes(batch, tokens, heads, nseq if packed else None, keep)
-    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    head = (_cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate), _cabi.ptr(beta), _cabi.ptr(initial_state),
-            _cabi.ptr(state) if want_state else None, _cabi.ptr(out), _cabi.ptr(aqk), _cabi.ptr(akk),
-            _cabi.ptr(rstd_q), _cabi.ptr(rstd_k), float(eps))
-    if packed:
-        _cabi.call("kda_chunk_fwd_qknorm", 3, *head, _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets), nseq, total,
-                   heads, 128, 128, capacity, _cabi.ptr(workspace), ws_bytes, int(keep), _cabi.stream())
-    else:
-        _cabi.call("kda_chunk_fwd_dense_qknorm", 3, *head, batch, tokens, heads, 128, 128, _cabi.ptr(workspace),
-                   ws_bytes, int(keep), _cabi.stream())
-    return out, state, aqk, akk, workspace, rstd_q, rstd_k
-
-
-@torch.library.impl(_lib, "kda_chunk_bwd_qknorm", "CUDA")
-def _chunk_bwd_qknorm(q, k, v, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_seqlens, chunk_offsets,
-                      d_output, d_final_state, initial_state, want_state_grad):
-    dq, dk, dv, dg, db, dh0 = _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets,
-                                              d_output, d_final_state, initial_state, want_state_grad,
-                                              saved=saved, rstd=(rstd_q.contiguous(), rstd_k.contiguous()))
-    if dh0 is None:
-        dh0 = torch.empty(0, dtype=torch.float32, device=q.device)
-    return dq, dk, dv, dg, db, dh0
-
-
-# The two operators above on one tensor [B, T, 3, H, 128] of q, k and v rows, as the layer's convolution leaves them:
+# kda_chunk_fwd_qknorm and its backward on one tensor [B, T, 3, H, 128] of q, k and v rows, as the layer's convolution leaves them:
 # no copies of q, k and v, and their gradients come back in one tensor of the same layout.
 @torch.library.impl(_lib_layer, "chunk_fwd_qkv", "CUDA")
 def _chunk_fwd_qkv(qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, want_state, keep, eps):
@@ -594,47 +446,6 @@ def _(gate, aqk, saved, cu_seqlens, chunk_offsets, d_output, d_final_state):
 # --------------------------------------------------------------------------------------------
 # recurrent scan
 # --------------------------------------------------------------------------------------------
-def _recurrent_impl(q, k, v, gate, beta, initial_state, cu_seqlens, state_indices, want_state):
-    _require_cuda(q, "the fused recurrent scan")
-    batch, tokens, heads, key_dim = q.shape
-    value_dim = v.shape[-1]
-    nseq = batch if cu_seqlens is None else cu_seqlens.shape[0] - 1
-    out = (torch.zeros if cu_seqlens is not None else torch.empty)(
-        v.shape, dtype=q.dtype, device=q.device)
-    final = None
-    slot_stride, num_slots = heads * key_dim * value_dim, 0
-    if state_indices is not None:
-        slot_stride, num_slots = initial_state.stride(0), initial_state.shape[0]
-    else:
-        if initial_state is not None:
-            initial_state = initial_state.float().contiguous()
-        if want_state:
-            final = torch.empty(nseq, heads, key_dim, value_dim, dtype=torch.float32,
-                                device=q.device)
-    _cabi.call("kda_recurrent_fwd", 1, _cabi.ptr(q), _cabi.ptr(k), _cabi.ptr(v), _cabi.ptr(gate),
-               _cabi.ptr(beta), _cabi.dt(q), _cabi.dt(k), _cabi.dt(v), _cabi.dt(gate),
-               _cabi.dt(beta), _cabi.ptr(initial_state), _cabi.ptr(final), _cabi.ptr(out),
-               _cabi.dt(out), _cabi.ptr(cu_seqlens), _cabi.ptr(state_indices), slot_stride,
-               num_slots, nseq, tokens, heads, key_dim, value_dim, float(key_dim) ** -0.5,
-               _cabi.stream())
-    return out, final
-
-
-@torch.library.impl(_lib, "kda_recurrent_fwd", "CUDA")
-def _recurrent_fwd(q, k, v, gate, beta, initial_state, cu_seqlens, autotune):
-    return _recurrent_impl(q, k, v, gate, beta, initial_state, cu_seqlens, None, True)
-
-
-@torch.library.impl(_lib, "kda_recurrent_fwd_no_state", "CUDA")
-def _recurrent_fwd_no_state(q, k, v, gate, beta, initial_state, cu_seqlens, autotune):
-    return _recurrent_impl(q, k, v, gate, beta, initial_state, cu_seqlens, None, False)[0]
-
-
-@torch.library.impl(_lib, "kda_recurrent_fwd_paged", "CUDA")
-def _recurrent_fwd_paged(q, k, v, gate, beta, state_cache, state_indices, cu_seqlens, autotune):
-    return _recurrent_impl(q, k, v, gate, beta, state_cache, cu_seqlens, state_indices, False)[0]
-
-
 @torch.library.impl(_lib_own, "chunk_scan", "CUDA")
 def _chunk_scan(q, k, v, gate, beta, initial_state, cu_seqlens, want_state):
     _require_cuda(q, "the fused recurrent scan")
@@ -926,26 +737,6 @@ def _widen(x):
 @torch.library.register_fake(f"{_NS_LAYER}::widen")
 def _(x):
     return x.new_empty(x.shape, dtype=torch.float32)
-
-
-@torch.library.impl(_lib_own, "decode_step", "CUDA")
-def _decode_step(x, weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta, activation,
-                 lower_bound, eps):
-    nseq, heads = x.shape[0], state_pool.shape[1]
-    x, weight, raw_gate, beta = x.contiguous(), weight.contiguous(), raw_gate.contiguous(), beta.contiguous()
-    A_log, dt_bias = A_log.float().contiguous(), dt_bias.float().contiguous()
-    out = torch.empty(nseq, heads, 128, dtype=x.dtype, device=x.device)
-    xp, wp, cp, bp = x.data_ptr(), weight.data_ptr(), conv_state.data_ptr(), dt_bias.data_ptr()
-    pool, width, dtype = state_pool.data_ptr(), weight.shape[1], _cabi.dt(x)
-    # 0: the whole step is one launch
-    need = _cabi.lib().kda_decode_step_scratch_bytes(xp | wp | cp | bp | pool | 4 * state_pool.stride(0), dtype, nseq,
-                                                     heads, width)
-    scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
-    _cabi.call("kda_decode_step", 2 if need else 1, xp, wp, cp, state_indices.data_ptr(), raw_gate.data_ptr(),
-               _cabi.dt(raw_gate), A_log.data_ptr(), bp, beta.data_ptr(), _cabi.dt(beta), pool, state_pool.stride(0),
-               _cabi.ptr(scratch), out.data_ptr(), dtype, nseq, heads, width, conv_state.shape[0],
-               state_pool.shape[0], _act_code(activation), lower_bound, eps, _cabi.stream())
-    return out
 
 
 @torch.library.register_fake(f"{_NS_OWN}::decode_step")
