@@ -68,6 +68,21 @@ Tensor empty(at::IntArrayRef shape, const Tensor& like, at::ScalarType dtype) {
 Tensor fresh(at::IntArrayRef shape, const Tensor& like, at::ScalarType dtype, bool zero) {
   return zero ? at::zeros(shape, like.options().dtype(dtype)) : empty(shape, like, dtype);
 }
+// zeroes the rows of [1, tokens, ...] results that no packed sequence covers
+void zero_unused_rows(std::initializer_list<Tensor> results, int64_t tokens, const OptTensor& cu, const OptTensor& co) {
+  void* buffers[8];
+  int64_t row_bytes[8];
+  int count = 0;
+  for (const Tensor& t : results) {
+    if (!t.defined()) continue;
+    buffers[count] = t.data_ptr();
+    row_bytes[count++] = t.numel() / std::max<int64_t>(tokens, 1) * t.element_size();
+  }
+  call("kda_b200/kda_zero_unused_rows", 1, [&] {
+    return kda_zero_unused_rows(buffers, row_bytes, count, iptr(cu), iptr(co), (int)kChunk, (int)(cu->size(0) - 1), tokens,
+                                stream());
+  });
+}
 // the largest number of chunks that `nseq` sequences can have in `tokens` tokens
 int64_t chunk_capacity(int64_t tokens, int64_t nseq) {
   TORCH_CHECK_VALUE(nseq >= 1, "num_sequences must be positive, got ", nseq);
@@ -111,13 +126,14 @@ Forward chunk_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, cons
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), gate = f32(gate_), beta = f32(beta_);
   const OptTensor h0 = f32(h0_);
   Forward f;
-  f.out = fresh(v.sizes(), v, v.scalar_type(), s.packed);
+  f.out = empty(v.sizes(), v, v.scalar_type());
   f.aqk = empty({s.batch, s.tokens, s.heads, kChunk}, q, q.scalar_type());
   f.akk = at::empty_like(f.aqk);
   if (norm) {
-    f.rstd_q = fresh({s.batch, s.tokens, s.heads}, q, at::kFloat, s.packed);
-    f.rstd_k = fresh({s.batch, s.tokens, s.heads}, q, at::kFloat, s.packed);
+    f.rstd_q = empty({s.batch, s.tokens, s.heads}, q, at::kFloat);
+    f.rstd_k = at::empty_like(f.rstd_q);
   }
+  if (s.packed) zero_unused_rows({f.out, f.rstd_q, f.rstd_k}, s.tokens, cu, co);
   if (want_state) f.state = empty({s.nseq, s.heads, kDim, kDim}, q, at::kFloat);
   const int64_t bytes = fwd_workspace(s.batch, s.tokens, s.heads, s.packed ? s.nseq : -1, keep);
   f.workspace = empty({bytes}, q, at::kByte);
@@ -214,8 +230,8 @@ struct Cotangents {
       call("kda_b200/kda_dense_offsets", 1, [&] { return kda_dense_offsets(base, (int)s.batch, (int)s.tokens, stream()); });
       cu = base; co = base + s.batch + 1;
     }
-    dg = s.packed ? at::zeros_like(gate) : at::empty_like(gate);
-    db = s.packed ? at::zeros_like(beta) : at::empty_like(beta);
+    dg = at::empty_like(gate);
+    db = at::empty_like(beta);
     if (want_state_grad) dh0 = empty({s.nseq, s.heads, kDim, kDim}, like, at::kFloat);
   }
   float* dh0_ptr() const { return dh0.defined() ? fptr(dh0) : nullptr; }
@@ -229,8 +245,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> chunk_backward(
   const Shape s(q_, 2, cu);
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
   const Cotangents c(s, q, gate, beta, saved, cu, co, d_out, d_state, h0, want_state_grad);
-  auto like = [&](const Tensor& t) { return s.packed ? at::zeros_like(t) : at::empty_like(t); };
-  const Tensor dq = like(q), dk = like(k), dv = like(v);
+  const Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
+  if (s.packed) zero_unused_rows({dq, dk, dv, c.dg, c.db}, s.tokens, cu, co);
   const int D = (int)kDim, H = (int)s.heads;
   if (rstd_q) {
     const Tensor rq = rstd_q->contiguous(), rk = rstd_k->contiguous();

@@ -82,6 +82,7 @@ _SIGNATURES = {
                                     c_void_p, c_int64, c_void_p]),
     "kda_chunk_bwd_state_saved": (c_int, [c_void_p] * 7 + [c_int, c_int64, c_int, c_int, c_int, c_int,
                                           c_void_p, c_int64, c_void_p]),
+    "kda_zero_unused_rows": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int64, c_void_p]),
     "kda_dense_offsets": (c_int, [c_void_p, c_int, c_int, c_void_p]),
     "kda_chunk_fwd_prepare": (c_int, [c_void_p] * 9 + [c_int, c_int64, c_int, c_int, c_void_p,
                                       c_int64, c_void_p]),

@@ -12,6 +12,8 @@ decode step) have that implementation in C++ (csrc/kda_torch.cpp), because their
 
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _cabi
@@ -175,6 +177,16 @@ def _fwd_workspace_bytes(batch, tokens, heads, packed_nseq, keep):
     return int(lib.kda_chunk_fwd_workspace_bytes(tokens, heads))
 
 
+def _zero_unused_rows(buffers, tokens, cu_seqlens, chunk_offsets=None, chunk_size=_CHUNK):
+    """Zero the rows of ``[1, tokens, ...]`` results that no packed sequence covers."""
+    count = len(buffers)
+    ptrs = (ctypes.c_void_p * count)(*(t.data_ptr() for t in buffers))
+    row_bytes = (ctypes.c_int64 * count)(*(t.numel() // max(tokens, 1) * t.element_size() for t in buffers))
+    _cabi.call("kda_zero_unused_rows", 1, ctypes.addressof(ptrs), ctypes.addressof(row_bytes), count,
+               _cabi.ptr(cu_seqlens), _cabi.ptr(chunk_offsets), chunk_size, cu_seqlens.shape[0] - 1, tokens,
+               _cabi.stream())
+
+
 def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_output,
                     d_final_state, initial_state, want_state_grad):
     """The backward pass that rebuilds the forward intermediates."""
@@ -198,9 +210,9 @@ def _chunk_bwd_impl(q, k, v, gate, beta, aqk, akk, cu_seqlens, chunk_offsets, d_
         d_final_state = d_final_state.float().contiguous()
     if initial_state is not None:
         initial_state = initial_state.float().contiguous()
-    alloc = torch.zeros_like if packed else torch.empty_like
-    dq, dk, dv = alloc(q), alloc(k), alloc(v)
-    dg, db = alloc(gate), alloc(beta)
+    dq, dk, dv, dg, db = (torch.empty_like(t) for t in (q, k, v, gate, beta))
+    if packed:
+        _zero_unused_rows((dq, dk, dv, dg, db), tokens, cu_seqlens, chunk_offsets)
     dh0 = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=q.device)
            if want_state_grad else None)
     ws_bytes = _cabi.lib().kda_chunk_bwd_workspace_bytes(total, heads, capacity)
@@ -277,12 +289,13 @@ def _chunk_fwd_qkv(qkv, gate, beta, initial_state, cu_seqlens, chunk_offsets, wa
     qkv, gate, beta = qkv.contiguous(), gate.float().contiguous(), beta.float().contiguous()
     if initial_state is not None:
         initial_state = initial_state.float().contiguous()
-    alloc = torch.zeros if packed else torch.empty
-    out = alloc(batch, tokens, heads, 128, dtype=qkv.dtype, device=qkv.device)
+    out = torch.empty(batch, tokens, heads, 128, dtype=qkv.dtype, device=qkv.device)
     aqk = torch.empty(batch, tokens, heads, _CHUNK, dtype=qkv.dtype, device=qkv.device)
     akk = torch.empty_like(aqk)
-    rstd_q = alloc(batch, tokens, heads, dtype=torch.float32, device=qkv.device)
-    rstd_k = alloc(batch, tokens, heads, dtype=torch.float32, device=qkv.device)
+    rstd_q = torch.empty(batch, tokens, heads, dtype=torch.float32, device=qkv.device)
+    rstd_k = torch.empty_like(rstd_q)
+    if packed:
+        _zero_unused_rows((out, rstd_q, rstd_k), tokens, cu_seqlens, chunk_offsets)
     state = (torch.empty(nseq, heads, 128, 128, dtype=torch.float32, device=qkv.device)
              if want_state else qkv.new_empty((0,), dtype=torch.float32))
     ws_bytes = _fwd_workspace_bytes(batch, tokens, heads, nseq if packed else None, keep)
@@ -316,8 +329,9 @@ def _chunk_bwd_qkv(qkv, gate, beta, aqk, akk, saved, rstd_q, rstd_k, cu_seqlens,
         d_final_state = d_final_state.float().contiguous()
     if initial_state is not None:
         initial_state = initial_state.float().contiguous()
-    alloc = torch.zeros_like if packed else torch.empty_like
-    dqkv, dg, db = alloc(qkv), alloc(gate), alloc(beta)
+    dqkv, dg, db = (torch.empty_like(t) for t in (qkv, gate, beta))
+    if packed:
+        _zero_unused_rows((dqkv, dg, db), tokens, cu_seqlens, chunk_offsets)
     dh0 = torch.empty((nseq, heads, 128, 128) if want_state_grad else (0,), dtype=torch.float32, device=qkv.device)
     ws_bytes = _cabi.lib().kda_chunk_bwd_workspace_bytes(total, heads, capacity)
     if saved.numel() < ws_bytes or saved.dtype != torch.uint8 or not saved.is_cuda:
@@ -520,8 +534,9 @@ def _gate_fwd(raw, A_log, dt_bias, cu_seqlens, chunk_offsets, chunk_size, lower_
     raw = raw.contiguous()
     batch, tokens, heads, dim = raw.shape
     nseq, chunks = _gate_chunks(raw, cu_seqlens, chunk_size)
-    alloc = torch.zeros if cu_seqlens is not None else torch.empty
-    out = alloc(raw.shape, dtype=torch.float32, device=raw.device)
+    out = torch.empty(raw.shape, dtype=torch.float32, device=raw.device)
+    if cu_seqlens is not None:
+        _zero_unused_rows((out,), tokens, cu_seqlens, chunk_offsets, chunk_size)
     _cabi.call("kda_gate_cumsum_fwd", 1, _cabi.ptr(raw), _cabi.dt(raw), _cabi.ptr(A_log.contiguous()),
                _cabi.ptr(dt_bias.contiguous()), _cabi.ptr(out), _cabi.ptr(cu_seqlens),
                _cabi.ptr(chunk_offsets), nseq, batch, tokens, heads, dim, chunk_size,
@@ -546,7 +561,9 @@ def _gate_bwd(raw, A_log, dt_bias, d_cumulative, cu_seqlens, chunk_offsets, chun
     d_cumulative = d_cumulative.float().contiguous()
     batch, tokens, heads, dim = raw.shape
     nseq, chunks = _gate_chunks(raw, cu_seqlens, chunk_size)
-    d_raw = (torch.zeros_like if cu_seqlens is not None else torch.empty_like)(raw)
+    d_raw = torch.empty_like(raw)
+    if cu_seqlens is not None:
+        _zero_unused_rows((d_raw,), tokens, cu_seqlens, chunk_offsets, chunk_size)
     rows = _cabi.lib().kda_gate_bwd_partial_rows(chunks)
     pa = torch.empty(max(rows, 1), heads * dim, dtype=torch.float32, device=raw.device)
     pb = torch.empty_like(pa)
@@ -663,7 +680,9 @@ def _act_code(activation):
 def _short_conv_fwd(x, weight, cu_seqlens=None, initial_state=None, *, activation=None):
     batch, tokens, channels = x.shape
     nseq = batch if cu_seqlens is None else cu_seqlens.shape[0] - 1
-    y = (torch.zeros_like if cu_seqlens is not None else torch.empty_like)(x)
+    y = torch.empty_like(x)
+    if cu_seqlens is not None:
+        _zero_unused_rows((y,), tokens, cu_seqlens)
     _cabi.call("kda_conv1d_fwd", 1, _cabi.ptr(x), _cabi.ptr(weight), _cabi.ptr(initial_state),
                _cabi.ptr(y), _cabi.dt(x), _cabi.ptr(cu_seqlens), nseq, batch, tokens, channels,
                weight.shape[1], _act_code(activation), _cabi.stream())
@@ -677,7 +696,9 @@ def _short_conv_bwd(x, weight, grad_output, cu_seqlens=None, initial_state=None,
     width = weight.shape[1]
     nseq = batch if cu_seqlens is None else cu_seqlens.shape[0] - 1
     grad_output = grad_output.to(x.dtype).contiguous()
-    dx = (torch.zeros_like if cu_seqlens is not None else torch.empty_like)(x)
+    dx = torch.empty_like(x)
+    if cu_seqlens is not None:
+        _zero_unused_rows((dx,), tokens, cu_seqlens)
     blocks = _cabi.lib().kda_conv1d_bwd_blocks(batch, tokens, int(cu_seqlens is not None))
     dw_part = torch.empty(blocks, channels, width, dtype=torch.float32, device=x.device)
     dstate = (torch.zeros(nseq, max(width - 1, 0), channels, dtype=torch.float32, device=x.device)

@@ -300,6 +300,13 @@ int kda_chunk_bwd_qkv_saved(const void* qkv, const float* cum_gate, const float*
                             const int32_t* cu_seqlens, const int32_t* chunk_offsets, int nseq, int64_t tokens, int heads,
                             int num_chunks, void* saved, int64_t saved_bytes, void* stream);
 
+/* Clears the rows of up to 8 row-major buffers of `tokens` rows (row_bytes and addresses even) that no
+ * packed sequence covers, before the kernels above write the others: those before cu_seqlens[0] and from cu_seqlens[nseq]
+ * on, or all of them if the offsets leave the buffer or contradict chunk_offsets (NULL: not checked).  The two arrays are
+ * read on the host. */
+int kda_zero_unused_rows(void* const* buffers, const int64_t* row_bytes, int count, const int32_t* cu_seqlens,
+                         const int32_t* chunk_offsets, int chunk_size, int nseq, int64_t tokens, void* stream);
+
 /* The packed description of a dense [batch, tokens] input: cu_seqlens [batch + 1] and, right behind it,
  * chunk_offsets [batch + 1] (int32, on the device). */
 int kda_dense_offsets(void* offsets, int batch, int tokens, void* stream);
