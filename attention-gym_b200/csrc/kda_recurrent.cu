@@ -22,8 +22,8 @@ namespace kda {
 // K > 128: bound by the latency of one token, the dependent chain of decay, reduction, three shuffles and update, so that NP
 // warps of their own fetch, publish and store (NP = 0: the computing warps do it).
 // A short scan of many sequences is bound by the state traffic and by how much of it two CTAs per SM
-// can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 141 us before, 60 us
-// now.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
+// can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 60 us, with four of half the columns 51
+// us.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
 // CUM: the gate is the cumulative one of chunk_kda; the per-token gate is its difference inside the
 // 64-token chunks of a sequence.
 // ------------------------------------------------------------------------------------------------
@@ -663,8 +663,9 @@ static int launch_block_scan(const ScanParams& p, bool cumulative, cudaStream_t 
 template <int KR, int VC, int NW, int NP, int MINB>
 static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream) {
   constexpr int CT = 4 * VC * NW, KP = 8 * KR;
-  // 24 KiB of operands in two buffers (K = 128: 8 tokens); the wide form also buffers 128 columns of v and o
-  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : 1024 / KP;
+  // 24 KiB of operands in two buffers (K = 128: 8 tokens, 4 where four CTAs share an SM); the wide form also buffers its
+  // columns of v and o
+  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : (MINB == 4 ? 512 : 1024) / KP;
   const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + CT - 1) / CT);
   if (blocks <= 0) return KDA_OK;
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
@@ -676,11 +677,19 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
 
 // Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length, a turn as
 // many slices as there are SMs.  Figures in us, both sides of each line (K = V = 128 unless said otherwise).
-// * wide: four columns per lane, 128 per CTA, 16-byte state accesses, two CTAs per SM, from more than two turns on; from more
-//   than one turn on for 2 to 8 tokens.  Below: blocks of four tokens, 16 columns per CTA.  Blocks / wide: 16 chains (128
-//   slices) 5.6 / 6.6 at 2 tokens, 12 / 27 at 32, 68 / 183 at 256; 32 chains 9.2 / 6.5 at 2, 10.1 / 10.0 at 8, 13.9 / 15.4 at 16,
-//   134 / 183 at 256; 48 chains (384) 12.7 / 6.4 at 2, 20 / 15.5 at 16, 56 / 49 at 64.  K = V = 32 up to four turns from 64 tokens
-//   on: 192 chains (384) 11.0 / 11.2 at 16, 25 / 36 at 64; 296 chains (592) 21.3 / 19.5 at 32, 109 / 135 at 256.
+// * wide: four columns per lane, 16-byte state accesses, sixteen warps per SM; below: blocks of four tokens, 16
+//   columns per CTA, whose time grows with every turn.  Blocks / wide, 2 to 8 tokens, wide above one turn: 16 chains (128 slices)
+//   5.6 / 6.6 at 2 tokens, 32 chains 9.2 / 6.5 at 2, 10.1 / 10.0 at 8; up to 15 tokens above two.  Above three turns from 16 tokens
+//   on: 48 chains (384) 14 / 16 at 16 tokens, 21 / 27 at 32, 56 chains (448) 17 / 16 and 26 / 27; four from 64 on: 72 chains (576)
+//   45 / 50 at 64, 151 / 185 at 256, 76 chains (608) 55 / 49 and 187 / 185.  K = V = 32 above two turns, 192 chains (384) 11 / 8 at
+//   16, 20 / 19 at 48; from 64 on above three: 192 chains 40 / 46 at 128, 224 chains (448) 51 / 46.
+//   128 columns per CTA and two CTAs per SM, or 64 and four, where 128 would leave half of a CTA without columns: 128 / 64 columns
+//   at V = 64, 1024 chains of 64 tokens, K = 64 172 / 100, K = 128 271 / 160; above V = 64 only if CTAs of 128 columns are more than
+//   two per SM: K = 72, V = 132, 8 tokens, 256 chains 25.5 / 22.0, 64 chains 9.4 / 10.5.  K = V = 32 runs 32 columns and eight CTAs per SM:
+//   2048 chains of 64 tokens 230 / 71.
+//   K over 64 also runs 64 columns for few tokens, where the states' way in and out is most of the time, so that more CTAs
+//   move states while others compute: up to 4 tokens (2048 chains of 4 tokens 58.9 / 55.4, of 6 72.6 / 74.7), up to 8 on average where
+//   lengths differ (48 sequences of 32 heads 54.3 / 50.6 at 4, 89.9 / 86.7 at 8, 104 / 108 at 12).
 // * many: state rows that are not 16-byte aligned, more than two turns: one column per lane, but 32 per CTA and two CTAs
 //   per SM.  K = 128, V = 130, one token at a time in 16 / 32 columns: 48 chains (432 slices) 15.8 / 10.1 at 3 tokens, 56 / 44 at
 //   64 (blocks of four: 56 at 64 and 384 slices).
@@ -693,7 +702,7 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
   const int64_t slices = (int64_t)p.nseq * p.H * ((p.V + 15) / 16);
   const int64_t tokens = p.cu_seqlens && p.nseq > 0 ? p.T / p.nseq : p.T;      // per sequence, on average
   const bool aligned = (((uintptr_t)p.h0 | (uintptr_t)p.ht) & 15) == 0 && p.V % 4 == 0 && p.slot_stride % 4 == 0;
-  const int turns = tokens >= 2 && tokens <= 8 ? 1 : (p.K <= 32 && tokens >= 64 ? 4 : 2);
+  const int turns = tokens >= 2 && tokens <= 8 ? 1 : 2 + (tokens >= 16 && p.K > 32) + (tokens >= 64);
   const bool wide = aligned && p.K <= 128 && slices > (int64_t)turns * sms;
   const bool many = !aligned && p.K <= 128 && slices > 2 * sms;
   const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || slices <= sms ? 1 : (p.K <= 32 ? 2 : 3));
@@ -705,8 +714,17 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
   }
   if (p.K > 128) return launch_scan<32, 1, 4, 4, 2>(p, cumulative, s);
   if (wide) {
-    if (p.K <= 32) return launch_scan<4, 4, 8, 0, 2>(p, cumulative, s);
-    if (p.K <= 64) return launch_scan<8, 4, 8, 0, 2>(p, cumulative, s);
+    const bool narrow = (p.V - 1) % 128 < 64 && (p.V <= 64 || (int64_t)p.nseq * p.H * ((p.V + 127) / 128) > 2 * sms);
+    if (p.K <= 32) {
+      if (p.V <= 32) return launch_scan<4, 4, 2, 0, 8>(p, cumulative, s);
+      if (narrow) return launch_scan<4, 4, 4, 0, 4>(p, cumulative, s);
+      return launch_scan<4, 4, 8, 0, 2>(p, cumulative, s);
+    }
+    if (p.K <= 64) {
+      if (narrow) return launch_scan<8, 4, 4, 0, 4>(p, cumulative, s);
+      return launch_scan<8, 4, 8, 0, 2>(p, cumulative, s);
+    }
+    if (narrow || tokens <= (p.cu_seqlens ? 8 : 4)) return launch_scan<16, 4, 4, 0, 4>(p, cumulative, s);
     return launch_scan<16, 4, 8, 0, 2>(p, cumulative, s);
   }
   if (many) {

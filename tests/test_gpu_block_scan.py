@@ -52,3 +52,18 @@ def test_mixed_dtypes_and_gates_that_forget():
     err = float((o.double().cpu() - want_o).abs().max() / want_o.abs().max())
     assert err < 2.0 ** -8 + TOL
     _close(s, want_s, "state")
+
+
+@pytest.mark.parametrize("kd,vd", [(128, 128), (96, 64), (72, 100), (65, 132)])
+def test_many_chains_of_few_tokens(kd, vd):
+    """64 columns per CTA and tiles of four tokens: lengths around 4 and 8 that average under 8, column counts around 64."""
+    lengths = [4, 1, 0, 3, 5, 8, 9, 20, 7, 2, 12, 16] * 2
+    inp = orc.make_inputs(1, sum(lengths), 4, kd, vd, seed=kd, with_state=True, lengths=lengths)
+    dev = {n: t.cuda() if torch.is_tensor(t) else t for n, t in inp.items()}
+    want_o, want_s = orc.recurrent_kda_ref(*(inp[n].double() for n in ("q", "k", "v", "gate_log2", "beta", "h0")),
+                                           inp["cu_seqlens"])
+    for call, gate in ((kda_b200.recurrent_kda, "gate_log2"), (kda_b200.chunk_kda, "cum_gate")):
+        o, s = call(dev["q"], dev["k"], dev["v"], dev[gate], dev["beta"], dev["h0"], cu_seqlens=dev["cu_seqlens"],
+                    output_final_state=True, **({"exact_fp32": True} if gate == "cum_gate" else {}))
+        _close(o, want_o, "output")
+        _close(s, want_s, "state")
