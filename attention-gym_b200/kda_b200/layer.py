@@ -34,7 +34,7 @@ import torch.nn.functional as F
 from .chunk_schedule import prepare_ragged_chunk_metadata
 from .fused import chunk_forward as _chunk_kda, chunk_forward_qkv as _chunk_kda_qkv
 from .masking import active_token_mask, mask_inactive_token_gradients, mask_inactive_tokens
-from .ops import widen_op
+from .ops import sum_gradients_op, widen_op
 from .preops import _bounded_gate_cumsum, causal_conv1d, gated_output_norm, l2norm
 from .reference_impl import reference_kda
 
@@ -54,6 +54,29 @@ class _CastWeight(torch.autograd.Function):
         if torch.is_grad_enabled():            # to be differentiated once more
             return grad.to(torch.float32)
         return widen_op(grad)
+
+
+class _FanOut(torch.autograd.Function):
+    """One activation for the four projections that read it; their gradients are added in one pass and rounded once."""
+
+    generate_vmap_rule = True
+
+    @staticmethod
+    def forward(x):
+        return tuple(x.view_as(x) for _ in range(4))
+
+    @staticmethod
+    def setup_context(ctx, inputs, output):
+        ctx.set_materialize_grads(False)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        grads = [g for g in grads if g is not None]
+        if len(grads) < 2:
+            return grads[0] if grads else None
+        if torch.is_grad_enabled():            # to be differentiated once more
+            return sum(grads[1:], grads[0])
+        return sum_gradients_op(grads)
 
 
 class KDAAttentionOutput(NamedTuple):
@@ -140,10 +163,11 @@ class KDAAttention(nn.Module):
                               groups=channels).transpose(1, 2))
         return out, (ext[:, tokens:].clone() if return_final_state else None)
 
-    def gate_projections(self, hidden):
+    def gate_projections(self, hidden, beta_hidden=None):
+        """``beta_hidden``: another alias of ``hidden``, so that the gradients of the two meet where all of them do."""
         batch, tokens, _ = hidden.shape
         raw = self._linear(self._linear(hidden, self.f_a_proj), self.f_b_proj)
-        beta = self._linear(hidden, self.beta_proj).view(batch, tokens, self.num_heads).float().sigmoid()
+        beta = self._linear(hidden if beta_hidden is None else beta_hidden, self.beta_proj).view(batch, tokens, self.num_heads).float().sigmoid()
         return raw.view(batch, tokens, self.num_heads, self.head_dim).contiguous(), beta
 
     def _reference_core(self, q, k, v, raw_gate, beta, initial_state, return_final_state):
@@ -181,12 +205,15 @@ class KDAAttention(nn.Module):
         mask = (active_token_mask(hidden_states, cu_seqlens)
                 if self.mask_inactive_capacity and cu_seqlens is not None else None)
         hidden = mask_inactive_tokens(hidden_states, mask).to(self.compute_dtype)
-        qkv = mask_inactive_token_gradients(self._linear(hidden, self.qkv_proj), mask)
+        fan = self.backend == "fused" and hidden.is_cuda and hidden.requires_grad and torch.is_grad_enabled()
+        for_qkv, for_gate, for_beta, for_output = _FanOut.apply(hidden) if fan else (hidden,) * 4
+        qkv = mask_inactive_token_gradients(self._linear(for_qkv, self.qkv_proj), mask)
         qkv, final_conv_state = self.short_convolution(qkv, initial_conv_state, cu_seqlens=cu_seqlens,
                                                        return_final_state=return_final_state)
         qkv = mask_inactive_tokens(qkv, mask)
         qkv = qkv.view(batch, tokens, 3, self.num_heads, self.head_dim)
-        raw_gate, beta = self.gate_projections(hidden)
+        own = fan and getattr(self.gate_projections, "__func__", None) is KDAAttention.gate_projections
+        raw_gate, beta = self.gate_projections(for_gate, for_beta) if own else self.gate_projections(for_gate)
         raw_gate = mask_inactive_token_gradients(raw_gate, mask)
         beta = mask_inactive_token_gradients(beta, mask)
         if self.backend == "reference":
@@ -208,7 +235,7 @@ class KDAAttention(nn.Module):
                                               metadata=metadata, output_final_state=return_final_state,
                                               fastmath=self.fastmath)
         out = mask_inactive_tokens(out, mask)
-        logits = self._linear(self._linear(hidden, self.g_a_proj), self.g_b_proj).view_as(out)
+        logits = self._linear(self._linear(for_output, self.g_a_proj), self.g_b_proj).view_as(out)
         if self.backend == "fused":
             gated = gated_output_norm(out, logits, self.output_norm_weight, self.rms_norm_eps)
         else:
