@@ -228,35 +228,6 @@ __global__ void __launch_bounds__(256) widen_kernel(const uint2* __restrict__ x,
   }
 }
 
-// The sum of up to four bf16 tensors in fp32, rounded once: the gradients that reach one activation from the projections that
-// read it.  Bound by memory, four reads and a write in one pass: 53 us for four tensors of 33.5 M elements; added pair by pair they
-// are three passes of three (93 us) and three roundings.
-struct SumParams { const uint4* in[4]; uint4* out; int count; int64_t n8; };
-__global__ void __launch_bounds__(256) sum_kernel(const SumParams p) {
-  const int64_t i0 = (int64_t)blockIdx.x * 512 + threadIdx.x;
-  uint4 raw[4][2];
-#pragma unroll
-  for (int t = 0; t < 4; ++t)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      raw[t][j] = t < p.count && i0 + 256 * j < p.n8 ? p.in[t][i0 + 256 * j] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    uint32_t o[4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 v = unpack_bf16(reinterpret_cast<const uint32_t*>(&raw[t][j])[h]);
-        acc.x = t ? acc.x + v.x : v.x; acc.y = t ? acc.y + v.y : v.y;
-      }
-      o[h] = pack_bf16(acc.x, acc.y);
-    }
-    if (i0 + 256 * j < p.n8) p.out[i0 + 256 * j] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-}
-
 static bool epilogue_vec_ok(int dtype, int dim, const void* a, const void* b, const void* c,
                             const void* d, const void* e) {
   const uintptr_t bits = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e;
@@ -328,22 +299,5 @@ extern "C" int kda_widen(const void* x, int dtype, float* y, int64_t n, void* st
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
   kda::widen_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
       reinterpret_cast<const uint2*>(x), dtype, reinterpret_cast<float4*>(y), n4);
-  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
-}
-
-extern "C" int kda_sum_bf16(const void* const* in, int count, void* out, int64_t n, void* stream) {
-  if (!in || !out || count < 1 || n < 0) return KDA_ERR_ARG;
-  if (count > 4 || n % 8 || ((uintptr_t)out & 15) != 0) return KDA_ERR_UNSUPPORTED;
-  kda::SumParams p{};
-  for (int i = 0; i < count; ++i) {
-    if (!in[i]) return KDA_ERR_ARG;
-    if (((uintptr_t)in[i] & 15) != 0) return KDA_ERR_UNSUPPORTED;
-    p.in[i] = reinterpret_cast<const uint4*>(in[i]);
-  }
-  p.out = reinterpret_cast<uint4*>(out); p.count = count; p.n8 = n / 8;
-  const int64_t blocks = (p.n8 + 511) / 512;
-  if (n == 0) return KDA_OK;
-  if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
-  kda::sum_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }

@@ -103,7 +103,6 @@ _SIGNATURES = {
     "kda_decode_prep": (c_int, [c_void_p] * 5 + [c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_float, c_float,
                                                                                       c_void_p]),
     "kda_widen": (c_int, [c_void_p, c_int, c_void_p, c_int64, c_void_p]),
-    "kda_sum_bf16": (c_int, [c_void_p, c_int, c_void_p, c_int64, c_void_p]),
     "kda_conv1d_decode": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
 }
 

@@ -34,7 +34,7 @@ import torch.nn.functional as F
 from .chunk_schedule import prepare_ragged_chunk_metadata
 from .fused import chunk_forward as _chunk_kda, chunk_forward_qkv as _chunk_kda_qkv
 from .masking import active_token_mask, mask_inactive_token_gradients, mask_inactive_tokens
-from .ops import sum_gradients_op, widen_op
+from .ops import widen_op
 from .preops import _bounded_gate_cumsum, causal_conv1d, gated_output_norm, l2norm
 from .reference_impl import reference_kda
 
@@ -54,29 +54,6 @@ class _CastWeight(torch.autograd.Function):
         if torch.is_grad_enabled():            # to be differentiated once more
             return grad.to(torch.float32)
         return widen_op(grad)
-
-
-class _FanOut(torch.autograd.Function):
-    """One activation for the four projections that read it; their gradients are added in one pass and rounded once."""
-
-    generate_vmap_rule = True
-
-    @staticmethod
-    def forward(x):
-        return tuple(x.view_as(x) for _ in range(4))
-
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        ctx.set_materialize_grads(False)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        grads = [g for g in grads if g is not None]
-        if len(grads) < 2:
-            return grads[0] if grads else None
-        if torch.is_grad_enabled():            # to be differentiated once more
-            return sum(grads[1:], grads[0])
-        return sum_gradients_op(grads)
 
 
 class KDAAttentionOutput(NamedTuple):
@@ -135,12 +112,15 @@ class KDAAttention(nn.Module):
         self.dt_bias = nn.Parameter(torch.zeros(num_heads, head_dim, device=device, dtype=torch.float32))
 
     # ---- stages -------------------------------------------------------------------------------
-    def _linear(self, x, layer):
+    def _cast(self, layer):
         weight = layer.weight
         if (self.backend == "fused" and type(weight) is nn.Parameter and weight.is_cuda and weight.requires_grad
                 and weight.dtype == torch.float32 and torch.is_grad_enabled()):
-            return F.linear(x, _CastWeight.apply(weight))
-        return F.linear(x, weight.to(self.compute_dtype))
+            return _CastWeight.apply(weight)
+        return weight.to(self.compute_dtype)
+
+    def _linear(self, x, layer):
+        return F.linear(x, self._cast(layer))
 
     def short_convolution(self, qkv, initial_state, *, cu_seqlens=None, return_final_state=False):
         batch, tokens, channels = qkv.shape
@@ -163,12 +143,26 @@ class KDAAttention(nn.Module):
                               groups=channels).transpose(1, 2))
         return out, (ext[:, tokens:].clone() if return_final_state else None)
 
-    def gate_projections(self, hidden, beta_hidden=None):
-        """``beta_hidden``: another alias of ``hidden``, so that the gradients of the two meet where all of them do."""
-        batch, tokens, _ = hidden.shape
-        raw = self._linear(self._linear(hidden, self.f_a_proj), self.f_b_proj)
-        beta = self._linear(hidden if beta_hidden is None else beta_hidden, self.beta_proj).view(batch, tokens, self.num_heads).float().sigmoid()
+    def gate_projections(self, hidden):
+        return self._gates(self._linear(hidden, self.f_a_proj), self._linear(hidden, self.beta_proj))
+
+    def _gates(self, low, beta_logits):
+        batch, tokens, _ = low.shape
+        raw = self._linear(low, self.f_b_proj)
+        beta = beta_logits.view(batch, tokens, self.num_heads).float().sigmoid()
         return raw.view(batch, tokens, self.num_heads, self.head_dim).contiguous(), beta
+
+    def _narrow_projections(self, hidden):
+        """``f_a_proj``, ``g_a_proj`` and ``beta_proj`` in one GEMM, or None.  Each of the three reads all of ``hidden`` for 128 columns
+        or fewer, forward and backward, and their input gradients have to be added.  8192 tokens of 4096 channels, us apart /
+        together: forward 61 / 24, weight gradients 54 / 23, input gradients 45 / 21, their sum 93 / 30; for that two small copies of
+        the weights and of the gradients, 10.  Only where the columns of every part start on 16 bytes."""
+        parts = (self.f_a_proj, self.g_a_proj, self.beta_proj)
+        own = getattr(self.gate_projections, "__func__", None) is KDAAttention.gate_projections
+        if self.backend != "fused" or not own or any(p.weight.shape[0] % 8 for p in parts):
+            return None
+        weights = [self._cast(p) for p in parts]
+        return F.linear(hidden, torch.cat(weights)).split([w.shape[0] for w in weights], -1)
 
     def _reference_core(self, q, k, v, raw_gate, beta, initial_state, return_final_state):
         """Eager fp32 evaluation of the normalisation, the gate and the recurrence (dense input)."""
@@ -205,15 +199,13 @@ class KDAAttention(nn.Module):
         mask = (active_token_mask(hidden_states, cu_seqlens)
                 if self.mask_inactive_capacity and cu_seqlens is not None else None)
         hidden = mask_inactive_tokens(hidden_states, mask).to(self.compute_dtype)
-        fan = self.backend == "fused" and hidden.is_cuda and hidden.requires_grad and torch.is_grad_enabled()
-        for_qkv, for_gate, for_beta, for_output = _FanOut.apply(hidden) if fan else (hidden,) * 4
-        qkv = mask_inactive_token_gradients(self._linear(for_qkv, self.qkv_proj), mask)
+        qkv = mask_inactive_token_gradients(self._linear(hidden, self.qkv_proj), mask)
         qkv, final_conv_state = self.short_convolution(qkv, initial_conv_state, cu_seqlens=cu_seqlens,
                                                        return_final_state=return_final_state)
         qkv = mask_inactive_tokens(qkv, mask)
         qkv = qkv.view(batch, tokens, 3, self.num_heads, self.head_dim)
-        own = fan and getattr(self.gate_projections, "__func__", None) is KDAAttention.gate_projections
-        raw_gate, beta = self.gate_projections(for_gate, for_beta) if own else self.gate_projections(for_gate)
+        narrow = self._narrow_projections(hidden)
+        raw_gate, beta = self.gate_projections(hidden) if narrow is None else self._gates(narrow[0], narrow[2])
         raw_gate = mask_inactive_token_gradients(raw_gate, mask)
         beta = mask_inactive_token_gradients(beta, mask)
         if self.backend == "reference":
@@ -235,7 +227,8 @@ class KDAAttention(nn.Module):
                                               metadata=metadata, output_final_state=return_final_state,
                                               fastmath=self.fastmath)
         out = mask_inactive_tokens(out, mask)
-        logits = self._linear(self._linear(for_output, self.g_a_proj), self.g_b_proj).view_as(out)
+        low = self._linear(hidden, self.g_a_proj) if narrow is None else narrow[1]
+        logits = self._linear(low, self.g_b_proj).view_as(out)
         if self.backend == "fused":
             gated = gated_output_norm(out, logits, self.output_norm_weight, self.rms_norm_eps)
         else:

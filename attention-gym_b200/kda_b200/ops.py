@@ -142,7 +142,6 @@ _lib_layer.define("chunk_bwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta
                 "-> (Tensor, Tensor, Tensor, Tensor)")
 # A 16-bit tensor as fp32 (the gradient of a weight that was cast for its GEMM).
 _lib_layer.define("widen(Tensor x) -> Tensor")
-_lib_layer.define("sum_gradients(Tensor[] grads) -> Tensor")
 
 
 _cabi.load_torch_library()
@@ -761,26 +760,6 @@ def _(x):
     return x.new_empty(x.shape, dtype=torch.float32)
 
 
-@torch.library.impl(_lib_layer, "sum_gradients", "CUDA")
-def _sum_gradients(grads):
-    first = grads[0]
-    if first.dtype != torch.bfloat16 or any(t.shape != first.shape or t.dtype != first.dtype for t in grads):
-        raise ValueError("sum_gradients takes bfloat16 tensors of one shape")
-    grads = [t.contiguous() for t in grads]
-    out = torch.empty(first.shape, dtype=first.dtype, device=first.device)
-    if out.numel() % 8 or len(grads) > 4 or any(t.data_ptr() % 16 for t in grads):
-        return out.copy_(sum(t.float() for t in grads))
-    ptrs = (ctypes.c_void_p * len(grads))(*(t.data_ptr() for t in grads))
-    if out.numel():
-        _cabi.call("kda_sum_bf16", 1, ctypes.addressof(ptrs), len(grads), out.data_ptr(), out.numel(), _cabi.stream())
-    return out
-
-
-@torch.library.register_fake(f"{_NS_LAYER}::sum_gradients")
-def _(grads):
-    return grads[0].new_empty(grads[0].shape)
-
-
 @torch.library.register_fake(f"{_NS_OWN}::decode_step")
 def _(x, weight, conv_state, state_pool, state_indices, raw_gate, A_log, dt_bias, beta, activation, lower_bound, eps):
     return x.new_empty((x.shape[0], state_pool.shape[1], 128))
@@ -826,7 +805,6 @@ chunk_bwd_with_state_grad_op = _ops.kda_chunk_bwd_with_state_grad.default
 chunk_fwd_qkv_op = torch.ops.kda_b200_layer.chunk_fwd_qkv.default
 chunk_bwd_qkv_op = torch.ops.kda_b200_layer.chunk_bwd_qkv.default
 widen_op = torch.ops.kda_b200_layer.widen.default
-sum_gradients_op = torch.ops.kda_b200_layer.sum_gradients.default
 chunk_scan_op = torch.ops.kda_b200_fused.chunk_scan.default
 decode_step_op = torch.ops.kda_b200_fused.decode_step.default
 recurrent_fwd_op = _ops.kda_recurrent_fwd.default

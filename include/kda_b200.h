@@ -391,10 +391,6 @@ int kda_conv1d_decode(const void* x, const void* weight, void* state, const int3
 /* y = x as fp32, n values of a 16-bit dtype (n a multiple of 8, both addresses 16-byte aligned). */
 int kda_widen(const void* x, int dtype, float* y, int64_t n, void* stream);
 
-/* out = the sum of `count` (1 to 4) bf16 tensors of n values, added in fp32 and rounded once (n a multiple of 8, all addresses
- * 16-byte aligned; out may be one of the inputs).  `in` is read on the host. */
-int kda_sum_bf16(const void* const* in, int count, void* out, int64_t n, void* stream);
-
 /* Decode-step preprocessing in one launch: the q | k | v projection x [N, 3 * H * 128] goes through the
  * depthwise causal convolution over the paged history conv_state [num_slots, W-1, 3 * H * 128] (advanced
  * in place; conv_state_indices as for kda_conv1d_decode, NULL = slot i for sequence i) and the
