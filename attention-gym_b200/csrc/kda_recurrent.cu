@@ -663,9 +663,9 @@ static int launch_block_scan(const ScanParams& p, bool cumulative, cudaStream_t 
 template <int KR, int VC, int NW, int NP, int MINB>
 static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream) {
   constexpr int CT = 4 * VC * NW, KP = 8 * KR;
-  // 24 KiB of operands in two buffers (K = 128: 8 tokens, 4 where four CTAs share an SM); the wide form also buffers its
+  // 24 KiB of operands in two buffers (K = 128: 8 tokens, 4 or 2 where four or eight CTAs share an SM); the wide form also buffers its
   // columns of v and o
-  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : (MINB == 4 ? 512 : 1024) / KP;
+  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : (2048 / MINB) / KP;
   const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + CT - 1) / CT);
   if (blocks <= 0) return KDA_OK;
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
@@ -690,6 +690,9 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
 //   K over 64 also runs 64 columns for few tokens, where the states' way in and out is most of the time, so that more CTAs
 //   move states while others compute: up to 4 tokens (2048 chains of 4 tokens 58.9 / 55.4, of 6 72.6 / 74.7), up to 8 on average where
 //   lengths differ (48 sequences of 32 heads 54.3 / 50.6 at 4, 89.9 / 86.7 at 8, 104 / 108 at 12).
+//   Up to 2 tokens 32 columns and eight CTAs: 64 columns / 32, 48 sequences 42.3 / 38.0 at 1, 45.3 / 43.0 at 2, 50.4 / 49.8 at 3, 51.6 /
+//   52.7 at 4; 128 sequences 101.6 / 91.3 at 1, 105.8 / 100.8 at 2.  Not for V up to 64 (2048 chains of 2 20.0 / 20.7) and the cumulative
+//   gate (39.6 / 43.7).
 // * many: state rows that are not 16-byte aligned, more than two turns: one column per lane, but 32 per CTA and two CTAs
 //   per SM.  K = 128, V = 130, one token at a time in 16 / 32 columns: 48 chains (432 slices) 15.8 / 10.1 at 3 tokens, 56 / 44 at
 //   64 (blocks of four: 56 at 64 and 384 slices).
@@ -724,6 +727,7 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
       if (narrow) return launch_scan<8, 4, 4, 0, 4>(p, cumulative, s);
       return launch_scan<8, 4, 8, 0, 2>(p, cumulative, s);
     }
+    if (tokens <= 2 && p.V > 64 && !cumulative) return launch_scan<16, 4, 2, 0, 8>(p, cumulative, s);
     if (narrow || tokens <= (p.cu_seqlens ? 8 : 4)) return launch_scan<16, 4, 4, 0, 4>(p, cumulative, s);
     return launch_scan<16, 4, 8, 0, 2>(p, cumulative, s);
   }

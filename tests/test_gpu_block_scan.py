@@ -55,9 +55,9 @@ def test_mixed_dtypes_and_gates_that_forget():
 
 
 @pytest.mark.parametrize("kd,vd", [(128, 128), (96, 64), (72, 100), (65, 132)])
-def test_many_chains_of_few_tokens(kd, vd):
-    """64 columns per CTA and tiles of four tokens: lengths around 4 and 8 that average under 8, column counts around 64."""
-    lengths = [4, 1, 0, 3, 5, 8, 9, 20, 7, 2, 12, 16] * 2
+@pytest.mark.parametrize("lengths", [[4, 1, 0, 3, 5, 8, 9, 20, 7, 2, 12, 16] * 2, [1, 2, 0, 3, 1, 1, 2, 5, 1, 2] * 4], ids=["few", "one"])
+def test_many_chains_of_few_tokens(kd, vd, lengths):
+    """64 or 32 columns per CTA and tiles of four or two tokens: lengths around these that average under 8 and under 2."""
     inp = orc.make_inputs(1, sum(lengths), 4, kd, vd, seed=kd, with_state=True, lengths=lengths)
     dev = {n: t.cuda() if torch.is_tensor(t) else t for n, t in inp.items()}
     want_o, want_s = orc.recurrent_kda_ref(*(inp[n].double() for n in ("q", "k", "v", "gate_log2", "beta", "h0")),
