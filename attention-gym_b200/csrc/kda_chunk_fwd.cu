@@ -259,8 +259,8 @@ extern "C" int kda_chunk_slice_map(const float* cum_gate, float* b_out, float* t
 // ------------------------------------------------------------------------------------------------
 namespace kda {
 
-int launch_state_affine(const float* M, const float* hin, const float* b, float* hout, int groups,
-                        int group, int64_t in_stride, int64_t out_stride, int K, int V, cudaStream_t s);
+int launch_state_chain(const float* M, const float* b, const float* h0, float* hin, float* fin, int rows, int heads, int segs,
+                       cudaStream_t s);
 
 static int g_row_segments = 0;   // 0 = choose; otherwise the forced number of segments per row (tests, tuning)
 
@@ -404,25 +404,8 @@ static int chunk_fwd_dense_impl(bool keep, float* rstd_q, float* rstd_k, float e
   rc = kda::launch_state_fwd(p, s);
   if (rc) return rc;
   // ---- chain along each row: h_in(0) = the row's initial state, h_in(s + 1) = M_s h_in(s) + b_s
-  const size_t row_bytes = (size_t)heads * 128 * 128 * 4;
-  cudaError_t e = initial_state
-      ? cudaMemcpy2DAsync(hin, row_bytes * pl.segs, initial_state, row_bytes, row_bytes, batch,
-                          cudaMemcpyDeviceToDevice, s)
-      : cudaMemset2DAsync(hin, row_bytes * pl.segs, 0, row_bytes, batch, s);
-  if (e != cudaSuccess) return KDA_ERR_LAUNCH;
-  const int64_t per_seg = (int64_t)heads * 128 * 128;
-  for (int sg = 0; sg + 1 < pl.segs; ++sg) {
-    rc = kda::launch_state_affine(trans + sg * per_seg, hin + sg * per_seg, b + sg * per_seg,
-                                  hin + (sg + 1) * per_seg, batch, heads, (int64_t)pl.segs * heads,
-                                  (int64_t)pl.segs * heads, 128, 128, s);
-    if (rc) return rc;
-  }
-  if (final_state) {
-    const int last = pl.segs - 1;
-    rc = kda::launch_state_affine(trans + last * per_seg, hin + last * per_seg, b + last * per_seg,
-                                  final_state, batch, heads, (int64_t)pl.segs * heads, heads, 128, 128, s);
-    if (rc) return rc;
-  }
+  rc = kda::launch_state_chain(trans, b, initial_state, hin, final_state, batch, heads, pl.segs, s);
+  if (rc) return rc;
   // ---- pass B: the leading chunks of every segment with its true entering state
   p.h0 = hin; p.ht = nullptr; p.trans_out = nullptr; p.limit_out = nullptr; p.limit_in = limit;
   return kda::launch_state_fwd(p, s);

@@ -18,16 +18,12 @@ template <bool VEC>
 __global__ void __launch_bounds__(128, 4) state_affine_kernel(const float* __restrict__ M,
                                                            const float* __restrict__ hin,
                                                            const float* __restrict__ b,
-                                                           float* __restrict__ hout, int K, int V,
-                                                           int group, int64_t in_stride,
-                                                           int64_t out_stride) {
+                                                           float* __restrict__ hout, int K, int V) {
   __shared__ __align__(16) float sM[32][kAffineSlab + 4];
   __shared__ __align__(16) float sH[kAffineSlab][32];
   const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, tid = threadIdx.x;
   const int tx = tid & 7, ty = tid >> 3;
-  // matrix blockIdx.z = (g, i) with i < group: inputs at g * in_stride + i, output at g * out_stride + i
-  const int64_t n = (int64_t)(blockIdx.z / group) * in_stride + blockIdx.z % group;
-  const int64_t no = (int64_t)(blockIdx.z / group) * out_stride + blockIdx.z % group;
+  const int64_t n = blockIdx.z;
   const float* Mn = M + n * K * K;
   const float* Hn = hin + n * K * V;
   auto copy = [](float* to, const float* from) {            // four values to shared memory, in flight together if VEC
@@ -72,21 +68,119 @@ __global__ void __launch_bounds__(128, 4) state_affine_kernel(const float* __res
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
-    *reinterpret_cast<float4*>(hout + no * K * V + (int64_t)(r0 + ty + 16 * i) * V + c0 + 4 * tx) =
+    *reinterpret_cast<float4*>(hout + n * K * V + (int64_t)(r0 + ty + 16 * i) * V + c0 + 4 * tx) =
         make_float4(acc[i][0] + bv[i].x, acc[i][1] + bv[i].y, acc[i][2] + bv[i].z, acc[i][3] + bv[i].w);
 }
 
-// `groups` x `group` products; the matrices of group g start at index g * in_stride (inputs) and
-// g * out_stride (output).
-int launch_state_affine(const float* M, const float* hin, const float* b, float* hout, int groups,
-                        int group, int64_t in_stride, int64_t out_stride, int K, int V, cudaStream_t s) {
-  if (groups <= 0 || group <= 0) return KDA_OK;
-  dim3 grid(V / 32, K / 32, groups * group);
-  if ((((uintptr_t)M | (uintptr_t)hin) & 15) == 0)
-    state_affine_kernel<true><<<grid, 128, 0, s>>>(M, hin, b, hout, K, V, group, in_stride, out_stride);
-  else
-    state_affine_kernel<false><<<grid, 128, 0, s>>>(M, hin, b, hout, K, V, group, in_stride, out_stride);
+// The chain of such maps along the segments of a row, K = V = 128: h(s + 1) = M_s h(s) + b_s from the row's initial state (zero if
+// NULL), every h(s) written to hin and the last one to fin (if given).  A column of h needs only the same column before it, so a
+// CTA carries COLS columns of one head through all segments in one launch, without waiting for any other; the next M is on its
+// way while one is multiplied.  A thread adds one or two rows x four columns in the order of K, as state_affine_kernel does.
+// Bound by the chain: loads, 128 steps and two barriers a map on one SM.  32 heads, four maps: 28 us, as four launches of that
+// kernel and the copy of the initial state 43; forward of 32768 tokens of 8 heads, eight maps, 475 us with launches, 370 with this
+// kernel (375 with 32 columns per CTA for so few heads).
+constexpr int kChainThreads = 512;
+constexpr int kChainPitch = 132;
+struct ChainParams {
+  const float* M; const float* b;      // [rows, segs, heads, 128, 128]
+  const float* h0;                     // [rows, heads, 128, 128] or NULL
+  float* hin;                          // [rows, segs, heads, 128, 128]
+  float* fin;                          // [rows, heads, 128, 128] or NULL
+  int heads, segs;
+};
+template <int COLS>
+__global__ void __launch_bounds__(kChainThreads) state_chain_kernel(const ChainParams p) {
+  constexpr int Q = COLS / 4, R = COLS / 16, SLICES = 128 / COLS;      // column quads; rows per thread, 128 / R apart
+  extern __shared__ __align__(16) float smem_chain[];
+  float* const sH = smem_chain + 2 * 128 * kChainPitch;       // [128][COLS]
+  const int tid = threadIdx.x, cq = 4 * (tid & (Q - 1)), r0 = tid / Q;
+  const int c0 = COLS * (blockIdx.x % SLICES), item = blockIdx.x / SLICES;
+  const int row = item / p.heads, head = item % p.heads;
+  auto state = [&](int sg) { return ((int64_t)(row * (int64_t)p.segs + sg) * p.heads + head) * 16384; };
+  auto fetch = [&](int sg) {
+    const float* m = p.M + state(sg);
+    float* to = smem_chain + (sg & 1) * 128 * kChainPitch;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+      const int e = tid + kChainThreads * l;
+      cp_async16(to + (e >> 5) * kChainPitch + 4 * (e & 31), m + 4 * e, true);
+    }
+    cp_async_commit();
+  };
+  const int maps = p.fin ? p.segs : p.segs - 1;
+  if (maps > 0) fetch(0);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int r = r0 + 64 * i;
+    const int64_t at = (int64_t)r * 128 + c0 + cq;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.h0) {                                               // (a caller's: it may start off a 16-byte address)
+      const float* h = p.h0 + (int64_t)item * 16384 + at;
+      x = make_float4(h[0], h[1], h[2], h[3]);
+    }
+    *reinterpret_cast<float4*>(sH + r * COLS + cq) = x;
+    *reinterpret_cast<float4*>(p.hin + state(0) + at) = x;
+  }
+  for (int sg = 0; sg < maps; ++sg) {
+    float4 bv[R], acc[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      bv[i] = *reinterpret_cast<const float4*>(p.b + state(sg) + (int64_t)(r0 + 64 * i) * 128 + c0 + cq);
+      acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (sg + 1 < maps) { fetch(sg + 1); cp_async_wait<1>(); }
+    else cp_async_wait<0>();
+    __syncthreads();                                          // M_s and h(s) are in shared memory
+    const float* m = smem_chain + (sg & 1) * 128 * kChainPitch + r0 * kChainPitch;
+#pragma unroll 4
+    for (int k = 0; k < 128; k += 4) {
+      float a[R][4];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(m + 64 * i * kChainPitch + k);
+        a[i][0] = x.x; a[i][1] = x.y; a[i][2] = x.z; a[i][3] = x.w;
+      }
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        const float4 y = *reinterpret_cast<const float4*>(sH + (k + d) * COLS + cq);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          acc[i].x = fmaf(a[i][d], y.x, acc[i].x); acc[i].y = fmaf(a[i][d], y.y, acc[i].y);
+          acc[i].z = fmaf(a[i][d], y.z, acc[i].z); acc[i].w = fmaf(a[i][d], y.w, acc[i].w);
+        }
+      }
+    }
+    __syncthreads();                                          // h(s) and this buffer of M have been read
+    float* to = sg + 1 < p.segs ? p.hin + state(sg + 1) : p.fin + (int64_t)item * 16384;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = r0 + 64 * i;
+      const float4 x = make_float4(acc[i].x + bv[i].x, acc[i].y + bv[i].y, acc[i].z + bv[i].z, acc[i].w + bv[i].w);
+      *reinterpret_cast<float4*>(sH + r * COLS + cq) = x;
+      *reinterpret_cast<float4*>(to + (int64_t)r * 128 + c0 + cq) = x;
+    }
+  }
+}
+
+template <int COLS>
+static int launch_chain(const ChainParams& p, int64_t chains, cudaStream_t s) {
+  constexpr int smem = (2 * 128 * kChainPitch + 128 * COLS) * 4;
+  if (chains * (128 / COLS) > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
+  if (cudaFuncSetAttribute(state_chain_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return KDA_ERR_LAUNCH;
+  state_chain_kernel<COLS><<<(unsigned)(chains * (128 / COLS)), kChainThreads, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
+}
+
+// One CTA fits an SM: 16 columns each while that leaves no CTA waiting, else 32.
+int launch_state_chain(const float* M, const float* b, const float* h0, float* hin, float* fin, int rows, int heads, int segs,
+                       cudaStream_t s) {
+  if ((((uintptr_t)M | (uintptr_t)b | (uintptr_t)hin | (uintptr_t)fin) & 15) != 0) return KDA_ERR_ARG;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const ChainParams p{M, b, h0, hin, fin, heads, segs};
+  const int64_t chains = (int64_t)rows * heads;
+  return chains * 8 <= sms ? launch_chain<16>(p, chains, s) : launch_chain<32>(p, chains, s);
 }
 
 }  // namespace kda
@@ -96,6 +190,10 @@ extern "C" int kda_state_affine(const float* transition, const float* h_in, cons
   if (!transition || !h_in || !b || !h_out || count < 0) return KDA_ERR_ARG;
   if (key_dim % 64 || value_dim % 64 || key_dim <= 0 || value_dim <= 0) return KDA_ERR_UNSUPPORTED;
   if (count == 0) return KDA_OK;
-  return kda::launch_state_affine(transition, h_in, b, h_out, 1, count, 0, 0, key_dim, value_dim,
-                                  (cudaStream_t)stream);
+  dim3 grid(value_dim / 32, key_dim / 32, count);
+  if ((((uintptr_t)transition | (uintptr_t)h_in) & 15) == 0)
+    kda::state_affine_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(transition, h_in, b, h_out, key_dim, value_dim);
+  else
+    kda::state_affine_kernel<false><<<grid, 128, 0, (cudaStream_t)stream>>>(transition, h_in, b, h_out, key_dim, value_dim);
+  return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }

@@ -1,9 +1,12 @@
-"""h_out = M h_in + b at the edges of its slabs of K, for matrices that start off 16-byte addresses, against fp64."""
+"""h_out = M h_in + b at the edges of its slabs of K, for matrices that start off 16-byte addresses, against fp64; and the chain of
+such maps along the segments of a row, with and without entering and leaving states."""
 
 import pytest
 import torch
 
+import kda_b200
 from kda_b200 import _cabi
+from oracle import kda_oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +27,25 @@ def test_affine(kd, vd, offset):
     # kd fused multiply-adds and one addition, each rounded to 2^-24 of a partial sum of absolute values
     bound = (kd + 1) * 2.0 ** -24 * (m64.abs() @ h64.abs() + b.double().abs())
     assert ((out.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("segments", [2, 3, 5])
+@pytest.mark.parametrize("initial,final", [(True, True), (True, False), (False, True), (False, False)])
+def test_chain_of_segments(segments, initial, final):
+    """The boundary states of two rows through all their segments, with gates that hardly forget, against the serial walk."""
+    inp = orc.make_inputs(2, 64 * 12 - 7, 3, 128, 128, seed=segments, with_state=True)
+    q, k, v = (inp[n].bfloat16().cuda() for n in ("q", "k", "v"))
+    gate, beta = 0.02 * inp["cum_gate"].cuda(), inp["beta"].cuda()
+    h0 = inp["h0"].cuda() if initial else None
+
+    def run(forced):
+        try:
+            assert _cabi.lib().kda_set_row_segments(forced) == 0
+            return kda_b200.chunk_kda(q, k, v, gate, beta, h0, output_final_state=final)
+        finally:
+            _cabi.lib().kda_set_row_segments(0)
+
+    serial, split = run(1), run(segments)
+    # two bf16 evaluations of the products of up to twelve chunks: a few roundings of 2^-9 of the largest value
+    for x, y in zip(split[:2 if final else 1], serial):
+        assert float((x.double() - y.double()).abs().max() / y.double().abs().max()) < 1e-2
