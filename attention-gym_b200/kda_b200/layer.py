@@ -158,7 +158,7 @@ class KDAAttention(nn.Module):
         together: forward 61 / 24, weight gradients 54 / 23, input gradients 45 / 21, their sum 93 / 30; for that two small copies of
         the weights and of the gradients, 10.  Only where the columns of every part start on 16 bytes."""
         parts = (self.f_a_proj, self.g_a_proj, self.beta_proj)
-        own = getattr(self.gate_projections, "__func__", None) is KDAAttention.gate_projections
+        own = getattr(self.gate_projections, "__func__", None) is _GATE_PROJECTIONS
         if self.backend != "fused" or not own or any(p.weight.shape[0] % 8 for p in parts):
             return None
         weights = [self._cast(p) for p in parts]
@@ -238,5 +238,7 @@ class KDAAttention(nn.Module):
         result = mask_inactive_token_gradients(result, mask)
         return KDAAttentionOutput(result.to(hidden_states.dtype), final_state, final_conv_state)
 
+
+_GATE_PROJECTIONS = KDAAttention.gate_projections      # a replaced one is called as it is
 
 __all__ = ["KDAAttention", "KDAAttentionOutput"]
