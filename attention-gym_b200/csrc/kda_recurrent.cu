@@ -831,3 +831,19 @@ extern "C" int kda_chunk_scan_fwd(const void* q, const void* k, const void* v, c
   p.scale = scale;
   return launch_scan_any(p, true, (cudaStream_t)stream);
 }
+
+// The state-streaming kernel on one token per state, in place, with one wait that runs out: from its state `step` on, warp `warp`
+// of the first CTA does not wait (0..15 arithmetic, 16 copies, 17..22 operands).
+extern "C" int kda_selftest_bounded_stream(const float* q, const float* k, const float* v, const float* gate, const float* beta,
+                                           float* states, float* out, int nseq, int warp, int step, void* stream) {
+  using namespace kda;
+  if (!q || !k || !v || !gate || !beta || !states || !out || nseq < 1 || warp < 0 || warp > 22 || step < 0) return KDA_ERR_ARG;
+  ScanParams p{};
+  p.q = q; p.k = k; p.v = v; p.g = gate; p.beta = beta;
+  p.dt_q = p.dt_k = p.dt_v = p.dt_g = p.dt_beta = p.dt_out = KDA_F32;
+  p.h0 = states; p.ht = states; p.out = out;
+  p.nseq = nseq; p.T = 1; p.H = 1; p.K = p.V = 128;
+  p.slot_stride = 128 * 128;
+  p.scale = 0.08838834764831845f;  // 128^-0.5
+  return stream_takes(p) ? launch_stream_short(p, warp, step, (cudaStream_t)stream) : KDA_ERR_UNSUPPORTED;
+}

@@ -69,6 +69,8 @@ int device_sms();
 // The state-streaming kernel (kda_stream.cu).  A scan it can take: K = V = 128, 16-byte aligned states in and out.
 bool stream_takes(const ScanParams& p);
 int launch_stream(const ScanParams& p, cudaStream_t stream);
+// The same with a wait that runs out (kda_selftest_bounded_stream).
+int launch_stream_short(const ScanParams& p, int warp, int step, cudaStream_t stream);
 // The whole decode step in one launch, if its tensors allow the vector form of the preprocessing.
 bool fused_decode_takes(const PrepDecodeParams& d, const ScanParams& p);
 int launch_fused_decode(const PrepDecodeParams& d, const ScanParams& p, cudaStream_t stream);

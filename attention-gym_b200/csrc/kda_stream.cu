@@ -17,6 +17,10 @@
 // us per step of a captured graph, 32 heads, 1 / 37 / 256 sequences (of measured copy bandwidth at 256): the fused step
 // 6.6 / 21.8 / 189 (87 %), against 9.3 / 27.6 / 204 as two overlapping launches with q, k, v and the gate in memory between
 // them; given operands 5.2 / 19.4 / 179 (91 %), against 5.7 / 22.6 / 191 with the states as 32-column slabs in four rings.
+// Every wait is bounded.  One that runs out records code 64 and stops the CTA: the others look for that while they
+// wait, the four warps of a column group decide together behind their barrier (a warp that left alone would leave them there),
+// a state that was not advanced completely is never handed to the copying warp, and that warp waits for the loads it has
+// issued before the shared memory goes back.
 // (Several tokens per sequence on the same ring: one state at a time has 1.1 us a token, 48 sequences of 1 to 8 tokens 72
 // against 66 us of the token scan.  Bulk-copied states under the token scan's layout, two persistent CTAs per SM: 80 us.)
 #include "kda_recurrent.cuh"
@@ -38,6 +42,20 @@ static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
+}
+
+// A bounded wait of the kernel: false if it ran out, or another warp of the CTA has given up meanwhile.
+__device__ __forceinline__ bool wait_unless(uint64_t* bar, uint32_t parity, volatile int* abort, int limit) {
+#pragma unroll 1
+  for (int spin = 0; spin < limit; ++spin) {
+    if (mbar_wait(bar, parity, 1)) return true;
+    if ((spin & 63) == 63 && *abort) return false;
+  }
+  return false;
+}
+__device__ __forceinline__ void give_up(volatile int* abort, int* error) {
+  *abort = 1;
+  if (error) atomicExch(error, 64);
 }
 
 // pool slot of work item n = (sequence, head); < 0: padding (a non-positive or out of range index)
@@ -100,8 +118,11 @@ __device__ __forceinline__ void publish(float* o, int half, int lane, float (&x)
   reinterpret_cast<float4*>(dst)[1] = make_float4(x[4], x[5], x[6], x[7]);
 }
 
-template <int W>
-__global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParams p, const PrepDecodeParams d, int* error) {
+// SHORT (the self-test): the waits of warp `warp` of CTA 0 have no polls from its state `step` on.
+struct ShortWait { int warp, step; };
+template <int W, bool SHORT = false>
+__global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParams p, const PrepDecodeParams d, int* error,
+                                                                 const ShortWait short_wait) {
   extern __shared__ __align__(128) unsigned char sm[];
   float* ring = reinterpret_cast<float*>(sm);
   float* ops = ring + kStages * kStateFloats;
@@ -111,7 +132,8 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
   uint64_t* op_full = done + kStages;                                    // [slot] the operands are there
   uint64_t* op_free = op_full + kSlots;                                  // [slot] they have been used
   volatile int* s_abort = reinterpret_cast<volatile int*>(op_free + kSlots);
-  static_assert(8 * (2 * kStages + 2 * kSlots) + 4 <= 256, "barriers");
+  volatile int* s_stop = s_abort + 1;                                    // [column group][step parity] a warp's wait ran out
+  static_assert(8 * (2 * kStages + 2 * kSlots) + 4 * (1 + 8) <= 256, "barriers");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int items = p.nseq * p.H, stride = (int)gridDim.x;
@@ -122,7 +144,11 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
     mbar_init_fence();
     *s_abort = 0;
   }
+  if (tid < 8) s_stop[tid] = 0;
   __syncthreads();
+  auto polls = [&](int step) {
+    return SHORT && blockIdx.x == 0 && warp == short_wait.warp && step >= short_wait.step ? 0 : kSpinLimit;
+  };
   if (warp == 16) {
     // ---- copies ------------------------------------------------------------------------------------------
     if (lane != 0) return;
@@ -147,9 +173,10 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
     };
     while (loads < kStages && find(n)) load(loads);
     uint32_t ph = 0;
-    for (int stores = 0; stores < loads; ++stores) {
+    int stores = 0;
+    for (; stores < loads; ++stores) {
       const bool more = find(n);                 // looked up before the wait
-      if (!mbar_wait(&done[st], ph)) { *s_abort = 1; break; }
+      if (!wait_unless(&done[st], ph, s_abort, polls(stores))) { give_up(s_abort, error); break; }
       bulk_store(dst + (st == 0 ? off0 : (st == 1 ? off1 : off2)), ring + st * kStateFloats, kStateBytes);
       tma_store_commit();
       if (more) {
@@ -158,6 +185,8 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
       }
       if (++st == kStages) { st = 0; ph ^= 1; }
     }
+    // (after a full run every load has been waited for) what is still on its way has to land in this CTA's shared memory
+    for (int l = stores; l < loads; ++l) mbar_wait(&full[l % kStages], (l / kStages) & 1);
     tma_store_wait_read();
     return;
   }
@@ -228,8 +257,10 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
         }
       }
       const int at = step - 1, slot = at % kSlots;
-      if (!mbar_wait(&op_free[slot], ((at / kSlots) & 1) ^ 1)) { *s_abort = 1; return; }
-      __syncwarp();
+      if (!__all_sync(0xffffffffu, wait_unless(&op_free[slot], ((at / kSlots) & 1) ^ 1, s_abort, polls(at)))) {
+        give_up(s_abort, error);
+        return;
+      }
       publish(ops + slot * kSlotFloats, half, lane, x, beta, p.scale);
       __syncwarp();
       if (lane == 0) mbar_arrive(&op_full[slot]);
@@ -247,13 +278,18 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
       if (wj == 0) store_from_float(p.out, p.dt_out, (int64_t)n * 128 + col, 0.f);
       continue;
     }
-    if (!mbar_wait(&full[st], ph)) *s_abort = 1;        // bounded: give up, do not hang
+    bool ready = wait_unless(&full[st], ph, s_abort, polls(step));
     float* S = ring + st * kStateFloats + 32 * wj * 128 + col;
     f32x2 s[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i] = pack2(S[2 * i * 128], S[(2 * i + 1) * 128]);
     const int slot = step % kSlots;
-    if (!mbar_wait(&op_full[slot], (step / kSlots) & 1)) *s_abort = 1;
+    ready = ready && wait_unless(&op_full[slot], (step / kSlots) & 1, s_abort, polls(step));
+    volatile int* stop = s_stop + 2 * grp + (step & 1);      // (a warp that is a step ahead writes the other one)
+    if (!ready) {
+      give_up(s_abort, error);
+      *stop = 1;
+    }
     const float* o = ops + slot * kSlotFloats;
     const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(o + 32 * wj);
     const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(o + 128 + 32 * wj);
@@ -276,6 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
     asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
     const float a = (r[0] + r[32]) + (r[64] + r[96]);
     const float delta = o[513] * (o[384 + col] - a);
+    if (*stop) break;                                        // the whole group, and this state stays as it was
     if (wj == 0) {
       const float out = fmaf(o[512], delta, (r[128] + r[160]) + (r[192] + r[224]));
       store_from_float(p.out, p.dt_out, (int64_t)n * 128 + col, out);
@@ -295,24 +332,22 @@ __global__ void __launch_bounds__(kThreads, 1) kda_stream_kernel(const ScanParam
     }
     ++step;
     if (++st == kStages) { st = 0; ph ^= 1; }
-    if (*s_abort) break;
   }
-  if (*s_abort && tid == 0 && error) atomicExch(error, 64);
 }
 
 __device__ int g_stream_error = 0;
 
-template <int W>
-int launch(const ScanParams& p, const PrepDecodeParams& d, cudaStream_t stream) {
+template <int W, bool SHORT = false>
+int launch(const ScanParams& p, const PrepDecodeParams& d, cudaStream_t stream, ShortWait short_wait = {}) {
   const int64_t items = (int64_t)p.nseq * p.H;
   if (items <= 0) return KDA_OK;
   int* error = nullptr;
   if (cudaGetSymbolAddress(reinterpret_cast<void**>(&error), g_stream_error) != cudaSuccess ||
-      cudaFuncSetAttribute(kda_stream_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+      cudaFuncSetAttribute(kda_stream_kernel<W, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
     return KDA_ERR_LAUNCH;
   const int sms = device_sms();
   StageScope timing(kStageRecurrent, stream);
-  kda_stream_kernel<W><<<(unsigned)(items < sms ? items : sms), kThreads, kSmemBytes, stream>>>(p, d, error);
+  kda_stream_kernel<W, SHORT><<<(unsigned)(items < sms ? items : sms), kThreads, kSmemBytes, stream>>>(p, d, error, short_wait);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
@@ -333,6 +368,10 @@ int launch_fused_decode(const PrepDecodeParams& d, const ScanParams& p, cudaStre
   if (d.W == 4) return launch<4>(p, d, stream);
   if (d.W == 3) return launch<3>(p, d, stream);
   return launch<2>(p, d, stream);
+}
+
+int launch_stream_short(const ScanParams& p, int warp, int step, cudaStream_t stream) {
+  return launch<0, true>(p, PrepDecodeParams{}, stream, ShortWait{warp, step});
 }
 
 int stream_error_word() {

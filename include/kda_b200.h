@@ -41,7 +41,7 @@ int kda_b200_version(void);
 
 /* Non-zero if a tensor-memory kernel abandoned a bounded barrier wait or met offsets that leave the
  * packed buffer since the last call (clears the flag); synchronises the device.  Byte 0: the state
- * walks, byte 1: the chunk backward kernel, byte 2: the prepare kernel, byte 3: the gate kernels.  Every wait in those kernels
+ * walks and, code 64, the state-streaming kernel of one-token calls, byte 1: the chunk backward kernel, byte 2: the prepare kernel, byte 3: the gate kernels.  Every wait in those kernels
  * polls a bounded number of times; one that runs out makes the CTA record a code here and leave, so
  * a lost arrival shows up as an error word, never as a hang.  Code 9: cu_seqlens / chunk_offsets
  * describe a sequence that does not lie inside the `tokens` rows of the buffers; its chunks were
@@ -49,10 +49,14 @@ int kda_b200_version(void);
  * counterpart of the reference's offset assertion (kda/chunk_scheduler.py:278-293), which the host
  * cannot check without a synchronisation.  kda_selftest_bounded_wait exercises exactly that path on purpose:
  * a one-warp kernel waits `poll_limit` polls on a barrier nothing arrives on, then returns with
- * code 2 in the error word; the context stays usable.  For tests and debugging; no reference
- * counterpart. */
+ * code 2 in the error word; the context stays usable.  kda_selftest_bounded_stream runs the state-streaming kernel on one token
+ * for each of nseq fp32 states [nseq, 128, 128] (operands [nseq, 128] and [nseq], fp32) in place, where one warp of the first CTA
+ * (0..15 arithmetic, 16 copies, 17..22 operands) gives up without waiting from the CTA's state `step` on: code 64, every state
+ * either as it was or advanced by its token.  For tests and debugging; no reference counterpart. */
 int kda_device_error_word(void);
 int kda_selftest_bounded_wait(int poll_limit, void* stream);
+int kda_selftest_bounded_stream(const float* q, const float* k, const float* v, const float* gate, const float* beta,
+                                float* states, float* out, int nseq, int warp, int step, void* stream);
 
 /* Optional per-kernel timing with CUDA events recorded on the launching stream (off by default).
  * kda_stage_timing_read synchronises the recorded events and fills launches[] / total_ms[] (arrays of
