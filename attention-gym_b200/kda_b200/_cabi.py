@@ -10,6 +10,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
@@ -129,15 +130,33 @@ def lib() -> ctypes.CDLL:
 
 
 _torch_lib = None
+_torch_lock = threading.Lock()
 
 
 def load_torch_library() -> None:
-    """Register the C++ implementations of the operators, once their library has been built."""
+    """Register the C++ implementations of the operators, at their first call (ops.py): importing the package maps neither library,
+    so that a missing or unusable one can be built and a stale one replaced."""
     global _torch_lib
-    if _torch_lib is None and os.path.exists(TORCH_LIB_PATH):
-        torch.ops.load_library(TORCH_LIB_PATH)
-        _torch_lib = ctypes.CDLL(TORCH_LIB_PATH)
-        _torch_lib.kda_torch_launches.restype = c_int64
+    with _torch_lock:
+        if _torch_lib is not None:
+            return
+        for path in (LIB_PATH, TORCH_LIB_PATH):
+            if not os.path.exists(path):
+                raise RuntimeError(f"{path} is missing: build it with `python -m kda_b200.build` "
+                                   "(there is no CPU or PyTorch fallback for the fused path)")
+        try:
+            torch.ops.load_library(TORCH_LIB_PATH)
+            handle = ctypes.CDLL(TORCH_LIB_PATH)
+        except OSError as error:
+            raise RuntimeError(f"{TORCH_LIB_PATH} cannot be loaded by torch {torch.__version__}: rebuild it with "
+                               f"`python -m kda_b200.build --force` ({error})") from error
+        handle.kda_torch_launches.restype = c_int64
+        _torch_lib = handle
+
+
+def mapped() -> bool:
+    """Whether this process already runs code of one of the libraries."""
+    return _lib is not None or _torch_lib is not None
 
 
 def __getattr__(name):

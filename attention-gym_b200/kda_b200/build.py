@@ -15,6 +15,8 @@ CSRC = os.path.join(os.path.dirname(HERE), "csrc")
 LIB_PATH = os.path.join(HERE, "libkda_b200.so")
 TORCH_LIB_PATH = os.path.join(HERE, "libkda_b200_torch.so")      # operators in C++ on top of it
 TORCH_SOURCE = "kda_torch.cpp"
+OBJ = os.path.join(HERE, "_obj")
+STAMP_PATH = os.path.join(OBJ, "torch_build")       # the torch that the operator library was built against
 SOURCES = [
     "kda_cabi.cu",
     "kda_recurrent.cu",
@@ -43,8 +45,23 @@ def _nvcc() -> str:
     return "nvcc"
 
 
+def _torch_build() -> str:
+    """What the operator library's C++ ABI hangs on."""
+    import torch
+
+    return f"{torch.__version__} cxx11={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+
+
+def _built_for() -> str:
+    try:
+        with open(STAMP_PATH) as f:
+            return f.read()
+    except OSError:
+        return ""
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH) or not os.path.exists(TORCH_LIB_PATH):
+    if not os.path.exists(LIB_PATH) or not os.path.exists(TORCH_LIB_PATH) or _built_for() != _torch_build():
         return True
     built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(TORCH_LIB_PATH))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
@@ -54,17 +71,21 @@ def needs_build() -> bool:
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every kernel for sm_100a into one shared library, and the C++ operators into a second one; returns the
-    path of the first."""
+    path of the first.  Both are linked aside and put in place together, so that a failed build leaves the old ones.  A process that
+    already runs the old code cannot take up the new one and is told so."""
+    from . import _cabi
+
     if not force and not needs_build():
         return LIB_PATH
     objs = []
     procs = []
-    os.makedirs(os.path.join(HERE, "_obj"), exist_ok=True)
+    linked = os.path.join(OBJ, "linked")
+    os.makedirs(linked, exist_ok=True)
     for src in SOURCES:
         path = os.path.join(CSRC, src)
         if not os.path.exists(path):
             raise FileNotFoundError(path)
-        obj = os.path.join(HERE, "_obj", src.replace(".cu", ".o"))
+        obj = os.path.join(OBJ, src.replace(".cu", ".o"))
         objs.append(obj)
         cmd = [_nvcc(), *NVCC_FLAGS, "-c", path, "-o", obj]
         if verbose:
@@ -76,15 +97,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(out.decode())
         if proc.returncode:
             raise RuntimeError(f"nvcc failed on {src}")
-    subprocess.check_call([_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-lcudart", "-ldl"])
-    _build_torch()
-    from . import _cabi
-
-    _cabi.load_torch_library()
+    new, new_torch = (os.path.join(linked, os.path.basename(p)) for p in (LIB_PATH, TORCH_LIB_PATH))
+    subprocess.check_call([_nvcc(), "-shared", "-o", new, *objs, "-lcudart", "-ldl"])
+    _build_torch(linked, new_torch)
+    os.replace(new, LIB_PATH)
+    os.replace(new_torch, TORCH_LIB_PATH)
+    with open(STAMP_PATH, "w") as f:
+        f.write(_torch_build())
+    if _cabi.mapped():
+        raise RuntimeError("the libraries were rebuilt, but this process runs the old ones: restart it")
     return LIB_PATH
 
 
-def _build_torch() -> None:
+def _build_torch(linked: str, path: str) -> None:
+    """The operators, against the library of the same name in `linked`."""
     import torch
 
     root = os.path.dirname(torch.__file__)
@@ -95,7 +121,7 @@ def _build_torch() -> None:
     subprocess.check_call([
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes),
-        os.path.join(CSRC, TORCH_SOURCE), "-o", TORCH_LIB_PATH, f"-L{HERE}", "-l:libkda_b200.so", f"-L{lib}", "-ltorch",
+        os.path.join(CSRC, TORCH_SOURCE), "-o", path, f"-L{linked}", "-l:libkda_b200.so", f"-L{lib}", "-ltorch",
         "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
 
 

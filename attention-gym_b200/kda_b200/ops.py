@@ -144,7 +144,34 @@ _lib_layer.define("chunk_bwd_qkv(Tensor qkv, Tensor cumulative_gate, Tensor beta
 _lib_layer.define("widen(Tensor x) -> Tensor")
 
 
-_cabi.load_torch_library()
+# The operators that csrc/kda_torch.cpp implements.  Their library is loaded by the first call of any of them: until it is, a call
+# on CUDA tensors comes out here, because a backend's own implementation precedes a composite one.
+_IN_CPP = {
+    _NS: ("kda_chunk_fwd", "kda_chunk_fwd_with_state", "kda_chunk_fwd_ragged", "kda_chunk_fwd_ragged_with_state",
+          "kda_chunk_fwd_saved", "kda_chunk_fwd_qknorm", "kda_chunk_bwd_saved", "kda_chunk_bwd_qknorm", "kda_recurrent_fwd",
+          "kda_recurrent_fwd_no_state", "kda_recurrent_fwd_paged"),
+    _NS_OWN: ("decode_step",),
+}
+
+
+def _load_at_first_call(library, namespace, name):
+    qualname = f"{namespace}::{name}"
+
+    def first_call(*args, **kwargs):
+        devices = {a.device.type for a in (*args, *kwargs.values()) if isinstance(a, torch.Tensor)}
+        if "cuda" not in devices:
+            raise NotImplementedError(f"Could not run '{qualname}' with arguments from {sorted(devices)}: it runs on CUDA tensors only")
+        _cabi.load_torch_library()
+        if not torch._C._dispatch_has_kernel_for_dispatch_key(qualname, "CUDA"):
+            raise RuntimeError(f"{_cabi.TORCH_LIB_PATH} does not implement {qualname}: rebuild it with `python -m kda_b200.build --force`")
+        return getattr(getattr(torch.ops, namespace), name).default(*args, **kwargs)
+
+    library.impl(name, first_call, "CompositeExplicitAutograd")
+
+
+for _namespace, _library in ((_NS, _lib), (_NS_OWN, _lib_own)):
+    for _name in _IN_CPP[_namespace]:
+        _load_at_first_call(_library, _namespace, _name)
 
 
 def _require_cuda(t: torch.Tensor, what: str):
