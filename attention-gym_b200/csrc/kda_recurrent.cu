@@ -19,8 +19,9 @@ namespace kda {
 // operands are fetched TT tokens at a time, one tile ahead of their use (raw bits in registers), and
 // published to shared memory as fp32 (q scaled, 2^g) with one barrier per tile.
 //
-// K > 128: bound by the latency of one token, the dependent chain of decay, reduction, three shuffles and update, so that NP
-// warps of their own fetch, publish and store (NP = 0: the computing warps do it).
+// A long scan of few sequences is bound by the latency of one token: the dependent chain of decay, reduction, three shuffles
+// and update.  So NP warps of their own fetch, publish and store (NP = 0: the computing warps do it), and up to K = 128 the next
+// token's operands are read from shared memory before the shuffles.  T = 512, H = 4, K = V = 64: 114 us without moving warps, 79 with.
 // A short scan of many sequences is bound by the state traffic and by how much of it two CTAs per SM
 // can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 60 us, with four of half the columns 51
 // us.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
@@ -33,6 +34,8 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
   constexpr int KP = 8 * KR, CT = 4 * VC * NW;
   constexpr int NE = TT * KP / NT;                 // operand elements per thread, array and tile
   constexpr int NV = (TT * CT + NT - 1) / NT;      // value and output elements per thread and tile
+  constexpr int NR = KR / 4;
+  constexpr bool kPrefetch = VC == 1 && KR <= 16 && NP > 0;
   static_assert(TT * KP % NT == 0 && TT <= 32, "tile split");
   __shared__ __align__(16) float s_q[2][TT][KP], s_k[2][TT][KP], s_d[2][TT][KP];
   __shared__ float s_v[2][TT][CT], s_o[2][TT][CT], s_beta[2][TT];
@@ -169,16 +172,31 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
     if (moves && more) fetch(t0 + TT);
     if (NP && moves && t0 > bos) flush(t0 - TT, b ^ 1, TT);
     if (computes) {
-#pragma unroll 1
+    // The operands of a long scan's next token are read from shared memory between the two halves of
+    // a step, where their latency hides behind the shuffles.
+    f32x2 q[KR / 2], k[KR / 2], d[KR / 2];
+    auto read = [&](int tok, f32x2 (&qd)[KR / 2], f32x2 (&kd)[KR / 2], f32x2 (&dd)[KR / 2]) {
+      const ulonglong2* qs = reinterpret_cast<const ulonglong2*>(s_q[b][tok]) + lk;
+      const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
+      const ulonglong2* ds = reinterpret_cast<const ulonglong2*>(s_d[b][tok]) + lk;
+#pragma unroll
+      for (int i = 0; i < NR; ++i) {
+        const ulonglong2 a = qs[8 * i], c = ks[8 * i], e = ds[8 * i];
+        qd[2 * i] = a.x; qd[2 * i + 1] = a.y;
+        kd[2 * i] = c.x; kd[2 * i + 1] = c.y;
+        dd[2 * i] = e.x; dd[2 * i + 1] = e.y;
+      }
+    };
+    if (kPrefetch) read(0, q, k, d);
+#pragma unroll(kPrefetch ? 2 : 1)
     for (int tok = 0; tok < ntok; ++tok) {
       f32x2 pk[VC], pq[VC], pqk = 0;       // (zero bits: +0, +0) even rows in the low half, odd in the high
 #pragma unroll
       for (int j = 0; j < VC; ++j) pk[j] = pq[j] = 0;
       const ulonglong2* ks = reinterpret_cast<const ulonglong2*>(s_k[b][tok]) + lk;
-      f32x2 q[KR / 2], k[KR / 2], d[KR / 2];
 #pragma unroll
       for (int i = 0; i < KR / 2; ++i) {
-        if (i % 2 == 0) {
+        if (!kPrefetch && i % 2 == 0) {
           const ulonglong2 x = reinterpret_cast<const ulonglong2*>(s_q[b][tok])[lk + 4 * i], y = ks[4 * i],
                            z = reinterpret_cast<const ulonglong2*>(s_d[b][tok])[lk + 4 * i];
           q[i] = x.x; q[i + 1] = x.y; k[i] = y.x; k[i + 1] = y.y; d[i] = z.x; d[i + 1] = z.y;
@@ -200,6 +218,8 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
         a[j] = y.x + y.y;
         o[j] = z.x + z.y;
       }
+      f32x2 qn[KR / 2], kn[KR / 2], dn[KR / 2];
+      if (kPrefetch) read(tok + 1 < TT ? tok + 1 : tok, qn, kn, dn);
 #pragma unroll
       for (int m = 4; m < 32; m <<= 1) {
 #pragma unroll
@@ -221,11 +241,15 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
       }
 #pragma unroll
       for (int i = 0; i < KR / 2; ++i) {
-        if (i % 2 == 0) { const ulonglong2 y = ks[4 * i]; k[i] = y.x; k[i + 1] = y.y; }      // read again: fewer registers
+        if (!kPrefetch && i % 2 == 0) { const ulonglong2 y = ks[4 * i]; k[i] = y.x; k[i + 1] = y.y; }      // read again: fewer registers
 #pragma unroll
         for (int j = 0; j < VC; ++j) S[i][j] = fma2(k[i], delta2[j], S[i][j]);
       }
       if (lk < VC) s_o[b][tok][wc + lk] = mine;
+      if (kPrefetch) {
+#pragma unroll
+        for (int i = 0; i < KR / 2; ++i) { q[i] = qn[i]; k[i] = kn[i]; d[i] = dn[i]; }
+      }
     }
     }
     if (moves && more) publish(b ^ 1, (int)min((int64_t)TT, eos - t0 - TT));   // those buffers were last read before the previous barrier
@@ -276,8 +300,10 @@ __global__ void __launch_bounds__(32 * (NW + NP), MINB) kda_scan_kernel(const Sc
 // thread (its products rounded before the sum) it was 3 to 8 % larger at gates that forget fast.  (The state is
 // rounded five times a block instead of eight.)
 // ------------------------------------------------------------------------------------------------
-// F32: every operand is fp32.
-template <int KR, bool CUM, bool F32>
+// Every operand is fp32.  (The same with a type test per operand and load, bf16 q, k and v: the moving warps took longer than the
+// computing ones, and at K = V = 128 nothing was left of the gain: 32 chains of 100 tokens 53.7 us, one token at a time 52.1; 4 chains of
+// 5 tokens 5.2 / 4.9.)
+template <int KR, bool CUM>
 __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams p) {
   constexpr int C = 4, KP = 8 * KR, NR = KR / 4, CT = 16;
   constexpr int LB = KP / 2, SW = (LB + 31) / 32;           // moving threads of a block (two channels each) and their warps
@@ -309,34 +335,26 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
   const float* sin = p.h0 ? p.h0 + (paged ? slot * p.slot_stride : slot * H * K * V) + (int64_t)head * K * V : nullptr;
   float* sout = paged ? const_cast<float*>(sin) : (p.ht ? p.ht + (slot * H + head) * K * V : nullptr);
 
-  // ---- operand tiles: raw bits in registers, two tiles ahead; a moving thread owns two channels of one block ----
-  // (one base address per operand and 32-bit offsets from it: with 64-bit index arithmetic and a type test for every
-  // element the moving warps took longer than the computing ones)
+  // ---- operand tiles: in registers, two tiles ahead; a moving thread owns two channels of one block ----
+  // (one base address per operand and 32-bit offsets from it: with 64-bit index arithmetic the moving warps took longer than the
+  // computing ones)
   const int blk0 = tid / LB, ch = 2 * (tid % LB), tok0 = C * blk0;       // (moving threads only)
   const bool in0 = ch < K, in1 = ch + 1 < K;
-  uint32_t rq[C][2], rk[C][2], rg[C][2], rp[2], rv[TT * CT / 128], rb = 0;
-  auto operand = [&](const void* base, int dt, int64_t at) {
-    return reinterpret_cast<const unsigned char*>(base) + at * (F32 ? 4 : dtype_size(dt));
-  };
-  auto bits = [&](const unsigned char* base, int dt, uint32_t off) -> uint32_t {
-    if (F32 || dt == KDA_F32) return *reinterpret_cast<const uint32_t*>(base + 4 * off);
-    return *reinterpret_cast<const unsigned short*>(base + 2 * off);
-  };
-  auto number = [&](uint32_t raw, int dt) { return F32 ? __uint_as_float(raw) : raw_to_float(raw, dt); };
+  float rq[C][2], rk[C][2], rg[C][2], rp[2], rv[TT * CT / 128], rb = 0.f;
+  auto operand = [](const void* base, int64_t at) { return reinterpret_cast<const float*>(base) + at; };
   const int64_t kat = (bos * H + head) * K + (in0 ? ch : 0), vat = (bos * H + head) * V + cta0;
-  const unsigned char *bq = operand(p.q, p.dt_q, kat), *bk = operand(p.k, p.dt_k, kat), *bg = operand(p.g, p.dt_g, kat),
-                      *bv = operand(p.v, p.dt_v, vat), *bb = operand(p.beta, p.dt_beta, bos * H + head);
+  const float *bq = operand(p.q, kat), *bk = operand(p.k, kat), *bg = operand(p.g, kat), *bv = operand(p.v, vat),
+              *bb = operand(p.beta, bos * H + head);
   const uint32_t krow = (uint32_t)H * K, vrow = (uint32_t)H * V;      // (a tile of rows is well below 2^31 bytes)
   auto fetch = [&](int64_t t0) {
     const int ntok = (int)min((int64_t)TT, eos - t0);
     const int64_t kt = (t0 - bos) * krow, vt0 = (t0 - bos) * vrow, bt0 = (t0 - bos) * H;
-    const unsigned char *q = bq + kt * (F32 ? 4 : dtype_size(p.dt_q)), *k = bk + kt * (F32 ? 4 : dtype_size(p.dt_k)),
-                        *g = bg + kt * (F32 ? 4 : dtype_size(p.dt_g)), *v = bv + vt0 * (F32 ? 4 : dtype_size(p.dt_v));
+    const float *q = bq + kt, *k = bk + kt, *g = bg + kt, *v = bv + vt0;
     // the gate before the block, unless the block starts a chunk (a block never straddles two)
     const bool before = CUM && tok0 < ntok && (((int)(t0 - bos) + tok0) & (kChunk - 1)) != 0;
-    const unsigned char* gp = g - (size_t)krow * (F32 ? 4 : dtype_size(p.dt_g));
-    rp[0] = before && in0 ? bits(gp, p.dt_g, tok0 * krow) : 0;
-    rp[1] = before && in1 ? bits(gp, p.dt_g, tok0 * krow + 1) : 0;
+    const float* gp = g - krow;
+    rp[0] = before && in0 ? gp[tok0 * krow] : 0.f;
+    rp[1] = before && in1 ? gp[tok0 * krow + 1] : 0.f;
 #pragma unroll
     for (int i = 0; i < C; ++i) {
       const bool live = tok0 + i < ntok;
@@ -344,17 +362,17 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const bool in = live && (u ? in1 : in0);
-        rq[i][u] = in ? bits(q, p.dt_q, off + u) : 0;
-        rk[i][u] = in ? bits(k, p.dt_k, off + u) : 0;
-        rg[i][u] = in ? bits(g, p.dt_g, off + u) : 0;
+        rq[i][u] = in ? q[off + u] : 0.f;
+        rk[i][u] = in ? k[off + u] : 0.f;
+        rg[i][u] = in ? g[off + u] : 0.f;
       }
     }
 #pragma unroll
     for (int n = 0; n < TT * CT / 128; ++n) {
       const int e = tid + n * 128, tok = e / CT, c = e % CT;
-      rv[n] = (tok < ntok && cta0 + c < V) ? bits(v, p.dt_v, (uint32_t)tok * vrow + c) : 0;
+      rv[n] = (tok < ntok && cta0 + c < V) ? v[(uint32_t)tok * vrow + c] : 0.f;
     }
-    rb = tid < ntok ? bits(bb + bt0 * (F32 ? 4 : dtype_size(p.dt_beta)), p.dt_beta, (uint32_t)tid * H) : 0;
+    rb = tid < ntok ? bb[bt0 + (uint32_t)tid * H] : 0.f;
   };
   auto publish = [&](int b, int ntok) {
     float q[C][2], k[C][2], d[C][2], kt[C][2], qt[C][2], kn[C][2], dc[2], x[16];
@@ -362,10 +380,10 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
     for (int u = 0; u < 2; ++u) {
 #pragma unroll
       for (int i = 0; i < C; ++i) {
-        q[i][u] = number(rq[i][u], p.dt_q) * p.scale;
-        k[i][u] = number(rk[i][u], p.dt_k);
-        float g = number(rg[i][u], p.dt_g);
-        if (CUM) g -= number(i == 0 ? rp[u] : rg[i == 0 ? 0 : i - 1][u], p.dt_g);
+        q[i][u] = rq[i][u] * p.scale;
+        k[i][u] = rk[i][u];
+        float g = rg[i][u];
+        if (CUM) g -= i == 0 ? rp[u] : rg[i == 0 ? 0 : i - 1][u];
         d[i][u] = tok0 + i < ntok ? exp2f(g) : 1.f;
       }
       const float d01 = d[0][u] * d[1][u], d12 = d[1][u] * d[2][u], d23 = d[2][u] * d[3][u], d123 = d12 * d[3][u];
@@ -414,9 +432,9 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
 #pragma unroll
     for (int n = 0; n < TT * CT / 128; ++n) {
       const int e = tid + n * 128;
-      s_v[b][e / CT][e % CT] = number(rv[n], p.dt_v);
+      s_v[b][e / CT][e % CT] = rv[n];
     }
-    if (tid < TT) s_beta[b][tid] = number(rb, p.dt_beta);
+    if (tid < TT) s_beta[b][tid] = rb;
   };
   auto flush = [&](int64_t t0, int b, int ntok) {      // the outputs of a tile
 #pragma unroll
@@ -652,11 +670,8 @@ static int launch_block_scan(const ScanParams& p, bool cumulative, cudaStream_t 
   if (blocks <= 0) return KDA_OK;
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
   StageScope timing(kStageRecurrent, stream);
-  const bool f32 = p.dt_q == KDA_F32 && p.dt_k == KDA_F32 && p.dt_v == KDA_F32 && p.dt_g == KDA_F32 && p.dt_beta == KDA_F32;
-  if (cumulative && f32) kda_block_scan_kernel<KR, true, true><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else if (cumulative) kda_block_scan_kernel<KR, true, false><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else if (f32) kda_block_scan_kernel<KR, false, true><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else kda_block_scan_kernel<KR, false, false><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  if (cumulative) kda_block_scan_kernel<KR, true><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  else kda_block_scan_kernel<KR, false><<<(unsigned)blocks, 256, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
@@ -665,7 +680,7 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
   constexpr int CT = 4 * VC * NW, KP = 8 * KR;
   // 24 KiB of operands in two buffers (K = 128: 8 tokens, 4 or 2 where four or eight CTAs share an SM); the wide form also buffers its
   // columns of v and o
-  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : (2048 / MINB) / KP;
+  constexpr int TT = KP <= 64 ? (VC > 1 ? 8 : 16) : (MINB <= 2 ? 1024 : 2048 / MINB) / KP;
   const int64_t blocks = (int64_t)p.nseq * p.H * ((p.V + CT - 1) / CT);
   if (blocks <= 0) return KDA_OK;
   if (blocks > 0x7fffffffLL) return KDA_ERR_UNSUPPORTED;
@@ -677,8 +692,16 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
 
 // Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length, a turn as
 // many slices as there are SMs.  Figures in us, both sides of each line (K = V = 128 unless said otherwise).
-// * wide: four columns per lane, 16-byte state accesses, sixteen warps per SM; below: blocks of four tokens, 16
-//   columns per CTA, whose time grows with every turn.  Blocks / wide, 2 to 8 tokens, wide above one turn: 16 chains (128 slices)
+// * narrow: one column per lane, 16 columns per CTA, the shortest chain from token to token; wide: four columns per lane, 16-byte state
+//   accesses, sixteen warps per SM.  bf16 q, k and v, narrow / wide above one turn up to 8 tokens: 32 chains (256 slices) 7.4 / 4.4 at 2
+//   tokens, 9.7 / 9.7 at 8; above two turns from there on: 32 chains 17.1 / 20.9 at 24, 123 / 183 at 256, 48 chains (384) 24.9 / 21.0 at 24.
+//   K = V = 32: one turn up to 6 tokens, 96 chains (192 slices) 3.8 / 3.6 at 2, 4.5 / 4.9 at 8; three from 48 tokens on, 192 chains (384) 16.7 /
+//   18.3 at 48, 65 / 86 at 256, 320 chains (640) 24 / 21 and 100 / 99.  These two and the unaligned form below add in the same order: from
+//   three tokens a sequence on, a sequence of 16-bit rows has the same bits in every batch.
+// * fp32 operands take blocks of four tokens where the above is narrow: 4 chains of 5 / 24 / 512 tokens 4.9 / 9.4 / 126 one at a time, 4.1 / 6.5 /
+//   74 in blocks.  Not for K = 32 and less above one turn, except from the cumulative gate: 96 chains (192 slices) of 24 tokens 6.9 / 8.7,
+//   cumulative 10.8 / 8.5.
+// * blocks or wide: the time of blocks grows with every turn.  Blocks / wide, 2 to 8 tokens, wide above one turn: 16 chains (128 slices)
 //   5.6 / 6.6 at 2 tokens, 32 chains 9.2 / 6.5 at 2, 10.1 / 10.0 at 8; up to 15 tokens above two.  Above three turns from 16 tokens
 //   on: 48 chains (384) 14 / 16 at 16 tokens, 21 / 27 at 32, 56 chains (448) 17 / 16 and 26 / 27; four from 64 on: 72 chains (576)
 //   45 / 50 at 64, 151 / 185 at 256, 76 chains (608) 55 / 49 and 187 / 185.  K = V = 32 above two turns, 192 chains (384) 11 / 8 at
@@ -705,10 +728,13 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
   const int64_t slices = (int64_t)p.nseq * p.H * ((p.V + 15) / 16);
   const int64_t tokens = p.cu_seqlens && p.nseq > 0 ? p.T / p.nseq : p.T;      // per sequence, on average
   const bool aligned = (((uintptr_t)p.h0 | (uintptr_t)p.ht) & 15) == 0 && p.V % 4 == 0 && p.slot_stride % 4 == 0;
-  const int turns = tokens >= 2 && tokens <= 8 ? 1 : 2 + (tokens >= 16 && p.K > 32) + (tokens >= 64);
+  const bool f32 = p.dt_q == KDA_F32 && p.dt_k == KDA_F32 && p.dt_v == KDA_F32 && p.dt_g == KDA_F32 && p.dt_beta == KDA_F32;
+  const bool blocks = f32 && p.K <= 128 && !(p.K <= 32 && !cumulative && slices > sms);
+  const int more = blocks ? (tokens >= 16 && p.K > 32) + (tokens >= 64) : p.K <= 32 && !cumulative && tokens >= 48;
+  const int turns = tokens >= 2 && tokens <= (p.K <= 32 ? 6 : 8) ? 1 : 2 + more;
   const bool wide = aligned && p.K <= 128 && slices > (int64_t)turns * sms;
   const bool many = !aligned && p.K <= 128 && slices > 2 * sms;
-  const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || slices <= sms ? 1 : (p.K <= 32 ? 2 : 3));
+  const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || slices <= sms ? 1 : (p.K <= 32 ? 1 + f32 : 2 + f32));
   if (!wide && !cumulative && tokens <= few) {
     if (p.K <= 32) return launch_short_scan<4>(p, s);
     if (p.K <= 64) return launch_short_scan<8>(p, s);
@@ -736,9 +762,14 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
     if (p.K <= 64) return launch_scan<8, 1, 8, 0, 2>(p, cumulative, s);
     return launch_scan<16, 1, 8, 0, 2>(p, cumulative, s);
   }
-  if (p.K <= 32) return launch_block_scan<4>(p, cumulative, s);
-  if (p.K <= 64) return launch_block_scan<8>(p, cumulative, s);
-  return launch_block_scan<16>(p, cumulative, s);
+  if (blocks) {
+    if (p.K <= 32) return launch_block_scan<4>(p, cumulative, s);
+    if (p.K <= 64) return launch_block_scan<8>(p, cumulative, s);
+    return launch_block_scan<16>(p, cumulative, s);
+  }
+  if (p.K <= 32) return launch_scan<4, 1, 4, 4, 1>(p, cumulative, s);
+  if (p.K <= 64) return launch_scan<8, 1, 4, 4, 1>(p, cumulative, s);
+  return launch_scan<16, 1, 4, 4, 1>(p, cumulative, s);
 }
 
 static int launch_recurrent(const ScanParams& p, cudaStream_t s) {

@@ -118,6 +118,10 @@ def recurrent_kda(q, k, v, gate, beta, initial_state=None, *, cu_seqlens=None,
     ``gate`` is the *per-token* log2 decay.  With ``state_indices`` (int32, one per sequence)
     ``initial_state`` is a paged pool ``[num_slots, H, K, V]`` advanced in place; entries <= 0 are
     padding (zero output rows, pool untouched).  Inference only.
+
+    The kernel is chosen by the call's shape, so the bits of a sequence may depend on what else is in the call: with 16-bit
+    q, k and v only below three tokens a sequence on average, with fp32 operands at any length (few chains are scanned in
+    blocks of four tokens).  All of them accumulate in fp32; the same call gives the same bits every time.
     """
     selected = resolve_impl(impl)
     validate_kda_inputs(q, k, v, gate, beta, None if state_indices is not None else initial_state,
