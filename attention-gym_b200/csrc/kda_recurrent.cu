@@ -6,6 +6,8 @@
 //     S <- diag(2^g) S ;  d = beta (v - S^T k) ;  S <- S + k d^T ;  o = scale S^T q
 // The two K-reductions of a step (S^T k and S^T q, both taken on the decayed state) share one
 // exchange:  o = scale (S_d^T q + (q.k) d).
+#include <type_traits>
+
 #include "kda_recurrent.cuh"
 #include "kda_timing.cuh"
 
@@ -469,7 +471,9 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
       if (t0 + 2 * TT < eos) fetch(t0 + 2 * TT);
       if (t0 > bos) flush(t0 - TT, b ^ 1, TT);
     } else {
-      for (int blk = 0; C * blk < ntok; ++blk) {
+      // a block of which `live` tokens exist (tail: fewer than C; its own copy, because the test costs 8 % of the chain)
+      auto block = [&](int blk, auto partial, int live) {
+        constexpr bool tail = decltype(partial)::value;
         const int tok0 = C * blk;
         f32x2 pa[C], po[C];
 #pragma unroll
@@ -518,7 +522,8 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
         const float e1 = bt.y * (vv[1][wc] - fmaf(w[0], e0, a[1]));
         const float e2 = bt.z * (vv[2][wc] - fmaf(w[2], e1, fmaf(w[1], e0, a[2])));
         const float e3 = bt.w * (vv[3][wc] - fmaf(w[5], e2, fmaf(w[4], e1, fmaf(w[3], e0, a[3]))));
-        const float e[C] = {e0, e1, e2, e3};
+        // (tokens past the end add nothing: their zero rows against an infinite state would give NaN)
+        const float e[C] = {e0, tail && live < 2 ? 0.f : e1, tail && live < 3 ? 0.f : e2, tail ? 0.f : e3};
         {
           const ulonglong2* dc = reinterpret_cast<const ulonglong2*>(s_dc[b][blk]) + lk;
 #pragma unroll
@@ -544,7 +549,9 @@ __global__ void __launch_bounds__(256, 1) kda_block_scan_kernel(const ScanParams
         o[2] = fmaf(w[11], e2, fmaf(w[10], e1, fmaf(w[9], e0, o[2])));
         o[3] = fmaf(w[15], e3, fmaf(w[14], e2, fmaf(w[13], e1, fmaf(w[12], e0, o[3]))));
         if (lk < C) s_o[b][tok0 + lk][wc] = lk == 0 ? o[0] : (lk == 1 ? o[1] : (lk == 2 ? o[2] : o[3]));
-      }
+      };
+      for (int blk = 0; blk < ntok / C; ++blk) block(blk, std::false_type{}, C);
+      if (ntok % C) block(ntok / C, std::true_type{}, ntok % C);
     }
     __syncthreads();
     if (moving && !more) flush(t0, b, ntok);
@@ -731,7 +738,7 @@ static int launch_scan_any(const ScanParams& p, bool cumulative, cudaStream_t s)
   const bool f32 = p.dt_q == KDA_F32 && p.dt_k == KDA_F32 && p.dt_v == KDA_F32 && p.dt_g == KDA_F32 && p.dt_beta == KDA_F32;
   const bool blocks = f32 && p.K <= 128 && !(p.K <= 32 && !cumulative && slices > sms);
   const int more = blocks ? (tokens >= 16 && p.K > 32) + (tokens >= 64) : p.K <= 32 && !cumulative && tokens >= 48;
-  const int turns = tokens >= 2 && tokens <= (p.K <= 32 ? 6 : 8) ? 1 : 2 + more;
+  const int turns = tokens >= 2 && tokens <= (p.K <= 32 && !cumulative ? 6 : 8) ? 1 : 2 + more;
   const bool wide = aligned && p.K <= 128 && slices > (int64_t)turns * sms;
   const bool many = !aligned && p.K <= 128 && slices > 2 * sms;
   const int few = p.K > 128 ? (slices > 2 * sms ? 2 : 1) : (many || slices <= sms ? 1 : (p.K <= 32 ? 1 + f32 : 2 + f32));
