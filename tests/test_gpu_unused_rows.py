@@ -93,3 +93,21 @@ def test_which_rows_are_cleared(offsets, chunks, kept):
     want[list(kept)] = True
     for b in buffers:
         assert torch.equal(b.cpu().bool().all(1), want) and torch.equal(b.cpu().bool().any(1), want)
+
+
+@pytest.mark.parametrize("rows", [-1, 0, 1])
+def test_where_clearing_rows_replaces_the_fill(rows):
+    """Either side of the size from which only the unused rows are cleared: zero there, one more launch beyond it."""
+    from kda_b200 import ops
+
+    tokens = ops._FILL_BYTES // (2 * 128 * 4) + rows
+    cu = torch.tensor([0, 100, tokens - 70], dtype=torch.int32, device="cuda")
+    raw = torch.randn(1, tokens, 2, 128, device="cuda").bfloat16()
+    a_log, bias = torch.zeros(2, device="cuda"), torch.zeros(2, 128, device="cuda")
+    kda_b200.bounded_gate_cumsum(raw, a_log, bias, cu_seqlens=cu)
+    _poison()
+    before = _cabi.launch_count
+    out = kda_b200.bounded_gate_cumsum(raw, a_log, bias, cu_seqlens=cu)
+    launches = _cabi.launch_count - before
+    assert torch.isfinite(out).all() and not out[:, -70:].any() and out[:, :-70].any(-1).all()
+    assert launches == (3 if rows > 0 else 2)            # the chunk offsets, the gate, and the clearing
