@@ -28,12 +28,15 @@ def test_sizes_and_addresses(n, offset):
     torch.library.opcheck(torch.ops.kda_b200_layer.widen.default, (t,), test_utils=("test_schema", "test_faketensor"))
 
 
-def test_layer_weight_gradients_are_those_of_a_plain_cast():
+@pytest.mark.parametrize("hidden,heads,large", [(256, 2, False), (2048, 32, True), (2040, 32, False)])
+def test_layer_weight_gradients_are_those_of_a_plain_cast(hidden, heads, large):
+    """Either side of the size from which a weight has its own way back."""
     torch.manual_seed(0)
-    layer = kda_b200.KDAAttention(256, 2, 128, device="cuda")
-    x = torch.randn(2, 70, 256, device="cuda").bfloat16()
+    layer = kda_b200.KDAAttention(hidden, heads, 128, device="cuda")
+    x = torch.randn(2, 70, hidden, device="cuda").bfloat16()
     w = layer.out_proj.weight
-    d = torch.randn(2, 70, 256, device="cuda").bfloat16()
+    d = torch.randn(2, 70, hidden, device="cuda").bfloat16()
+    assert (type(layer._cast(layer.out_proj).grad_fn).__name__ == "_CastWeightBackward") == large
     seen = {}
     hook = layer.out_proj.weight.register_hook(lambda g: seen.setdefault("grad", g))
     inner = {}
