@@ -162,10 +162,12 @@ class KDAAttention(nn.Module):
         """``f_a_proj``, ``g_a_proj`` and ``beta_proj`` in one GEMM, or None.  Each of the three reads all of ``hidden`` for 128 columns
         or fewer, forward and backward, and their input gradients have to be added.  8192 tokens of 4096 channels, us apart /
         together: forward 61 / 24, weight gradients 54 / 23, input gradients 45 / 21, their sum 93 / 30; for that two small copies of
-        the weights and of the gradients, 10.  Only where the columns of every part start on 16 bytes."""
+        the weights and of the gradients, 10.  Only where the columns of every part start on 16 bytes, the weights are plain
+        tensors (not sharded or quantised ones, which may not concatenate) and the class's own methods do the projections."""
         parts = (self.f_a_proj, self.g_a_proj, self.beta_proj)
-        own = getattr(self.gate_projections, "__func__", None) is _GATE_PROJECTIONS
-        if self.backend != "fused" or not own or any(p.weight.shape[0] % 8 for p in parts):
+        own = all(getattr(type(self), name) is method and name not in self.__dict__ for name, method in _PROJECTIONS.items())
+        plain = all(type(p.weight) in (nn.Parameter, torch.Tensor) for p in parts)
+        if self.backend != "fused" or not own or not plain or any(p.weight.shape[0] % 8 for p in parts):
             return None
         weights = [self._cast(p) for p in parts]
         return F.linear(hidden, torch.cat(weights)).split([w.shape[0] for w in weights], -1)
@@ -245,6 +247,7 @@ class KDAAttention(nn.Module):
         return KDAAttentionOutput(result.to(hidden_states.dtype), final_state, final_conv_state)
 
 
-_GATE_PROJECTIONS = KDAAttention.gate_projections      # a replaced one is called as it is
+# replaced ones, in a subclass or on an object, are called for every projection (compared on the class, which a trace can do too)
+_PROJECTIONS = {name: getattr(KDAAttention, name) for name in ("gate_projections", "_linear", "_cast")}
 
 __all__ = ["KDAAttention", "KDAAttentionOutput"]

@@ -65,3 +65,34 @@ def test_only_some_weights_train():
         layer(x).hidden_states.backward(d)
         assert layer.f_a_proj.weight.grad is None and layer.beta_proj.weight.grad is None
     _close(joint.g_a_proj.weight.grad, apart.g_a_proj.weight.grad, "g_a_proj")
+
+
+class _OwnLinear(kda_b200.KDAAttention):
+    def _linear(self, x, layer):
+        self.seen = getattr(self, "seen", []) + [layer]
+        return super()._linear(x, layer)
+
+
+def test_a_replaced_linear_sees_every_projection():
+    torch.manual_seed(1)
+    plain = kda_b200.KDAAttention(256, 8, 128, device="cuda")
+    own = _OwnLinear(256, 8, 128, device="cuda")
+    own.load_state_dict(plain.state_dict())
+    x = torch.randn(2, 70, 256, device="cuda").bfloat16()
+    _close(own(x).hidden_states, plain(x).hidden_states, "output")
+    want = {own.qkv_proj, own.f_a_proj, own.f_b_proj, own.beta_proj, own.g_a_proj, own.g_b_proj, own.out_proj}
+    assert set(own.seen) == want and len(own.seen) == len(want)
+    plain._linear = lambda inputs, layer: _OwnLinear._linear(own, inputs, layer)         # replaced on the object
+    assert plain._narrow_projections(x) is None
+
+
+class _Marked(torch.Tensor):
+    pass
+
+
+def test_weights_of_another_tensor_class_stay_apart():
+    layer = kda_b200.KDAAttention(256, 8, 128, device="cuda")
+    x = torch.randn(1, 8, 256, device="cuda").bfloat16()
+    assert layer._narrow_projections(x) is not None
+    layer.f_a_proj.weight = torch.nn.Parameter(layer.f_a_proj.weight.detach().as_subclass(_Marked))
+    assert layer._narrow_projections(x) is None

@@ -1,5 +1,5 @@
-"""KDAAttention traced as one graph, forward and backward, with the bits of the eager call: small weights that are cast by ``.to``, and
-weights that have their own way back to fp32."""
+"""KDAAttention traced as one graph, forward and backward, with the bits of the eager call: small weights that are cast by ``.to``,
+weights that have their own way back to fp32, and the narrow projections apart or in one GEMM."""
 
 import pytest
 import torch
@@ -9,7 +9,7 @@ import kda_b200
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("hidden,heads", [(256, 2), (2048, 33)])
+@pytest.mark.parametrize("hidden,heads", [(256, 2), (2048, 33), (256, 8), (2048, 32)])
 def test_one_graph(hidden, heads):
     torch.manual_seed(heads)
     layer = kda_b200.KDAAttention(hidden, heads, 128, device="cuda")
