@@ -225,15 +225,16 @@ class KDAAttention(nn.Module):
             gate = _bounded_gate_cumsum(raw_gate, self.A_log, self.dt_bias, chunk_size=self.chunk_size,
                                         lower_bound=self.lower_bound, fastmath=self.fastmath,
                                         metadata=metadata)
-            if self.fuse_qk_norm:
+            if self.fuse_qk_norm and qkv.dtype == torch.bfloat16:      # (what the class's own convolution returns)
                 out, final_state = _chunk_kda_qkv(qkv, gate, beta, initial_state, metadata=metadata,
                                                   output_final_state=return_final_state)
             else:
                 q, k, v = qkv.unbind(2)
-                q, k = l2norm(q.contiguous()), l2norm(k.contiguous())
+                if not self.fuse_qk_norm:
+                    q, k = l2norm(q.contiguous()), l2norm(k.contiguous())
                 out, final_state = _chunk_kda(q, k, v.contiguous(), gate, beta, initial_state,
                                               metadata=metadata, output_final_state=return_final_state,
-                                              fastmath=self.fastmath)
+                                              fastmath=self.fastmath, normalize_qk=self.fuse_qk_norm)
         out = mask_inactive_tokens(out, mask)
         low = self._linear(hidden, self.g_a_proj) if narrow is None else narrow[1]
         logits = self._linear(low, self.g_b_proj).view_as(out)
