@@ -810,9 +810,9 @@ extern "C" int kda_recurrent_fwd(const void* q, const void* k, const void* v, co
 }
 
 extern "C" int64_t kda_decode_step_scratch_bytes(int64_t address_bits, int dtype, int nseq, int heads, int width) {
-  const bool fused = dtype != KDA_F32 && width >= 2 && width <= 4 && (address_bits & 15) == 0 &&
-                     (int64_t)nseq * heads < (1 << 24);
-  return fused || nseq <= 0 || heads <= 0 ? 0 : (int64_t)nseq * heads * 128 * (3 * kda::dtype_size(dtype) + 4);
+  const int64_t states = (int64_t)nseq * heads;
+  return nseq <= 0 || heads <= 0 || kda::decode_fuses(address_bits, dtype, states, width)
+             ? 0 : states * 128 * (3 * kda::dtype_size(dtype) + 4);
 }
 
 // One decode step: one launch where the vector form of the preprocessing applies; else preprocessing and state
@@ -838,7 +838,9 @@ extern "C" int kda_decode_step(const void* x, const void* conv_weight, void* con
   d.x = x; d.w = conv_weight; d.conv_state = conv_state; d.raw_gate = raw_gate; d.A_log = A_log; d.dt_bias = dt_bias;
   d.state_indices = state_indices; d.dt = dtype; d.dt_gate = dt_gate; d.nseq = nseq; d.H = heads; d.W = width;
   d.num_slots = conv_slots; d.act = activation; d.lower_bound = lower_bound; d.eps = eps;
-  if (fused_decode_takes(d, p)) return launch_fused_decode(d, p, (cudaStream_t)stream);
+  const uintptr_t bits = (uintptr_t)x | (uintptr_t)conv_weight | (uintptr_t)conv_state | (uintptr_t)dt_bias |
+                         (uintptr_t)state_pool | (uintptr_t)(4 * slot_stride);
+  if (decode_fuses((int64_t)bits, dtype, (int64_t)nseq * heads, width)) return launch_fused_decode(d, p, (cudaStream_t)stream);
   if (!scratch) return KDA_ERR_SCRATCH;
   const int64_t elems = (int64_t)nseq * heads * 128;
   unsigned char* q = reinterpret_cast<unsigned char*>(scratch);

@@ -71,8 +71,12 @@ bool stream_takes(const ScanParams& p);
 int launch_stream(const ScanParams& p, cudaStream_t stream);
 // The same with a wait that runs out (kda_selftest_bounded_stream).
 int launch_stream_short(const ScanParams& p, int warp, int step, cudaStream_t stream);
-// The whole decode step in one launch, if its tensors allow the vector form of the preprocessing.
-bool fused_decode_takes(const PrepDecodeParams& d, const ScanParams& p);
+// Whether a decode step of `states` (sequence, head) pairs runs in one launch: the vector form of the preprocessing and whole states
+// by bulk copies.  address_bits: all addresses and the slot stride in bytes, or-ed together.  (Slots that overlap need no
+// exception: as in the two launches, only states of the same call must not.)
+inline bool decode_fuses(int64_t address_bits, int dtype, int64_t states, int width) {
+  return dtype != KDA_F32 && width >= 2 && width <= 4 && (address_bits & 15) == 0 && states < (1 << 24);
+}
 int launch_fused_decode(const PrepDecodeParams& d, const ScanParams& p, cudaStream_t stream);
 int stream_error_word();
 

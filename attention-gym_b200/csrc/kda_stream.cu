@@ -360,10 +360,6 @@ bool stream_takes(const ScanParams& p) {
 }
 int launch_stream(const ScanParams& p, cudaStream_t stream) { return launch<0>(p, PrepDecodeParams{}, stream); }
 
-bool fused_decode_takes(const PrepDecodeParams& d, const ScanParams& p) {
-  const uintptr_t bits = (uintptr_t)d.x | (uintptr_t)d.w | (uintptr_t)d.conv_state | (uintptr_t)d.dt_bias;
-  return d.dt != KDA_F32 && d.W >= 2 && d.W <= 4 && (bits & 15) == 0 && p.state_indices && stream_takes(p);
-}
 int launch_fused_decode(const PrepDecodeParams& d, const ScanParams& p, cudaStream_t stream) {
   if (d.W == 4) return launch<4>(p, d, stream);
   if (d.W == 3) return launch<3>(p, d, stream);
