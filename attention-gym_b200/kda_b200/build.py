@@ -109,6 +109,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def _cxx_runtime() -> list:
+    """The C++ runtime that torch runs in this process.  Named before the compiler's own: a compiler that finds only a static one
+    would give the library a second runtime, and formatting a number into an error message then crashes the process."""
+    with open("/proc/self/maps") as f:
+        return sorted({line.split()[-1] for line in f if "/libstdc++.so" in line})[:1]
+
+
 def _build_torch(linked: str, path: str) -> None:
     """The operators, against the library of the same name in `linked`."""
     import torch
@@ -122,7 +129,7 @@ def _build_torch(linked: str, path: str) -> None:
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes),
         os.path.join(CSRC, TORCH_SOURCE), "-o", path, f"-L{linked}", "-l:libkda_b200.so", f"-L{lib}", "-ltorch",
-        "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
+        "-ltorch_cpu", "-lc10", "-lc10_cuda", *_cxx_runtime(), "-Wl,-rpath,$ORIGIN"])
 
 
 if __name__ == "__main__":

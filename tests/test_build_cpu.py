@@ -117,3 +117,27 @@ def test_operators_refuse_cpu_tensors_as_before():
     x = torch.zeros(1, 64, 1, 128, dtype=torch.bfloat16)
     with pytest.raises(NotImplementedError, match="Could not run 'kda_b200::kda_chunk_fwd'"):
         torch.ops.kda_b200.kda_chunk_fwd(x, x, x, x.float(), x[..., 0].float(), None, True)
+
+
+def test_a_refusal_whose_message_holds_a_number():
+    """An exception of the operator library with a formatted number, in a process of its own: it must not crash.  (The CUDA
+    implementation is called with CPU tensors; it refuses them before it touches one.)"""
+    import __graft_entry__  # noqa: F401  (path setup)
+    from kda_b200 import build
+
+    build.build()
+    said = subprocess.run([sys.executable, "-c", textwrap.dedent("""\
+        import torch, kda_b200
+        from kda_b200 import _cabi
+        _cabi.load_torch_library()
+        q = torch.zeros(1, 64, 2, 128, dtype=torch.bfloat16)
+        gate, beta, tape = torch.zeros(1, 64, 2, 128), torch.zeros(1, 64, 2), torch.zeros(1, 64, 2, 64, dtype=torch.bfloat16)
+        saved, offsets = torch.zeros(2 ** 20, dtype=torch.uint8), torch.zeros(1, dtype=torch.int32)      # no sequence at all
+        cuda = torch._C.DispatchKeySet(torch._C.DispatchKey.CUDA)
+        try:
+            torch.ops.kda_b200.kda_chunk_bwd_saved.default.redispatch(
+                cuda, q, q, q, gate, beta, tape, tape, saved, offsets, offsets, None, None, None, False)
+        except ValueError as error:
+            print("refused:", error)
+        """)], env=dict(os.environ, PYTHONPATH=os.path.join(ROOT, "attention-gym_b200")), capture_output=True, text=True)
+    assert "refused: num_sequences must be positive, got 0" in said.stdout, (said.returncode, said.stderr[-500:])
