@@ -107,8 +107,9 @@ struct Forward { Tensor out, state, aqk, akk, workspace, rstd_q, rstd_k; };
 struct Shape {
   int64_t batch, tokens, heads, nseq, capacity;
   bool packed;
-  Shape(const Tensor& x, int64_t head_dim, const OptTensor& cu) {
-    batch = x.size(0); tokens = x.size(1); heads = x.size(head_dim);
+  Shape(const Tensor& x, const OptTensor& cu) {
+    TORCH_CHECK_VALUE(x.dim() == 4, "expected q [B, T, H, 128], got ", x.sizes());
+    batch = x.size(0); tokens = x.size(1); heads = x.size(2);
     packed = cu.has_value();
     TORCH_CHECK_VALUE(!packed || batch == 1, "packed cu_seqlens require batch size one");
     nseq = packed ? cu->size(0) - 1 : batch;
@@ -122,7 +123,7 @@ Forward chunk_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, cons
                       const OptTensor& h0_, const OptTensor& cu, const OptTensor& co, bool want_state, bool keep, bool norm,
                       double eps) {
   check_core(q_, k_, v_);
-  const Shape s(q_, 2, cu);
+  const Shape s(q_, cu);
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous(), gate = f32(gate_), beta = f32(beta_);
   const OptTensor h0 = f32(h0_);
   Forward f;
@@ -242,7 +243,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> chunk_backward(
     const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& gate, const Tensor& beta, const Tensor& aqk,
     const Tensor& akk, const Tensor& saved, const OptTensor& rstd_q, const OptTensor& rstd_k, const OptTensor& cu,
     const OptTensor& co, const OptTensor& d_out, const OptTensor& d_state, const OptTensor& h0, bool want_state_grad) {
-  const Shape s(q_, 2, cu);
+  const Shape s(q_, cu);
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
   const Cotangents c(s, q, gate, beta, saved, cu, co, d_out, d_state, h0, want_state_grad);
   const Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
@@ -284,6 +285,7 @@ std::pair<Tensor, Tensor> recurrent(const Tensor& q, const Tensor& k, const Tens
                                     const Tensor& beta, const OptTensor& h0_, const OptTensor& cu, const OptTensor& slots,
                                     bool want_state) {
   TORCH_CHECK_VALUE(q.is_cuda(), "the fused recurrent scan requires CUDA tensors");
+  TORCH_CHECK_VALUE(q.dim() == 4, "expected q [B, T, H, K], got ", q.sizes());
   const int64_t batch = q.size(0), tokens = q.size(1), heads = q.size(2), K = q.size(3), V = v.size(-1);
   const int64_t nseq = cu ? cu->size(0) - 1 : batch;
   const Tensor out = fresh(v.sizes(), q, q.scalar_type(), cu.has_value());
