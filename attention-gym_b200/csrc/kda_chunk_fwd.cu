@@ -503,7 +503,7 @@ extern "C" int kda_zero_unused_rows(void* const* buffers, const int64_t* row_byt
   }
   p.count = count; p.nseq = nseq; p.chunk = chunk_size; p.cu_seqlens = cu_seqlens; p.chunk_offsets = chunk_offsets; p.tokens = tokens;
   if (tokens == 0) return KDA_OK;
-  kda::zero_rows_kernel<<<2 * 148, 256, 0, (cudaStream_t)stream>>>(p);
+  kda::zero_rows_kernel<<<2 * kda::device_sms(), 256, 0, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 

@@ -21,6 +21,8 @@ constexpr int kChunk = 64;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
+int device_sms();      // of the current device
+
 typedef __nv_bfloat16 bf16;
 typedef __nv_bfloat162 bf162;
 

@@ -176,11 +176,9 @@ static int launch_chain(const ChainParams& p, int64_t chains, cudaStream_t s) {
 int launch_state_chain(const float* M, const float* b, const float* h0, float* hin, float* fin, int rows, int heads, int segs,
                        cudaStream_t s) {
   if ((((uintptr_t)M | (uintptr_t)b | (uintptr_t)hin | (uintptr_t)fin) & 15) != 0) return KDA_ERR_ARG;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const ChainParams p{M, b, h0, hin, fin, heads, segs};
   const int64_t chains = (int64_t)rows * heads;
-  return chains * 8 <= sms ? launch_chain<16>(p, chains, s) : launch_chain<32>(p, chains, s);
+  return chains * 8 <= device_sms() ? launch_chain<16>(p, chains, s) : launch_chain<32>(p, chains, s);
 }
 
 }  // namespace kda

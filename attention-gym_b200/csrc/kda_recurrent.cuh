@@ -64,8 +64,6 @@ __device__ __forceinline__ float decode_gate(float a, float raw, float bias, flo
   return lower_bound / (1.f + expf(-z)) * kLog2e;
 }
 
-int device_sms();
-
 // The state-streaming kernel (kda_stream.cu).  A scan it can take: K = V = 128, 16-byte aligned states in and out.
 bool stream_takes(const ScanParams& p);
 int launch_stream(const ScanParams& p, cudaStream_t stream);
