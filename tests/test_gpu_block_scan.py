@@ -1,6 +1,6 @@
-"""The scan in blocks of four tokens where its blocks, tiles and moving warps end: token counts around 4, 8, 16 and 32, head
-sizes around its row groups (32, 64, 128) and column slices (16), chunk boundaries of the cumulative gate, mixed dtypes,
-gates that forget at once; against the fp64 recurrence."""
+"""The scan in blocks of four tokens (fp32 operands) where its blocks, tiles and moving warps end: token counts around 4, 8, 16 and 32,
+head sizes around its row groups (32, 64, 128) and column slices (16), chunk boundaries of the cumulative gate, gates that forget at
+once; the wide forms with each number of columns per block; against the fp64 recurrence."""
 
 import pytest
 import torch
@@ -10,9 +10,9 @@ from oracle import kda_oracle as orc
 
 pytestmark = pytest.mark.gpu
 
-# fp32 sums of at most 128 terms over at most 200 tokens of a contracting recurrence: 200 * 128 * 2^-24 = 1.5e-3 of the
-# largest value bounds the worst case
-TOL = 1.5e-3
+# fp32 sums of at most 128 terms over at most 200 tokens of a contracting recurrence, whose roundings of 2^-24 have either sign:
+# sqrt(200 * 128) * 2^-24 = 1e-5 of the largest value
+TOL = 1e-5
 
 
 def _close(got, want, what):
@@ -52,6 +52,36 @@ def test_mixed_dtypes_and_gates_that_forget():
     err = float((o.double().cpu() - want_o).abs().max() / want_o.abs().max())
     assert err < 2.0 ** -8 + TOL
     _close(s, want_s, "state")
+
+
+@pytest.mark.parametrize("dtypes", ["mixed", "fp32"])
+def test_forgetting_in_every_form(dtypes):
+    """Decays of zero inside a block of fp32 operands, and token by token for the others."""
+    inp = orc.make_inputs(1, 45, 2, 48, 24, seed=4, with_state=True)
+    if dtypes == "mixed":
+        inp["k"] = inp["k"].bfloat16()
+    inp["gate_log2"][:, 6] = -300.0
+    inp["gate_log2"][:, 11:13] = float("-inf")
+    args = [inp[n] for n in ("q", "k", "v", "gate_log2", "beta", "h0")]
+    want_o, want_s = orc.recurrent_kda_ref(*(x.double() for x in args))
+    o, s = kda_b200.recurrent_kda(*(x.cuda() for x in args), output_final_state=True)
+    _close(o, want_o, "output")
+    _close(s, want_s, "state")
+
+
+@pytest.mark.parametrize("kd,vd", [(32, 40), (32, 64), (20, 100), (32, 128), (17, 196)])
+@pytest.mark.parametrize("heads,lengths", [(8, [4, 1, 0, 3, 5, 8, 9, 20, 7, 2, 12, 16] * 4), (4, [1, 2, 0, 3, 1, 1, 2, 5, 1, 2] * 12)], ids=["few", "one"])
+def test_small_keys_in_the_wide_forms(kd, vd, heads, lengths):
+    """Keys of at most 32 rows against more than 32 columns: 64 and 128 columns per block, with a last block of few columns."""
+    inp = orc.make_inputs(1, sum(lengths), heads, kd, vd, seed=vd, with_state=True, lengths=lengths)
+    dev = {n: t.cuda() if torch.is_tensor(t) else t for n, t in inp.items()}
+    want_o, want_s = orc.recurrent_kda_ref(*(inp[n].double() for n in ("q", "k", "v", "gate_log2", "beta", "h0")),
+                                           inp["cu_seqlens"])
+    for call, gate in ((kda_b200.recurrent_kda, "gate_log2"), (kda_b200.chunk_kda, "cum_gate")):
+        o, s = call(dev["q"], dev["k"], dev["v"], dev[gate], dev["beta"], dev["h0"], cu_seqlens=dev["cu_seqlens"],
+                    output_final_state=True, **({"exact_fp32": True} if gate == "cum_gate" else {}))
+        _close(o, want_o, "output")
+        _close(s, want_s, "state")
 
 
 @pytest.mark.parametrize("kd,vd", [(128, 128), (96, 64), (72, 100), (65, 132)])

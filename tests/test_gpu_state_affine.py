@@ -1,5 +1,5 @@
 """h_out = M h_in + b at the edges of its slabs of K, for matrices that start off 16-byte addresses, against fp64; and the chain of
-such maps along the segments of a row, with and without entering and leaving states."""
+such maps along the segments of a row, with and without entering and leaving states, 16 and 32 columns per block."""
 
 import pytest
 import torch
@@ -48,4 +48,29 @@ def test_chain_of_segments(segments, initial, final):
     serial, split = run(1), run(segments)
     # two bf16 evaluations of the products of up to twelve chunks: a few roundings of 2^-9 of the largest value
     for x, y in zip(split[:2 if final else 1], serial):
+        assert float((x.double() - y.double()).abs().max() / y.double().abs().max()) < 1e-2
+
+
+@pytest.mark.parametrize("rows,heads", [(1, 32), (2, 10)])
+@pytest.mark.parametrize("segments", [2, 5])
+def test_both_widths_of_the_chain(rows, heads, segments):
+    """Many chains take 32 columns per block, two rows per thread, few 16.  Both add in the order of K: the first three heads of the large
+    call have the bits of a call of their own, and it agrees with the serial walk."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert rows * heads * 8 > sms >= rows * 3 * 8
+    inp = orc.make_inputs(rows, 64 * 12 - 7, heads, 128, 128, seed=heads, with_state=True)
+    q, k, v = (inp[n].bfloat16().cuda() for n in ("q", "k", "v"))
+    args = (q, k, v, 0.02 * inp["cum_gate"].cuda(), inp["beta"].cuda(), inp["h0"].cuda())
+
+    def run(forced, some):
+        part = [x[:, :, :some].contiguous() for x in args[:5]] + [args[5][:, :some].contiguous()]
+        try:
+            assert _cabi.lib().kda_set_row_segments(forced) == 0
+            return kda_b200.chunk_kda(*part, output_final_state=True)
+        finally:
+            _cabi.lib().kda_set_row_segments(0)
+
+    (out, state), (few, few_state), serial = run(segments, heads), run(segments, 3), run(1, heads)
+    assert torch.equal(out[:, :, :3], few) and torch.equal(state[:, :3], few_state)
+    for x, y in zip((out, state), serial):
         assert float((x.double() - y.double()).abs().max() / y.double().abs().max()) < 1e-2
