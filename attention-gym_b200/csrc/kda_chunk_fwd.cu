@@ -449,7 +449,7 @@ extern "C" int kda_chunk_fwd_dense_qknorm(const void* q, const void* k, const vo
 // Rows of packed results that no sequence writes stay zero: the unused tail of a fixed-capacity buffer, which only the
 // device knows.  Every block checks the offsets (a few KB that hit L2) and clears its share of the rows before the first and
 // behind the last sequence; offsets that the chunk kernels would skip, because they leave the buffer or contradict one
-// another, clear all rows.  (Filling the results first: 11.5 GB, 1.9 ms of a training step of 279046 tokens, H = 32.)
+// another, clear all rows.  (Filling the results first: 13.8 GB, 2.9 ms of a training step of 279046 tokens, H = 32.)
 // ------------------------------------------------------------------------------------------------
 namespace kda {
 constexpr int kZeroBuffers = 8;

@@ -25,8 +25,8 @@ namespace kda {
 // and update.  So NP warps of their own fetch, publish and store (NP = 0: the computing warps do it), and up to K = 128 the next
 // token's operands are read from shared memory before the shuffles.  T = 512, H = 4, K = V = 64: 114 us without moving warps, 79 with.
 // A short scan of many sequences is bound by the state traffic and by how much of it two CTAs per SM
-// can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 60 us, with four of half the columns 51
-// us.  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
+// can keep in flight: 48 sequences of 1 to 8 tokens, H = 32, K = V = 128 (212 MB): 58.9 us, with four of half the columns 57.6
+// (60.9 and 59.5 over four pools in turn).  (Three CTAs of half the columns per lane: 74 us; asking the next CTA's state into L2: no change.)
 // CUM: the gate is the cumulative one of chunk_kda; the per-token gate is its difference inside the
 // 64-token chunks of a sequence.
 // ------------------------------------------------------------------------------------------------
@@ -697,8 +697,8 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
   return cudaGetLastError() == cudaSuccess ? KDA_OK : KDA_ERR_LAUNCH;
 }
 
-// Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length, a turn as
-// many slices as there are SMs.  Figures in us, both sides of each line (K = V = 128 unless said otherwise).
+// Which form a scan takes; `slices` is the number of 16-column slices of all chains, `tokens` the average length (of a packed call the
+// capacity of its buffer over its sequences: their lengths are on the device), a turn as many slices as there are SMs.  Figures in us, both sides of each line (K = V = 128 unless said otherwise).
 // * narrow: one column per lane, 16 columns per CTA, the shortest chain from token to token; wide: four columns per lane, 16-byte state
 //   accesses, sixteen warps per SM.  bf16 q, k and v, narrow / wide above one turn up to 8 tokens: 32 chains (256 slices) 7.4 / 4.4 at 2
 //   tokens, 9.7 / 9.7 at 8; above two turns from there on: 32 chains 17.1 / 20.9 at 24, 123 / 183 at 256, 48 chains (384) 24.9 / 21.0 at 24.
@@ -717,7 +717,8 @@ static int launch_scan(const ScanParams& p, bool cumulative, cudaStream_t stream
 //   at V = 64, 1024 chains of 64 tokens, K = 64 172 / 100, K = 128 271 / 160; above V = 64 only if CTAs of 128 columns are more than
 //   two per SM: K = 72, V = 132, 8 tokens, 256 chains 25.5 / 22.0, 64 chains 9.4 / 10.5.  K = V = 32 runs 32 columns and eight CTAs per SM:
 //   2048 chains of 64 tokens 230 / 71.
-//   K over 64 also runs 64 columns for few tokens, where the states' way in and out is most of the time, so that more CTAs
+//   K = 64, V = 128 keeps 128 columns: 64 would gain up to four turns (48 chains, 384 slices, 6.2 / 5.7 at 6 tokens, 25.1 / 24.1 at 48) and
+//   lose above (80 chains, 640 slices, 6.2 / 6.7 and 25.4 / 28.9).  K over 64 also runs 64 columns for few tokens, where the states' way in and out is most of the time, so that more CTAs
 //   move states while others compute: up to 4 tokens (2048 chains of 4 tokens 58.9 / 55.4, of 6 72.6 / 74.7), up to 8 on average where
 //   lengths differ (48 sequences of 32 heads 54.3 / 50.6 at 4, 89.9 / 86.7 at 8, 104 / 108 at 12).
 //   Up to 2 tokens 32 columns and eight CTAs: 64 columns / 32, 48 sequences 42.3 / 38.0 at 1, 45.3 / 43.0 at 2, 50.4 / 49.8 at 3, 51.6 /

@@ -14,7 +14,8 @@
 //                 the packed arithmetic.  The two K-reductions cross the four warps of a column group through shared
 //                 memory, one named barrier per state
 //
-// us per step of a captured graph, 32 heads, 1 / 37 / 256 sequences (of measured copy bandwidth at 256): the fused step
+// us per step of a captured graph, 32 heads, 1 / 37 / 256 sequences (of measured copy bandwidth at 256; the 78 MB of 37 sequences stay in
+// L2 when one pool is advanced again and again, over four pools in turn the fused step takes 32): the fused step
 // 6.6 / 21.8 / 189 (87 %), against 9.3 / 27.6 / 204 as two overlapping launches with q, k, v and the gate in memory between
 // them; given operands 5.2 / 19.4 / 179 (91 %), against 5.7 / 22.6 / 191 with the states as 32-column slabs in four rings.
 // Every wait is bounded.  One that runs out records code 64 and stops the CTA: the others look for that while they
@@ -22,7 +23,7 @@
 // a state that was not advanced completely is never handed to the copying warp, and that warp waits for the loads it has
 // issued before the shared memory goes back.
 // (Several tokens per sequence on the same ring: one state at a time has 1.1 us a token, 48 sequences of 1 to 8 tokens 72
-// against 66 us of the token scan.  Bulk-copied states under the token scan's layout, two persistent CTAs per SM: 80 us.)
+// against 58 us of the token scan.  Bulk-copied states under the token scan's layout, two persistent CTAs per SM: 80 us.)
 #include "kda_recurrent.cuh"
 #include "kda_sm100.cuh"
 #include "kda_timing.cuh"
