@@ -23,6 +23,15 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 int device_sms();      // of the current device
 
+// Whether all of these addresses (NULL among them) are multiples of `bytes`: what a kernel's vector loads and stores need, asked on
+// the host, because a misaligned one takes the context down.
+template <typename... P>
+inline bool aligned_to(uintptr_t bytes, P... p) {
+  return (((uintptr_t)p | ...) & (bytes - 1)) == 0;
+}
+// of four values of a dtype
+inline uintptr_t four_bytes(int dtype) { return dtype == KDA_F32 ? 16 : 8; }
+
 typedef __nv_bfloat16 bf16;
 typedef __nv_bfloat162 bf162;
 

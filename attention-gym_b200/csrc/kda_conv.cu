@@ -847,9 +847,11 @@ __global__ void __launch_bounds__(128) conv_bwd_dx_edge_kernel(const ConvParams 
   }
 }
 
-static int conv_check(const ConvParams& p) {
+static int conv_check(const ConvParams& p, int dtype) {
   if (!p.x || !p.w || p.C <= 0 || p.W < 1 || p.W > WMAX || p.batch < 1 || p.T < 1) return KDA_ERR_ARG;
   if (p.cu_seqlens && p.batch != 1) return KDA_ERR_ARG;
+  if (!aligned_to(16, p.x, p.y, p.state, p.dy, p.dx, p.dpre)) return KDA_ERR_ARG;
+  if (p.W == 4 && !aligned_to(four_bytes(dtype), p.w)) return KDA_ERR_ARG;      // (four taps at once)
   return KDA_OK;
 }
 
@@ -930,7 +932,7 @@ extern "C" int kda_conv1d_fwd(const void* x, const void* weight, const void* ini
   p.x = x; p.w = weight; p.y = y; p.state = initial_state; p.cu_seqlens = cu_seqlens; p.nseq = nseq;
   p.batch = batch; p.T = tokens; p.C = channels; p.W = width; p.act = activation;
   if (!y) return KDA_ERR_ARG;
-  int rc = kda::conv_check(p);
+  int rc = kda::conv_check(p, dtype);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == KDA_BF16) return kda::conv_fwd_launch<__nv_bfloat16>(p, s);
@@ -959,7 +961,7 @@ extern "C" int kda_conv1d_bwd(const void* x, const void* weight, const void* ini
   p.dw_part = dw_partial; p.dstate = dstate; p.cu_seqlens = cu_seqlens; p.nseq = nseq;
   p.batch = batch; p.T = tokens; p.C = channels; p.W = width; p.act = activation;
   if (!dy || !dx || !dw_partial) return KDA_ERR_ARG;     // dpre_scratch is needed only when width != 4
-  int rc = kda::conv_check(p);
+  int rc = kda::conv_check(p, dtype);
   if (rc) return rc;
   int64_t blocks = conv_bwd_launch_blocks(batch, tokens, cu_seqlens != nullptr);
   cudaStream_t s = (cudaStream_t)stream;
@@ -975,6 +977,7 @@ extern "C" int kda_conv1d_decode(const void* x, const void* weight, void* state,
   if (!x || !weight || !state || !y || nseq < 0 || channels <= 0 || width < 2 || width > kda::WMAX)
     return KDA_ERR_ARG;
   if (nseq == 0) return KDA_OK;
+  if (!kda::aligned_to(16, x, state, y)) return KDA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   int n = dtype == KDA_F32 ? 4 : 8;
   if (channels % n) return KDA_ERR_UNSUPPORTED;

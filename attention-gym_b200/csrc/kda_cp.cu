@@ -188,6 +188,7 @@ extern "C" int kda_state_affine(const float* transition, const float* h_in, cons
   if (!transition || !h_in || !b || !h_out || count < 0) return KDA_ERR_ARG;
   if (key_dim % 64 || value_dim % 64 || key_dim <= 0 || value_dim <= 0) return KDA_ERR_UNSUPPORTED;
   if (count == 0) return KDA_OK;
+  if (!kda::aligned_to(16, b, h_out)) return KDA_ERR_ARG;
   dim3 grid(value_dim / 32, key_dim / 32, count);
   if ((((uintptr_t)transition | (uintptr_t)h_in) & 15) == 0)
     kda::state_affine_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(transition, h_in, b, h_out, key_dim, value_dim);

@@ -500,6 +500,7 @@ extern "C" int kda_gate_cumsum_fwd(const void* raw_gate, int dt_raw, const float
                                    int heads, int dim, int chunk_size, float lower_bound,
                                    int64_t num_chunks, void* stream) {
   if (!raw_gate || !A_log || !dt_bias || !out) return KDA_ERR_ARG;
+  if (!kda::aligned_to(kda::four_bytes(dt_raw), raw_gate) || !kda::aligned_to(16, dt_bias, out)) return KDA_ERR_ARG;
   kda::GateParams p{};
   int rc = gate_common(p, cu_seqlens, chunk_offsets, nseq, batch, tokens, heads, dim, chunk_size,
                        num_chunks);
@@ -526,6 +527,9 @@ extern "C" int kda_gate_cumsum_bwd(const void* raw_gate, int dt_raw, const float
                                    int chunk_size, float lower_bound, int64_t num_chunks,
                                    void* stream) {
   if (!raw_gate || !A_log || !dt_bias || !d_cumulative || !d_raw || !dA_partial || !dbias_partial)
+    return KDA_ERR_ARG;
+  if (!kda::aligned_to(kda::four_bytes(dt_raw), raw_gate, d_raw) ||
+      !kda::aligned_to(16, dt_bias, d_cumulative, dA_partial, dbias_partial))
     return KDA_ERR_ARG;
   kda::GateParams p{};
   int rc = gate_common(p, cu_seqlens, chunk_offsets, nseq, batch, tokens, heads, dim, chunk_size,
@@ -557,6 +561,7 @@ extern "C" int kda_l2norm_fwd(const void* x, int dtype, void* y, float* rstd, in
                               int dim, float eps, void* stream) {
   if (!x || !y || rows < 0 || dim <= 0 || dim % 4) return KDA_ERR_ARG;
   if (rows == 0) return KDA_OK;
+  if (!kda::aligned_to(kda::four_bytes(dtype), x, y)) return KDA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = dtype != KDA_F32 && (dim == 64 || dim == 128 || dim == 256) &&
                    ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0;
@@ -578,6 +583,7 @@ extern "C" int kda_l2norm_bwd(const void* y, const float* rstd, const void* dy, 
                               int64_t rows, int dim, void* stream) {
   if (!y || !rstd || !dy || !dx || rows < 0 || dim <= 0 || dim % 4) return KDA_ERR_ARG;
   if (rows == 0) return KDA_OK;
+  if (!kda::aligned_to(kda::four_bytes(dtype), y, dy, dx)) return KDA_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = dtype != KDA_F32 && (dim == 64 || dim == 128 || dim == 256) &&
                    ((uintptr_t)y & 15) == 0 && ((uintptr_t)dy & 15) == 0 && ((uintptr_t)dx & 15) == 0;

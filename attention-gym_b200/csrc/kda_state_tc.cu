@@ -503,6 +503,7 @@ int launch_state_fwd_tc(const bf16* w, const bf16* u, const bf16* kg, const bf16
                         bf16* vnew_out, const int32_t* cu, const int32_t* co, int nseq, int H,
                         int64_t tokens, int chunks, cudaStream_t s) {
   if (nseq == 0) return KDA_OK;
+  if (!aligned_to(16, h0, ht, trans_out)) return KDA_ERR_ARG;
   StateTcParams p;
   int* error = nullptr;
   if (cudaGetSymbolAddress(reinterpret_cast<void**>(&error), g_state_tc_error) != cudaSuccess)
@@ -812,6 +813,7 @@ int launch_state_bwd_tc(const bf16* w, const bf16* kg, const bf16* qg, const bf1
                         const int32_t* cu, const int32_t* co, int nseq, int H, int64_t tokens,
                         int chunks, cudaStream_t s) {
   if (nseq == 0) return KDA_OK;
+  if (!aligned_to(16, dht, dh0)) return KDA_ERR_ARG;
   StateBwdTcParams p;
   const int64_t cols = (int64_t)H * D;
   if (!make_tensor_map(&p.tm_w, w, tokens, cols, 64) || !make_tensor_map(&p.tm_kg, kg, tokens, cols, 64) ||

@@ -31,7 +31,7 @@ extern "C" {
 #define KDA_F16 2
 
 #define KDA_OK 0
-#define KDA_ERR_ARG (-1)         /* null pointer, bad size or inconsistent arguments */
+#define KDA_ERR_ARG (-1)         /* null pointer, bad size, an address off the alignment that vector loads need, or inconsistent arguments */
 #define KDA_ERR_UNSUPPORTED (-2) /* shape outside what the kernels are built for */
 #define KDA_ERR_LAUNCH (-3)      /* the CUDA runtime refused the launch */
 #define KDA_ERR_SCRATCH (-4)     /* the problem needs more scratch than the built-in array holds */
